@@ -41,26 +41,26 @@ def listed():
     N, K = SHAPES[0]
     return [
         # the training step of one Linear at the batch of the published configuration (32 x 512 tokens), noise given as a tensor
-        {"name": "linear step, 16384 tokens", "kind": "linear_step", "M": 16384, "N": N, "K": K, "rank": 16, "noise": "tensor", "straight": True},
+        {"name": "linear_step_16384", "kind": "linear_step", "M": 16384, "N": N, "K": K, "rank": 16, "noise": "tensor", "straight": True},
         # the same call on a short ragged batch, down projection, larger LoRA rank, sampled noise
-        {"name": "linear step, 1000 tokens", "kind": "linear_step", "M": 1000, "N": K, "K": N, "rank": 32, "noise": "hash", "straight": True},
+        {"name": "linear_step_1000", "kind": "linear_step", "M": 1000, "N": K, "K": N, "rank": 32, "noise": "hash", "straight": True},
         # a program written for the reference: its soft and hard functions under autograd, its tensor layouts
-        {"name": "reference api, soft", "kind": "api_soft", "M": 2048, "N": 4096, "K": 2560, "bias": False},
-        {"name": "reference api, hard", "kind": "api_hard", "M": 512, "N": N, "K": K, "bias": True},
+        {"name": "api_soft_2048", "kind": "api_soft", "M": 2048, "N": 4096, "K": 2560, "bias": False},
+        {"name": "api_hard_512", "kind": "api_hard", "M": 512, "N": N, "K": K, "bias": True},
         # inference of one Linear for a single token
-        {"name": "linear inference, 1 token", "kind": "linear_eval", "M": 1, "N": N, "K": K, "rank": 0},
+        {"name": "linear_eval_1", "kind": "linear_eval", "M": 1, "N": N, "K": K, "rank": 0},
         # fine-tuning of a decoder layer with LoRA, forward and backward
-        {"name": "layer training, 8 x 512", "kind": "layers", "B": 8, "S": 512, "layers": 1, "rank": 16},
+        {"name": "layers_8x512", "kind": "layers", "B": 8, "S": 512, "layers": 1, "rank": 16},
         # a batch of prompts through a palettized model
-        {"name": "qwen prefill, 4 x 1024", "kind": "qwen_prefill", "B": 4, "S": 1024, "layers": 2},
+        {"name": "qwen_prefill_4x1024", "kind": "qwen_prefill", "B": 4, "S": 1024, "layers": 2},
         # token decode of a palettized model: one user, and a full batch
-        {"name": "qwen decode, 1 x 2048", "kind": "qwen_decode", "B": 1, "T": 2048, "layers": 4},
-        {"name": "qwen decode, 64 x 1024", "kind": "qwen_decode", "B": 64, "T": 1024, "layers": 4},
+        {"name": "qwen_decode_1x2048", "kind": "qwen_decode", "B": 1, "T": 2048, "layers": 4},
+        {"name": "qwen_decode_64x1024", "kind": "qwen_decode", "B": 64, "T": 1024, "layers": 4},
         # a hybrid decoder with one layer of each kind: prompts, and a full batch of single tokens
-        {"name": "gopunex prefill, 2 x 1024", "kind": "hybrid_prefill", "design": "Gopunex", "size": "medium", "B": 2, "S": 1024},
-        {"name": "gopunex decode, 64 x 1024", "kind": "hybrid_decode", "design": "Gopunex", "size": "medium", "B": 64, "T": 1024},
+        {"name": "gopunex_prefill_2x1024", "kind": "hybrid_prefill", "design": "Gopunex", "size": "medium", "B": 2, "S": 1024},
+        {"name": "gopunex_decode_64x1024", "kind": "hybrid_decode", "design": "Gopunex", "size": "medium", "B": 64, "T": 1024},
         # a request served by the engine: a ragged prompt, then token by token
-        {"name": "latodra request, 1000 + 16", "kind": "request", "design": "Latodra", "size": "medium", "prompt": 1000, "new": 16},
+        {"name": "latodra_request_1000", "kind": "request", "design": "Latodra", "size": "medium", "prompt": 1000, "new": 16},
     ]
 
 
