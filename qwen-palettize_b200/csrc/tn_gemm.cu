@@ -67,7 +67,9 @@ struct TnParams {
     unsigned long long* prof;  // diagnostics build: [gridDim][8] cycle counters of the MMA thread
 };
 
-constexpr int kTnThreads = 320;  // warp 0: TMA, warp 1: MMA, warps 2..9: epilogue
+// Warp 0: TMA, warp 1: MMA, then EW epilogue warps. Sixteen of them (four per scheduler) where the soft epilogue is what the launch waits
+// for, eight where it runs in the shadow of a long main loop or does little (launch_tn_gemm).
+constexpr int tn_threads(int ew) { return 64 + 32 * ew; }
 constexpr int kTnStages = 4;
 constexpr uint32_t kTnABytes = 128 * 64 * 2;  // 2 boxes of [64 m][64 i]
 constexpr uint32_t kTnBBytes = 256 * 64 * 2;  // 4 boxes of [64 m][64 j]
@@ -87,12 +89,14 @@ __device__ __forceinline__ float warp_sum(float v) {
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, o);
     return v;
 }
-__device__ __forceinline__ void epi_bar_sync() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
+template <int EW>
+__device__ __forceinline__ void epi_bar_sync() { asm volatile("bar.sync 1, %0;" ::"n"(32 * EW) : "memory"); }
 
-template <int EPI, typename LogitT, bool ROWS_K, bool PAIR>
-__global__ void __launch_bounds__(kTnThreads, 1)
+template <int EPI, typename LogitT, bool ROWS_K, bool PAIR, int EW>
+__global__ void __launch_bounds__(tn_threads(EW), 1)
 tn_gemm_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant__ CUtensorMap tmQ,
                const __grid_constant__ CUtensorMap tmS0, const __grid_constant__ CUtensorMap tmS1, const TnParams p) {
+    constexpr int kBatch = 64 / EW;   // columns an epilogue warp has in flight
     constexpr int kStages = PAIR ? kTnStagesPair : kTnStages;
     constexpr uint32_t kBBytes = PAIR ? kTnBBytesPair : kTnBBytes;
     constexpr uint32_t kStageBytes = kTnABytes + kBBytes;
@@ -131,7 +135,7 @@ tn_gemm_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant__ 
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(acc_full(b), 1);
-            mbar_init(acc_empty(b), PAIR ? 16 : 8);
+            mbar_init(acc_empty(b), PAIR ? 2 * EW : EW);
         }
         *abort_flag = 0;
         mbar_fence_init();
@@ -307,12 +311,11 @@ tn_gemm_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant__ 
         }
     } else {
         // ------------------------------------------------------------------ epilogue warps
-        // Eight warps: warp w reads TMEM lanes 32*(w%4).., and the two warps of a lane group split the
-        // 256 columns in halves. Columns are processed 8 at a time: all global loads of a batch are issued
-        // before any arithmetic, so that each thread keeps 16 x 16 bytes in flight.
+        // Warp w reads TMEM lanes 32*(w%4).., and the EW / 4 warps of a lane group split the 256 columns. Columns are
+        // processed kBatch at a time: all global loads of a batch are issued before any arithmetic.
         const int lane_group = warp & 3;
-        const int col_half = (warp - 2) >> 2;
-        const int ew = warp - 2;  // 0..7
+        const int col_part = (warp - 2) >> 2;
+        const int ew = warp - 2;  // 0..EW - 1
         bool ok = true;
         int lt = 0;
         for (int t = unit; t < n_tiles && ok; t += n_units, ++lt) {
@@ -325,10 +328,10 @@ tn_gemm_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant__ 
             if (!ok) break;
             tc_fence_after_sync();
             const int row = ti * 128 + lane_group * 32 + lane;  // D row of this thread
-            const int wcols = c_num >> 1;  // columns per epilogue warp: 128, or 64 in a half tile
-            const uint32_t trow = tmem_base + ((uint32_t)(lane_group * 32) << 16) + buf * 256u + col_half * wcols;
+            const int wcols = c_num / (EW / 4);  // columns per epilogue warp
+            const uint32_t trow = tmem_base + ((uint32_t)(lane_group * 32) << 16) + buf * 256u + col_part * wcols;
             const bool row_ok = row < p.I;
-            const int colbase = (PAIR && job >= 0) ? col_half * wcols : tj * 256 + c_off + col_half * wcols;
+            const int colbase = (PAIR && job >= 0) ? col_part * wcols : tj * 256 + c_off + col_part * wcols;
 
             if (EPI == EPI_STORE || job >= 0) {
                 float* o_ptr = (job < 0) ? p.out : p.side[job].out;
@@ -351,19 +354,20 @@ tn_gemm_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant__ 
             } else if (ROWS_K) {
                 // Interleaved logits [N, K, 4], one palette per (n, 256-wide k group): D rows are input columns k
                 // (the 32 lanes of a warp read 32 consecutive float4 = 512 contiguous bytes), D columns are weight
-                // rows n, each with its own palette. The palette gradient of a column is a sum over lanes: the 32
-                // partials of a batch (8 columns x 4 entries) are reduced with a 31-shuffle transposing butterfly.
+                // rows n, each with its own palette. The palette gradient of a column is a sum over lanes: the
+                // partials of a batch (kBatch columns x 4 entries) are reduced with a transposing butterfly.
                 const int k = row;
                 const int kgi = (row_ok ? k : 0) / p.gs_k;
-                const float* lbase = reinterpret_cast<const float*>(p.logits) + (long long)k * p.ls_row;
-                float* dbase = p.dlogits ? reinterpret_cast<float*>(p.dlogits) + (long long)k * p.ls_row : nullptr;
-                const float* nbase = p.noise ? p.noise + (long long)k * p.ns_row : nullptr;
+                // running addresses of the batch's first column
+                const float* lcol = reinterpret_cast<const float*>(p.logits) + (long long)k * p.ls_row + (long long)colbase * p.ls_col;
+                float* dcol = p.dlogits ? reinterpret_cast<float*>(p.dlogits) + (long long)k * p.ls_row + (long long)colbase * p.ls_col : nullptr;
+                const float* ncol = p.noise ? p.noise + (long long)k * p.ns_row + (long long)colbase * p.ns_col : nullptr;
+                const long long pal_step = 4ll * p.n_kgroups;
+                const __nv_bfloat16* pcol = p.palette + (long long)colbase * pal_step + 4 * kgi;
 #pragma unroll 1
-                for (int c0 = 0; c0 < wcols; c0 += 8) {
-                    uint32_t v[8];
-                    tmem_ld_32x8(trow + c0, v);
+                for (int c0 = 0; c0 < wcols; c0 += kBatch) {
                     const int nb = colbase + c0;  // first n of the batch
-                    // fused reduce-scatter: the 8 rows of a batch have one owner (rows_per_rank % 8 == 0); its buffer, this
+                    // fused reduce-scatter: the rows of a batch have one owner (rows_per_rank % 8 == 0); its buffer, this
                     // rank's slot (or the accumulator) and this thread's k folded into one base pointer per batch
                     float* sbase = nullptr;
                     if (p.world > 1 && nb < p.J) {
@@ -371,33 +375,33 @@ tn_gemm_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant__ 
                         sbase = p.peer_stage[owner] + (p.scatter_add ? 0ll : (long long)p.rank * p.shard_elems) +
                                 ((long long)(nb - owner * p.rows_per_rank) * p.I + k) * 4;
                     }
-                    float4 lv[8], gv[8];
-                    uint2 praw[8];
-                    uint32_t hbyte[8];
+                    float4 lv[kBatch], gv[kBatch];
+                    uint2 praw[kBatch];
+                    uint32_t hbyte[kBatch];
                     // ---- phase 1: issue every load of the batch
 #pragma unroll
-                    for (int c = 0; c < 8; ++c) {
-                        const int n = nb + c;
-                        const bool valid = row_ok && n < p.J;
+                    for (int c = 0; c < kBatch; ++c) {
+                        const bool valid = row_ok && nb + c < p.J;
                         lv[c] = make_float4(0.f, 0.f, 0.f, 0.f);
                         gv[c] = make_float4(0.f, 0.f, 0.f, 0.f);
                         praw[c] = make_uint2(0u, 0u);
                         hbyte[c] = 0;
                         if (valid) {
                             if (EPI == EPI_SOFT) {
-                                praw[c] = __ldg(reinterpret_cast<const uint2*>(p.palette + ((long long)n * p.n_kgroups + kgi) * 4));
-                                lv[c] = __ldcs(reinterpret_cast<const float4*>(lbase + (long long)n * p.ls_col));
-                                if (p.noise_mode == NOISE_TENSOR)
-                                    gv[c] = __ldcs(reinterpret_cast<const float4*>(nbase + (long long)n * p.ns_col));
+                                praw[c] = __ldg(reinterpret_cast<const uint2*>(pcol + c * pal_step));
+                                lv[c] = __ldcs(reinterpret_cast<const float4*>(lcol + c * p.ls_col));
+                                if (p.noise_mode == NOISE_TENSOR) gv[c] = __ldcs(reinterpret_cast<const float4*>(ncol + c * p.ns_col));
                             } else {
-                                hbyte[c] = __ldg(p.packed + (long long)n * p.packed_pitch + (k >> 2));
+                                hbyte[c] = __ldg(p.packed + (long long)(nb + c) * p.packed_pitch + (k >> 2));
                             }
                         }
                     }
+                    uint32_t v[kBatch];
+                    tmem_ld_cols(trow + c0, v);
                     // ---- phase 2: arithmetic and stores
-                    float part[32];
+                    float part[4 * kBatch];
 #pragma unroll
-                    for (int c = 0; c < 8; ++c) {
+                    for (int c = 0; c < kBatch; ++c) {
                         const int n = nb + c;
                         const bool valid = row_ok && n < p.J;
                         const float dw = valid ? __uint_as_float(v[c]) : 0.f;
@@ -431,8 +435,8 @@ tn_gemm_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant__ 
                                 } else {
                                     *reinterpret_cast<float4*>(dst) = make_float4(dl[0], dl[1], dl[2], dl[3]);
                                 }
-                            } else if (valid && dbase != nullptr)
-                                __stcs(reinterpret_cast<float4*>(dbase + (long long)n * p.ls_col), make_float4(dl[0], dl[1], dl[2], dl[3]));
+                            } else if (valid && dcol != nullptr)
+                                __stcs(reinterpret_cast<float4*>(dcol + c * p.ls_col), make_float4(dl[0], dl[1], dl[2], dl[3]));
                         } else {
                             const int idx = (hbyte[c] >> (2 * (k & 3))) & 3;
 #pragma unroll
@@ -440,22 +444,29 @@ tn_gemm_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant__ 
                         }
                     }
                     if (p.dpalette != nullptr) {
-                        // transposing butterfly: afterwards lane L holds the sum over all 32 lanes of part[L]
+                        // transposing butterfly: the values per lane halve until one is left, plain sums then; lane L ends up with
+                        // the sum over all 32 lanes of part[L / (32 / values)]
+                        constexpr int kVals = 4 * kBatch;
 #pragma unroll
-                        for (int s = 16; s >= 1; s >>= 1) {
+                        for (int s = 16, h = kVals / 2; s >= 1; s >>= 1, h >>= 1) {
                             const bool up = (lane & s) != 0;
+                            if (h == 0) part[0] += __shfl_xor_sync(0xFFFFFFFFu, part[0], s);
 #pragma unroll
-                            for (int j = 0; j < s; ++j) {
-                                const float send = up ? part[j] : part[j + s];
-                                const float keep = up ? part[j + s] : part[j];
+                            for (int j = 0; j < h; ++j) {
+                                const float send = up ? part[j] : part[j + h];
+                                const float keep = up ? part[j + h] : part[j];
                                 part[j] = keep + __shfl_xor_sync(0xFFFFFFFFu, send, s);
                             }
                         }
-                        red[(lane_group * 256 + col_half * wcols + c0) * 4 + lane] = part[0];
+                        if (lane % (32 / kVals) == 0) red[(lane_group * 256 + col_part * wcols + c0) * 4 + lane / (32 / kVals)] = part[0];
                     }
+                    lcol += kBatch * p.ls_col;
+                    pcol += kBatch * pal_step;
+                    if (dcol != nullptr) dcol += kBatch * p.ls_col;
+                    if (ncol != nullptr) ncol += kBatch * p.ns_col;
                 }
                 if (p.dpalette != nullptr) {
-                    epi_bar_sync();
+                    epi_bar_sync<EW>();
                     // one thread per column: add the four lane groups' partials in a fixed order
                     const int et = threadIdx.x - 64;  // 0..255
                     const int n = tj * 256 + c_off + et;
@@ -469,7 +480,7 @@ tn_gemm_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant__ 
                             atomicAdd(p.dpalette + pg + q, s);
                         }
                     }
-                    epi_bar_sync();
+                    epi_bar_sync<EW>();
                 }
             } else {
                 // D rows are weight rows n, columns are input columns k. A thread owns one n and walks k, so the
@@ -489,53 +500,53 @@ tn_gemm_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant__ 
                     cpal[2] = __uint_as_float(praw.y << 16);
                     cpal[3] = __uint_as_float(praw.y & 0xFFFF0000u);
                 }
-                const LogitT* lrow = reinterpret_cast<const LogitT*>(p.logits) + (long long)n * p.ls_row;
-                LogitT* drow = p.dlogits ? reinterpret_cast<LogitT*>(p.dlogits) + (long long)n * p.ls_row : nullptr;
-                const float* nrow = p.noise ? p.noise + (long long)n * p.ns_row : nullptr;
+                // running addresses of the batch's first column
+                const LogitT* lcol = reinterpret_cast<const LogitT*>(p.logits) + (long long)n * p.ls_row + (long long)colbase * p.ls_col;
+                LogitT* dcol = p.dlogits ? reinterpret_cast<LogitT*>(p.dlogits) + (long long)n * p.ls_row + (long long)colbase * p.ls_col : nullptr;
+                const float* ncol = p.noise ? p.noise + (long long)n * p.ns_row + (long long)colbase * p.ns_col : nullptr;
                 const uint8_t* prow = p.packed ? p.packed + (long long)n * p.packed_pitch : nullptr;
                 float acc[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll 1
-                for (int c0 = 0; c0 < wcols; c0 += 8) {
-                    uint32_t v[8];
-                    tmem_ld_32x8(trow + c0, v);
+                for (int c0 = 0; c0 < wcols; c0 += kBatch) {
                     const int kb = colbase + c0;  // first k of the batch
-                    float l[8][4], g[8][4];
+                    LogitT l[kBatch][4];
+                    float g[kBatch][4];
                     uint32_t hard_bits = 0;
                     // ---- phase 1: issue every load of the batch
                     if (EPI == EPI_SOFT) {
 #pragma unroll
-                        for (int c = 0; c < 8; ++c) {
+                        for (int c = 0; c < kBatch; ++c) {
                             const bool valid = row_ok && (kb + c) < p.J;
 #pragma unroll
-                            for (int q = 0; q < 4; ++q) { l[c][q] = 0.f; g[c][q] = 0.f; }
+                            for (int q = 0; q < 4; ++q) { from_f32(l[c][q], 0.f); g[c][q] = 0.f; }
                             if (valid) {
-                                const long long lo = (long long)(kb + c) * p.ls_col;
                                 if (vec_l) {
-                                    const float4 lv = __ldcs(reinterpret_cast<const float4*>(reinterpret_cast<const float*>(lrow) + lo));
-                                    l[c][0] = lv.x; l[c][1] = lv.y; l[c][2] = lv.z; l[c][3] = lv.w;
+                                    const float4 lv = __ldcs(reinterpret_cast<const float4*>(reinterpret_cast<const float*>(lcol + c * p.ls_col)));
+                                    from_f32(l[c][0], lv.x); from_f32(l[c][1], lv.y); from_f32(l[c][2], lv.z); from_f32(l[c][3], lv.w);
                                 } else {
 #pragma unroll
-                                    for (int q = 0; q < 4; ++q) l[c][q] = to_f32(lrow[lo + q * p.ls_p]);
+                                    for (int q = 0; q < 4; ++q) l[c][q] = __ldcs(lcol + c * p.ls_col + q * p.ls_p);
                                 }
                                 if (p.noise_mode == NOISE_TENSOR) {
-                                    const long long no = (long long)(kb + c) * p.ns_col;
                                     if (vec_n) {
-                                        const float4 gv = __ldcs(reinterpret_cast<const float4*>(nrow + no));
+                                        const float4 gv = __ldcs(reinterpret_cast<const float4*>(ncol + c * p.ns_col));
                                         g[c][0] = gv.x; g[c][1] = gv.y; g[c][2] = gv.z; g[c][3] = gv.w;
                                     } else {
 #pragma unroll
-                                        for (int q = 0; q < 4; ++q) g[c][q] = __ldcs(nrow + no + q * p.ns_p);
+                                        for (int q = 0; q < 4; ++q) g[c][q] = __ldcs(ncol + c * p.ns_col + q * p.ns_p);
                                     }
                                 }
                             }
                         }
                     } else if (row_ok && kb < p.J) {
-                        // 8 consecutive k = 16 bits of the packed row
-                        hard_bits = __ldg(reinterpret_cast<const unsigned short*>(prow + (kb >> 2)));
+                        // kBatch consecutive k = 16 or 8 bits of the packed row
+                        hard_bits = kBatch == 8 ? (uint32_t)__ldg(reinterpret_cast<const unsigned short*>(prow + (kb >> 2))) : (uint32_t)__ldg(prow + (kb >> 2));
                     }
+                    uint32_t v[kBatch];
+                    tmem_ld_cols(trow + c0, v);
                     // ---- phase 2: arithmetic and stores
 #pragma unroll
-                    for (int c = 0; c < 8; ++c) {
+                    for (int c = 0; c < kBatch; ++c) {
                         const bool valid = row_ok && (kb + c) < p.J;
                         const float dw = valid ? __uint_as_float(v[c]) : 0.f;
                         if (EPI == EPI_SOFT) {
@@ -544,7 +555,8 @@ tn_gemm_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant__ 
 #pragma unroll
                                 for (int q = 0; q < 4; ++q) g[c][q] = gumbel_hash(p.seed, e + q);
                             }
-                            const Soft4 s4 = soft4(l[c], g[c], cpal, p.inv_tau);
+                            const float lf[4] = {to_f32(l[c][0]), to_f32(l[c][1]), to_f32(l[c][2]), to_f32(l[c][3])};
+                            const Soft4 s4 = soft4(lf, g[c], cpal, p.inv_tau);
                             float dl[4];
 #pragma unroll
                             for (int q = 0; q < 4; ++q) {
@@ -552,14 +564,12 @@ tn_gemm_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant__ 
                                 acc[q] += cq;
                                 dl[q] = cq * (cpal[q] - s4.w_soft);
                             }
-                            if (valid && drow != nullptr) {
-                                const long long lo = (long long)(kb + c) * p.ls_col;
+                            if (valid && dcol != nullptr) {
                                 if (vec_l) {
-                                    __stcs(reinterpret_cast<float4*>(reinterpret_cast<float*>(drow) + lo),
-                                           make_float4(dl[0], dl[1], dl[2], dl[3]));
+                                    __stcs(reinterpret_cast<float4*>(reinterpret_cast<float*>(dcol + c * p.ls_col)), make_float4(dl[0], dl[1], dl[2], dl[3]));
                                 } else {
 #pragma unroll
-                                    for (int q = 0; q < 4; ++q) from_f32(drow[lo + q * p.ls_p], dl[q]);
+                                    for (int q = 0; q < 4; ++q) from_f32(dcol[c * p.ls_col + q * p.ls_p], dl[q]);
                                 }
                             }
                         } else {
@@ -568,10 +578,13 @@ tn_gemm_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant__ 
                             for (int q = 0; q < 4; ++q) acc[q] += (q == idx) ? dw : 0.f;
                         }
                     }
+                    lcol += kBatch * p.ls_col;
+                    if (dcol != nullptr) dcol += kBatch * p.ls_col;
+                    if (ncol != nullptr) ncol += kBatch * p.ns_col;
                 }
                 if (p.dpalette != nullptr) {
                     if (p.gs_n == 1) {
-                        // this thread's row has its own palette: the two column halves add up in either order
+                        // this thread's row has its own palette: the column parts add up in any order
                         if (row_ok) {
 #pragma unroll
                             for (int q = 0; q < 4; ++q) atomicAdd(p.dpalette + pg + q, acc[q]);
@@ -583,15 +596,15 @@ tn_gemm_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant__ 
                             const float s = warp_sum(acc[q]);
                             if (lane == 0) red[ew * 4 + q] = s;
                         }
-                        epi_bar_sync();
+                        epi_bar_sync<EW>();
                         const int et = threadIdx.x - 64;
                         if (et < 4 && ti * 128 < p.I) {
                             float s = 0.f;
 #pragma unroll
-                            for (int w8 = 0; w8 < 8; ++w8) s += red[w8 * 4 + et];
+                            for (int w = 0; w < EW; ++w) s += red[w * 4 + et];
                             atomicAdd(p.dpalette + pg - 0 + et, s);
                         }
-                        epi_bar_sync();
+                        epi_bar_sync<EW>();
                     }
                 }
             }
@@ -615,10 +628,18 @@ tn_gemm_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant__ 
 // host side
 // ---------------------------------------------------------------------------------------------
 
-template <int EPI, typename LogitT, bool ROWS_K, bool PAIR>
+// From this many tokens on the main loop of a tile (256 x 256, 0.33 us per 64 tokens) is longer than its soft epilogue with eight warps
+// (interleaved fp32 logits, 60 us), which then runs in its shadow. Measured at 9728 x 2560, noise tensor / sampled noise, eight against
+// sixteen warps: 512 tokens 320 / 336 against 288 / 260 us, 4096: 352 / 374 against 316 / 306, 8192: 435 / 443 against 417 / 410,
+// 10240: 493 / 491 against 488 / 483, 16384: 712 / 708 against 766 / -. Planar fp16 logits (4096 x 2560, 2048 tokens) take 125 us per
+// tile with eight warps, longer than any main loop: 309 against 126 us, always sixteen. The hard epilogue has 45 against 40 us at
+// 512 tokens: always eight.
+constexpr int kTnLongLoop = 10241;
+
+template <int EPI, typename LogitT, bool ROWS_K, bool PAIR, int EW>
 static int launch_tn_t(const TnArgs& a, const TnParams& p, const CUtensorMap& tmP, const CUtensorMap& tmQ,
                        const CUtensorMap& tmS0, const CUtensorMap& tmS1, int grid, cudaStream_t stream) {
-    auto kern = tn_gemm_kernel<EPI, LogitT, ROWS_K, PAIR>;
+    auto kern = tn_gemm_kernel<EPI, LogitT, ROWS_K, PAIR, EW>;
     constexpr uint32_t smem = PAIR ? kTnSmemBytesPair : kTnSmemBytes;
     static bool attr_set[64] = {};
     int dev = 0;
@@ -629,7 +650,7 @@ static int launch_tn_t(const TnArgs& a, const TnParams& p, const CUtensorMap& tm
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(kTnThreads);
+    cfg.blockDim = dim3(tn_threads(EW));
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
@@ -782,23 +803,16 @@ int launch_tn_gemm(const TnArgs& a, cudaStream_t stream) {
         }
     }
     const int ctas = pair ? 2 * grid : grid;
-    switch (a.epi) {
-        case EPI_STORE: return launch_tn_t<EPI_STORE, float, false, false>(a, p, tmP, tmQ, tmS0, tmS1, ctas, stream);
-        case EPI_HARD:
-            if (pair) return a.rows_are_k ? launch_tn_t<EPI_HARD, float, true, true>(a, p, tmP, tmQ, tmS0, tmS1, ctas, stream)
-                                          : launch_tn_t<EPI_HARD, float, false, true>(a, p, tmP, tmQ, tmS0, tmS1, ctas, stream);
-            return a.rows_are_k ? launch_tn_t<EPI_HARD, float, true, false>(a, p, tmP, tmQ, tmS0, tmS1, ctas, stream)
-                                : launch_tn_t<EPI_HARD, float, false, false>(a, p, tmP, tmQ, tmS0, tmS1, ctas, stream);
-        case EPI_SOFT:
-            if (pair) {
-                if (a.rows_are_k) return launch_tn_t<EPI_SOFT, float, true, true>(a, p, tmP, tmQ, tmS0, tmS1, ctas, stream);
-                return a.logits_f16 ? launch_tn_t<EPI_SOFT, __half, false, true>(a, p, tmP, tmQ, tmS0, tmS1, ctas, stream)
-                                    : launch_tn_t<EPI_SOFT, float, false, true>(a, p, tmP, tmQ, tmS0, tmS1, ctas, stream);
-            }
-            if (a.rows_are_k) return launch_tn_t<EPI_SOFT, float, true, false>(a, p, tmP, tmQ, tmS0, tmS1, ctas, stream);
-            return a.logits_f16 ? launch_tn_t<EPI_SOFT, __half, false, false>(a, p, tmP, tmQ, tmS0, tmS1, ctas, stream)
-                                : launch_tn_t<EPI_SOFT, float, false, false>(a, p, tmP, tmQ, tmS0, tmS1, ctas, stream);
+#define PLZ_TN(EPI, T, ROWS_K, EW) \
+    return pair ? launch_tn_t<EPI, T, ROWS_K, true, EW>(a, p, tmP, tmQ, tmS0, tmS1, ctas, stream) : launch_tn_t<EPI, T, ROWS_K, false, EW>(a, p, tmP, tmQ, tmS0, tmS1, ctas, stream)
+    if (a.epi == EPI_STORE) return launch_tn_t<EPI_STORE, float, false, false, 8>(a, p, tmP, tmQ, tmS0, tmS1, ctas, stream);
+    if (a.epi == EPI_HARD) { if (a.rows_are_k) PLZ_TN(EPI_HARD, float, true, 8); else PLZ_TN(EPI_HARD, float, false, 8); }
+    if (a.epi == EPI_SOFT) {
+        const bool long_loop = a.M >= kTnLongLoop;
+        if (!a.rows_are_k) { if (a.logits_f16) PLZ_TN(EPI_SOFT, __half, false, 16); else PLZ_TN(EPI_SOFT, float, false, 16); }
+        if (long_loop) PLZ_TN(EPI_SOFT, float, true, 8); else PLZ_TN(EPI_SOFT, float, true, 16);
     }
+#undef PLZ_TN
     set_last_error("tn_gemm: unknown epilogue %d", a.epi);
     return PLZ_ERR_UNSUPPORTED;
 }
