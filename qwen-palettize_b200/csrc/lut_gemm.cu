@@ -661,6 +661,23 @@ int launch_lut_gemm(const LutGemmArgs& a, cudaStream_t stream) {
         if ((uintptr_t)a.palette & 7) { set_last_error("lut_gemm: palette must be 8-byte aligned"); return PLZ_ERR_BAD_ALIGN; }
         if (a.gs_k % 64 || a.Wk % a.gs_k || a.Wk % 64) { set_last_error("lut_gemm: K group size %d must be a multiple of 64 dividing K=%d", a.gs_k, a.Wk); return PLZ_ERR_BAD_SHAPE; }
     }
+    // Few rows: the swapped form with the reduction split over a cluster (narrow_gemm.cu). A 128 x 256 tile per CTA is as good only where the
+    // tiles alone fill the chip (dense, wide outputs: 32768 x 2560 at 64 rows 31 against 36 us) or where the reduction is short and
+    // the rows many (6144 x 1024 at 128 rows 11 / 13); else 64 rows of 9728 x 2560 / 2560 x 9728 / 1024 x 2560 take 20 / 58 / 18 us here
+    // and 16 / 17 / 9 there, packed weights 32 / 122 / 30 and 18 / 22 / 9.
+    const bool own = !decode && ((a.M >= 32 && a.J >= 128 * 148) || (a.M > 64 && a.R < 2048 && a.J > 1024));
+    if (!own && a.M <= 128 && (a.bmode == B_TMA_K || a.bmode == B_DECODE_K) && a.fuse != 1 && !a.col_scale && !a.row_scale && a.sm_limit <= 0 && g_cta_limit <= 0) {
+        NarrowArgs n = {};
+        n.M = a.M; n.K = a.R; n.x = a.A; n.ldx = a.lda; n.count = 1;
+        n.mat[0].N = a.J; n.mat[0].w = a.Bdense; n.mat[0].ldw = a.ldb; n.mat[0].y = a.out; n.mat[0].ldy = a.ld_out;
+        if (decode) { n.mat[0].packed = a.packed; n.mat[0].pitch = a.packed_pitch; n.mat[0].palette = a.palette; n.gs_n = a.gs_n; n.gs_k = a.gs_k; }
+        n.r2 = a.r2; n.x2 = a.A2; n.ldx2 = a.lda2; n.w2 = a.B2; n.ldw2 = a.ldb2;
+        n.bias = a.fuse == 2 || a.fuse == 3 ? a.bias : nullptr;
+        n.act = a.fuse == 4 ? 2 : a.fuse == 3 ? a.act : 0;
+        n.alpha = a.alpha;
+        const int rc = launch_narrow_gemm(n, stream);
+        if (rc != PLZ_ERR_UNSUPPORTED) return rc;
+    }
     if (decode && a.fuse == 0) {
         // the large products run on CTA pairs (lut_gemm_pair.cu); everything else, and shapes it declines, stays here
         const int rc = launch_lut_gemm_pair(a, stream);

@@ -1,0 +1,397 @@
+// Linear products with few rows, y[m, n] = sum_k x[m, k] W[n, k] for M <= 128: token decode and short portions. What such a launch cannot do
+// without is one pass over W, so everything here serves that stream.
+//
+//   shape     The operands change sides: 128 rows of W are the 128 TMEM lanes, the tokens are the N side (16 .. 128 columns). A tile of 128
+//             weight rows and all tokens is shared by a cluster of up to eight CTAs that split the reduction, because N / 128 tiles alone
+//             leave most SMs idle (2560 rows are 20 tiles). Each CTA leaves its partial tile in its own shared memory and every CTA of the
+//             cluster adds up its share of the outputs over distributed shared memory, in rank order: no workspace, no atomics, the same
+//             bits on every run.
+//   operands  dense bf16 W by TMA (requested before the wait on the previous kernel of the stream), or packed 2-bit indices: a decode
+//             thread is one weight row, fetches the 16 bytes of a block of 64 columns several blocks ahead and writes the decoded row to
+//             TMEM, from where it is the A operand (lane = row: no shared memory, no swizzle, no proxy fence in between). x by TMA.
+//             Shared memory and TMEM are kept to half of an SM's, so that two CTAs share one and hide each other's start and end.
+//   extra     an optional block of up to 64 more reduction elements (the LoRA up-projection: t [M, r] against B [N, r]).
+//
+// Accumulating into the tile the previous MMA still writes costs a TMEM round trip, so the four MMAs of a block go to several accumulators,
+// as many as fit, which the epilogue adds.
+#include "attention_tiles.cuh"
+#include "seq_math.cuh"
+
+namespace plz {
+namespace {
+
+constexpr int kNgMaxMats = 4;
+constexpr int kNgDecodeWarps = 8;                 // two groups of 128 threads, blocks alternate between them
+constexpr uint32_t kNgWBytes = 128 * 64 * 2;
+// shared memory of the stages; two CTAs per SM. LUT: four x tiles of 128 tokens and the W tile of the extra block
+template <bool LUT>
+constexpr uint32_t kNgRingBytes = LUT ? 80 * 1024 : 96 * 1024;
+constexpr int kNgMaxStages = 8;
+constexpr int kNgAhead = 4;                       // blocks of packed indices a decode thread has in flight
+
+struct NarrowMat {
+    int N, first_tile;
+    const uint8_t* packed; long long pitch; const __nv_bfloat16* palette;
+    void* y; long long ldy;
+};
+struct NarrowParams {
+    int M, npad, n_acc, stages;
+    uint32_t tmem_cols;
+    int group_blocks, group_shift; // blocks of 64 columns per palette group, its logarithm or -1
+    int nkb, n_blocks;             // blocks of 64 columns of W; the same plus the extra block
+    int count; NarrowMat mat[kNgMaxMats];
+    int gs_n, gs_k, n_kgroups;
+    const __nv_bfloat16* bias; int act, y_f32; float alpha;
+    StatusWord* status;
+};
+
+__device__ __forceinline__ uint32_t cluster_nctarank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ uint32_t map_rank(uint32_t addr, uint32_t rank) {
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr) {
+    float4 v;
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+    return v;
+}
+
+template <bool LUT>
+constexpr int kNgThreads = 64 + 32 * (LUT ? kNgDecodeWarps : 4);
+
+template <bool LUT>
+__global__ void __launch_bounds__(kNgThreads<LUT>, 2)
+narrow_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX2,
+                   const __grid_constant__ CUtensorMap tmW2, const NarrowParams p) {
+    extern __shared__ uint8_t smem_raw[];
+    const uint32_t raw = smem_u32(smem_raw);
+    const uint32_t base = (raw + 1023u) & ~1023u;
+    uint8_t* smem = smem_raw + (base - raw);
+    // dense: a stage is a W tile and an x tile; LUT: x tiles, behind them one W tile for the extra block (W is decoded to TMEM)
+    const uint32_t x_bytes = (uint32_t)p.npad * 128u, stage_bytes = (LUT ? 0u : kNgWBytes) + x_bytes;
+    const uint32_t w2_off = LUT ? (uint32_t)p.stages * x_bytes : 0u;
+    const uint32_t bar_off = kNgRingBytes<LUT>;
+    auto full = [&](int s) { return base + bar_off + 8u * s; };
+    auto empty = [&](int s) { return base + bar_off + 8u * (kNgMaxStages + s); };
+    const uint32_t acc_full = base + bar_off + 8u * (2 * kNgMaxStages);
+    volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem + bar_off + 8 * (2 * kNgMaxStages + 1));
+    volatile uint32_t* abort_flag = tmem_slot + 1;
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int n_ranks = (int)cluster_nctarank(), rank = (int)cluster_ctarank();
+    const int tile = (int)blockIdx.x / n_ranks;
+    int mi = 0;
+#pragma unroll
+    for (int i = 1; i < kNgMaxMats; ++i)
+        if (i < p.count && tile >= p.mat[i].first_tile) mi = i;
+    const NarrowMat& mat = p.mat[mi];
+    const int n0 = (tile - mat.first_tile) * 128;
+    const int b_begin = (int)((long long)rank * p.n_blocks / n_ranks), b_end = (int)((long long)(rank + 1) * p.n_blocks / n_ranks);
+    const int nb = b_end - b_begin;        // at least one: the cluster is no larger than the number of blocks
+
+    // the bytes of both copies of a stage are announced with the first one
+    auto load_w = [&](int it, int s) {
+        const int b = b_begin + it;
+        const bool extra = b >= p.nkb, by_tma = !LUT || extra;
+        mbar_arrive_expect_tx(full(s), x_bytes + (by_tma ? kNgWBytes : 0u));
+        if (by_tma) tma_load_2d(base + (LUT ? w2_off : s * stage_bytes), extra ? &tmW2 : &tmW, full(s), extra ? 0 : b * 64, n0);
+    };
+    auto load_x = [&](int it, int s) {
+        const int b = b_begin + it;
+        const bool extra = b >= p.nkb;
+        tma_load_2d(base + s * stage_bytes + (LUT ? 0u : kNgWBytes), extra ? &tmX2 : &tmX, full(s), extra ? 0 : b * 64, 0);
+    };
+    const int pre = nb < p.stages ? nb : p.stages;
+
+    // weights do not depend on the previous kernel and do not wait for this block's own set-up either
+    constexpr int kAhead = LUT ? kNgAhead : 1;
+    const int row = (warp & 3) * 32 + lane;                         // decode: thread = one weight row = its TMEM lane
+    const int grp = LUT && warp >= 6 ? 1 : 0;
+    const int nw = b_end < p.nkb ? nb : p.nkb - b_begin;            // blocks of W in this CTA's range
+    const bool row_ok = n0 + row < mat.N;
+    const uint8_t* prow = LUT ? mat.packed + (row_ok ? (long long)(n0 + row) * mat.pitch : 0ll) + (long long)b_begin * 16 : nullptr;
+    const __nv_bfloat16* pal = LUT ? mat.palette + (row_ok ? (long long)((n0 + row) / p.gs_n) * p.n_kgroups * 4 : 0ll) : nullptr;
+    uint4 w[kAhead];
+    uint2 pr[kAhead];
+    auto fetch = [&](int it, int j) {
+        w[j] = make_uint4(0u, 0u, 0u, 0u);
+        pr[j] = make_uint2(0u, 0u);
+        if (row_ok && it < nw) {
+            const int kg = p.group_shift >= 0 ? (b_begin + it) >> p.group_shift : (b_begin + it) / p.group_blocks;
+            w[j] = __ldg(reinterpret_cast<const uint4*>(prow + it * 16));
+            pr[j] = __ldg(reinterpret_cast<const uint2*>(pal + kg * 4));
+        }
+    };
+    if (LUT && warp >= 2) {
+#pragma unroll
+        for (int j = 0; j < kAhead; ++j) fetch(grp + 2 * j, j);
+    }
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < kNgMaxStages; ++s) {
+            mbar_init(full(s), LUT ? 1 + kNgDecodeWarps / 2 : 1);
+            mbar_init(empty(s), 1);
+        }
+        mbar_init(acc_full, 1);
+        *abort_flag = 0;
+        mbar_fence_init();
+        tma_prefetch_desc(&tmX);
+        if (p.n_blocks > p.nkb) { tma_prefetch_desc(&tmX2); tma_prefetch_desc(&tmW2); }
+        for (int it = 0; it < pre; ++it) load_w(it, it);
+    }
+    if (warp == 1) { tmem_alloc(smem_u32((const void*)tmem_slot), p.tmem_cols); tmem_relinquish(); }
+    tc_fence_before_sync();
+    __syncthreads();
+    tc_fence_after_sync();
+    const uint32_t tmem_base = *tmem_slot;
+    const uint32_t tmem_w = tmem_base + (uint32_t)(p.n_acc * p.npad);      // LUT: 32 columns per stage
+    pdl_launch_dependents();
+
+    if (warp == 0) {
+        if (lane == 0) {
+            pdl_wait();
+            for (int it = 0; it < pre; ++it) load_x(it, it);
+            bool ok = true;
+            int issued = pre;
+            for (int it = pre; it < nb; ++it) {
+                const int s = it % p.stages;
+                ok = mbar_wait(empty(s), ((it / p.stages) & 1) ^ 1u, abort_flag, p.status, ST_TIMEOUT_EMPTY, 0);
+                if (!ok) break;
+                load_w(it, s);
+                load_x(it, s);
+                issued = it + 1;
+            }
+            if (!ok) {
+                // copies in flight get a bounded chance to land before the CTA exits
+                const uint64_t t0 = globaltimer_ns();
+                for (int it = issued > p.stages ? issued - p.stages : 0; it < issued; ++it)
+                    while (!mbar_try_wait(full(it % p.stages), (it / p.stages) & 1))
+                        if (globaltimer_ns() - t0 > 100000000ull) { report(p.status, ST_TIMEOUT_DRAIN, 0); break; }
+            }
+        }
+    } else if (warp == 1) {
+        if (lane == 0) {
+            const uint32_t idesc = make_idesc(128, p.npad, 0, 0);
+            bool ok = true;
+            for (int it = 0; it < nb && ok; ++it) {
+                const int s = it % p.stages;
+                ok = mbar_wait(full(s), (it / p.stages) & 1, abort_flag, p.status, ST_TIMEOUT_FULL, 1);
+                if (!ok) break;
+                tc_fence_after_sync();
+                const bool from_tmem = LUT && b_begin + it < p.nkb;
+                const uint32_t sw = base + (LUT ? w2_off : s * stage_bytes), sx = base + s * stage_bytes + (LUT ? 0u : kNgWBytes);
+                const uint64_t ad = make_sdesc(sw, 16u, 1024u), bd = make_sdesc(sx, 16u, 1024u);
+#pragma unroll
+                for (int ks = 0; ks < 4; ++ks) {
+                    const uint32_t d = tmem_base + (uint32_t)((ks & (p.n_acc - 1)) * p.npad), more = (it > 0 || ks >= p.n_acc) ? 1u : 0u;
+                    if (from_tmem) umma_ts(d, tmem_w + s * 32u + ks * 8u, (uint32_t)bd + ks * 2u, (uint32_t)(bd >> 32), idesc, more);
+                    else umma_bf16_words<1>(d, (uint32_t)ad + ks * 2u, (uint32_t)(ad >> 32), (uint32_t)bd + ks * 2u, (uint32_t)(bd >> 32), idesc, more);
+                }
+                umma_commit(empty(s));
+            }
+            if (ok) umma_commit(acc_full);
+        }
+    } else {
+        bool ok = true;
+        if (LUT) {
+            // ------------------------------------------------------ decode; the two groups of four warps take blocks in turn
+            for (int it0 = grp; it0 < nb && ok; it0 += 2 * kAhead) {
+#pragma unroll
+                for (int j = 0; j < kAhead; ++j) {
+                    const int it = it0 + 2 * j;
+                    if (it >= nb || !ok) continue;
+                    const int s = it % p.stages;
+                    ok = mbar_wait(empty(s), ((it / p.stages) & 1) ^ 1u, abort_flag, p.status, ST_TIMEOUT_EMPTY, 3);
+                    if (!ok) continue;
+                    if (it < nw) {
+                        uint32_t o[32];
+                        const PalRegs pl = pal_split(pr[j].x, pr[j].y);
+                        decode16(w[j].x, pl, o);
+                        decode16(w[j].y, pl, o + 8);
+                        decode16(w[j].z, pl, o + 16);
+                        decode16(w[j].w, pl, o + 24);
+                        fetch(it + 2 * kAhead, j);
+                        tc_fence_after_sync();
+                        tmem_st_32x32(tmem_w + ((uint32_t)((warp & 3) * 32) << 16) + s * 32u, o);
+                        tc_fence_before_sync();
+                    }
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(full(s));
+                }
+            }
+        }
+        // ---------------------------------------------------------- this CTA's partial tile: [token][weight row] in the ring's space
+        if (warp < 6) {
+            if (ok) ok = mbar_wait(acc_full, 0, abort_flag, p.status, ST_TIMEOUT_ACCUM, 4);
+            if (ok) {
+                tc_fence_after_sync();
+                const int lg = warp & 3;
+                float* part = reinterpret_cast<float*>(smem) + lg * 32 + lane;
+                for (int c0 = 0; c0 < p.npad && c0 < p.M; c0 += 16) {
+                    float sum[16];
+                    for (int a = 0; a < p.n_acc; ++a) {
+                        uint32_t v[16];
+                        tmem_ld_32x16(tmem_base + ((uint32_t)(lg * 32) << 16) + a * p.npad + c0, v);
+#pragma unroll
+                        for (int c = 0; c < 16; ++c) sum[c] = a == 0 ? __uint_as_float(v[c]) : sum[c] + __uint_as_float(v[c]);
+                    }
+#pragma unroll
+                    for (int c = 0; c < 16; ++c)
+                        if (c0 + c < p.M) part[(c0 + c) * 128] = sum[c];
+                }
+            }
+        }
+    }
+    tc_fence_before_sync();
+    __syncwarp();
+    cluster_sync_all();        // every CTA's partial tile is complete and visible
+    pdl_wait();                // outputs may be what the previous kernel still reads
+    {
+        uint32_t from[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) from[i] = map_rank(base, i < n_ranks ? i : 0);
+        const int units = p.M * 32;       // (token, 4 weight rows)
+        const int u1 = (int)((long long)(rank + 1) * units / n_ranks);
+        for (int u = (int)((long long)rank * units / n_ranks) + threadIdx.x; u < u1; u += kNgThreads<LUT>) {
+            const int m = u >> 5, r = (u & 31) * 4, n = n0 + r;
+            float v[4] = {0.f, 0.f, 0.f, 0.f};
+            float4 f[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+                if (i < n_ranks) f[i] = ld_cluster_f4(from[i] + (uint32_t)u * 16u);
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+                if (i < n_ranks) { v[0] += f[i].x; v[1] += f[i].y; v[2] += f[i].z; v[3] += f[i].w; }
+            if (n >= mat.N) continue;
+            if (p.act == ACT_GLU_GELU) {      // N is even
+                const long long o = (long long)m * mat.ldy + (n >> 1);
+                const float a = gelu_tanh_f(v[0]) * v[1], b = gelu_tanh_f(v[2]) * v[3];
+                if (p.y_f32) {
+                    float* y = (float*)mat.y + o;
+                    y[0] = a;
+                    if (n + 2 < mat.N) y[1] = b;
+                } else {
+                    __nv_bfloat16* y = (__nv_bfloat16*)mat.y + o;
+                    y[0] = __float2bfloat16_rn(a);
+                    if (n + 2 < mat.N) y[1] = __float2bfloat16_rn(b);
+                }
+                continue;
+            }
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                v[e] *= p.alpha;
+                if (p.bias && n + e < mat.N) v[e] += __bfloat162float(p.bias[n + e]);
+                v[e] = activate(v[e], p.act);
+            }
+            const long long o = (long long)m * mat.ldy + n;
+            if (p.y_f32) {
+                float* y = (float*)mat.y + o;
+                if (n + 3 < mat.N && !((uintptr_t)y & 15)) { *reinterpret_cast<float4*>(y) = make_float4(v[0], v[1], v[2], v[3]); continue; }
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    if (n + e < mat.N) y[e] = v[e];
+            } else {
+                __nv_bfloat16* y = (__nv_bfloat16*)mat.y + o;
+                if (n + 3 < mat.N && !((uintptr_t)y & 7)) { *reinterpret_cast<uint2*>(y) = make_uint2(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3])); continue; }
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    if (n + e < mat.N) y[e] = __float2bfloat16_rn(v[e]);
+            }
+        }
+    }
+    cluster_sync_all();        // nobody leaves while its partial tile may still be read
+    if (warp == 1) { tc_fence_after_sync(); tmem_dealloc(tmem_base, p.tmem_cols); }
+}
+
+// CTAs per tile: the shortest schedule when tiles * c CTAs of ceil(blocks / c) blocks each, plus about four for start, sum and end, are dealt
+// to the SMs.
+int cluster_size(int tiles, int blocks, int sms) {
+    int best = 1;
+    long long best_cost = 0;
+    for (int c = 1; c <= 8; ++c) {
+        if (c > 1 && blocks / c < 2) break;
+        if (c == 5 || c == 7) continue;           // leave SMs of a processing cluster without a partner
+        const long long rounds = ((long long)tiles * c + sms - 1) / sms;
+        const long long cost = rounds * ((blocks + c - 1) / c + 4);
+        if (c == 1 || cost < best_cost) { best = c; best_cost = cost; }
+    }
+    return best;
+}
+
+template <bool LUT>
+int launch_ng(const NarrowParams& p, int tiles, int ranks, const CUtensorMap (&tm)[4], cudaStream_t stream) {
+    auto kern = narrow_gemm_kernel<LUT>;
+    constexpr uint32_t smem = kNgRingBytes<LUT> + 256 + 1024;
+    static bool attr_set[64] = {};
+    int dev = 0;
+    PLZ_CUDA_CHECK(cudaGetDevice(&dev));
+    if (!attr_set[dev & 63]) {
+        PLZ_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        attr_set[dev & 63] = true;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(tiles * ranks)); cfg.blockDim = dim3(kNgThreads<LUT>); cfg.dynamicSmemBytes = smem; cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)ranks; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr; cfg.numAttrs = g_smallm_overlap ? 2 : 1;
+    PLZ_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kern, tm[0], tm[1], tm[2], tm[3], p));
+    ++g_launch_count;
+    return PLZ_OK;
+}
+
+}  // namespace
+
+// PLZ_ERR_UNSUPPORTED: not a call for this kernel.
+int launch_narrow_gemm(const NarrowArgs& a, cudaStream_t stream) {
+    const bool lut = a.mat[0].packed != nullptr;
+    if (a.M < 1 || a.M > 128 || a.count < 1 || a.count > kNgMaxMats || (!lut && a.count != 1) || a.K < 8 || a.K % (lut ? 64 : 8)) return PLZ_ERR_UNSUPPORTED;
+    if (a.r2 < 0 || a.r2 > 64 || a.r2 % 8 || (a.r2 && a.count != 1)) return PLZ_ERR_UNSUPPORTED;
+    if (((uintptr_t)a.x & 15) || a.ldx % 8) return PLZ_ERR_UNSUPPORTED;
+    if (lut && (a.gs_n <= 0 || a.gs_k <= 0 || a.gs_k % 64 || a.K % a.gs_k)) return PLZ_ERR_UNSUPPORTED;
+    if (!lut && (((uintptr_t)a.mat[0].w & 15) || a.mat[0].ldw % 8)) return PLZ_ERR_UNSUPPORTED;
+    NarrowParams p = {};
+    p.M = a.M; p.npad = a.M <= 16 ? 16 : a.M <= 32 ? 32 : a.M <= 64 ? 64 : 128;
+    if (lut) {      // 256 TMEM columns: accumulators, then 32 columns per stage
+        p.n_acc = p.npad <= 32 ? 4 : p.npad == 64 ? 2 : 1;
+        p.stages = (256 - p.n_acc * p.npad) / 32;
+        p.tmem_cols = 256;
+        p.group_blocks = a.gs_k / 64; p.group_shift = -1;
+        for (int i = 0; i < 16; ++i) if (p.group_blocks == 1 << i) p.group_shift = i;
+    } else {
+        p.n_acc = p.npad <= 64 ? 4 : 2;
+        p.stages = (int)(kNgRingBytes<false> / (kNgWBytes + (uint32_t)p.npad * 128u));
+        p.tmem_cols = (uint32_t)(p.n_acc * p.npad);     // 64, 128 or 256
+    }
+    if (p.stages > kNgMaxStages) p.stages = kNgMaxStages;
+    p.nkb = (a.K + 63) / 64; p.n_blocks = p.nkb + (a.r2 > 0 ? 1 : 0);
+    p.count = a.count;
+    p.gs_n = a.gs_n; p.gs_k = a.gs_k; p.n_kgroups = lut ? a.K / a.gs_k : 0;
+    p.bias = (const __nv_bfloat16*)a.bias; p.act = a.act; p.y_f32 = a.y_f32; p.alpha = a.alpha;
+    p.status = device_status_ptr();
+    int tiles = 0, rc;
+    for (int i = 0; i < a.count; ++i) {
+        const NarrowArgs::Mat& s = a.mat[i];
+        if (s.N < 1 || (a.act == ACT_GLU_GELU && s.N % 2) || (lut && (((uintptr_t)s.packed & 15) || s.pitch % 16 || ((uintptr_t)s.palette & 7)))) return PLZ_ERR_UNSUPPORTED;
+        p.mat[i] = NarrowMat{s.N, tiles, (const uint8_t*)s.packed, s.pitch, (const __nv_bfloat16*)s.palette, s.y, s.ldy};
+        tiles += (s.N + 127) / 128;
+    }
+    CUtensorMap tm[4];
+    if ((rc = make_tmap_bf16(&tm[0], a.x, a.M, a.K, a.ldx, 64, (uint32_t)p.npad))) return rc;
+    tm[1] = tm[2] = tm[3] = tm[0];
+    if (!lut && (rc = make_tmap_bf16(&tm[1], a.mat[0].w, a.mat[0].N, a.K, a.mat[0].ldw, 64, 128))) return rc;
+    if (a.r2) {
+        if ((rc = make_tmap_bf16(&tm[2], a.x2, a.M, a.r2, a.ldx2, 64, (uint32_t)p.npad))) return rc;
+        if ((rc = make_tmap_bf16(&tm[3], a.w2, a.mat[0].N, a.r2, a.ldw2, 64, 128))) return rc;
+    }
+    const int ranks = cluster_size(tiles, p.n_blocks, seq_sm_count());
+    return lut ? launch_ng<true>(p, tiles, ranks, tm, stream) : launch_ng<false>(p, tiles, ranks, tm, stream);
+}
+
+}  // namespace plz

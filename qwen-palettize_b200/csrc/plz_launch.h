@@ -35,6 +35,24 @@ int launch_lut_gemm_pair(const LutGemmArgs& a, cudaStream_t stream);
 extern int g_pair_gemm;  // 0: keep every product on the single-CTA kernel
 extern int g_cta_limit;
 
+// ---- narrow_gemm.cu: M <= 128, operands swapped, reduction split over a cluster --------------------
+struct NarrowArgs {
+    int M, K;
+    const void* x; long long ldx;
+    int count;                        // matrices sharing x (dense: 1)
+    struct Mat {
+        int N;
+        const void* w; long long ldw;                                  // dense bf16 [N, K]
+        const void* packed; long long pitch; const void* palette;      // or packed 2-bit indices
+        void* y; long long ldy;
+    } mat[4];
+    int gs_n, gs_k;
+    int r2; const void* x2; long long ldx2; const void* w2; long long ldw2;   // extra block: x2 [M, r2], w2 [N, r2]
+    const void* bias; int act;        // bf16 [N], SeqAct
+    int y_f32; float alpha;           // y = act(alpha * sum + bias)
+};
+int launch_narrow_gemm(const NarrowArgs& a, cudaStream_t stream);   // PLZ_ERR_UNSUPPORTED: not a call for it
+
 // ---- tn_gemm.cu -------------------------------------------------------------------------------
 enum Epi { EPI_STORE = 0, EPI_SOFT = 1, EPI_HARD = 2 };
 struct TnArgs {

@@ -7,7 +7,8 @@
 //                        Both also serve one small product per head (grid y = head, z = group of 16 rows).
 //   linear_tile_kernel   any shape and both types on the CUDA cores, fp32 products and sums: the 32-bit mode, and bf16 shapes
 //                        that the tensor-core path's 16-byte rows exclude.
-//   launch_seq_linear    picks one of them or the tcgen05 GEMM (lut_gemm.cu, dense B, bias and activation in its epilogue).
+//   launch_seq_linear    picks one of them, the swapped tcgen05 form (narrow_gemm.cu) or the tcgen05 GEMM (lut_gemm.cu, dense B, bias and
+//                        activation in its epilogue).
 #include "seq_math.cuh"
 
 namespace plz {
@@ -294,6 +295,15 @@ int launch_tile(const LinParams& p, int heads, cudaStream_t stream) {
     return PLZ_OK;
 }
 
+// 2 to 16 rows: narrow_gemm.cu streams large weights faster (its time hardly grows with the rows), but starts and ends later than the
+// register kernels here. us here / there in a decode chain: 8 rows 9728 x 2560 17.8 / 12.7, 4096 x 2560 8.3 / 9.7, 32768 x 2560
+// 61 / 31, 2560 x 9728 28 / 15; 16 rows 20 / 12, 8.3 / 7.5, 73 / 30, 1024 x 2560 6.3 / 5.1, 6144 x 1024 4.4 / 6.3. One row: 12.6 / 11.4
+// alone, but a served request (16 tokens, 14 Linears each) took 4.70 ms there and 4.62 ms here.
+bool rows_on_tensor_cores(int M, int N, int K) {
+    const long long size = (long long)N * K;
+    return M >= 2 && (size >= (1ll << 24) || (M > 8 && K >= 2048 && size >= (1ll << 21)));
+}
+
 }  // namespace
 
 int launch_seq_linear(int dtype, const void* x, long long ldx, int M, int K, const void* w, long long ldw, int N, const void* bias, int act,
@@ -307,6 +317,14 @@ int launch_seq_linear(int dtype, const void* x, long long ldx, int M, int K, con
     p.x = x; p.ldx = ldx; p.w = w; p.ldw = ldw; p.bias = bias; p.y = y; p.ldy = ldy; p.M = M; p.N = N; p.K = K; p.act = act;
     const int per16 = dtype == 0 ? 8 : 4;
     const bool vec = K % 8 == 0 && ldx % per16 == 0 && ldw % per16 == 0 && !((uintptr_t)x & 15) && !((uintptr_t)w & 15);
+    if (dtype == 0 && M <= 16 && vec && rows_on_tensor_cores(M, N, K)) {
+        NarrowArgs n = {};
+        n.M = M; n.K = K; n.x = x; n.ldx = ldx; n.count = 1;
+        n.mat[0].N = N; n.mat[0].w = w; n.mat[0].ldw = ldw; n.mat[0].y = y; n.mat[0].ldy = ldy;
+        n.bias = bias; n.act = act; n.y_f32 = y_f32; n.alpha = 1.0f;
+        const int rc = launch_narrow_gemm(n, stream);
+        if (rc != PLZ_ERR_UNSUPPORTED) return rc;
+    }
     if (dtype == 0 && M > 1 && M <= 16 && vec) return y_f32 ? launch_skinny<float>(p, 1, stream) : launch_skinny<__nv_bfloat16>(p, 1, stream);
     if (M <= 8 && vec) {
         if (dtype == 1) return launch_rows<float, float>(p, 1, stream);

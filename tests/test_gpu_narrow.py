@@ -1,0 +1,75 @@
+"""Linear products with 1 to 128 rows on the swapped tcgen05 kernel (csrc/narrow_gemm.cu): edges of its tiles, clusters and epilogues, against
+the same product in 64 bits. One bf16 rounding of the result bounds every element by 2^-8 of it; sums over K in fp32 add at most K 2^-24 of the sum
+of magnitudes."""
+import pytest
+import torch
+
+import plz_ops as ops
+import seq_ops as S
+
+pytestmark = pytest.mark.gpu
+
+
+def check(y, ref, mag, K, half_ulp=2.0 ** -8):
+    bound = half_ulp * ref.abs() + K * 2.0 ** -24 * mag + 1e-30
+    assert bool(((y.double() - ref).abs() <= bound).all())
+
+
+# rows around the MMA widths 16 / 32 / 64 / 128, outputs around a 128-row tile, reductions of one block, of ragged last blocks, and long enough
+# for clusters of several CTAs (2560 x 1000: split; 20000 columns: no split)
+@pytest.mark.parametrize("M,N,K", [(17, 8, 8), (17, 136, 72), (32, 128, 64), (33, 120, 200), (64, 1032, 2560), (65, 264, 2056), (128, 2560, 1000), (127, 1000, 4096), (24, 20000, 320), (16, 1024, 2560), (9, 1000, 2104)])
+def test_dense(M, N, K):
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    x = torch.randn(M, K, generator=g, device="cuda").bfloat16()
+    w = torch.randn(N, K, generator=g, device="cuda").bfloat16()
+    b = torch.randn(N, generator=g, device="cuda").bfloat16()
+    ref, mag = x.double() @ w.double().T, x.double().abs() @ w.double().abs().T
+    check(S.linear(x, w), ref, mag, K)
+    check(S.linear(x, w, b), ref + b.double(), mag + b.double().abs(), K)
+    y = S.linear(x, w, act=S.ACT_RELU2)
+    r = ref.clamp(min=0)
+    assert bool(((y.double() - r * r).abs() <= 2.0 ** -8 * r * r + (2 * r + 1) * (K * 2.0 ** -24 * mag) + 1e-30).all())
+    if M <= 16:
+        check(S.linear(x, w, out_f32=True), ref, mag, K, 2.0 ** -24)
+    out = torch.full((M, N + 24), 7.0, device="cuda", dtype=torch.bfloat16)      # a pitched destination: nothing beside it is written
+    S.linear(x, w, out=out[:, 8:8 + N])
+    check(out[:, 8:8 + N], ref, mag, K)
+    assert bool((out[:, :8] == 7).all()) and bool((out[:, 8 + N:] == 7).all())
+
+
+@pytest.mark.parametrize("M,N,K", [(20, 6, 64), (64, 1032, 2560), (100, 130, 2304)])
+def test_gated_pairs(M, N, K):
+    g = torch.Generator(device="cuda").manual_seed(N)
+    x = torch.randn(M, K, generator=g, device="cuda").bfloat16()
+    w = (torch.randn(2 * N, K, generator=g, device="cuda") * K ** -0.5).bfloat16()
+    z = x.double() @ w.double().T
+    ref = torch.nn.functional.gelu(z[:, 0::2], approximate="tanh") * z[:, 1::2]
+    y = S.linear(x, w, act=S.ACT_GLU_GELU)
+    # |d gelu| <= 1.13; each of the two factors carries K 2^-24 times the row's magnitude
+    mag = x.double().abs() @ w.double().abs().T
+    slack = K * 2.0 ** -24 * (1.13 * mag[:, 0::2] * z[:, 1::2].abs() + mag[:, 1::2] * z[:, 0::2].abs()) + 1e-6 * ref.abs() + 1e-7
+    assert bool(((y.double() - ref).abs() <= 2.0 ** -8 * ref.abs() + slack).all())
+
+
+# palette groups of 64, 192 (no power of two), 256 columns and of the whole reduction with 256 shared rows; LoRA ranks that fill part of a block
+@pytest.mark.parametrize("M,N,K,gs_n,gs_k,rank", [(17, 8, 64, 1, 64, 0), (33, 136, 384, 1, 192, 8), (64, 2560, 2560, 1, 256, 16), (128, 1000, 1024, 1, 256, 64), (1, 512, 2560, 256, 2560, 32),
+                                                  (65, 768, 2624, 256, 2624, 0), (16, 520, 9728, 1, 256, 0), (40, 9728, 320, 1, 64, 16)])
+def test_packed(M, N, K, gs_n, gs_k, rank):
+    g = torch.Generator(device="cuda").manual_seed(K)
+    idx = torch.randint(0, 4, (N, K), generator=g, device="cuda", dtype=torch.int8)
+    pal = torch.randn((N // gs_n) * (K // gs_k), 4, generator=g, device="cuda").bfloat16()
+    w = ops.PackedWeight(ops.pack_indices(idx, n_major=True), pal, N, K, gs_n, gs_k)
+    x = torch.randn(M, K, generator=g, device="cuda").bfloat16()
+    W = torch.gather(pal.view(N // gs_n, 1, K // gs_k, 1, 4).expand(-1, gs_n, -1, gs_k, -1).reshape(N, K, 4), 2, idx.long()[:, :, None])[:, :, 0].double()
+    ref, mag = x.double() @ W.T, x.double().abs() @ W.abs().T
+    if rank:
+        a, b = torch.randn(rank, K, generator=g, device="cuda").bfloat16(), torch.randn(N, rank, generator=g, device="cuda").bfloat16()
+        y, t = ops.hard_forward(w, x, (a, b, 0.5))
+        check(t, 0.5 * x.double() @ a.double().T, 0.5 * x.double().abs() @ a.double().abs().T, K)
+        ref, mag = ref + t.double() @ b.double().T, mag + t.double().abs() @ b.double().abs().T
+    else:
+        y = ops.hard_forward(w, x)[0]
+        if 16 < M <= 64:
+            check(ops.hard_forward_smallm(w, x), ref, mag, K)
+    check(y, ref, mag, K + rank)
+    assert torch.equal(y, ops.hard_forward(w, x, (a, b, 0.5) if rank else None)[0])
