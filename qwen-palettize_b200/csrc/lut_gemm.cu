@@ -678,7 +678,7 @@ int launch_lut_gemm(const LutGemmArgs& a, cudaStream_t stream) {
         const int rc = launch_narrow_gemm(n, stream);
         if (rc != PLZ_ERR_UNSUPPORTED) return rc;
     }
-    if (decode && a.fuse == 0) {
+    if (decode) {
         // the large products run on CTA pairs (lut_gemm_pair.cu); everything else, and shapes it declines, stays here
         const int rc = launch_lut_gemm_pair(a, stream);
         if (rc != PLZ_ERR_UNSUPPORTED) return rc;

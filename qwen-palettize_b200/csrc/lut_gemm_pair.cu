@@ -20,11 +20,17 @@
 //
 // Synchronisation (every barrier named here lives at the same shared-memory offset in both CTAs):
 //   full[s]     leader's copy: the leader's producer announces both CTAs' TMA bytes (each CTA's copies complete on the
-//               LEADER's barrier) and every decode warp of BOTH CTAs arrives once (remote arrive from the peer)
+//               LEADER's barrier) and the decode warps of one group of BOTH CTAs arrive once (remote arrive from the peer)
 //   empty[s]    own copy in each CTA: tcgen05.commit of the leader, multicast to both CTAs
 //   acc_full[b] own copy in each CTA: tcgen05.commit multicast after the last reduction block of a tile
 //   acc_empty[b] leader's copy: one arrival per epilogue warp of BOTH CTAs
 // No load uses cluster multicast: every CTA issues its own plain TMA copies.
+//
+// Tiles narrower than 256 columns (plan_pair_tiles). A launch ends when its last wave does, and a wave of a few tiles costs as much as a full one:
+// 4096 x 2560 outputs are 160 tiles on 74 pairs, two full waves and one with twelve tiles. So where the tiles of the last wave, cut in halves of
+// 128 columns, still fit one wave, they are; and a launch with fewer tiles than pairs takes the narrowest tile (32-column steps) that still
+// fits one wave. Below 128 columns the rows of A, 32 KB per stage and CTA, arrive no faster than the tensor cores would use them up.
+// The order of every sum is that of a 256-column tile.
 //
 // Replaces, in the reference: fused_lut_linear_fwd_tc_kernel (scripts/fused_lut_kernel.cu:309),
 // fused_lut_linear_bwd_grad_x_tc_kernel (:551) and the cuBLAS calls of the soft path
@@ -40,12 +46,15 @@ namespace {
 struct PairParams {
     int M, J, R;
     int n_extra;             // 0 or 1 extra 64-wide reduction block from (A2, B2)
-    int tiles_m, tiles_j, n_tiles;
+    int tiles_j, tile_w;     // column tiles of tile_w columns
+    int n_whole, n_items;    // items [0, n_whole) are whole tiles, the others halves of 128 columns of the tiles behind (tile_w = 256 then)
     const uint8_t* packed; long long packed_pitch;
     const __nv_bfloat16* palette;
     int gs_n, gs_k, n_kgroups, gs_n_shift;
+    int gs_k_shift;          // log2(gs_k / 64) or -1
     int Wn, Wk;
     float alpha;
+    const __nv_bfloat16* bias;   // optional [J], added in fp32 before the rounding
     StatusWord* status;
     unsigned long long* prof;  // diagnostics build: [gridDim][8] cycle counters (MMA thread 0..4, one decode thread 5..6)
 };
@@ -68,7 +77,8 @@ constexpr uint32_t kSmemBytes = kBarOff + 1024 + 256;
 template <int BMODE>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 lut_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmA2,
-                     const __grid_constant__ CUtensorMap tmB2, const __grid_constant__ CUtensorMap tmD, const PairParams p) {
+                     const __grid_constant__ CUtensorMap tmB2, const __grid_constant__ CUtensorMap tmD, const __grid_constant__ CUtensorMap tmD32,
+                     const PairParams p) {
     constexpr bool kBMn = (BMODE == B_DECODE_MN);
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
@@ -95,7 +105,7 @@ lut_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < kStages; ++s) {
-            mbar_init(full(s), 1 + 2 * kDecodeWarps);
+            mbar_init(full(s), 1 + kDecodeWarps);   // half of the decode warps of both CTAs
             mbar_init(empty(s), 1);
         }
         for (int b = 0; b < 2; ++b) {
@@ -106,6 +116,7 @@ lut_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
         mbar_fence_init();
         tma_prefetch_desc(&tmA);
         tma_prefetch_desc(&tmD);
+        if (p.tile_w & 32) tma_prefetch_desc(&tmD32);
         if (p.n_extra) { tma_prefetch_desc(&tmA2); tma_prefetch_desc(&tmB2); }
     }
     if (warp == 1) {
@@ -118,9 +129,12 @@ lut_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
 
-    auto tile_origin = [&](int t, int& m0, int& j0) {
-        j0 = (t % p.tiles_j) * 256;
-        m0 = (t / p.tiles_j) * 256;
+    auto item_width = [&](int t) { return t < p.n_whole ? p.tile_w : 128; };
+    auto item_origin = [&](int t, int& m0, int& j0) {
+        const int cut = t - p.n_whole;                       // >= 0: a half tile
+        const int tile = cut < 0 ? t : p.n_whole + (cut >> 1);
+        j0 = (tile % p.tiles_j) * p.tile_w + (cut < 0 ? 0 : (cut & 1) * 128);
+        m0 = (tile / p.tiles_j) * 256;
     };
 
     if (warp == 0) {
@@ -129,11 +143,11 @@ lut_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
             bool ok = true;
             int s = 0;
             uint32_t ph = 0;
-            for (int t = pair; t < p.n_tiles && ok; t += n_pairs) {
+            for (int t = pair; t < p.n_items && ok; t += n_pairs) {
                 int m0, j0;
-                tile_origin(t, m0, j0);
+                item_origin(t, m0, j0);
                 const int mrow = m0 + 128 * (int)rank;
-                const int jr = j0 + 128 * (int)rank;
+                const int jr = j0 + (item_width(t) >> 1) * (int)rank;
                 for (int it = 0; it < nkb_total; ++it) {
                     ok = mbar_wait(empty(s), ph ^ 1u, abort_flag, p.status, ST_TIMEOUT_EMPTY, 0);
                     if (!ok) break;
@@ -162,7 +176,7 @@ lut_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
     } else if (warp == 1) {
         // ------------------------------------------------------------- MMA issuer (leader only)
         if (rank == 0 && lane == 0) {
-            const uint32_t idesc = make_idesc(256, 256, 0, kBMn ? 1 : 0);
+            const uint32_t idesc_whole = make_idesc(256, p.tile_w, 0, kBMn ? 1 : 0), idesc_half = make_idesc(256, 128, 0, kBMn ? 1 : 0);
             // descriptor words of stage 0; a stage is kStageBytes >> 4 = 4096 further in the low word
             const uint64_t ad0 = make_sdesc(base, 16u, 1024u);
             const uint64_t bd0 = kBMn ? make_sdesc(base + kABytes, kBlkBytes, 1024u) : make_sdesc(base + kABytes, 16u, 1024u);
@@ -174,8 +188,9 @@ lut_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
             uint32_t ph = 0;
             long long wait_f = 0, wait_t = 0;
             const long long t_begin = PLZ_PROF_ON(p.prof) ? clock64() : 0;
-            for (int t = pair; t < p.n_tiles && ok; t += n_pairs, ++lt) {
+            for (int t = pair; t < p.n_items && ok; t += n_pairs, ++lt) {
                 const uint32_t d_tmem = tmem_base + (uint32_t)(lt & 1) * 256u;
+                const uint32_t idesc = t < p.n_whole ? idesc_whole : idesc_half;
                 const long long c_t = PLZ_PROF_ON(p.prof) ? clock64() : 0;
                 ok = mbar_wait_lean(acc_empty(lt & 1), ((lt >> 1) & 1) ^ 1u, abort_flag, p.status, ST_TIMEOUT_ACCUM, 1);
                 if (PLZ_PROF_ON(p.prof)) wait_t += clock64() - c_t;
@@ -217,113 +232,124 @@ lut_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
         }
     } else if (warp < kFirstEpiWarp) {
         // ------------------------------------------------------------- decode warps
-        // 512 threads produce this CTA's half of the B stage, 128 columns x 128 reduction elements: 32 weights (eight bytes of
-        // packed indices, four 16-byte chunks of a 128-byte operand row) per thread and stage.
-        //   forward  (rows of the operand = n, two 64-wide k blocks):  block b = t / 256, row n = (t % 256) / 2, half h = t % 2
-        //   backward (rows of the operand = n of the stage, two 64-wide k column blocks): block b = t / 256, row = (t % 256) / 2, h
+        // Two groups of eight warps take the stages in turn: what a warp does per stage is a chain (wait, decode, store, proxy fence, arrive) of
+        // about 0.7 us, as long as the MMAs of a whole stage, so with all warps on every stage it set the pace of narrow tiles.
+        // 1000 rows, 2560 x 9728: 65 us with 256-column tiles and all warps on a stage, 58 with 160 columns, 52 with two groups; input gradient at
+        // 512 rows 58 / 53 / 51 us; 4096 rows, 9728 x 2560 177 / 176 / 165 us.
+        // The 256 threads of a group produce this CTA's half of the B stage, 128 columns x 128 reduction elements: 64 weights (twice eight bytes
+        // of packed indices, eight 16-byte chunks of 128-byte operand rows) per thread, in the two 64-wide blocks b = 0, 1
+        //   forward  (rows of the operand = n, blocks along k):                  row n = t / 2, half h = t % 2
+        //   backward (rows of the operand = n of the stage, blocks of k columns): row = t / 2, h
         // Eight consecutive lanes cover four rows x two halves of one block, whose swizzled chunk positions are all different.
-        // The index / palette loads run three stages ahead of the stage being written, ACROSS tile boundaries: the sequence
+        // The index / palette loads run two of the group's stages ahead of the one being written, ACROSS tile boundaries: the sequence
         // of (tile, stage) positions of this pair is one stream, so a new tile does not start with an exposed load latency.
-        const int t = threadIdx.x - 64;
-        const int h = t & 1;
-        const int rr = (t & 255) >> 1;
-        const int b = t >> 8;
+        const int grp = (threadIdx.x - 64) >> 8, t = (threadIdx.x - 64) & 255;
+        const int h = t & 1, rr = t >> 1;
         const int blocks_per_kgroup = p.gs_k / 64;
-        const int dj = n_pairs % p.tiles_j;                 // column-tile step from one tile of this pair to its next
-        // Position in the stream of (tile, stage) pairs of this CTA pair, with the running addresses of this thread's
-        // loads: per stage the index pointer moves by a constant (32 bytes along k in the forward product, 128 rows in the
-        // backward one), so a load costs a compare and an add instead of the full address arithmetic.
         struct Pos {
-            int tile, it, tj, kg, cnt;
-            const uint8_t* ip;            // packed indices of this thread at stage `it`
-            const __nv_bfloat16* pp;      // forward: palettes of this thread's row; backward: palette base + fixed k group
-            bool ok;                      // the fixed coordinate (forward: n, backward: k) lies inside the matrix
+            int tile, it;
+            const uint8_t* ip;            // packed indices of this thread at stage 0 of the tile, block 0
+            const __nv_bfloat16* pp;      // forward: palettes of this thread's row; backward: palette base
+            int kg0, kg1;                 // backward: k groups of the two blocks
+            bool ok0, ok1;                // the fixed coordinate (forward: n, backward: k of the block) lies inside the matrix and the tile
         };
-        const int koff = b * 64 + h * 32;
-        // number of stages for which the running coordinate stays inside the matrix (forward: k, backward: n)
-        const int it_lim = kBMn ? ((p.Wn - rr + kBK - 1) / kBK) : ((p.Wk - koff + kBK - 1) / kBK);
-        const long long ip_step = kBMn ? (long long)kBK * p.packed_pitch : (long long)(kBK / 4);
         auto set_tile = [&](Pos& q) {
-            const int jr = q.tj * 256 + 128 * (int)rank;
+            int m0, j0;
+            item_origin(q.tile, m0, j0);
+            const int half = item_width(q.tile) >> 1;       // columns of this CTA; threads beyond them have nothing to fetch
+            const int jr = j0 + half * (int)rank;
             if (kBMn) {
-                const int k = jr + koff;
-                q.ok = k < p.Wk;
-                q.kg = q.ok ? (k / p.gs_k) : 0;
-                q.cnt = 0;
+                const int k = jr + h * 32;
+                q.ok0 = k < p.Wk && h * 32 < half;
+                q.ok1 = k + 64 < p.Wk && h * 32 + 64 < half;
+                q.kg0 = q.ok0 ? k / p.gs_k : 0;
+                q.kg1 = q.ok1 ? (k + 64) / p.gs_k : 0;
                 q.ip = p.packed + (long long)rr * p.packed_pitch + (k >> 2);
-                q.pp = p.palette + (long long)q.kg * 4;
+                q.pp = p.palette;
             } else {
                 const int n = jr + rr;
-                q.ok = n < p.Wn;
-                q.kg = b / blocks_per_kgroup; q.cnt = b % blocks_per_kgroup;
-                q.ip = p.packed + (long long)n * p.packed_pitch + (koff >> 2);
-                const int ng = q.ok ? ((p.gs_n_shift >= 0) ? (n >> p.gs_n_shift) : (n / p.gs_n)) : 0;
+                q.ok0 = q.ok1 = n < p.Wn && rr < half;
+                q.ip = p.packed + (long long)n * p.packed_pitch + h * 8;
+                const int ng = q.ok0 ? ((p.gs_n_shift >= 0) ? (n >> p.gs_n_shift) : (n / p.gs_n)) : 0;
                 q.pp = p.palette + (long long)ng * p.n_kgroups * 4;
             }
         };
-        auto pos_next = [&](Pos& q) {
-            if (++q.it == nkb_total) {
-                q.it = 0; q.tile += n_pairs; q.tj += dj; if (q.tj >= p.tiles_j) q.tj -= p.tiles_j;
-                set_tile(q);
-            } else {
-                q.ip += ip_step;
-                if (!kBMn) {
-                    q.cnt += 2;
-                    while (q.cnt >= blocks_per_kgroup) { q.cnt -= blocks_per_kgroup; ++q.kg; }
-                }
-            }
+        auto normalise = [&](int& tile, int& it) {          // true: another tile
+            bool moved = false;
+            while (it >= nkb_total) { it -= nkb_total; tile += n_pairs; moved = true; }
+            return moved;
         };
-        auto load_pos = [&](const Pos& q, uint2& idx, uint2& pal) {
-            idx = make_uint2(0u, 0u); pal = make_uint2(0u, 0u);
-            if (!q.ok || q.it >= it_lim || q.it >= nkb || q.tile >= p.n_tiles) return;
-            idx = __ldg(reinterpret_cast<const uint2*>(q.ip));
+        auto load_pos = [&](const Pos& q, uint2 (&idx)[2], uint2 (&pal)[2]) {
+            idx[0] = idx[1] = pal[0] = pal[1] = make_uint2(0u, 0u);
+            if (q.it >= nkb || q.tile >= p.n_items) return;
             if (kBMn) {
                 const int n = q.it * kBK + rr;
+                if (n >= p.Wn) return;
+                const uint8_t* ip = q.ip + (long long)(q.it * kBK) * p.packed_pitch;
                 const int ng = (p.gs_n_shift >= 0) ? (n >> p.gs_n_shift) : (n / p.gs_n);
-                pal = __ldg(reinterpret_cast<const uint2*>(q.pp + (long long)ng * p.n_kgroups * 4));
-            } else {
-                pal = __ldg(reinterpret_cast<const uint2*>(q.pp + q.kg * 4));
+                const __nv_bfloat16* pp = q.pp + (long long)ng * p.n_kgroups * 4;
+                if (q.ok0) { idx[0] = __ldg(reinterpret_cast<const uint2*>(ip)); pal[0] = __ldg(reinterpret_cast<const uint2*>(pp + q.kg0 * 4)); }
+                if (q.ok1) { idx[1] = __ldg(reinterpret_cast<const uint2*>(ip + 16)); pal[1] = __ldg(reinterpret_cast<const uint2*>(pp + q.kg1 * 4)); }
+            } else if (q.ok0) {
+                const int kb = q.it * 2;                    // blocks of 64 along k
+                const uint8_t* ip = q.ip + q.it * (kBK / 4);
+                int g0, g1;
+                if (p.gs_k_shift >= 0) { g0 = kb >> p.gs_k_shift; g1 = (kb + 1) >> p.gs_k_shift; }
+                else { g0 = kb / blocks_per_kgroup; g1 = (kb + 1) / blocks_per_kgroup; }
+                if (kb * 64 + h * 32 < p.Wk) { idx[0] = __ldg(reinterpret_cast<const uint2*>(ip)); pal[0] = __ldg(reinterpret_cast<const uint2*>(q.pp + g0 * 4)); }
+                if (kb * 64 + 64 + h * 32 < p.Wk) { idx[1] = __ldg(reinterpret_cast<const uint2*>(ip + 16)); pal[1] = __ldg(reinterpret_cast<const uint2*>(q.pp + g1 * 4)); }
             }
         };
-        // The stream is walked three stages per trip (= the ring), so ring stage and queue slot of every step are compile-time
-        // constants: no slot is ever copied, which would make the copy wait for a load that has just been issued.
-        static_assert(kStages == 3, "the decode loop is unrolled by the depth of the ring");
-        uint2 idx_q[3], pal_q[3];
-        Pos pf; pf.tile = pair; pf.it = 0; pf.tj = pair % p.tiles_j; set_tile(pf);
-        int c_tile = pair, c_it = 0;   // the position being written
+        // Two stages per trip, so that the queue slot of every step is a compile-time constant: no slot is ever copied, which would make
+        // the copy wait for a load that has just been issued.
+        uint2 idx_q[2][2], pal_q[2][2];
+        Pos pf; pf.tile = pair; pf.it = grp;
+        normalise(pf.tile, pf.it);
+        set_tile(pf);
+        int c_tile = pf.tile, c_it = pf.it;   // the position being written
+        auto pos_next = [&](Pos& q) {
+            q.it += 2;
+            if (normalise(q.tile, q.it) && q.tile < p.n_items) set_tile(q);
+        };
 #pragma unroll
-        for (int u = 0; u < 3; ++u) { load_pos(pf, idx_q[u], pal_q[u]); pos_next(pf); }
+        for (int u = 0; u < 2; ++u) { load_pos(pf, idx_q[u], pal_q[u]); pos_next(pf); }
+        int s = grp;                          // ring slot and phase of the stage being written
+        uint32_t ph = 0;
         bool ok = true;
-        for (int g0 = 0; ok && c_tile < p.n_tiles; g0 += 3) {
-            const uint32_t ph = (uint32_t)((g0 / 3) & 1);
+        while (ok && c_tile < p.n_items) {
 #pragma unroll
-            for (int u = 0; u < 3; ++u) {
-                if (c_tile >= p.n_tiles) break;
+            for (int u = 0; u < 2; ++u) {
+                if (!ok || c_tile >= p.n_items) break;
                 const bool is_extra = c_it >= nkb;
-                if (++c_it == nkb_total) { c_it = 0; c_tile += n_pairs; }
-                const uint2 idx_cur = idx_q[u], pal_cur = pal_q[u];
+                const int half = item_width(c_tile) >> 1;
+                uint2 idx[2] = {idx_q[u][0], idx_q[u][1]}, pl[2] = {pal_q[u][0], pal_q[u][1]};
                 load_pos(pf, idx_q[u], pal_q[u]);
                 pos_next(pf);
-                ok = mbar_wait(empty(u), ph ^ 1u, abort_flag, p.status, ST_TIMEOUT_EMPTY, 3);
+                ok = mbar_wait(empty(s), ph ^ 1u, abort_flag, p.status, ST_TIMEOUT_EMPTY, 3);
                 if (!ok) break;
-                if (is_extra) {
-                    // the LoRA block comes by TMA; arrive all the same, after the stage is free, to keep the phases in step
-                    if (lane == 0) mbar_arrive_cluster(lead_full(u));
-                    continue;
-                }
-                uint8_t* row = smem + u * kStageBytes + kABytes + b * kBlkBytes + rr * 128;
-                const PalRegs pal = pal_split(pal_cur.x, pal_cur.y);
-                const uint32_t w[2] = {idx_cur.x, idx_cur.y};
+                if (!is_extra) {              // the LoRA block comes by TMA; arrive all the same, after the stage is free, to keep the phases in step
 #pragma unroll
-                for (int i = 0; i < 2; ++i) {
-                    uint32_t o[8];
-                    decode16(w[i], pal, o);
-                    *reinterpret_cast<uint4*>(row + (((4 * h + 2 * i) ^ (rr & 7)) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
-                    *reinterpret_cast<uint4*>(row + (((4 * h + 2 * i + 1) ^ (rr & 7)) << 4)) = make_uint4(o[4], o[5], o[6], o[7]);
+                    for (int b = 0; b < 2; ++b) {
+                        if ((kBMn ? b * 64 + h * 32 : rr) >= half) continue;
+                        uint8_t* row = smem + s * kStageBytes + kABytes + b * kBlkBytes + rr * 128;
+                        const PalRegs pal = pal_split(pl[b].x, pl[b].y);
+                        const uint32_t w[2] = {idx[b].x, idx[b].y};
+#pragma unroll
+                        for (int i = 0; i < 2; ++i) {
+                            uint32_t o[8];
+                            decode16(w[i], pal, o);
+                            *reinterpret_cast<uint4*>(row + (((4 * h + 2 * i) ^ (rr & 7)) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
+                            *reinterpret_cast<uint4*>(row + (((4 * h + 2 * i + 1) ^ (rr & 7)) << 4)) = make_uint4(o[4], o[5], o[6], o[7]);
+                        }
+                    }
+                    fence_proxy_async_smem();
+                    __syncwarp();
                 }
-                fence_proxy_async_smem();
-                __syncwarp();
-                if (lane == 0) mbar_arrive_cluster(lead_full(u));
+                if (lane == 0) mbar_arrive_cluster(lead_full(s));
+                s += 2;
+                if (s >= kStages) { s -= kStages; ph ^= 1u; }
+                c_it += 2;
+                normalise(c_tile, c_it);
             }
         }
     } else {
@@ -336,24 +362,26 @@ lut_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
         const uint32_t stage_u32 = base + kEpiOff + e * kEpiStageBytes;
         bool ok = true;
         int lt = 0;
-        for (int t = pair; t < p.n_tiles && ok; t += n_pairs, ++lt) {
+        for (int t = pair; t < p.n_items && ok; t += n_pairs, ++lt) {
             int m0, j0;
-            tile_origin(t, m0, j0);
+            item_origin(t, m0, j0);
+            const int w = item_width(t);
             const int buf = lt & 1;
             const int mrow = m0 + 128 * (int)rank + lane_group * 32;
             ok = mbar_wait(acc_full(buf), (lt >> 1) & 1, abort_flag, p.status, ST_TIMEOUT_ACCUM, 4);
             if (!ok) break;
             tc_fence_after_sync();
 #pragma unroll 1
-            for (int b = 0; b < 4; ++b) {
-                const int col = b * 64;
+            for (int col = 0; col < w; col += 64) {
+                const bool wide = col + 32 < w;            // a box of 64 columns, or the last 32 of a tile
                 if (lane == 0) tma_store_wait_read();
                 __syncwarp();
 #pragma unroll
                 for (int c = 0; c < 2; ++c) {
+                    if (c == 1 && !wide) break;
                     uint32_t v[32];
                     tmem_ld_32x32(tmem_base + ((uint32_t)(lane_group * 32) << 16) + buf * 256u + col + c * 32, v);
-                    if (b == 3 && c == 1) {
+                    if (col + 32 * (c + 1) >= w) {
                         // last read of this accumulator: hand it back to the MMA thread of the leader
                         tc_fence_before_sync();
                         __syncwarp();
@@ -361,18 +389,24 @@ lut_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
                     }
 #pragma unroll
                     for (int g = 0; g < 4; ++g) {
-                        uint4 o;
-                        o.x = pack_bf16x2(__uint_as_float(v[g * 8 + 0]) * p.alpha, __uint_as_float(v[g * 8 + 1]) * p.alpha);
-                        o.y = pack_bf16x2(__uint_as_float(v[g * 8 + 2]) * p.alpha, __uint_as_float(v[g * 8 + 3]) * p.alpha);
-                        o.z = pack_bf16x2(__uint_as_float(v[g * 8 + 4]) * p.alpha, __uint_as_float(v[g * 8 + 5]) * p.alpha);
-                        o.w = pack_bf16x2(__uint_as_float(v[g * 8 + 6]) * p.alpha, __uint_as_float(v[g * 8 + 7]) * p.alpha);
-                        *reinterpret_cast<uint4*>(stage + swz128(lane, c * 4 + g)) = o;
+                        float f[8];
+                        uint4 bb = make_uint4(0u, 0u, 0u, 0u);
+                        const int jc = j0 + col + c * 32 + g * 8;      // J is a multiple of 8
+                        if (p.bias != nullptr && jc < p.J) bb = __ldg(reinterpret_cast<const uint4*>(p.bias + jc));
+                        const uint32_t bw[4] = {bb.x, bb.y, bb.z, bb.w};
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            f[2 * i] = __uint_as_float(v[g * 8 + 2 * i]) * p.alpha + __uint_as_float(bw[i] << 16);
+                            f[2 * i + 1] = __uint_as_float(v[g * 8 + 2 * i + 1]) * p.alpha + __uint_as_float(bw[i] & 0xFFFF0000u);
+                        }
+                        const uint32_t at = wide ? swz128(lane, c * 4 + g) : (uint32_t)(lane * 64 + ((g ^ ((lane >> 1) & 3)) << 4));
+                        *reinterpret_cast<uint4*>(stage + at) = make_uint4(pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]), pack_bf16x2(f[4], f[5]), pack_bf16x2(f[6], f[7]));
                     }
                 }
                 fence_proxy_async_smem();
                 __syncwarp();
                 if (lane == 0 && j0 + col < p.J && mrow < p.M) {
-                    tma_store_2d(&tmD, stage_u32, j0 + col, mrow);
+                    tma_store_2d(wide ? &tmD : &tmD32, stage_u32, j0 + col, mrow);
                     tma_store_commit();
                 }
             }
@@ -392,7 +426,7 @@ lut_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
 
 template <int BMODE>
 int launch_pair_t(const LutGemmArgs& a, cudaStream_t stream) {
-    CUtensorMap tmA, tmA2, tmB2, tmD;
+    CUtensorMap tmA, tmA2, tmB2, tmD, tmD32;
     int rc;
     if ((rc = make_tmap_bf16(&tmA, a.A, a.M, a.R, a.lda, 64, 128))) return rc;
     tmA2 = tmA; tmB2 = tmA;
@@ -405,19 +439,19 @@ int launch_pair_t(const LutGemmArgs& a, cudaStream_t stream) {
         }
     }
     if ((rc = make_tmap_bf16(&tmD, a.out, a.M, a.J, a.ld_out, 64, 32))) return rc;
+    if ((rc = make_tmap_bf16(&tmD32, a.out, a.M, a.J, a.ld_out, 32, 32))) return rc;
     PairParams p = {};
     p.M = a.M; p.J = a.J; p.R = a.R; p.n_extra = a.r2 > 0 ? 1 : 0;
-    p.tiles_j = (a.J + 255) / 256;
-    p.tiles_m = (a.M + 255) / 256;
-    p.n_tiles = p.tiles_m * p.tiles_j;
     p.packed = (const uint8_t*)a.packed; p.packed_pitch = a.packed_pitch;
     p.palette = (const __nv_bfloat16*)a.palette;
     p.gs_n = a.gs_n > 0 ? a.gs_n : 1; p.gs_k = a.gs_k > 0 ? a.gs_k : kBK;
     p.n_kgroups = a.gs_k > 0 ? (a.Wk / a.gs_k) : 1;
     p.gs_n_shift = -1;
     for (int sh = 0; sh < 31; ++sh) if ((1 << sh) == p.gs_n) p.gs_n_shift = sh;
+    p.gs_k_shift = -1;
+    for (int sh = 0; sh < 26; ++sh) if ((64ll << sh) == p.gs_k) p.gs_k_shift = sh;
     p.Wn = a.Wn; p.Wk = a.Wk;
-    p.alpha = a.alpha;
+    p.alpha = a.alpha; p.bias = (const __nv_bfloat16*)a.bias;
     p.status = device_status_ptr();
     p.prof = (unsigned long long*)a.prof;
     auto kern = lut_gemm_pair_kernel<BMODE>;
@@ -432,25 +466,51 @@ int launch_pair_t(const LutGemmArgs& a, cudaStream_t stream) {
     if (a.sm_limit > 0 && a.sm_limit < sms) sms = a.sm_limit;
     if (g_cta_limit > 0 && g_cta_limit < sms) sms = g_cta_limit;
     int pairs = sms / 2;
-    if (pairs > p.n_tiles) pairs = p.n_tiles;
     if (pairs < 1) return PLZ_ERR_UNSUPPORTED;
+    // backward product: a decode thread's 32 columns start at a multiple of 32 (8-byte loads of indices, one palette group)
+    const PairTiles pt = plan_pair_tiles(a.M, a.J, pairs, BMODE == B_DECODE_MN ? 64 : 32);
+    p.tiles_j = pt.tiles_j; p.tile_w = pt.tile_w; p.n_whole = pt.n_whole; p.n_items = pt.n_items;
+    if (pairs > p.n_items) pairs = p.n_items;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2 * pairs);
     cfg.blockDim = dim3(kThreads);
     cfg.dynamicSmemBytes = kSmemBytes;
     cfg.stream = stream;
-    PLZ_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kern, tmA, tmA2, tmB2, tmD, p));
+    PLZ_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kern, tmA, tmA2, tmB2, tmD, tmD32, p));
     ++g_launch_count;
     return PLZ_OK;
 }
 
 }  // namespace
 
+// Waves of a launch in units of a 256-column tile, the shortest of
+//   whole tiles, the last wave cut in halves where the halves fit one wave;
+//   fewer tiles than pairs: the narrowest tile that fits one wave.
+PairTiles plan_pair_tiles(int M, int J, int pairs, int step) {
+    const int tiles_m = (M + 255) / 256;
+    PairTiles t;
+    t.tile_w = 256; t.tiles_j = (J + 255) / 256;
+    const int tiles = tiles_m * t.tiles_j;
+    t.n_whole = t.n_items = tiles;
+    if (tiles <= pairs) {
+        for (int w = 128; w < 256; w += step) {
+            const int tj = (J + w - 1) / w;
+            if (tiles_m * tj <= pairs) { t.tile_w = w; t.tiles_j = tj; t.n_whole = t.n_items = tiles_m * tj; break; }
+        }
+        return t;
+    }
+    const int rem = tiles % pairs;
+    if (rem > 0 && 2 * rem <= pairs) { t.n_whole = tiles - rem; t.n_items = t.n_whole + 2 * rem; }
+    return t;
+}
+
 // PLZ_ERR_UNSUPPORTED: not a shape for this kernel, the caller falls back to the single-CTA kernel.
 int launch_lut_gemm_pair(const LutGemmArgs& a, cudaStream_t stream) {
     if (!g_pair_gemm) return PLZ_ERR_UNSUPPORTED;
     if (a.bmode != B_DECODE_K && a.bmode != B_DECODE_MN) return PLZ_ERR_UNSUPPORTED;
-    if (a.fuse != 0 || a.M < 256 || a.J < 256) return PLZ_ERR_UNSUPPORTED;
+    const bool plain = a.fuse == 0 || (a.fuse == 2 && !a.col_scale && !a.row_scale);   // fuse 2 without norm factors: at most a bias
+    if (!plain || a.M < 256 || a.J < 256) return PLZ_ERR_UNSUPPORTED;
+    if ((uintptr_t)a.bias & 15) return PLZ_ERR_UNSUPPORTED;
     if (a.bmode == B_DECODE_MN && (a.J % 16)) return PLZ_ERR_UNSUPPORTED;
     if (a.bmode == B_DECODE_K && (a.Wk % 16)) return PLZ_ERR_UNSUPPORTED;
     return a.bmode == B_DECODE_K ? launch_pair_t<B_DECODE_K>(a, stream) : launch_pair_t<B_DECODE_MN>(a, stream);
