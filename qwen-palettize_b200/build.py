@@ -9,7 +9,7 @@ import sys
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
-SOURCES = ["api.cu", "lut_gemm.cu", "lut_gemm_pair.cu", "narrow_gemm.cu", "tn_gemm.cu", "elementwise.cu", "gemv.cu", "smallm_mma.cu", "train_ops.cu", "soft_tensors.cu", "attention.cu", "attention_decode.cu", "layer_ops.cu",
+SOURCES = ["api.cu", "lut_gemm.cu", "lut_gemm_pair.cu", "dense_gemm_pair.cu", "narrow_gemm.cu", "tn_gemm.cu", "elementwise.cu", "gemv.cu", "smallm_mma.cu", "train_ops.cu", "soft_tensors.cu", "attention.cu", "attention_decode.cu", "layer_ops.cu",
            "seq_linear.cu", "seq_ops.cu", "seq_recurrent.cu", "seq_chunk.cu", "seq_scan.cu", "attention_bias.cu", "attention_bias_tc.cu",
            "latent_ops.cu", "latent_attention.cu", "latent_attention_tc.cu"]
 PRECISE = {"narrow_gemm.cu", "seq_linear.cu", "seq_ops.cu", "seq_recurrent.cu", "seq_chunk.cu", "seq_scan.cu", "attention_bias.cu", "latent_ops.cu", "latent_attention.cu"}   # compiled without --use_fast_math

@@ -683,6 +683,10 @@ int launch_lut_gemm(const LutGemmArgs& a, cudaStream_t stream) {
         const int rc = launch_lut_gemm_pair(a, stream);
         if (rc != PLZ_ERR_UNSUPPORTED) return rc;
     }
+    if (!decode) {
+        const int rc = launch_dense_gemm_pair(a, stream);
+        if (rc != PLZ_ERR_UNSUPPORTED) return rc;
+    }
     // narrow outputs (the rank-16/32 LoRA products) are bound by streaming A: 128-row tiles give twice the CTAs
     const bool big = a.M > 128 && a.J > 64;
     const bool narrow = !decode && a.J <= 64 && a.r2 == 0;

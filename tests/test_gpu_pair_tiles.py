@@ -1,9 +1,10 @@
-"""Products on CTA pairs (csrc/lut_gemm_pair.cu) with every tile width its plan chooses on 74 pairs, against the same product in 64 bits. One
+"""Products on CTA pairs (csrc/lut_gemm_pair.cu, csrc/dense_gemm_pair.cu) with every tile width its plan chooses on 74 pairs, against the same product in 64 bits. One
 bf16 rounding of the result bounds every element by 2^-8 of it; sums over K in fp32 add at most K 2^-24 of the sum of magnitudes."""
 import pytest
 import torch
 
 import plz_ops as ops
+import seq_ops as S
 
 pytestmark = pytest.mark.gpu
 
@@ -51,3 +52,39 @@ def test_tile_widths(M, J, R, rank):
         dx = ops.backward_dx(w, x)[0]
     check(dx, ref, mag, R + rank)
 
+
+# the dense counterpart (csrc/dense_gemm_pair.cu): the same widths, gated outputs in steps of 64, reductions that end inside a stage or a block
+@pytest.mark.parametrize("M,J,R,rank", [(256, 256, 128, 0), (1000, 2560, 200, 0), (1000, 2560, 192, 16), (1000, 3200, 72, 0), (900, 3904, 64, 64),
+                                        (1024, 4544, 1000, 0), (4800, 1024, 192, 0), (1000, 9664, 128, 0), (300, 1088, 328, 0)])
+def test_dense_tile_widths(M, J, R, rank):
+    g = torch.Generator(device="cuda").manual_seed(M + J)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda").bfloat16()
+    x, w, bias = rnd(M, R), rnd(J, R), rnd(J)
+    z, mag = x.double() @ w.double().T, x.double().abs() @ w.double().abs().T
+    if rank:
+        lora = (rnd(rank, R), rnd(J, rank), 0.5)
+        y, t = ops.dense_forward(w, x, lora)
+        check(y, z + t.double() @ lora[1].double().T, mag + t.double().abs() @ lora[1].double().abs().T, R + rank)
+    else:
+        out = torch.full((M, J + 16), 7.0, device="cuda", dtype=torch.bfloat16)
+        S.linear(x, w, out=out[:, 8:8 + J])
+        check(out[:, 8:8 + J], z, mag, R)
+        assert bool((out[:, :8] == 7).all()) and bool((out[:, 8 + J:] == 7).all())
+        check(S.linear(x, w, bias), z + bias.double(), mag + bias.double().abs(), R)
+        y, r = S.linear(x, w, act=S.ACT_RELU2), z.clamp(min=0)
+        assert bool(((y.double() - r * r).abs() <= 2.0 ** -8 * r * r + (2 * r + 1) * (R * 2.0 ** -24 * mag) + 1e-30).all())
+        w2 = (w * R ** -0.5).bfloat16()
+        z, mag = x.double() @ w2.double().T, x.double().abs() @ w2.double().abs().T
+        ref = torch.nn.functional.gelu(z[:, 0::2], approximate="tanh") * z[:, 1::2]
+        # |d gelu| <= 1.13; each of the two factors carries R 2^-24 times the row's magnitude, the fast exp and divide 2^-20 of the gate
+        slack = R * 2.0 ** -24 * (1.13 * mag[:, 0::2] * z[:, 1::2].abs() + mag[:, 1::2] * z[:, 0::2].abs()) + 2.0 ** -20 * (z[:, 0::2] * z[:, 1::2]).abs() + 1e-7
+        assert bool(((S.linear(x, w2, act=S.ACT_GLU_GELU).double() - ref).abs() <= 2.0 ** -8 * ref.abs() + slack).all())
+    # reduction over the rows of the matrix
+    if R % 64 == 0:
+        wt = rnd(R, J)
+        lora = (rnd(rank, J), rnd(R, rank), 0.5) if rank else None
+        dx, dt = ops.dense_backward_dx(wt, x, lora)
+        ref, mag = x.double() @ wt.double(), x.double().abs() @ wt.double().abs()
+        if rank:
+            ref, mag = ref + dt.double() @ lora[0].double(), mag + dt.double().abs() @ lora[0].double().abs()
+        check(dx, ref, mag, R + rank)
