@@ -1,8 +1,15 @@
 // Attention of one new token per sequence against a key / value cache (token decode), and the embedding-row gather that
-// opens a forward pass. Both are single passes bound by HBM: a decode step reads every cached key and value once
-// (B * T * Hkv * 128 * 2 * 2 bytes per layer), no tensor core involved.
+// opens a forward pass. Both are single passes that should be bound by HBM: a decode step reads every cached key and value once
+// (B * T * Hkv * 128 * 2 * 2 bytes per layer).
 //
-//   attn_decode_partial_kernel  grid (splits, Hkv, B), 4 warps. The sequence is cut into `splits` contiguous chunks so that
+//   attn_decode_mma_kernel  bf16, head sizes above 64 and up to 128. With scores and sums on FMAs (the kernel below) a step of 64 sequences over 1025
+//     tokens of 8 key / value heads issued about 1000 instructions per 16 tokens and warp and took 68 us for 268 MB, bound by issue. Here the
+//     scores are mma.sync m16n8k16 (A = the query heads of the group, 4 of 16 rows used; B = 8 keys straight from memory, the order of
+//     the dimensions permuted alike on both sides so that a lane's operands are whole 16-byte loads): products of bf16 are exact and sums
+//     are fp32 as before. The weights stay fp32: they pass through shared memory (16 tokens x 4 heads per warp and step) to the lanes that
+//     hold the values, and weight x value runs on packed fp32 pairs.
+//     Keys and values are requested one step ahead. 69 -> 51 us (5.3 TB/s); one sequence of 2049 tokens 6.2 -> 5.5 us.
+//   attn_decode_partial_kernel  the other types and sizes: grid (splits, Hkv, B), 4 warps. The sequence is cut into `splits` contiguous chunks so that
 //     the launch has a few CTAs per SM whatever B is. Inside a CTA a warp takes 8 tokens per step: 16 lanes per token, each
 //     lane the 16 bytes (8 dims) of the key and of the value row that belong to it, so one load instruction of a warp covers
 //     two whole 256-byte rows, and four such loads for K and four for V are in flight per lane before anything is used. The
@@ -10,6 +17,7 @@
 //     slots) are summed over the 16 lanes by recursive halving (15 shuffles, after which lane i owns score i), so exp2 is
 //     evaluated once per score; online softmax (running max and sum per head) across steps; the warps' partial results meet in
 //     shared memory. With one split the CTA writes the bf16 output itself, else an unnormalised fp32 partial (o, max, sum).
+//     Both kernels share the grid, the split and the merge.
 //   attn_decode_combine_kernel  merges the splits.
 //
 // Template parameters widen it: element type (bf16, fp32), lanes per token (8, 16, 32: head sizes up to 64, 128, 256, key and value
@@ -69,6 +77,36 @@ template <> struct Chunk<float> {
 };
 __device__ __forceinline__ void store_elem(__nv_bfloat16* p, float v) { *p = __float2bfloat16_rn(v); }
 __device__ __forceinline__ void store_elem(float* p, float v) { *p = v; }
+
+// the warps' partial results of a CTA, unnormalised (o, max, sum) per head: thread d takes dimension d (and d + 128) of every head
+template <typename T, bool EXT, int D>
+__device__ __forceinline__ void merge_warps(const DecParams& p, const float (&sm_o)[kDecWarps][4][D], const float (&sm_ml)[kDecWarps][4][2], int split, int b,
+                                            int head0, int G, int dv) {
+    for (int d = threadIdx.x; d < dv; d += kDecWarps * 32) {
+        for (int g = 0; g < G; ++g) {
+            float M = kNegBig;
+#pragma unroll
+            for (int w = 0; w < kDecWarps; ++w) M = fmaxf(M, sm_ml[w][g][0]);
+            const bool sink = EXT && p.sink && p.splits == 1;
+            if (sink) M = fmaxf(M, 0.f);
+            float acc = 0.f, l = sink ? ex2(-M) : 0.f;
+#pragma unroll
+            for (int w = 0; w < kDecWarps; ++w) {
+                const float c = ex2(sm_ml[w][g][0] - M);
+                acc = fmaf(c, sm_o[w][g][d], acc);
+                l = fmaf(c, sm_ml[w][g][1], l);
+            }
+            const int head = head0 + g;
+            if (p.splits == 1) {
+                store_elem((T*)p.out + (long long)b * p.ldo + (long long)head * dv + d, l > 0.f ? acc / l : 0.f);
+            } else {
+                const long long slot = ((long long)b * p.Hq + head) * p.splits + split;
+                p.ws_o[slot * dv + d] = acc;
+                if (d == 0) { p.ws_ml[slot * 2] = M; p.ws_ml[slot * 2 + 1] = l; }
+            }
+        }
+    }
+}
 
 // T: element type; LPT: lanes per token (head sizes up to 8 * LPT); EXT: the head sizes, bias, sink and length of the params
 template <typename T, int LPT, bool EXT>
@@ -199,31 +237,169 @@ attn_decode_partial_kernel(const DecParams p) {
         if (u_own == 0) { sm_ml[warp][g_own][0] = m_own; sm_ml[warp][g_own][1] = l_own; }
     }
     __syncthreads();
-    // merge the warps: thread d takes dimension d (and d + 128) of every head
-    for (int d = threadIdx.x; d < dv; d += kDecWarps * 32) {
-        for (int g = 0; g < G; ++g) {
-            float M = kNegBig;
+    merge_warps<T, EXT, D>(p, sm_o, sm_ml, split, b, head0, G, dv);
+}
+
+__device__ __forceinline__ uint64_t pack2(float lo, float hi) { uint64_t r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi)); return r; }
+__device__ __forceinline__ void unpack2(uint64_t v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) { uint64_t d; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c)); return d; }
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) { uint64_t d; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
+__device__ __forceinline__ uint32_t word(const uint4& v, int i) { return i == 0 ? v.x : i == 1 ? v.y : i == 2 ? v.z : v.w; }
+
+// A warp takes 16 tokens per step. Scores: lane (g, t) = (lane / 4, lane % 4) loads chunks t, t + 4, t + 8, t + 12 (of 8 dimensions) of the keys of tokens
+// g and g + 8, and of query head g; words 2 h, 2 h + 1 of a chunk are the operand registers of one MMA. It ends up with the scores of head g for tokens
+// 2 t, 2 t + 1, 2 t + 8, 2 t + 9. Values: lane (tl, dl) = (lane / 16, lane % 16) holds dimensions 8 dl .. of tokens 2 u + tl, as in the kernel above.
+template <bool EXT>
+__global__ void __launch_bounds__(kDecWarps * 32, 4)
+attn_decode_mma_kernel(const DecParams p) {
+    constexpr int D = 128, kStep = 16;
+    __shared__ float sm_o[kDecWarps][4][D];
+    __shared__ float sm_ml[kDecWarps][4][2];
+    __shared__ float4 sm_p[kDecWarps][kStep];       // weights of a step: token -> four heads
+    __shared__ uint4 sm_q[8][17];                   // query heads (rows of absent heads zero)
+    const int split = blockIdx.x, hk = blockIdx.y / p.passes, g0 = (blockIdx.y % p.passes) * 4, b = blockIdx.z;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3, tl = lane >> 4, dl = lane & 15;
+    const int G = min(4, p.group - g0);
+    const int head0 = hk * p.group + g0;
+    const int dk = EXT ? p.dk : 128, dv = EXT ? p.dv : 128;
+    const bool in_v = !EXT || dl * 8 < dv;
+    pdl_launch_dependents();
+    pdl_wait();
+    const int T_all = EXT ? *p.pos + 1 : p.T;
+    int chunk = p.chunk;
+    if (EXT) chunk = ((T_all + p.splits - 1) / p.splits + kCtaStep - 1) / kCtaStep * kCtaStep;
+    const int t0 = split * chunk, t1 = min(T_all, t0 + chunk);
+
+    for (int i = threadIdx.x; i < 8 * 16; i += kDecWarps * 32) {
+        const int h = i >> 4, c = i & 15;
+        uint4 v = make_uint4(0u, 0u, 0u, 0u);
+        if (h < G && (!EXT || c * 8 < dk)) v = __ldcs(reinterpret_cast<const uint4*>((const __nv_bfloat16*)p.q + (long long)b * p.ldq + (long long)(head0 + h) * dk + c * 8));
+        sm_q[h][c] = v;
+    }
+    __syncthreads();
+    uint64_t o[4][4];
 #pragma unroll
-            for (int w = 0; w < kDecWarps; ++w) M = fmaxf(M, sm_ml[w][g][0]);
-            const bool sink = EXT && p.sink && p.splits == 1;
-            if (sink) M = fmaxf(M, 0.f);
-            float acc = 0.f, l = sink ? ex2(-M) : 0.f;
+    for (int h = 0; h < 4; ++h)
 #pragma unroll
-            for (int w = 0; w < kDecWarps; ++w) {
-                const float c = ex2(sm_ml[w][g][0] - M);
-                acc = fmaf(c, sm_o[w][g][d], acc);
-                l = fmaf(c, sm_ml[w][g][1], l);
-            }
-            const int head = head0 + g;
-            if (p.splits == 1) {
-                store_elem((T*)p.out + (long long)b * p.ldo + (long long)head * dv + d, l > 0.f ? acc / l : 0.f);
-            } else {
-                const long long slot = ((long long)b * p.Hq + head) * p.splits + split;
-                p.ws_o[slot * dv + d] = acc;
-                if (d == 0) { p.ws_ml[slot * 2] = M; p.ws_ml[slot * 2 + 1] = l; }
+        for (int d = 0; d < 4; ++d) o[h][d] = 0ull;
+    float m_own = kNegBig, l_own = 0.f;             // of head g, this lane's share of the sum
+    const __nv_bfloat16* kb = (const __nv_bfloat16*)p.k + (long long)b * p.k_batch + (long long)hk * dk + t * 8;
+    const __nv_bfloat16* vb = (const __nv_bfloat16*)p.v + (long long)b * p.v_batch + (long long)hk * dv + dl * 8;
+    const float* brow = nullptr;
+    if (EXT && p.bias && g < G) brow = p.bias + (long long)(head0 + g) * p.ldb;
+
+    uint4 kr[2][4], vr[8];
+    float bias[4];
+    auto load_k = [&](int base) {
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            const int tok = base + 8 * r + g;
+            const __nv_bfloat16* row = kb + (long long)tok * p.k_tok;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                kr[r][j] = make_uint4(0u, 0u, 0u, 0u);
+                if (tok < t1 && (!EXT || (t + 4 * j) * 8 < dk)) kr[r][j] = __ldcs(reinterpret_cast<const uint4*>(row + 32 * j));
             }
         }
+        if (EXT && p.bias) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int tok = base + (i >> 1) * 8 + 2 * t + (i & 1);
+                bias[i] = brow && tok < t1 ? __ldg(brow + min(T_all - 1 - tok, p.n_bias - 1)) : 0.f;
+            }
+        }
+    };
+    auto load_v = [&](int base) {
+        const __nv_bfloat16* row = vb + (long long)(base + tl) * p.v_tok;
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            vr[u] = make_uint4(0u, 0u, 0u, 0u);
+            if (base + 2 * u + tl < t1 && in_v) vr[u] = __ldcs(reinterpret_cast<const uint4*>(row));
+            row += 2 * p.v_tok;
+        }
+    };
+    // keys and values of a step are requested one step ahead, each as soon as the registers of the step before are used up
+    load_k(t0 + warp * kStep);
+    load_v(t0 + warp * kStep);
+    for (int base = t0 + warp * kStep; base < t1; base += kDecWarps * kStep) {
+        float s[4];
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            float c[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const uint4 q = sm_q[g][t + 4 * j];
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+                    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+                                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+                                 : "r"(word(q, 2 * h)), "r"(0u), "r"(word(q, 2 * h + 1)), "r"(0u), "r"(word(kr[r][j], 2 * h)), "r"(word(kr[r][j], 2 * h + 1)));
+            }
+            s[2 * r] = c[0]; s[2 * r + 1] = c[1];
+        }
+        float mx = m_own;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int tok = base + (i >> 1) * 8 + 2 * t + (i & 1);
+            s[i] *= p.scale_log2e;
+            if (EXT && p.bias) s[i] = fmaf(bias[i], kLog2eDec, s[i]);
+            if (tok >= t1) s[i] = kNegBig;
+            mx = fmaxf(mx, s[i]);
+        }
+        load_k(base + kDecWarps * kStep);
+        mx = fmaxf(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, 1));
+        mx = fmaxf(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, 2));
+        const float corr = ex2(m_own - mx);
+        const bool grew = mx > m_own;
+        m_own = mx;
+        l_own *= corr;
+        __syncwarp();                               // the previous step's weights have been read
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int at = (i >> 1) * 8 + 2 * t + (i & 1);
+            const float w = base + at < t1 ? ex2(s[i] - mx) : 0.f;
+            l_own += w;
+            if (g < 4) reinterpret_cast<float*>(&sm_p[warp][at])[g] = w;
+        }
+        if (__any_sync(0xFFFFFFFFu, grew)) {
+#pragma unroll
+            for (int h = 0; h < 4; ++h) {
+                const float ch = __shfl_sync(0xFFFFFFFFu, corr, 4 * h);
+                const uint64_t c2 = pack2(ch, ch);
+#pragma unroll
+                for (int d = 0; d < 4; ++d) o[h][d] = mul2(o[h][d], c2);
+            }
+        }
+        __syncwarp();
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            const float4 w = sm_p[warp][2 * u + tl];
+            const uint64_t w2[4] = {pack2(w.x, w.x), pack2(w.y, w.y), pack2(w.z, w.z), pack2(w.w, w.w)};
+#pragma unroll
+            for (int d = 0; d < 4; ++d) {
+                const uint32_t v = word(vr[u], d);
+                const uint64_t v2 = pack2(__uint_as_float(v << 16), __uint_as_float(v & 0xFFFF0000u));
+#pragma unroll
+                for (int h = 0; h < 4; ++h) o[h][d] = fma2(w2[h], v2, o[h][d]);
+            }
+        }
+        load_v(base + kDecWarps * kStep);
     }
+    l_own += __shfl_xor_sync(0xFFFFFFFFu, l_own, 1);
+    l_own += __shfl_xor_sync(0xFFFFFFFFu, l_own, 2);
+    if (t == 0 && g < 4) { sm_ml[warp][g][0] = m_own; sm_ml[warp][g][1] = l_own; }
+#pragma unroll
+    for (int h = 0; h < 4; ++h)
+#pragma unroll
+        for (int d = 0; d < 4; ++d) {
+            float lo, hi;
+            unpack2(o[h][d], lo, hi);
+            lo += __shfl_xor_sync(0xFFFFFFFFu, lo, 16);      // the two token slots
+            hi += __shfl_xor_sync(0xFFFFFFFFu, hi, 16);
+            if (tl == 0) { sm_o[warp][h][dl * 8 + 2 * d] = lo; sm_o[warp][h][dl * 8 + 2 * d + 1] = hi; }
+        }
+    __syncthreads();
+    merge_warps<__nv_bfloat16, EXT, D>(p, sm_o, sm_ml, split, b, head0, G, dv);
 }
 
 // Merge of the splits: one block per (head, sequence), thread d = dimension d (and d + 128). The weights exp2(m_s - M) of the
@@ -324,7 +500,7 @@ int launch_attn_decode(const AttnDecodeArgs& a, cudaStream_t stream) {
     p.ws_ml = p.ws_o ? p.ws_o + (long long)a.B * a.Hq * p.splits * 128 : nullptr;
     p.T = a.T; p.Hq = a.Hq; p.Hkv = a.Hkv; p.group = a.Hq / a.Hkv; p.passes = (p.group + 3) / 4;
     p.scale_log2e = a.scale * kLog2eDec;
-    PLZ_LAUNCH_CHAIN((attn_decode_partial_kernel<__nv_bfloat16, 16, false>), dim3(p.splits, a.Hkv * p.passes, a.B), dim3(kDecWarps * 32), 0, stream, p);
+    PLZ_LAUNCH_CHAIN(attn_decode_mma_kernel<false>, dim3(p.splits, a.Hkv * p.passes, a.B), dim3(kDecWarps * 32), 0, stream, p);
     if (p.splits > 1) {
         PLZ_LAUNCH_CHAIN(attn_decode_combine_kernel<__nv_bfloat16>, dim3(a.Hq, a.B), dim3(128), 0, stream, (const float*)p.ws_o, (const float*)p.ws_ml,
                          p.splits, a.Hq, 128, 0, (__nv_bfloat16*)p.out, p.ldo);
@@ -355,7 +531,8 @@ static int launch_attn_bias_decode_t(const AttnBiasArgs& a, int cap, float* ws, 
     const dim3 grid(p.splits, a.G * p.passes, a.B), block(kDecWarps * 32);
     const int d = a.dk > a.dv ? a.dk : a.dv;
     if (d <= 64) PLZ_LAUNCH_CHAIN((attn_decode_partial_kernel<T, 8, true>), grid, block, 0, stream, p);
-    else if (d <= 128) PLZ_LAUNCH_CHAIN((attn_decode_partial_kernel<T, 16, true>), grid, block, 0, stream, p);
+    else if (d <= 128 && sizeof(T) == 2) PLZ_LAUNCH_CHAIN(attn_decode_mma_kernel<true>, grid, block, 0, stream, p);
+    else if (d <= 128) PLZ_LAUNCH_CHAIN((attn_decode_partial_kernel<float, 16, true>), grid, block, 0, stream, p);
     else PLZ_LAUNCH_CHAIN((attn_decode_partial_kernel<T, 32, true>), grid, block, 0, stream, p);
     if (p.splits > 1) {
         PLZ_LAUNCH_CHAIN(attn_decode_combine_kernel<T>, dim3(a.H, a.B), dim3(128), 0, stream, (const float*)p.ws_o, (const float*)p.ws_ml, p.splits, a.H,
