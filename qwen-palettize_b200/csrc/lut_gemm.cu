@@ -678,6 +678,16 @@ int launch_lut_gemm(const LutGemmArgs& a, cudaStream_t stream) {
         const int rc = launch_narrow_gemm(n, stream);
         if (rc != PLZ_ERR_UNSUPPORTED) return rc;
     }
+    // Outputs of at most 64 columns (the LoRA products x A^T and dY B): bound by streaming A, and 128 rows a CTA leave a launch of a few thousand
+    // rows with a few CTAs that stream one tile each. The narrow kernel turned round shares a tile among a cluster.
+    if (!decode && a.J <= 64 && a.r2 == 0 && a.fuse == 0 && a.sm_limit <= 0 && g_cta_limit <= 0) {
+        NarrowArgs n = {};
+        n.transposed = 1; n.x_mn = a.bmode == B_TMA_MN;
+        n.M = a.J; n.K = a.R; n.x = a.Bdense; n.ldx = a.ldb; n.count = 1;
+        n.mat[0].N = a.M; n.mat[0].w = a.A; n.mat[0].ldw = a.lda; n.mat[0].y = a.out; n.mat[0].ldy = a.ld_out; n.alpha = a.alpha;
+        const int rc = launch_narrow_gemm(n, stream);
+        if (rc != PLZ_ERR_UNSUPPORTED) return rc;
+    }
     if (decode) {
         // the large products run on CTA pairs (lut_gemm_pair.cu); everything else, and shapes it declines, stays here
         const int rc = launch_lut_gemm_pair(a, stream);

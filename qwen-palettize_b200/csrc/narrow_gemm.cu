@@ -10,6 +10,9 @@
 //             thread is one weight row, fetches the 16 bytes of a block of 64 columns several blocks ahead and writes the decoded row to
 //             TMEM, from where it is the A operand (lane = row: no shared memory, no swizzle, no proxy fence in between). x by TMA.
 //             Shared memory and TMEM are kept to half of an SM's, so that two CTAs share one and hide each other's start and end.
+//   turned    (transposed) W is an activation matrix of any number of rows and x the few rows of a LoRA factor, t = s x A^T and dt = s dY B: the
+//             same launch with y stored [row of W][row of x], x from [M, K] or (x_mn) from [K, M].
+//             Rank 32, 1000 rows: K = 9728 33 -> 13 us, 2560 rows of B 12 -> 8 us; rank 16, 4096 rows: 9728 33 / 35 -> 24 us.
 //   extra     an optional block of up to 64 more reduction elements (the LoRA up-projection: t [M, r] against B [N, r]).
 //
 // Accumulating into the tile the previous MMA still writes costs a TMEM round trip, so the four MMAs of a block go to several accumulators,
@@ -36,6 +39,8 @@ struct NarrowMat {
 };
 struct NarrowParams {
     int M, npad, n_acc, stages;
+    int x_mn, transposed;
+    uint32_t x_bytes;              // of a tile of x
     uint32_t tmem_cols;
     int group_blocks, group_shift; // blocks of 64 columns per palette group, its logarithm or -1
     int nkb, n_blocks;             // blocks of 64 columns of W; the same plus the extra block
@@ -73,7 +78,7 @@ narrow_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
     const uint32_t base = (raw + 1023u) & ~1023u;
     uint8_t* smem = smem_raw + (base - raw);
     // dense: a stage is a W tile and an x tile; LUT: x tiles, behind them one W tile for the extra block (W is decoded to TMEM)
-    const uint32_t x_bytes = (uint32_t)p.npad * 128u, stage_bytes = (LUT ? 0u : kNgWBytes) + x_bytes;
+    const uint32_t x_bytes = p.x_bytes, stage_bytes = (LUT ? 0u : kNgWBytes) + x_bytes;
     const uint32_t w2_off = LUT ? (uint32_t)p.stages * x_bytes : 0u;
     const uint32_t bar_off = kNgRingBytes<LUT>;
     auto full = [&](int s) { return base + bar_off + 8u * s; };
@@ -104,7 +109,8 @@ narrow_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
     auto load_x = [&](int it, int s) {
         const int b = b_begin + it;
         const bool extra = b >= p.nkb;
-        tma_load_2d(base + s * stage_bytes + (LUT ? 0u : kNgWBytes), extra ? &tmX2 : &tmX, full(s), extra ? 0 : b * 64, 0);
+        const bool mn = !LUT && p.x_mn;
+        tma_load_2d(base + s * stage_bytes + (LUT ? 0u : kNgWBytes), extra ? &tmX2 : &tmX, full(s), extra || mn ? 0 : b * 64, mn ? b * 64 : 0);
     };
     const int pre = nb < p.stages ? nb : p.stages;
 
@@ -175,7 +181,8 @@ narrow_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
         }
     } else if (warp == 1) {
         if (lane == 0) {
-            const uint32_t idesc = make_idesc(128, p.npad, 0, 0);
+            const bool mn = !LUT && p.x_mn;
+            const uint32_t idesc = make_idesc(128, p.npad, 0, mn ? 1 : 0), x_step = mn ? 2048u >> 4 : 2u;   // 16 reduction elements of x
             bool ok = true;
             for (int it = 0; it < nb && ok; ++it) {
                 const int s = it % p.stages;
@@ -189,7 +196,7 @@ narrow_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
                 for (int ks = 0; ks < 4; ++ks) {
                     const uint32_t d = tmem_base + (uint32_t)((ks & (p.n_acc - 1)) * p.npad), more = (it > 0 || ks >= p.n_acc) ? 1u : 0u;
                     if (from_tmem) umma_ts(d, tmem_w + s * 32u + ks * 8u, (uint32_t)bd + ks * 2u, (uint32_t)(bd >> 32), idesc, more);
-                    else umma_bf16_words<1>(d, (uint32_t)ad + ks * 2u, (uint32_t)(ad >> 32), (uint32_t)bd + ks * 2u, (uint32_t)(bd >> 32), idesc, more);
+                    else umma_bf16_words<1>(d, (uint32_t)ad + ks * 2u, (uint32_t)(ad >> 32), (uint32_t)bd + ks * x_step, (uint32_t)(bd >> 32), idesc, more);
                 }
                 umma_commit(empty(s));
             }
@@ -224,7 +231,8 @@ narrow_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
                 }
             }
         }
-        // ---------------------------------------------------------- this CTA's partial tile: [token][weight row] in the ring's space
+        // ---------------------------------------------------------- this CTA's partial tile in the ring's space: [token][weight row], transposed
+        // [weight row][npad tokens]
         if (warp < 6) {
             if (ok) ok = mbar_wait(acc_full, 0, abort_flag, p.status, ST_TIMEOUT_ACCUM, 4);
             if (ok) {
@@ -238,6 +246,12 @@ narrow_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
                         tmem_ld_32x16(tmem_base + ((uint32_t)(lg * 32) << 16) + a * p.npad + c0, v);
 #pragma unroll
                         for (int c = 0; c < 16; ++c) sum[c] = a == 0 ? __uint_as_float(v[c]) : sum[c] + __uint_as_float(v[c]);
+                    }
+                    if (!LUT && p.transposed) {
+                        float4* to = reinterpret_cast<float4*>(smem) + ((lg * 32 + lane) * p.npad + c0) / 4;
+#pragma unroll
+                        for (int c = 0; c < 16; c += 4) to[c / 4] = make_float4(sum[c], sum[c + 1], sum[c + 2], sum[c + 3]);
+                        continue;
                     }
 #pragma unroll
                     for (int c = 0; c < 16; ++c)
@@ -254,10 +268,11 @@ narrow_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
         uint32_t from[8];
 #pragma unroll
         for (int i = 0; i < 8; ++i) from[i] = map_rank(base, i < n_ranks ? i : 0);
-        const int units = p.M * 32;       // (token, 4 weight rows)
+        const bool turned = !LUT && p.transposed;
+        const int quads = p.npad / 4, units = turned ? 128 * quads : p.M * 32;       // (token, 4 weight rows); turned: (weight row, 4 tokens)
         const int u1 = (int)((long long)(rank + 1) * units / n_ranks);
         for (int u = (int)((long long)rank * units / n_ranks) + threadIdx.x; u < u1; u += kNgThreads<LUT>) {
-            const int m = u >> 5, r = (u & 31) * 4, n = n0 + r;
+            const int m = turned ? u % quads * 4 : u >> 5, r = turned ? u / quads : (u & 31) * 4, n = n0 + r;
             float v[4] = {0.f, 0.f, 0.f, 0.f};
             float4 f[8];
 #pragma unroll
@@ -267,6 +282,18 @@ narrow_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
             for (int i = 0; i < 8; ++i)
                 if (i < n_ranks) { v[0] += f[i].x; v[1] += f[i].y; v[2] += f[i].z; v[3] += f[i].w; }
             if (n >= mat.N) continue;
+            if (turned) {
+                __nv_bfloat16* y = (__nv_bfloat16*)mat.y + (long long)n * mat.ldy + m;
+#pragma unroll
+                for (int e = 0; e < 4; ++e) v[e] *= p.alpha;
+                if (m + 3 < p.M && !((uintptr_t)y & 7)) *reinterpret_cast<uint2*>(y) = make_uint2(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]));
+                else {
+#pragma unroll
+                    for (int e = 0; e < 4; ++e)
+                        if (m + e < p.M) y[e] = __float2bfloat16_rn(v[e]);
+                }
+                continue;
+            }
             if (p.act == ACT_GLU_GELU) {      // N is even
                 const long long o = (long long)m * mat.ldy + (n >> 1);
                 const float a = gelu_tanh_f(v[0]) * v[1], b = gelu_tanh_f(v[2]) * v[3];
@@ -340,7 +367,7 @@ int launch_ng(const NarrowParams& p, int tiles, int ranks, const CUtensorMap (&t
     attr[0].val.clusterDim.x = (unsigned)ranks; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[1].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr; cfg.numAttrs = g_smallm_overlap ? 2 : 1;
+    cfg.attrs = attr; cfg.numAttrs = g_smallm_overlap && !p.transposed ? 2 : 1;   // transposed: W is what the previous kernel wrote
     PLZ_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kern, tm[0], tm[1], tm[2], tm[3], p));
     ++g_launch_count;
     return PLZ_OK;
@@ -352,12 +379,15 @@ int launch_ng(const NarrowParams& p, int tiles, int ranks, const CUtensorMap (&t
 int launch_narrow_gemm(const NarrowArgs& a, cudaStream_t stream) {
     const bool lut = a.mat[0].packed != nullptr;
     if (a.M < 1 || a.M > 128 || a.count < 1 || a.count > kNgMaxMats || (!lut && a.count != 1) || a.K < 8 || a.K % (lut ? 64 : 8)) return PLZ_ERR_UNSUPPORTED;
+    if ((a.transposed || a.x_mn) && (lut || a.count != 1 || a.r2 || a.bias || a.act || a.y_f32 || !a.transposed || (a.x_mn && a.M > 64))) return PLZ_ERR_UNSUPPORTED;
     if (a.r2 < 0 || a.r2 > 64 || a.r2 % 8 || (a.r2 && a.count != 1)) return PLZ_ERR_UNSUPPORTED;
     if (((uintptr_t)a.x & 15) || a.ldx % 8) return PLZ_ERR_UNSUPPORTED;
     if (lut && (a.gs_n <= 0 || a.gs_k <= 0 || a.gs_k % 64 || a.K % a.gs_k)) return PLZ_ERR_UNSUPPORTED;
     if (!lut && (((uintptr_t)a.mat[0].w & 15) || a.mat[0].ldw % 8)) return PLZ_ERR_UNSUPPORTED;
     NarrowParams p = {};
     p.M = a.M; p.npad = a.M <= 16 ? 16 : a.M <= 32 ? 32 : a.M <= 64 ? 64 : 128;
+    p.x_mn = a.x_mn; p.transposed = a.transposed;
+    p.x_bytes = a.x_mn ? 64u * 128u : (uint32_t)p.npad * 128u;       // x_mn: 64 reduction rows of 64 columns
     if (lut) {      // 256 TMEM columns: accumulators, then 32 columns per stage
         p.n_acc = p.npad <= 32 ? 4 : p.npad == 64 ? 2 : 1;
         p.stages = (256 - p.n_acc * p.npad) / 32;
@@ -366,7 +396,7 @@ int launch_narrow_gemm(const NarrowArgs& a, cudaStream_t stream) {
         for (int i = 0; i < 16; ++i) if (p.group_blocks == 1 << i) p.group_shift = i;
     } else {
         p.n_acc = p.npad <= 64 ? 4 : 2;
-        p.stages = (int)(kNgRingBytes<false> / (kNgWBytes + (uint32_t)p.npad * 128u));
+        p.stages = (int)(kNgRingBytes<false> / (kNgWBytes + p.x_bytes));
         p.tmem_cols = (uint32_t)(p.n_acc * p.npad);     // 64, 128 or 256
     }
     if (p.stages > kNgMaxStages) p.stages = kNgMaxStages;
@@ -383,7 +413,7 @@ int launch_narrow_gemm(const NarrowArgs& a, cudaStream_t stream) {
         tiles += (s.N + 127) / 128;
     }
     CUtensorMap tm[4];
-    if ((rc = make_tmap_bf16(&tm[0], a.x, a.M, a.K, a.ldx, 64, (uint32_t)p.npad))) return rc;
+    if ((rc = a.x_mn ? make_tmap_bf16(&tm[0], a.x, a.K, a.M, a.ldx, 64, 64) : make_tmap_bf16(&tm[0], a.x, a.M, a.K, a.ldx, 64, (uint32_t)p.npad))) return rc;
     tm[1] = tm[2] = tm[3] = tm[0];
     if (!lut && (rc = make_tmap_bf16(&tm[1], a.mat[0].w, a.mat[0].N, a.K, a.mat[0].ldw, 64, 128))) return rc;
     if (a.r2) {

@@ -43,7 +43,8 @@ extern int g_cta_limit;
 // ---- narrow_gemm.cu: M <= 128, operands swapped, reduction split over a cluster --------------------
 struct NarrowArgs {
     int M, K;
-    const void* x; long long ldx;
+    const void* x; long long ldx;     // bf16 [M, K], or [K, M] with x_mn
+    int x_mn, transposed;             // transposed: y [N, M]; W may be any previous kernel's output, any N
     int count;                        // matrices sharing x (dense: 1)
     struct Mat {
         int N;

@@ -73,3 +73,16 @@ def test_packed(M, N, K, gs_n, gs_k, rank):
             check(ops.hard_forward_smallm(w, x), ref, mag, K)
     check(y, ref, mag, K + rank)
     assert torch.equal(y, ops.hard_forward(w, x, (a, b, 0.5) if rank else None)[0])
+
+
+# x A^T and dY B of a LoRA branch: rows around a 128-row tile, ranks around the MMA widths, reductions of one block, of a few, and split over a cluster
+@pytest.mark.parametrize("M,K,rank", [(1, 64, 8), (127, 128, 16), (129, 192, 24), (1000, 9728, 32), (300, 2560, 64), (4097, 1024, 40), (20000, 256, 16)])
+def test_lora_factors(M, K, rank):
+    g = torch.Generator(device="cuda").manual_seed(M + K)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda").bfloat16()
+    x, a, b = rnd(M, K + 8)[:, :K], rnd(rank, K), rnd(K, rank)
+    ref, mag = 0.5 * x.double() @ b.double(), 0.5 * x.double().abs() @ b.double().abs()
+    check(ops.lora_dt((a, b, 0.5), x), ref, mag, K)
+    w = ops.PackedWeight(ops.pack_indices(torch.zeros(64, K, dtype=torch.int8, device="cuda"), n_major=True), torch.zeros(64, 4, device="cuda", dtype=torch.bfloat16), 64, K, 1, K)
+    t = ops.hard_forward(w, x, (a, rnd(64, rank), 0.5))[1]
+    check(t, 0.5 * x.double() @ a.double().T, 0.5 * x.double().abs() @ a.double().abs().T, K)
