@@ -367,6 +367,29 @@ int32_t plz_attn_decode(const void* q, int64_t ldq, const void* k_cache, const v
 int32_t plz_embed_gather(const void* table, int64_t ldt, const int64_t* ids, int64_t n, int32_t width, int64_t vocab, void* out, int64_t ldo,
                          int32_t* bad, void* stream);
 
+/* One token per sequence through all decoder layers of a hard-palettized model (embedding rows -> layers -> final norm) as one call: the
+ * chain of the entry points of this header that a caller would make itself, without its cost per call. Linears take 1..64 rows
+ * (B <= 64). The new key and value go to position T - 1 of the caches, attention reads positions [0, T).
+ * ws: plz_decode_ws_bytes of scratch, 16-byte aligned; h / h1: the residual stream after the last layer and its final norm, bf16
+ * [B, hidden] contiguous. All members are 8 bytes so that a caller can fill a layer as a row of integers. */
+typedef struct plz_decode_linear { int64_t N, K, gs_n, gs_k; const void* packed; int64_t packed_pitch; const void* palette; } plz_decode_linear_t;
+typedef struct plz_decode_layer {
+    plz_decode_linear_t q, k, v, o, gate, up, down;
+    const void *input_ln, *post_ln, *q_norm, *k_norm;   /* bf16 [hidden], [hidden], [128], [128] */
+    void *k_cache, *v_cache;                            /* bf16, position 0 of sequence 0 */
+} plz_decode_layer_t;
+typedef struct plz_decode {
+    int64_t B, T, n_layers, hidden, intermediate, n_heads, n_kv_heads, head_dim;
+    int64_t batch_stride, tok_stride;                   /* of both caches, elements */
+    const void* embed; int64_t ld_embed, vocab; const int64_t* ids;
+    const float *cos_row, *sin_row;                     /* [64] of position T - 1 */
+    const void* final_norm;
+    void *h, *h1, *ws; int64_t ws_bytes;
+    double eps;
+} plz_decode_t;
+int64_t plz_decode_ws_bytes(int32_t B, int32_t T, int32_t hidden, int32_t intermediate, int32_t n_heads, int32_t n_kv_heads);
+int32_t plz_decode_hidden(const plz_decode_t* a, const plz_decode_layer_t* layers, void* stream);
+
 /* ---- element-wise ops of a decoder layer -------------------------------------------------------
  * The reference has no code for these (it calls the HuggingFace decoder layer, scripts/train_qwen.py:1259-1266);
  * semantics follow transformers' Qwen3RMSNorm / Qwen3Attention (q_norm, k_norm, apply_rotary_pos_emb) / Qwen3MLP.

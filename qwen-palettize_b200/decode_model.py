@@ -194,33 +194,15 @@ class PalettizedQwen:
         return h, last
 
     # ---- decode --------------------------------------------------------------------------------------------------
-    def _small(self, ws, x, outs=None):
-        if x.shape[0] <= 16:
-            return ops.hard_forward_smallm_multi(ws, x, outs)
-        return [ops.hard_forward_smallm(w, x, out=(outs[i] if outs is not None else None)) for i, w in enumerate(ws)]
-
     def decode_hidden(self, ids: torch.Tensor, cache: KVCache, pos: int | None = None):
         """One token per sequence (ids int64 [B]) at position pos (default: cache.length): writes its key / value into the cache
         and returns (final hidden state, its final RMSNorm), bf16 [B, hidden] each. Does not advance cache.length."""
         c = self.cfg
-        B = ids.shape[0]
         pos = cache.length if pos is None else pos
         assert pos < cache.k.shape[2] and pos < self.cos.shape[0]
         cos, sin = self.cos[pos:pos + 1], self.sin[pos:pos + 1]
-        h = ops.embed_gather(self.embed, ids)
-        h1, _ = ops.rmsnorm_forward(h, self.layers[0]["input_ln"], c.eps)
-        n = len(self.layers)
-        for li, L in enumerate(self.layers):
-            q_raw, k_raw, _ = self._small([L["q"], L["k"], L["v"]], h1, [None, None, cache.v[li, :, pos]])
-            q, _ = ops.qknorm_rope_forward2(q_raw, L["q_norm"], c.n_heads, k_raw, L["k_norm"], c.n_kv_heads, cos, sin, 1, c.eps,
-                                            out_k=cache.k[li, :, pos])
-            a = ops.attention_decode(q, cache.k[li], cache.v[li], pos + 1, c.n_heads, c.n_kv_heads, c.head_dim)
-            x2, h2 = ops.add_rmsnorm_forward(h, self._small([L["o"]], a)[0], L["post_ln"], c.eps)
-            gate, up = self._small([L["gate"], L["up"]], h2)
-            d = self._small([L["down"]], ops.swiglu_forward(gate, up))[0]
-            # the residual add closes the layer and the same pass applies the next layer's (or the final) norm
-            h, h1 = ops.add_rmsnorm_forward(x2, d, self.layers[li + 1]["input_ln"] if li + 1 < n else self.final_norm, c.eps)
-        return h, h1
+        return ops.decode_hidden(ids, self.embed, self.layers, ("q", "k", "v", "o", "gate", "up", "down"), ("input_ln", "post_ln", "q_norm", "k_norm"),
+                                 cache.k, cache.v, pos + 1, self.final_norm, cos, sin, c.n_heads, c.n_kv_heads, c.intermediate, c.eps)
 
     def decode_step(self, ids: torch.Tensor, cache: KVCache) -> torch.Tensor:
         """Logits bf16 [B, vocab] of the next token after ids (int64 [B]); advances the cache by one position."""

@@ -94,6 +94,12 @@ class LatentPrep(C.Structure):
                 ("q_rank", C.c_int32), ("R", C.c_int32), ("dr", C.c_int32), ("cap", C.c_int32), ("eps", C.c_float)]
 
 
+class Decode(C.Structure):
+    _fields_ = [(n, C.c_int64) for n in ("B", "T", "n_layers", "hidden", "intermediate", "n_heads", "n_kv_heads", "head_dim", "batch_stride", "tok_stride")] + [
+        ("embed", C.c_void_p), ("ld_embed", C.c_int64), ("vocab", C.c_int64), ("ids", C.c_void_p), ("cos_row", C.c_void_p), ("sin_row", C.c_void_p),
+        ("final_norm", C.c_void_p), ("h", C.c_void_p), ("h1", C.c_void_p), ("ws", C.c_void_p), ("ws_bytes", C.c_int64), ("eps", C.c_double)]
+
+
 class Rotate(C.Structure):
     _fields_ = [("x", C.c_void_p), ("ldx", C.c_int64), ("xh", C.c_int64), ("out", C.c_void_p), ("ldo", C.c_int64), ("oh", C.c_int64), ("pos", C.c_void_p),
                 ("freq", C.c_void_p), ("pairs", C.c_int32), ("m", C.c_float), ("B", C.c_int32), ("n", C.c_int32), ("H", C.c_int32), ("dr", C.c_int32)]
@@ -159,6 +165,8 @@ SIGNATURES = {
     "plz_attn_bwd": [_P, _I64, _P, _I64, _P, _I64, _P, _P, _I64, _P, _I32, _I32, _I32, _I32, _I32, _F, _P, _P, _P, _P, _P],
     "plz_attn_decode_ws_bytes": [_I32, _I32, _I32, _I32],
     "plz_attn_decode": [_P, _I64, _P, _P, _I64, _I64, _I32, _I32, _I32, _I32, _I32, _F, _P, _I64, _P, _I64, _P],
+    "plz_decode_ws_bytes": [_I32, _I32, _I32, _I32, _I32, _I32],
+    "plz_decode_hidden": [C.POINTER(Decode), _P, _P],
     "plz_embed_gather": [_P, _I64, _P, _I64, _I32, _I64, _P, _I64, _P, _P],
     "plz_rmsnorm_fwd": [_P, _I64, _P, _I32, _I32, _F, _P, _I64, _P, _P],
     "plz_add_rmsnorm_fwd": [_P, _I64, _P, _I64, _P, _I64, _P, _I32, _I32, _F, _P, _I64, _P, _P],
@@ -189,7 +197,7 @@ SIGNATURES = {
     "plz_sample": [_P, _I64, _I32, _I32, _F, _I32, C.c_uint32, _P, _P, _P],
     "plz_distill_loss": [_P, _I64, _P, _I64, _I32, _I32, _F, _F, _F, _P, _P, _P, _I64, _I32, _P],
 }
-_RESTYPES = {"plz_last_error": C.c_char_p, "plz_launch_count": C.c_uint64, "plz_attn_decode_ws_bytes": C.c_int64,
+_RESTYPES = {"plz_last_error": C.c_char_p, "plz_launch_count": C.c_uint64, "plz_attn_decode_ws_bytes": C.c_int64, "plz_decode_ws_bytes": C.c_int64,
              "plz_attn_bias_ws_bytes": C.c_int64, "plz_chunk_ws_bytes": C.c_int64, "plz_latent_attn_ws_bytes": C.c_int64}
 
 

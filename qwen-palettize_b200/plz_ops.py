@@ -546,6 +546,39 @@ def attention_decode(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tens
     return out
 
 
+def decode_hidden(ids: torch.Tensor, embed: torch.Tensor, layers, names, norms, k_cache: torch.Tensor, v_cache: torch.Tensor, T: int, final_norm: torch.Tensor,
+                  cos: torch.Tensor, sin: torch.Tensor, n_heads: int, n_kv_heads: int, intermediate: int, eps: float):
+    """One token per sequence through all layers of a hard-palettized model, one native call. ids int64 [B]; layers: dicts with the PackedWeight of
+    `names` (q, k, v, o, gate, up, down) and the vectors of `norms` (input, post-attention, q, k); caches bf16 [n_layers, B, T_max, n_kv_heads * 128],
+    position T - 1 is written; cos / sin: the table rows of that position. Returns (residual stream, its final norm), bf16 [B, hidden]."""
+    assert embed.dtype == torch.bfloat16 and embed.dim() == 2 and embed.stride(1) == 1 and ids.dtype == torch.int64
+    ids = ids.reshape(-1).contiguous()
+    B, hidden, dev = ids.numel(), embed.shape[1], embed.device
+    P._need_cuda(ids, embed, final_norm, cos, sin, k_cache, v_cache)
+    assert k_cache.dtype == v_cache.dtype == torch.bfloat16 and k_cache.shape == v_cache.shape and k_cache.stride() == v_cache.stride()
+    n, st = len(layers), k_cache.stride()
+    assert k_cache.dim() == 4 and k_cache.shape[0] >= n and k_cache.shape[1] == B and k_cache.shape[3] == n_kv_heads * 128 and st[3] == 1 and 0 < T <= k_cache.shape[2]
+    rows, k0, v0 = [], k_cache.data_ptr(), v_cache.data_ptr()
+    for i, L in enumerate(layers):
+        for name in names:
+            w = L[name]
+            packed, palette = w.packed, w.palette
+            P._need_cuda(packed, palette)
+            assert packed.dtype == torch.uint8 and packed.dim() == 2 and packed.stride(1) == 1
+            assert palette.dtype == torch.bfloat16 and palette.is_contiguous() and palette.numel() == (w.N // w.gs_n) * (w.K // w.gs_k) * 4, "palette size does not match the grouping"
+            rows += (w.N, w.K, w.gs_n, w.gs_k, packed.data_ptr(), packed.stride(0), palette.data_ptr())
+        rows += [L[name].data_ptr() if L[name] is not None else 0 for name in norms]
+        rows += (k0 + 2 * i * st[0], v0 + 2 * i * st[0])
+    lib = P.lib()
+    out = torch.empty(2, B, hidden, dtype=torch.bfloat16, device=dev)
+    nbytes = int(lib.plz_decode_ws_bytes(B, T, hidden, intermediate, n_heads, n_kv_heads))
+    ws = torch.empty(nbytes, dtype=torch.uint8, device=dev)
+    a = P.Decode(B, T, n, hidden, intermediate, n_heads, n_kv_heads, 128, st[1], st[2], embed.data_ptr(), embed.stride(0), embed.shape[0], ids.data_ptr(),
+                 cos.data_ptr(), sin.data_ptr(), final_norm.data_ptr() if final_norm is not None else None, out[0].data_ptr(), out[1].data_ptr(), ws.data_ptr(), nbytes, eps)
+    P.check(lib.plz_decode_hidden(C.byref(a), (C.c_int64 * len(rows))(*rows), P.stream_ptr()), "plz_decode_hidden")
+    return out[0], out[1]
+
+
 def embed_gather(table: torch.Tensor, ids: torch.Tensor) -> torch.Tensor:
     """table[ids] for a bf16 [vocab, width] table and int64 ids (any shape); returns bf16 [ids.numel(), width]."""
     assert table.dtype == torch.bfloat16 and table.dim() == 2 and table.stride(1) == 1 and ids.dtype == torch.int64
