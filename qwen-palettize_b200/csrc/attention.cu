@@ -302,20 +302,35 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 __global__ void __launch_bounds__(256)
 attn_dsum_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ d_o, long long ld, int B, int S, int Hq,
                  float* __restrict__ dsum) {
-    const int lane = threadIdx.x & 31;
-    const long long row = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);   // over B * S * Hq
-    if (row >= (long long)B * S * Hq) return;
-    const int h = (int)(row % Hq);
-    const long long tok = row / Hq;
-    const uint2 a = *reinterpret_cast<const uint2*>(o + tok * ld + h * kD + lane * 4);
-    const uint2 g = *reinterpret_cast<const uint2*>(d_o + tok * ld + h * kD + lane * 4);
-    float s = __uint_as_float(a.x << 16) * __uint_as_float(g.x << 16) + __uint_as_float(a.x & 0xFFFF0000u) * __uint_as_float(g.x & 0xFFFF0000u) +
-              __uint_as_float(a.y << 16) * __uint_as_float(g.y << 16) + __uint_as_float(a.y & 0xFFFF0000u) * __uint_as_float(g.y & 0xFFFF0000u);
+    // sixteen lanes per (token, head) row, eight rows of a warp at once: four 16-byte loads of each operand in flight per lane (4096 tokens x 32
+    // heads 23 -> 18 us against one row per warp)
+    const int lane = threadIdx.x & 31, l = lane & 15;
+    const long long rows = (long long)B * S * Hq, row0 = ((long long)blockIdx.x * 8 + (threadIdx.x >> 5)) * 8 + (lane >> 4);
+    uint4 a[4], g[4];
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xFFFFFFFFu, s, off);
-    if (lane == 0) {
-        const int b = (int)(tok / S), sidx = (int)(tok % S);
-        dsum[((long long)b * Hq + h) * S + sidx] = s;
+    for (int i = 0; i < 4; ++i) {
+        const long long row = row0 + 2 * i;
+        a[i] = g[i] = make_uint4(0u, 0u, 0u, 0u);
+        if (row < rows) {
+            const long long at = row / Hq * ld + row % Hq * kD + l * 8;
+            a[i] = __ldcs(reinterpret_cast<const uint4*>(o + at));
+            g[i] = *reinterpret_cast<const uint4*>(d_o + at);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const uint32_t aw[4] = {a[i].x, a[i].y, a[i].z, a[i].w}, gw[4] = {g[i].x, g[i].y, g[i].z, g[i].w};
+        float s = 0.f;
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+            s += __uint_as_float(aw[e] << 16) * __uint_as_float(gw[e] << 16) + __uint_as_float(aw[e] & 0xFFFF0000u) * __uint_as_float(gw[e] & 0xFFFF0000u);
+#pragma unroll
+        for (int off = 8; off > 0; off >>= 1) s += __shfl_xor_sync(0xFFFFFFFFu, s, off);
+        const long long row = row0 + 2 * i;
+        if (l == 0 && row < rows) {
+            const long long tok = row / Hq;
+            dsum[(tok / S * Hq + row % Hq) * S + tok % S] = s;
+        }
     }
 }
 
@@ -653,7 +668,7 @@ int launch_attn_bwd(const AttnArgs& a, cudaStream_t stream) {
         once = true;
     }
     const long long n_rows = (long long)a.B * a.S * a.Hq;
-    attn_dsum_kernel<<<(unsigned)((n_rows + 7) / 8), 256, 0, stream>>>((const __nv_bfloat16*)a.o, (const __nv_bfloat16*)a.d_o, a.ldo, a.B, a.S,
+    attn_dsum_kernel<<<(unsigned)((n_rows + 63) / 64), 256, 0, stream>>>((const __nv_bfloat16*)a.o, (const __nv_bfloat16*)a.d_o, a.ldo, a.B, a.S,
                                                                        a.Hq, a.dsum);
     PLZ_LAUNCH_CHECK();
     attn_bwd_dq_kernel<<<dim3(a.S / kT, a.Hq, a.B), kBwdThreads, kDqSmem, stream>>>(tmQ, tmK, tmV, tmdO, tmdQ, p);

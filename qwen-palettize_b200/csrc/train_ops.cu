@@ -330,10 +330,91 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, const __n
     }
 }
 
+// The same with 16-byte accesses, a thread per eight columns and two rows at a time (K % 8 == 0, K <= 8192, rows aligned to 16 bytes): one barrier
+// per two rows instead of two per row, and dg added up by vector reductions of few blocks. 4096 x 2560 31 -> 24 us.
+constexpr int kNorm8MaxK = 8192;
+__global__ void __launch_bounds__(1024)
+rmsnorm_bwd8_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, const __nv_bfloat16* __restrict__ dh, long long lddh, const float* __restrict__ rstd,
+                    const __nv_bfloat16* __restrict__ g, int M, int K, __nv_bfloat16* __restrict__ dx, long long lddx, float* __restrict__ dg) {
+    __shared__ float2 red[2][32];
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, n_warps = blockDim.x >> 5, c = threadIdx.x * 8;
+    const bool in = c < K;
+    auto unpack = [](const uint4& v, float (&f)[8]) {
+        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) { f[2 * i] = __uint_as_float(w[i] << 16); f[2 * i + 1] = __uint_as_float(w[i] & 0xFFFF0000u); }
+    };
+    const uint4 gv = in ? (g ? *reinterpret_cast<const uint4*>(g + c) : make_uint4(0x3F803F80u, 0x3F803F80u, 0x3F803F80u, 0x3F803F80u)) : make_uint4(0u, 0u, 0u, 0u);
+    float acc[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) acc[e] = 0.f;
+    int buf = 0;
+    for (long long row = 2 * (long long)blockIdx.x; row < M; row += 2 * (long long)gridDim.x, buf ^= 1) {
+        uint4 xr[2], dr[2];
+        float rs[2], s[2];
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            xr[r] = dr[r] = make_uint4(0u, 0u, 0u, 0u);
+            rs[r] = 0.f;
+            if (row + r < M) {
+                rs[r] = rstd[row + r];
+                if (in) {
+                    xr[r] = __ldcs(reinterpret_cast<const uint4*>(x + (row + r) * ldx + c));
+                    dr[r] = __ldcs(reinterpret_cast<const uint4*>(dh + (row + r) * lddh + c));
+                }
+            }
+        }
+        float gf[8];
+        unpack(gv, gf);
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            float xf[8], df[8];
+            unpack(xr[r], xf);
+            unpack(dr[r], df);
+            s[r] = 0.f;
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                s[r] += xf[e] * gf[e] * df[e];
+                acc[e] += df[e] * xf[e] * rs[r];
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) s[r] += __shfl_xor_sync(0xFFFFFFFFu, s[r], o);
+        }
+        if (lane == 0) red[buf][wib] = make_float2(s[0], s[1]);
+        __syncthreads();      // whoever writes the other buffer next has everybody's reads of it behind this barrier
+        float2 tot = make_float2(0.f, 0.f);
+        for (int w = 0; w < n_warps; ++w) { const float2 v = red[buf][w]; tot.x += v.x; tot.y += v.y; }
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            if (row + r >= M || !in) continue;
+            const float coef = (r ? tot.y : tot.x) * rs[r] * rs[r] * rs[r] / (float)K;
+            float xf[8], df[8], o[8];
+            unpack(xr[r], xf);
+            unpack(dr[r], df);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) o[e] = rs[r] * gf[e] * df[e] - xf[e] * coef;
+            *reinterpret_cast<uint4*>(dx + (row + r) * lddx + c) =
+                make_uint4(pack_bf16x2(o[0], o[1]), pack_bf16x2(o[2], o[3]), pack_bf16x2(o[4], o[5]), pack_bf16x2(o[6], o[7]));
+        }
+    }
+    if (dg && in) {
+        atomicAdd(reinterpret_cast<float4*>(dg + c), make_float4(acc[0], acc[1], acc[2], acc[3]));
+        atomicAdd(reinterpret_cast<float4*>(dg + c + 4), make_float4(acc[4], acc[5], acc[6], acc[7]));
+    }
+}
+
 int launch_rmsnorm_bwd(const void* x, long long ldx, const void* dh, long long lddh, const float* rstd, const void* g, int M, int K,
                        void* dx, long long lddx, float* dg, cudaStream_t stream) {
     if (M <= 0) return PLZ_OK;
     if (K > 512 * kNormPairsMax) { set_last_error("rmsnorm_bwd: K=%d exceeds %d", K, 512 * kNormPairsMax); return PLZ_ERR_TOO_LARGE; }
+    if (K % 8 == 0 && K <= kNorm8MaxK && !(((uintptr_t)x | (uintptr_t)dh | (uintptr_t)g | (uintptr_t)dx | (uintptr_t)dg) & 15) && !((ldx | lddh | lddx) & 7)) {
+        const int threads = (K / 8 + 31) / 32 * 32, per_sm = threads <= 320 ? 3 : threads <= 512 ? 2 : 1;
+        int blocks = (M + 1) / 2;
+        if (blocks > per_sm * sm_count_of_current_device()) blocks = per_sm * sm_count_of_current_device();
+        rmsnorm_bwd8_kernel<<<blocks, threads, 0, stream>>>((const __nv_bfloat16*)x, ldx, (const __nv_bfloat16*)dh, lddh, rstd, (const __nv_bfloat16*)g, M, K, (__nv_bfloat16*)dx, lddx, dg);
+        PLZ_LAUNCH_CHECK();
+        return PLZ_OK;
+    }
     int blocks = M < sm_count_of_current_device() * 8 ? M : sm_count_of_current_device() * 8;
     const __nv_bfloat16 *xp = (const __nv_bfloat16*)x, *dp = (const __nv_bfloat16*)dh, *gp = (const __nv_bfloat16*)g;
     if (K <= 512 * 5) rmsnorm_bwd_kernel<5><<<blocks, 256, 0, stream>>>(xp, ldx, dp, lddh, rstd, gp, M, K, (__nv_bfloat16*)dx, lddx, dg);

@@ -85,6 +85,16 @@ def _mat(x: torch.Tensor, cols: int):
     return x
 
 
+def _zeros(shapes, device):
+    """Zeroed fp32 tensors of the given shapes (None: None), cleared by one launch; each starts at a multiple of 16 bytes."""
+    sizes = [0 if s is None else (s[0] * s[1] + 3) // 4 * 4 for s in shapes]
+    flat, at, out = torch.zeros(sum(sizes), dtype=torch.float32, device=device), 0, []
+    for s, n in zip(shapes, sizes):
+        out.append(None if s is None else flat[at:at + s[0] * s[1]].view(s))
+        at += n
+    return out
+
+
 def hard_forward(w: PackedWeight, x: torch.Tensor, lora=None):
     """y = x W^T (+ LoRA).  Returns (y, t) where t = scale * x A^T (None without LoRA)."""
     _mat(x, w.K)
@@ -209,18 +219,17 @@ def backward_dw_soft(w: PackedWeight, x: torch.Tensor, dy: torch.Tensor, logits:
     dlog = torch.empty_like(logits) if want_dlogits else None
     if dlog is not None:
         assert dlog.stride() == logits.stride()
-    dpal = torch.zeros(w.palette.numel() // 4, 4, dtype=torch.float32, device=x.device) if want_dpalette else None
     d = w.desc()
     if lora_ws is not None:
         t, dt = lora_ws
         r = t.shape[1]
-        da = torch.zeros(r, w.K, dtype=torch.float32, device=x.device)
-        db = torch.zeros(w.N, r, dtype=torch.float32, device=x.device)
+        dpal, da, db = _zeros([(w.palette.numel() // 4, 4) if want_dpalette else None, (r, w.K), (w.N, r)], x.device)
         P.check(P.lib().plz_bwd_dw_soft_lora(C.byref(d), x.data_ptr(), x.stride(0), dy.data_ptr(), dy.stride(0), M, C.byref(ld),
                                              C.byref(nd), float(tau), dlog.data_ptr() if dlog is not None else None,
                                              dpal.data_ptr() if dpal is not None else None, t.data_ptr(), dt.data_ptr(), r,
                                              da.data_ptr(), db.data_ptr(), P.stream_ptr()), "plz_bwd_dw_soft_lora")
         return dlog, dpal, da, db
+    dpal = torch.zeros(w.palette.numel() // 4, 4, dtype=torch.float32, device=x.device) if want_dpalette else None
     P.check(P.lib().plz_bwd_dw_soft(C.byref(d), x.data_ptr(), x.stride(0), dy.data_ptr(), dy.stride(0), M, C.byref(ld),
                                     C.byref(nd), float(tau), dlog.data_ptr() if dlog is not None else None,
                                     dpal.data_ptr() if dpal is not None else None, P.stream_ptr()), "plz_bwd_dw_soft")
@@ -687,9 +696,7 @@ def backward_dw_hard_lora(w: PackedWeight, x: torch.Tensor, dy: torch.Tensor, t:
     """(dPalette fp32 [groups, 4], dA fp32 [r, K], dB fp32 [N, r]) of a hard palettized Linear with LoRA, one launch."""
     _mat(x, w.K), _mat(dy, w.N)
     r = t.shape[1]
-    dpal = torch.zeros(w.palette.numel() // 4, 4, dtype=torch.float32, device=x.device)
-    da = torch.zeros(r, w.K, dtype=torch.float32, device=x.device)
-    db = torch.zeros(w.N, r, dtype=torch.float32, device=x.device)
+    dpal, da, db = _zeros([(w.palette.numel() // 4, 4), (r, w.K), (w.N, r)], x.device)
     d = w.desc()
     P.check(P.lib().plz_bwd_dw_hard_lora(C.byref(d), x.data_ptr(), x.stride(0), dy.data_ptr(), dy.stride(0), x.shape[0], dpal.data_ptr(),
                                          t.data_ptr(), dt.data_ptr(), r, da.data_ptr(), db.data_ptr(), P.stream_ptr()), "plz_bwd_dw_hard_lora")
