@@ -407,8 +407,8 @@ attn_decode_mma_kernel(const DecParams p) {
 // independent loads.
 template <typename T>
 __global__ void __launch_bounds__(128)
-attn_decode_combine_kernel(const float* __restrict__ ws_o, const float* __restrict__ ws_ml, int splits, int Hq, int dv, int sink,
-                           T* __restrict__ out, long long ldo) {
+attn_decode_combine_kernel(const float* ws_o, const float* ws_ml, int splits, int Hq, int dv, int sink,
+                           T* out, long long ldo) {
     __shared__ float wgt[kMaxSplits];
     __shared__ float red[8];
     const int head = blockIdx.x, b = blockIdx.y, t = threadIdx.x, lane = t & 31, wib = t >> 5;

@@ -120,7 +120,7 @@ latent_rows_kernel(const RowsParams p) {
 // once. A split without keys has weight 0 and was not written: the first one, which always has some, is read in its place.
 template <typename T, int V>
 __global__ void __launch_bounds__(128)
-latent_combine_kernel(const LatentParams p, T* __restrict__ o, long long ldo) {
+latent_combine_kernel(const LatentParams p, T* o, long long ldo) {
     __shared__ float wgt[kLatMaxSplits];
     __shared__ float red[8];
     __shared__ float sum[4][32 * V];

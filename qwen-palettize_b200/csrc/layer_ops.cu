@@ -25,9 +25,9 @@ __device__ __forceinline__ float round_bf16(float v) { return __bfloat162float(_
 // of rows: token decode, where one warp per row would leave the row's 5 KB to 32 lanes).
 template <bool BLOCK, bool ADD>
 __global__ void __launch_bounds__(256)
-rms_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, const __nv_bfloat16* __restrict__ addend, long long lda,
-           __nv_bfloat16* __restrict__ sum_out, long long lds, const __nv_bfloat16* __restrict__ g, int M, int K, float eps,
-           __nv_bfloat16* __restrict__ h, long long ldh, float* __restrict__ rstd) {
+rms_kernel(const __nv_bfloat16* x, long long ldx, const __nv_bfloat16* addend, long long lda,
+           __nv_bfloat16* sum_out, long long lds, const __nv_bfloat16* g, int M, int K, float eps,
+           __nv_bfloat16* h, long long ldh, float* rstd) {
     __shared__ float part[8];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const int t = BLOCK ? (int)threadIdx.x : lane, team = BLOCK ? 256 : 32;
@@ -288,8 +288,8 @@ qknorm_rope_bwd16_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, con
 
 // act = silu(gate) * up, bf16, eight elements per thread and step
 __global__ void __launch_bounds__(256)
-swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gate, long long ldg, const __nv_bfloat16* __restrict__ up, long long ldu, int M, int N,
-                  __nv_bfloat16* __restrict__ act, long long lda) {
+swiglu_fwd_kernel(const __nv_bfloat16* gate, long long ldg, const __nv_bfloat16* up, long long ldu, int M, int N,
+                  __nv_bfloat16* act, long long lda) {
     const int vec = N >> 3;
     const long long total = (long long)M * vec;
     pdl_launch_dependents();
@@ -313,8 +313,8 @@ swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gate, long long ldg, const _
 
 // out = a + b (+ c), bf16 rows, fp32 sum rounded once
 __global__ void __launch_bounds__(256)
-add_kernel(const __nv_bfloat16* __restrict__ a, long long lda, const __nv_bfloat16* __restrict__ b, long long ldb,
-           const __nv_bfloat16* __restrict__ c3, long long ldc, int M, int N, __nv_bfloat16* __restrict__ out, long long ldo) {
+add_kernel(const __nv_bfloat16* a, long long lda, const __nv_bfloat16* b, long long ldb,
+           const __nv_bfloat16* c3, long long ldc, int M, int N, __nv_bfloat16* out, long long ldo) {
     const int vec = N >> 3;
     const long long total = (long long)M * vec;
     pdl_launch_dependents();

@@ -46,6 +46,8 @@ struct StatusWord {
 // Programmatic dependent launch: let the next kernel of the stream start (it will wait for this one to finish before it
 // reads what this one writes), and wait for the previous kernel to have finished. Both are no-ops in a launch without the
 // programmatic-stream-serialization attribute.
+// What an earlier kernel writes must reach a kernel that waits here through plain pointers: loads through const __restrict__ parameters and __ldg count
+// as invariant, and the compiler moves them above the wait.
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
