@@ -9,6 +9,8 @@
 //     mbarrier so that its items start as soon as its 16 rows have landed.  Loading the rows into registers with
 //     ordinary 16-byte loads instead was measured to take 4400 cycles just to ISSUE (the SM's outstanding-load
 //     capacity, not HBM, was the limit), and one bulk copy per row 50 cycles of issue each;
+//     The strip's palettes come with it, where rows have their own and copies of 16 bytes can fetch them: loaded into registers after the wait on
+//     the previous kernel of the stream, they cost another trip to HBM: 9728 x 2560, one row 8.6 -> 8.2 us alone, 8.8 -> 8.2 on average in a decode chain.
 //   * while the rows are in flight all warps stage x in shared memory, in the permuted order below;
 //   * a work item is 16 rows x 256 input columns (one palette group per row); the items are dealt round-robin to the
 //     warps (32 of them up to eight rows, 16 beyond).  Weights go from shared memory straight into mma.sync.m16n8k16 A fragments (the 128-row tcgen05 tile
@@ -58,6 +60,7 @@ struct SmallmParams {
     int gs_n_shift, gs_k_shift;          // log2 of gs_n / gs_k when they are powers of two, else -1 (division)
     int rows_per_cta, rows_alloc;        // rows_alloc: packed rows reserved in shared memory (rows_per_cta up to 16)
     StatusWord* status;
+    uint32_t pal_bytes;                  // bytes of a row's palettes in shared memory, behind the packed rows; 0: loaded into registers
     uint32_t x_pitch;                    // bytes per token row of the staged x (K * 2 + 32)
     unsigned long long* prof;            // optional [gridDim][8] cycle counters of warp 0 (diagnostics)
 };
@@ -99,7 +102,8 @@ lut_smallm_mma_kernel(const SmallmParams p) {
     const int rows_pad = strips * 16;
     const uint32_t row_bytes = (uint32_t)p.K >> 2;
     uint8_t* wsm = smem + kHeader;          // rows back to back (row_bytes each), as in global memory
-    uint8_t* xs = wsm + (size_t)p.rows_alloc * row_bytes;
+    uint8_t* pal_sm = wsm + (size_t)p.rows_alloc * row_bytes;
+    uint8_t* xs = pal_sm + (size_t)p.rows_alloc * p.pal_bytes;
     float* acc_s = reinterpret_cast<float*>(xs + (size_t)p.M * p.x_pitch);
 
     const long long t_entry = PLZ_PROF_ON(p.prof) ? clock64() : 0;
@@ -114,7 +118,7 @@ lut_smallm_mma_kernel(const SmallmParams p) {
         if (PLZ_PROF_ON(p.prof) && threadIdx.x == 0) p.prof[8ull * blockIdx.x + 5] = clock64() - t_entry;
         for (int s = lane; s < strips; s += 32) {
             const int a = s * 16, b = min(rows, a + 16);
-            mbar_arrive_expect_tx(bar0 + 8u * s, (uint32_t)(b - a) * row_bytes);
+            mbar_arrive_expect_tx(bar0 + 8u * s, (uint32_t)(b - a) * (row_bytes + p.pal_bytes));
             int r = a;
             while (r < b) {
                 const int mi = mat_of(p, r0 + r), lr = r0 + r - p.row_start[mi];
@@ -123,6 +127,8 @@ lut_smallm_mma_kernel(const SmallmParams p) {
                 if (pitch == (long long)row_bytes) n = min(b - r, p.row_start[mi + 1] - (r0 + r));
                 bulk_load(smem_u32(wsm) + (uint32_t)r * row_bytes, p.packed[mi] + (long long)lr * pitch, (uint32_t)n * row_bytes,
                           bar0 + 8u * s);
+                if (p.pal_bytes)
+                    bulk_load(smem_u32(pal_sm) + (uint32_t)r * p.pal_bytes, p.palette[mi] + (long long)lr * p.n_kgroups * 4, (uint32_t)n * p.pal_bytes, bar0 + 8u * s);
                 r += n;
             }
         }
@@ -160,6 +166,7 @@ lut_smallm_mma_kernel(const SmallmParams p) {
     };
     int s_cur = 0, kg_cur = warp;  // (strip, k group) of the warp's next item
     while (kg_cur >= kgs) { kg_cur -= kgs; ++s_cur; }
+    if (!p.pal_bytes) load_palettes(warp, s_cur, kg_cur);      // weights too: ahead of the wait
     const long long t_a = PLZ_PROF_ON(p.prof) ? clock64() : 0;
     asm volatile("griddepcontrol.wait;" ::: "memory");
     {
@@ -179,7 +186,7 @@ lut_smallm_mma_kernel(const SmallmParams p) {
                 uint4 v[8];
 #pragma unroll
                 for (int u = 0; u < 8; ++u)
-                    if (m0 + u < p.M) v[u] = __ldg(reinterpret_cast<const uint4*>(src + (long long)(m0 + u) * p.ldx));
+                    if (m0 + u < p.M) v[u] = *reinterpret_cast<const uint4*>(src + (long long)(m0 + u) * p.ldx);
 #pragma unroll
                 for (int u = 0; u < 8; ++u) {
                     if (m0 + u < p.M) {
@@ -194,7 +201,6 @@ lut_smallm_mma_kernel(const SmallmParams p) {
             }
         }
     }
-    load_palettes(warp, s_cur, kg_cur);
     for (int i = threadIdx.x; i < rows_pad * 8 * MT; i += kThreads) acc_s[i] = 0.f;
     const long long t_pro = PLZ_PROF_ON(p.prof) ? clock64() : 0;
     __syncthreads();
@@ -208,7 +214,7 @@ lut_smallm_mma_kernel(const SmallmParams p) {
         xs_base[mt] = smem_u32(xs) + (uint32_t)((mt * 8 + g) < p.M ? (mt * 8 + g) : 0) * p.x_pitch + (uint32_t)t * 8u;
     const uint32_t w_base = smem_u32(wsm) + (uint32_t)g * row_bytes + (uint32_t)t * 16u;
     for (int first = warp; ok && first < n_items; first += kBatch * kWarps) {
-        if (first != warp) load_palettes(first, s_cur, kg_cur);
+        if (!p.pal_bytes && first != warp) load_palettes(first, s_cur, kg_cur);
 #pragma unroll
         for (int q = 0; q < kBatch; ++q) {
             const int item = first + q * kWarps;
@@ -227,6 +233,12 @@ lut_smallm_mma_kernel(const SmallmParams p) {
             for (int mt = 0; mt < MT; ++mt) {
                 d[mt][0] = d[mt][1] = d[mt][2] = d[mt][3] = 0.f;
                 e_acc[mt][0] = e_acc[mt][1] = e_acc[mt][2] = e_acc[mt][3] = 0.f;
+            }
+            if (p.pal_bytes) {       // rows past the last one read what lies behind, for outputs that are not written
+                const int pg = p.gs_k_shift >= 0 ? ((kg << 8) >> p.gs_k_shift) : ((kg << 8) / p.gs_k);
+                const uint32_t at = smem_u32(pal_sm) + (uint32_t)(s * 16 + g) * p.pal_bytes + (uint32_t)pg * 8u;
+                asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(pa[q].x), "=r"(pa[q].y) : "r"(at));
+                asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(pb[q].x), "=r"(pb[q].y) : "r"(at + 8u * p.pal_bytes));
             }
             uint32_t wra[4], wrb[4];
             const uint32_t wadr = w_base + (uint32_t)(s * 16) * row_bytes + (uint32_t)kg * 64u;
@@ -257,10 +269,15 @@ lut_smallm_mma_kernel(const SmallmParams p) {
             float* o = acc_s + (size_t)(s * 16 + g) * (8 * MT) + 2 * t;
 #pragma unroll
             for (int mt = 0; mt < MT; ++mt) {
-                atomicAdd(o + mt * 8, d[mt][0] + e_acc[mt][0]);
-                atomicAdd(o + mt * 8 + 1, d[mt][1] + e_acc[mt][1]);
-                atomicAdd(o + 8 * (8 * MT) + mt * 8, d[mt][2] + e_acc[mt][2]);
-                atomicAdd(o + 8 * (8 * MT) + mt * 8 + 1, d[mt][3] + e_acc[mt][3]);
+                const int m = mt * 8 + 2 * t;                    // columns of rows of x that there are
+                if (m < p.M) {
+                    atomicAdd(o + mt * 8, d[mt][0] + e_acc[mt][0]);
+                    atomicAdd(o + 8 * (8 * MT) + mt * 8, d[mt][2] + e_acc[mt][2]);
+                }
+                if (m + 1 < p.M) {
+                    atomicAdd(o + mt * 8 + 1, d[mt][1] + e_acc[mt][1]);
+                    atomicAdd(o + 8 * (8 * MT) + mt * 8 + 1, d[mt][3] + e_acc[mt][3]);
+                }
             }
         }
     }
@@ -333,11 +350,20 @@ int launch_lut_smallm_mma_multi(const GemvArgs* mats, int count, cudaStream_t st
     // reserved; when that does not fit, reserve the exact rows and make the tail at least that long.
     const size_t rb = (size_t)a.K / 4;
     const size_t tail = (size_t)a.M * p.x_pitch + (size_t)rows_pad * 8 * mt * sizeof(float);
-    size_t smem = kHeader + (size_t)rows_pad * rb + tail;
-    p.rows_alloc = rows_pad;
-    if (smem > 227u * 1024u) {
-        p.rows_alloc = rows_per_cta;
-        smem = kHeader + (size_t)rows_per_cta * rb + (tail > 16 * rb ? tail : 16 * rb);
+    p.pal_bytes = a.gs_n == 1 && p.n_kgroups % 2 == 0 ? (uint32_t)p.n_kgroups * 8u : 0u;
+    for (int i = 0; i < count; ++i)
+        if ((uintptr_t)mats[i].palette & 15) p.pal_bytes = 0;
+    size_t smem = 0;
+    for (int form = p.pal_bytes ? 0 : 1; form < 2; ++form) {       // the palettes only where they fit
+        if (form == 1) p.pal_bytes = 0;
+        const size_t row = rb + p.pal_bytes;
+        p.rows_alloc = rows_pad;
+        smem = kHeader + (size_t)rows_pad * row + tail;
+        if (smem > 227u * 1024u) {
+            p.rows_alloc = rows_per_cta;
+            smem = kHeader + (size_t)rows_per_cta * row + (tail > 16 * rb ? tail : 16 * rb);
+        }
+        if (smem <= 227u * 1024u) break;
     }
     if (rows_pad / 16 > (kHeader - 16) / 8) return PLZ_ERR_UNSUPPORTED;
     if (smem > 227u * 1024u) {
