@@ -8,7 +8,8 @@
 //             bits on every run.
 //   operands  dense bf16 W by TMA (requested before the wait on the previous kernel of the stream), or packed 2-bit indices: a decode
 //             thread is one weight row, fetches the 16 bytes of a block of 64 columns several blocks ahead and writes the decoded row to
-//             TMEM, from where it is the A operand (lane = row: no shared memory, no swizzle, no proxy fence in between). x by TMA.
+//             TMEM, from where it is the A operand (lane = row: no shared memory, no swizzle, no proxy fence in between). x by TMA into a
+//             ring of its own, since TMEM has room for a few blocks of W only. A block takes a CTA 0.6 us, whatever the rows: the decode.
 //             Shared memory and TMEM are kept to half of an SM's, so that two CTAs share one and hide each other's start and end.
 //   turned    (transposed) W is an activation matrix of any number of rows and x the few rows of a LoRA factor, t = s x A^T and dt = s dY B: the
 //             same launch with y stored [row of W][row of x], x from [M, K] or (x_mn) from [K, M].
@@ -29,7 +30,9 @@ constexpr uint32_t kNgWBytes = 128 * 64 * 2;
 // shared memory of the stages; two CTAs per SM. LUT: four x tiles of 128 tokens and the W tile of the extra block
 template <bool LUT>
 constexpr uint32_t kNgRingBytes = LUT ? 80 * 1024 : 96 * 1024;
-constexpr int kNgMaxStages = 8;
+constexpr int kNgMaxStages = 16;                  // slots for copies
+constexpr int kNgMaxW = 8;                        // blocks of decoded W in TMEM
+constexpr uint32_t kNgBarBytes = 512;
 constexpr int kNgAhead = 4;                       // blocks of packed indices a decode thread has in flight
 
 struct NarrowMat {
@@ -38,7 +41,7 @@ struct NarrowMat {
     void* y; long long ldy;
 };
 struct NarrowParams {
-    int M, npad, n_acc, stages;
+    int M, npad, n_acc, stages, w_stages;   // slots for copies (dense: W and x, LUT: x), LUT: blocks of W in TMEM
     int x_mn, transposed;
     uint32_t x_bytes;              // of a tile of x
     uint32_t tmem_cols;
@@ -83,8 +86,12 @@ narrow_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
     const uint32_t bar_off = kNgRingBytes<LUT>;
     auto full = [&](int s) { return base + bar_off + 8u * s; };
     auto empty = [&](int s) { return base + bar_off + 8u * (kNgMaxStages + s); };
-    const uint32_t acc_full = base + bar_off + 8u * (2 * kNgMaxStages);
-    volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem + bar_off + 8 * (2 * kNgMaxStages + 1));
+    auto full_w = [&](int s) { return base + bar_off + 8u * (2 * kNgMaxStages + s); };             // LUT only
+    auto empty_w = [&](int s) { return base + bar_off + 8u * (2 * kNgMaxStages + kNgMaxW + s); };
+    constexpr int kBars = 2 * kNgMaxStages + 2 * kNgMaxW + 1;
+    static_assert(8 * kBars + 8 <= kNgBarBytes, "barriers");
+    const uint32_t acc_full = base + bar_off + 8u * (kBars - 1);
+    volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem + bar_off + 8 * kBars);
     volatile uint32_t* abort_flag = tmem_slot + 1;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -139,8 +146,12 @@ narrow_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
     }
     if (threadIdx.x == 0) {
         for (int s = 0; s < kNgMaxStages; ++s) {
-            mbar_init(full(s), LUT ? 1 + kNgDecodeWarps / 2 : 1);
+            mbar_init(full(s), 1);
             mbar_init(empty(s), 1);
+        }
+        for (int s = 0; LUT && s < kNgMaxW; ++s) {
+            mbar_init(full_w(s), kNgDecodeWarps / 2);
+            mbar_init(empty_w(s), 1);
         }
         mbar_init(acc_full, 1);
         *abort_flag = 0;
@@ -184,9 +195,11 @@ narrow_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
             const bool mn = !LUT && p.x_mn;
             const uint32_t idesc = make_idesc(128, p.npad, 0, mn ? 1 : 0), x_step = mn ? 2048u >> 4 : 2u;   // 16 reduction elements of x
             bool ok = true;
+            int s = 0, iw = 0;
+            uint32_t ph = 0, phw = 0;
             for (int it = 0; it < nb && ok; ++it) {
-                const int s = it % p.stages;
-                ok = mbar_wait(full(s), (it / p.stages) & 1, abort_flag, p.status, ST_TIMEOUT_FULL, 1);
+                ok = mbar_wait(full(s), ph, abort_flag, p.status, ST_TIMEOUT_FULL, 1);
+                if (LUT && ok) ok = mbar_wait(full_w(iw), phw, abort_flag, p.status, ST_TIMEOUT_FULL, 1);
                 if (!ok) break;
                 tc_fence_after_sync();
                 const bool from_tmem = LUT && b_begin + it < p.nkb;
@@ -195,10 +208,13 @@ narrow_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
 #pragma unroll
                 for (int ks = 0; ks < 4; ++ks) {
                     const uint32_t d = tmem_base + (uint32_t)((ks & (p.n_acc - 1)) * p.npad), more = (it > 0 || ks >= p.n_acc) ? 1u : 0u;
-                    if (from_tmem) umma_ts(d, tmem_w + s * 32u + ks * 8u, (uint32_t)bd + ks * 2u, (uint32_t)(bd >> 32), idesc, more);
+                    if (from_tmem) umma_ts(d, tmem_w + iw * 32u + ks * 8u, (uint32_t)bd + ks * 2u, (uint32_t)(bd >> 32), idesc, more);
                     else umma_bf16_words<1>(d, (uint32_t)ad + ks * 2u, (uint32_t)(ad >> 32), (uint32_t)bd + ks * x_step, (uint32_t)(bd >> 32), idesc, more);
                 }
                 umma_commit(empty(s));
+                if (LUT) umma_commit(empty_w(iw));
+                if (++s == p.stages) { s = 0; ph ^= 1u; }
+                if (LUT && ++iw == p.w_stages) { iw = 0; phw ^= 1u; }
             }
             if (ok) umma_commit(acc_full);
         }
@@ -211,8 +227,8 @@ narrow_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
                 for (int j = 0; j < kAhead; ++j) {
                     const int it = it0 + 2 * j;
                     if (it >= nb || !ok) continue;
-                    const int s = it % p.stages;
-                    ok = mbar_wait(empty(s), ((it / p.stages) & 1) ^ 1u, abort_flag, p.status, ST_TIMEOUT_EMPTY, 3);
+                    const int s = it % p.w_stages;       // an even number of blocks: a group always writes the same ones
+                    ok = mbar_wait(empty_w(s), ((it / p.w_stages) & 1) ^ 1u, abort_flag, p.status, ST_TIMEOUT_EMPTY, 3);
                     if (!ok) continue;
                     if (it < nw) {
                         uint32_t o[32];
@@ -227,7 +243,7 @@ narrow_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
                         tc_fence_before_sync();
                     }
                     __syncwarp();
-                    if (lane == 0) mbar_arrive(full(s));
+                    if (lane == 0) mbar_arrive(full_w(s));
                 }
             }
         }
@@ -334,16 +350,19 @@ narrow_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
     if (warp == 1) { tc_fence_after_sync(); tmem_dealloc(tmem_base, p.tmem_cols); }
 }
 
-// CTAs per tile: the shortest schedule when tiles * c CTAs of ceil(blocks / c) blocks each, plus about four for start, sum and end, are dealt
-// to the SMs.
-int cluster_size(int tiles, int blocks, int sms) {
+// CTAs per tile: the shortest schedule when tiles * c CTAs of ceil(blocks / c) blocks each, plus about `fixed` for start, sum and end, are dealt to
+// two places per SM, of which clusters can fill about nine tenths. Two CTAs of an SM slow each other down a little. Measured over 8 to 152
+// tiles, 40 to 152 blocks, 20 to 128 rows: within 5 % of the best of 1 .. 8. A rule that counted one place per SM gave 2560 x 9728 packed 22 us at 64 rows
+// for 19, 6144 x 2560 14.7 for 12.7, 19456 x 2560 36 for 33.
+int cluster_size(int tiles, int blocks, int sms, int fixed) {
     int best = 1;
-    long long best_cost = 0;
+    double best_cost = 0;
     for (int c = 1; c <= 8; ++c) {
         if (c > 1 && blocks / c < 2) break;
         if (c == 5 || c == 7) continue;           // leave SMs of a processing cluster without a partner
-        const long long rounds = ((long long)tiles * c + sms - 1) / sms;
-        const long long cost = rounds * ((blocks + c - 1) / c + 4);
+        const long long ctas = (long long)tiles * c, places = c > 1 ? 2 * sms * 9 / 10 : 2 * sms;
+        const double shared = ctas <= sms ? 0.0 : ctas >= 2 * sms ? 1.0 : (double)(ctas - sms) / sms;
+        const double cost = (double)((ctas + places - 1) / places) * ((blocks + c - 1) / c + fixed) * (1.0 + 0.3 * shared);
         if (c == 1 || cost < best_cost) { best = c; best_cost = cost; }
     }
     return best;
@@ -352,7 +371,7 @@ int cluster_size(int tiles, int blocks, int sms) {
 template <bool LUT>
 int launch_ng(const NarrowParams& p, int tiles, int ranks, const CUtensorMap (&tm)[4], cudaStream_t stream) {
     auto kern = narrow_gemm_kernel<LUT>;
-    constexpr uint32_t smem = kNgRingBytes<LUT> + 256 + 1024;
+    constexpr uint32_t smem = kNgRingBytes<LUT> + kNgBarBytes + 1024;
     static bool attr_set[64] = {};
     int dev = 0;
     PLZ_CUDA_CHECK(cudaGetDevice(&dev));
@@ -390,7 +409,8 @@ int launch_narrow_gemm(const NarrowArgs& a, cudaStream_t stream) {
     p.x_bytes = a.x_mn ? 64u * 128u : (uint32_t)p.npad * 128u;       // x_mn: 64 reduction rows of 64 columns
     if (lut) {      // 256 TMEM columns: accumulators, then 32 columns per stage
         p.n_acc = p.npad <= 32 ? 4 : p.npad == 64 ? 2 : 1;
-        p.stages = (256 - p.n_acc * p.npad) / 32;
+        p.w_stages = (256 - p.n_acc * p.npad) / 32;                              // 4 or 6
+        p.stages = (int)((kNgRingBytes<true> - kNgWBytes) / p.x_bytes);      // behind them the W tile of the extra block
         p.tmem_cols = 256;
         p.group_blocks = a.gs_k / 64; p.group_shift = -1;
         for (int i = 0; i < 16; ++i) if (p.group_blocks == 1 << i) p.group_shift = i;
@@ -420,7 +440,7 @@ int launch_narrow_gemm(const NarrowArgs& a, cudaStream_t stream) {
         if ((rc = make_tmap_bf16(&tm[2], a.x2, a.M, a.r2, a.ldx2, 64, (uint32_t)p.npad))) return rc;
         if ((rc = make_tmap_bf16(&tm[3], a.w2, a.mat[0].N, a.r2, a.ldw2, 64, 128))) return rc;
     }
-    const int ranks = cluster_size(tiles, p.n_blocks, seq_sm_count());
+    const int ranks = cluster_size(tiles, p.n_blocks, seq_sm_count(), 12);
     return lut ? launch_ng<true>(p, tiles, ranks, tm, stream) : launch_ng<false>(p, tiles, ranks, tm, stream);
 }
 
