@@ -9,7 +9,7 @@
 //   operands  dense bf16 W by TMA (requested before the wait on the previous kernel of the stream), or packed 2-bit indices: a decode
 //             thread is one weight row, fetches the 16 bytes of a block of 64 columns several blocks ahead and writes the decoded row to
 //             TMEM, from where it is the A operand (lane = row: no shared memory, no swizzle, no proxy fence in between). x by TMA into a
-//             ring of its own, since TMEM has room for a few blocks of W only. A block takes a CTA 0.6 us, whatever the rows: the decode.
+//             ring of its own, since TMEM has room for a few blocks of W only. A single issuing lane took 0.6 us a block (see there).
 //             Shared memory and TMEM are kept to half of an SM's, so that two CTAs share one and hide each other's start and end.
 //   turned    (transposed) W is an activation matrix of any number of rows and x the few rows of a LoRA factor, t = s x A^T and dt = s dY B: the
 //             same launch with y stored [row of W][row of x], x from [M, K] or (x_mn) from [K, M].
@@ -94,7 +94,8 @@ narrow_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem + bar_off + 8 * kBars);
     volatile uint32_t* abort_flag = tmem_slot + 1;
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    // the warp's number as a value the compiler knows to be uniform: what the issuing warp computes then stays in uniform registers
+    const int warp = __shfl_sync(0xFFFFFFFFu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     const int n_ranks = (int)cluster_nctarank(), rank = (int)cluster_ctarank();
     const int tile = (int)blockIdx.x / n_ranks;
     int mi = 0;
@@ -191,33 +192,50 @@ narrow_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            const bool mn = !LUT && p.x_mn;
-            const uint32_t idesc = make_idesc(128, p.npad, 0, mn ? 1 : 0), x_step = mn ? 2048u >> 4 : 2u;   // 16 reduction elements of x
-            bool ok = true;
-            int s = 0, iw = 0;
-            uint32_t ph = 0, phw = 0;
-            for (int it = 0; it < nb && ok; ++it) {
-                ok = mbar_wait(full(s), ph, abort_flag, p.status, ST_TIMEOUT_FULL, 1);
-                if (LUT && ok) ok = mbar_wait(full_w(iw), phw, abort_flag, p.status, ST_TIMEOUT_FULL, 1);
-                if (!ok) break;
-                tc_fence_after_sync();
-                const bool from_tmem = LUT && b_begin + it < p.nkb;
-                const uint32_t sw = base + (LUT ? w2_off : s * stage_bytes), sx = base + s * stage_bytes + (LUT ? 0u : kNgWBytes);
-                const uint64_t ad = make_sdesc(sw, 16u, 1024u), bd = make_sdesc(sx, 16u, 1024u);
-#pragma unroll
-                for (int ks = 0; ks < 4; ++ks) {
-                    const uint32_t d = tmem_base + (uint32_t)((ks & (p.n_acc - 1)) * p.npad), more = (it > 0 || ks >= p.n_acc) ? 1u : 0u;
-                    if (from_tmem) umma_ts(d, tmem_w + iw * 32u + ks * 8u, (uint32_t)bd + ks * 2u, (uint32_t)(bd >> 32), idesc, more);
-                    else umma_bf16_words<1>(d, (uint32_t)ad + ks * 2u, (uint32_t)(ad >> 32), (uint32_t)bd + ks * x_step, (uint32_t)(bd >> 32), idesc, more);
+        // The whole warp walks the blocks and one elected lane issues. In a branch of one lane the operands of every MMA live in vector registers
+        // and are moved to uniform ones first: 630 clocks for the four MMAs and two commits of a block, longer than all else. Packed, 64 rows: 19456 x 2560 33 -> 24 us,
+        // 2560 x 9728 18.8 -> 14.1, 1024 x 2560 7.7 -> 6.3.
+        const bool mn = !LUT && p.x_mn;
+        const uint32_t idesc = make_idesc(128, p.npad, 0, mn ? 1 : 0), x_step = mn ? 2048u >> 4 : 2u;   // 16 reduction elements of x
+        const uint64_t desc = make_sdesc(base, 16u, 1024u);
+        const uint32_t hi = (uint32_t)(desc >> 32), lo0 = (uint32_t)desc, slot = stage_bytes >> 4, x_off = LUT ? 0u : kNgWBytes >> 4;
+        const uint32_t d1 = tmem_base + (p.n_acc > 1 ? (uint32_t)p.npad : 0u), d2 = tmem_base + (p.n_acc > 2 ? 2u * (uint32_t)p.npad : 0u),
+                       d3 = p.n_acc > 2 ? tmem_base + 3u * (uint32_t)p.npad : d1;
+        bool ok = true;
+        int s = 0, iw = 0;
+        uint32_t ph = 0, phw = 0, lo = lo0;
+        for (int it = 0; it < nb; ++it) {
+            ok = mbar_wait(full(s), ph, abort_flag, p.status, ST_TIMEOUT_FULL, 1);
+            if (LUT && ok) ok = mbar_wait(full_w(iw), phw, abort_flag, p.status, ST_TIMEOUT_FULL, 1);
+            ok = __all_sync(0xFFFFFFFFu, ok);
+            if (!ok) break;
+            tc_fence_after_sync();
+            const bool from_tmem = LUT && b_begin + it < p.nkb;
+            const uint32_t xd = lo + x_off, wd = LUT ? lo0 + (w2_off >> 4) : lo, wt = tmem_w + iw * 32u;
+            const uint32_t first = it > 0 ? 1u : 0u;             // accumulators start with their first MMA
+            const uint32_t m1 = p.n_acc > 1 ? first : 1u, m2 = p.n_acc > 2 ? first : 1u;
+            if (elect_one()) {
+                if (from_tmem) {
+                    umma_ts(tmem_base, wt, xd, hi, idesc, first);
+                    umma_ts(d1, wt + 8u, xd + 2u, hi, idesc, m1);
+                    umma_ts(d2, wt + 16u, xd + 4u, hi, idesc, m2);
+                    umma_ts(d3, wt + 24u, xd + 6u, hi, idesc, m2);
+                } else {
+                    umma_bf16_words<1>(tmem_base, wd, hi, xd, hi, idesc, first);
+                    umma_bf16_words<1>(d1, wd + 2u, hi, xd + x_step, hi, idesc, m1);
+                    umma_bf16_words<1>(d2, wd + 4u, hi, xd + 2u * x_step, hi, idesc, m2);
+                    umma_bf16_words<1>(d3, wd + 6u, hi, xd + 3u * x_step, hi, idesc, m2);
                 }
                 umma_commit(empty(s));
                 if (LUT) umma_commit(empty_w(iw));
-                if (++s == p.stages) { s = 0; ph ^= 1u; }
-                if (LUT && ++iw == p.w_stages) { iw = 0; phw ^= 1u; }
             }
-            if (ok) umma_commit(acc_full);
+            __syncwarp();
+            lo += slot;
+            if (++s == p.stages) { s = 0; ph ^= 1u; lo = lo0; }
+            if (LUT && ++iw == p.w_stages) { iw = 0; phw ^= 1u; }
         }
+        if (ok && elect_one()) umma_commit(acc_full);
+        __syncwarp();
     } else {
         bool ok = true;
         if (LUT) {
