@@ -5,7 +5,7 @@
 // Bound by the tensor cores where the tiles fill the waves. Against a CTA per 256 x 256 tile (lut_gemm.cu) an SM reads 8 instead of 12 KB of
 // operands per 128 x 256 x 16 of work and holds two accumulators, so that a tile's epilogue runs under the next one's main loop; a last wave
 // of few tiles is cut, and few tiles are made narrow enough to fill the chip once.
-// us there / here: 1000 rows, 2560 x 9728 97 / 51, 19456 x 2560 gated 90 / 74; 2048 rows, 2560 x 9728 103 / 96, 9728 x 2560 88 / 78.
+// us there / here: 1000 rows, 2560 x 9728 97 / 49, 19456 x 2560 gated 90 / 72; 2048 rows, 2560 x 9728 103 / 90, 9728 x 2560 88 / 73.
 #include "plz_launch.h"
 
 namespace plz {
@@ -59,7 +59,8 @@ dense_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem + kDpBarOff + 8 * (2 * kDpStages + 4));
     volatile uint32_t* abort_flag = tmem_slot + 1;
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xFFFFFFFFu, (int)(threadIdx.x >> 5), 0);   // uniform to the compiler too
+    const int lane = threadIdx.x & 31;
     const int rank = (int)cluster_ctarank();
     const uint32_t lead_bar_base = leader_addr(bar_base);
     const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
@@ -139,7 +140,8 @@ dense_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------- MMA issuer (leader only)
-        if (rank == 0 && lane == 0) {
+        // the whole warp walks the stages and one elected lane issues (narrow_gemm.cu: operands stay in uniform registers)
+        if (rank == 0) {
             const uint32_t idesc_whole = make_idesc(256, p.tile_w, 0, BMN ? 1 : 0), idesc_half = make_idesc(256, 128, 0, BMN ? 1 : 0);
             const uint64_t ad0 = make_sdesc(base, 16u, 1024u);
             const uint64_t bd0 = BMN ? make_sdesc(base + kDpABytes, kDpBlkBytes, 1024u) : make_sdesc(base + kDpABytes, 16u, 1024u);
@@ -151,28 +153,33 @@ dense_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
             for (int t = pair; t < p.n_items && ok; t += n_pairs, ++lt) {
                 const uint32_t d_tmem = tmem_base + (uint32_t)(lt & 1) * 256u;
                 const uint32_t idesc = t < p.n_whole ? idesc_whole : idesc_half;
-                ok = mbar_wait_lean(acc_empty(lt & 1), ((lt >> 1) & 1) ^ 1u, abort_flag, p.status, ST_TIMEOUT_ACCUM, 1);
+                ok = __all_sync(0xFFFFFFFFu, mbar_wait_lean(acc_empty(lt & 1), ((lt >> 1) & 1) ^ 1u, abort_flag, p.status, ST_TIMEOUT_ACCUM, 1));
                 if (!ok) break;
                 tc_fence_after_sync();
                 for (int it = 0; it < nkb_total; ++it) {
-                    ok = mbar_wait_lean(full(s), ph, abort_flag, p.status, ST_TIMEOUT_FULL, 1);
+                    ok = __all_sync(0xFFFFFFFFu, mbar_wait_lean(full(s), ph, abort_flag, p.status, ST_TIMEOUT_FULL, 1));
                     if (!ok) break;
                     tc_fence_after_sync();
                     // k step ks: A and K-major B advance 32 bytes inside a 64-wide block and one block after four steps;
-                    // MN-major B advances 16 rows of 128 bytes
-                    const int steps = it < nkb ? 8 : 4;
+                    // MN-major B advances 16 rows of 128 bytes. The LoRA block is 64 wide: four steps
+                    const uint32_t more = it > 0 ? 1u : 0u;
+                    if (elect_one()) {
 #pragma unroll
-                    for (int ks = 0; ks < 8; ++ks) {
-                        if (ks >= steps) break;
-                        const uint32_t offk = (uint32_t)((ks >> 2) * (kDpBlkBytes >> 4) + (ks & 3) * 2);
-                        const uint32_t offb = BMN ? (uint32_t)(ks * (2048 >> 4)) : offk;
-                        umma_bf16_words<2>(d_tmem, a_lo + offk, a_hi, b_lo + offb, b_hi, idesc, (ks > 0) ? 1u : (it > 0 ? 1u : 0u));
+                        for (int ks = 0; ks < 4; ++ks)
+                            umma_bf16_words<2>(d_tmem, a_lo + ks * 2, a_hi, b_lo + (BMN ? ks * (2048 >> 4) : ks * 2), b_hi, idesc, ks > 0 ? 1u : more);
+                        if (it < nkb) {
+#pragma unroll
+                            for (int ks = 0; ks < 4; ++ks)
+                                umma_bf16_words<2>(d_tmem, a_lo + (kDpBlkBytes >> 4) + ks * 2, a_hi, b_lo + (BMN ? (ks + 4) * (2048 >> 4) : (int)(kDpBlkBytes >> 4) + ks * 2), b_hi, idesc, 1u);
+                        }
+                        umma_commit_pair(empty(s));
                     }
-                    umma_commit_pair(empty(s));
+                    __syncwarp();
                     if (++s == kDpStages) { s = 0; ph ^= 1u; a_lo = a_lo0; b_lo = b_lo0; }
                     else { a_lo += kDpStageBytes >> 4; b_lo += kDpStageBytes >> 4; }
                 }
-                if (ok) umma_commit_pair(acc_full(lt & 1));
+                if (ok && elect_one()) umma_commit_pair(acc_full(lt & 1));
+                __syncwarp();
             }
         }
     } else {

@@ -92,7 +92,7 @@ lut_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem + kBarOff + 8 * (2 * kStages + 4));
     volatile uint32_t* abort_flag = tmem_slot + 1;
 
-    const int warp = threadIdx.x >> 5;
+    const int warp = __shfl_sync(0xFFFFFFFFu, (int)(threadIdx.x >> 5), 0);   // uniform to the compiler too
     const int lane = threadIdx.x & 31;
     const uint32_t rank = cluster_ctarank();   // 0 = leader
     const uint32_t lead_bar_base = leader_addr(bar_base);   // the leader's barrier block as a shared::cluster address
@@ -175,7 +175,9 @@ lut_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------- MMA issuer (leader only)
-        if (rank == 0 && lane == 0) {
+        // the whole warp walks the stages and one elected lane issues (narrow_gemm.cu: operands stay in uniform registers): 1000 rows,
+        // 2560 x 9728 52 -> 46 us, input gradient at 512 rows 51 -> 40, 4096 rows, 9728 x 2560 165 -> 149
+        if (rank == 0) {
             const uint32_t idesc_whole = make_idesc(256, p.tile_w, 0, kBMn ? 1 : 0), idesc_half = make_idesc(256, 128, 0, kBMn ? 1 : 0);
             // descriptor words of stage 0; a stage is kStageBytes >> 4 = 4096 further in the low word
             const uint64_t ad0 = make_sdesc(base, 16u, 1024u);
@@ -192,40 +194,38 @@ lut_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
                 const uint32_t d_tmem = tmem_base + (uint32_t)(lt & 1) * 256u;
                 const uint32_t idesc = t < p.n_whole ? idesc_whole : idesc_half;
                 const long long c_t = PLZ_PROF_ON(p.prof) ? clock64() : 0;
-                ok = mbar_wait_lean(acc_empty(lt & 1), ((lt >> 1) & 1) ^ 1u, abort_flag, p.status, ST_TIMEOUT_ACCUM, 1);
+                ok = __all_sync(0xFFFFFFFFu, mbar_wait_lean(acc_empty(lt & 1), ((lt >> 1) & 1) ^ 1u, abort_flag, p.status, ST_TIMEOUT_ACCUM, 1));
                 if (PLZ_PROF_ON(p.prof)) wait_t += clock64() - c_t;
                 if (!ok) break;
                 tc_fence_after_sync();
                 for (int it = 0; it < nkb_total; ++it) {
                     const long long c0 = PLZ_PROF_ON(p.prof) ? clock64() : 0;
-                    ok = mbar_wait_lean(full(s), ph, abort_flag, p.status, ST_TIMEOUT_FULL, 1);
+                    ok = __all_sync(0xFFFFFFFFu, mbar_wait_lean(full(s), ph, abort_flag, p.status, ST_TIMEOUT_FULL, 1));
                     if (PLZ_PROF_ON(p.prof)) wait_f += clock64() - c0;
                     if (!ok) break;
                     tc_fence_after_sync();
                     // k step ks: A and K-major B advance 32 bytes inside a 64-wide block and one block (16 KB) after four
-                    // steps; MN-major B advances 16 rows of 128 bytes
-                    if (it < nkb) {
+                    // steps; MN-major B advances 16 rows of 128 bytes. The LoRA block is 64 wide: four steps
+                    const uint32_t more = it > 0 ? 1u : 0u;
+                    if (elect_one()) {
 #pragma unroll
-                        for (int ks = 0; ks < 8; ++ks) {
-                            const uint32_t offk = (uint32_t)((ks >> 2) * (kBlkBytes >> 4) + (ks & 3) * 2);
-                            const uint32_t offb = kBMn ? (uint32_t)(ks * (2048 >> 4)) : offk;
-                            umma_bf16_words<2>(d_tmem, a_lo + offk, a_hi, b_lo + offb, b_hi, idesc, (ks > 0) ? 1u : (it > 0 ? 1u : 0u));
-                        }
-                    } else {
+                        for (int ks = 0; ks < 4; ++ks)
+                            umma_bf16_words<2>(d_tmem, a_lo + ks * 2, a_hi, b_lo + (kBMn ? ks * (2048 >> 4) : ks * 2), b_hi, idesc, ks > 0 ? 1u : more);
+                        if (it < nkb) {
 #pragma unroll
-                        for (int ks = 0; ks < 4; ++ks) {   // the LoRA block is 64 wide
-                            const uint32_t offk = (uint32_t)(ks * 2);
-                            const uint32_t offb = kBMn ? (uint32_t)(ks * (2048 >> 4)) : offk;
-                            umma_bf16_words<2>(d_tmem, a_lo + offk, a_hi, b_lo + offb, b_hi, idesc, 1u);
+                            for (int ks = 0; ks < 4; ++ks)
+                                umma_bf16_words<2>(d_tmem, a_lo + (kBlkBytes >> 4) + ks * 2, a_hi, b_lo + (kBMn ? (ks + 4) * (2048 >> 4) : (int)(kBlkBytes >> 4) + ks * 2), b_hi, idesc, 1u);
                         }
+                        umma_commit_pair(empty(s));
                     }
-                    umma_commit_pair(empty(s));
+                    __syncwarp();
                     if (++s == kStages) { s = 0; ph ^= 1u; a_lo = a_lo0; b_lo = b_lo0; }
                     else { a_lo += kStageBytes >> 4; b_lo += kStageBytes >> 4; }
                 }
-                if (ok) umma_commit_pair(acc_full(lt & 1));
+                if (ok && elect_one()) umma_commit_pair(acc_full(lt & 1));
+                __syncwarp();
             }
-            if (PLZ_PROF_ON(p.prof)) {
+            if (PLZ_PROF_ON(p.prof) && lane == 0) {
                 unsigned long long* o = p.prof + 8ull * blockIdx.x;
                 o[0] = wait_f; o[1] = 0; o[2] = wait_t; o[3] = clock64() - t_begin; o[4] = lt;
             }

@@ -114,7 +114,7 @@ tn_gemm_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant__ 
         smem + kStages * kStageBytes + kTnRedBytes + 8 * (2 * kStages + 4));
     volatile uint32_t* abort_flag = tmem_slot + 1;
 
-    const int warp = threadIdx.x >> 5;
+    const int warp = __shfl_sync(0xFFFFFFFFu, (int)(threadIdx.x >> 5), 0);   // uniform to the compiler too
     const int lane = threadIdx.x & 31;
     // PAIR: the two CTAs of a cluster share every work item; full[] and acc_empty[] are used in the leader's copy only
     // (remote arrivals / TMA completions from the partner), empty[] and acc_full[] in each CTA's own copy (multicast commit)
@@ -264,7 +264,8 @@ tn_gemm_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant__ 
         // MMA issuer (PAIR: the leader's only). Kept lean on purpose: a lone thread retires a dependent instruction every
         // five or six cycles and an MMA lasts 128, so the descriptor words are precomputed (one integer add per operand
         // and MMA) and the usual, already-completed barrier costs a single try_wait.
-        if (lane == 0 && rank == 0) {
+        // the whole warp walks the stages and one elected lane issues (narrow_gemm.cu: operands stay in uniform registers)
+        if (rank == 0) {
             bool ok = true;
             int lt = 0, s = 0;
             uint32_t ph = 0;
@@ -284,27 +285,31 @@ tn_gemm_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant__ 
                 const uint32_t idesc = make_idesc(PAIR ? 256 : 128, c_num, 1, 1);
                 const uint32_t d_tmem = tmem_base + buf * 256u;
                 const long long c_t = PLZ_PROF_ON(p.prof) ? clock64() : 0;
-                ok = mbar_wait_lean(acc_empty(buf), ((lt >> 1) & 1) ^ 1u, abort_flag, p.status, ST_TIMEOUT_ACCUM, 1);
+                ok = __all_sync(0xFFFFFFFFu, mbar_wait_lean(acc_empty(buf), ((lt >> 1) & 1) ^ 1u, abort_flag, p.status, ST_TIMEOUT_ACCUM, 1));
                 if (PLZ_PROF_ON(p.prof)) wait_t += clock64() - c_t;
                 if (!ok) break;
                 tc_fence_after_sync();
                 for (int it = 0; it < nkb; ++it) {
                     const long long c_f = PLZ_PROF_ON(p.prof) ? clock64() : 0;
-                    ok = mbar_wait_lean(full(s), ph, abort_flag, p.status, ST_TIMEOUT_FULL, 1);
+                    ok = __all_sync(0xFFFFFFFFu, mbar_wait_lean(full(s), ph, abort_flag, p.status, ST_TIMEOUT_FULL, 1));
                     if (PLZ_PROF_ON(p.prof)) { wait_f += clock64() - c_f; ++n_st; }
                     if (!ok) break;
                     tc_fence_after_sync();
+                    const uint32_t more = it > 0 ? 1u : 0u;
+                    if (elect_one()) {
 #pragma unroll
-                    for (int ks = 0; ks < 4; ++ks)   // 16 rows of m = 2048 bytes per step in both MN-major operands
-                        umma_bf16_words<PAIR ? 2 : 1>(d_tmem, a_lo + ks * 128u, a_hi, b_lo + ks * 128u, b_hi, idesc,
-                                                     (ks > 0) ? 1u : (it > 0 ? 1u : 0u));
-                    if (PAIR) umma_commit_pair(empty(s)); else umma_commit(empty(s));
+                        for (int ks = 0; ks < 4; ++ks)   // 16 rows of m = 2048 bytes per step in both MN-major operands
+                            umma_bf16_words<PAIR ? 2 : 1>(d_tmem, a_lo + ks * 128u, a_hi, b_lo + ks * 128u, b_hi, idesc, ks > 0 ? 1u : more);
+                        if (PAIR) umma_commit_pair(empty(s)); else umma_commit(empty(s));
+                    }
+                    __syncwarp();
                     if (++s == kStages) { s = 0; ph ^= 1u; a_lo = a_lo0; b_lo = b_lo0; }
                     else { a_lo += kStageBytes >> 4; b_lo += kStageBytes >> 4; }
                 }
-                if (ok) { if (PAIR) umma_commit_pair(acc_full(buf)); else umma_commit(acc_full(buf)); }
+                if (ok && elect_one()) { if (PAIR) umma_commit_pair(acc_full(buf)); else umma_commit(acc_full(buf)); }
+                __syncwarp();
             }
-            if (PLZ_PROF_ON(p.prof)) {
+            if (PLZ_PROF_ON(p.prof) && lane == 0) {
                 unsigned long long* o = p.prof + 8ull * blockIdx.x;
                 o[0] = wait_f; o[1] = n_st; o[2] = wait_t; o[3] = clock64() - t_begin; o[4] = lt;
             }
