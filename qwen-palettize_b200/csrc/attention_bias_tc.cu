@@ -234,7 +234,7 @@ attn_bias_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem + C::OFF_BAR + 128);
     volatile uint32_t* abort_flag = tmem_slot + 1;
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xFFFFFFFFu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;   // uniform to the compiler too
     const int n_qt = (p.n + kT - 1) / kT;
     const int n_pairs = (n_qt + 1) / 2;
     const int pi = n_pairs - 1 - (int)blockIdx.x;   // heavy pairs first
@@ -264,61 +264,62 @@ attn_bias_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     auto tO = [&](int g) { return tmem + 256u + 128u * g; };
 
     if (warp == 8) {
-        if (lane == 0) {
-            tma_prefetch_desc(&tmQ); tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmV);
-            mbar_arrive_expect_tx(q_full, hasB ? 2 * C::QK : C::QK);
-            load_boxes2<DKB>(sQ0, &tmQ, &tmQ2, p.k1_blocks, q_full, h, h, qtA * kT, b);
-            if (hasB) load_boxes2<DKB>(sQ0 + C::QS, &tmQ, &tmQ2, p.k1_blocks, q_full, h, h, qtB * kT, b);
+        // the whole warp walks the tiles and one elected lane issues (narrow_gemm.cu: operands stay in uniform registers)
+        {
+            if (elect_one()) { tma_prefetch_desc(&tmQ); tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmV); }
+            if (elect_one()) { mbar_arrive_expect_tx(q_full, hasB ? 2 * C::QK : C::QK); }
+            if (elect_one()) { load_boxes2<DKB>(sQ0, &tmQ, &tmQ2, p.k1_blocks, q_full, h, h, qtA * kT, b); }
+            if (hasB && elect_one()) load_boxes2<DKB>(sQ0 + C::QS, &tmQ, &tmQ2, p.k1_blocks, q_full, h, h, qtB * kT, b);
             bool ok = true;
             for (int j = 0; j < 2 && j < n_kv; ++j) {
-                mbar_arrive_expect_tx(k_full0 + 8 * j, C::QK);
-                load_boxes2<DKB>(sK0 + j * C::QK, &tmK, &tmK2, p.k1_blocks, k_full0 + 8 * j, hk, 0, j * kT, b);
+                if (elect_one()) { mbar_arrive_expect_tx(k_full0 + 8 * j, C::QK); }
+                if (elect_one()) { load_boxes2<DKB>(sK0 + j * C::QK, &tmK, &tmK2, p.k1_blocks, k_full0 + 8 * j, hk, 0, j * kT, b); }
             }
-            mbar_arrive_expect_tx(v_full, C::V);
-            load_boxes<DVB>(sV, &tmV, v_full, hk, 0, b);
-            ok = mbar_wait(q_full, 0, abort_flag, p.status, ST_TIMEOUT_FULL, 10);
-            if (ok) ok = mbar_wait(k_full0, 0, abort_flag, p.status, ST_TIMEOUT_FULL, 11);
+            if (elect_one()) { mbar_arrive_expect_tx(v_full, C::V); }
+            if (elect_one()) { load_boxes<DVB>(sV, &tmV, v_full, hk, 0, b); }
+            ok = mbar_wait_warp(q_full, 0, abort_flag, p.status, ST_TIMEOUT_FULL, 10);
+            if (ok) ok = mbar_wait_warp(k_full0, 0, abort_flag, p.status, ST_TIMEOUT_FULL, 11);
             if (ok) {
                 tc_fence_after_sync();
-                mma_qk<DKB>(tS(0), sQ0, sK0, p.k_steps);
-                umma_commit(s_full(0));
-                if (hasB) { mma_qk<DKB>(tS(1), sQ0 + C::QS, sK0, p.k_steps); umma_commit(s_full(1)); }
+                if (elect_one()) { mma_qk<DKB>(tS(0), sQ0, sK0, p.k_steps); }
+                if (elect_one()) { umma_commit(s_full(0)); }
+                if (hasB && elect_one()) { mma_qk<DKB>(tS(1), sQ0 + C::QS, sK0, p.k_steps); umma_commit(s_full(1)); }
             }
             for (int j = 0; j < n_kv && ok; ++j) {
                 const int s = j & 1, s1 = (j + 1) & 1;
-                ok = mbar_wait(v_full, j & 1, abort_flag, p.status, ST_TIMEOUT_FULL, 15);
+                ok = mbar_wait_warp(v_full, j & 1, abort_flag, p.status, ST_TIMEOUT_FULL, 15);
                 if (!ok) break;
 #pragma unroll
                 for (int g = 0; g < 2; ++g) {
                     const int n_g = g == 0 ? n_kvA : n_kv;
                     if ((g == 1 && !hasB) || j >= n_g) continue;
-                    ok = mbar_wait(p_full(g), j & 1, abort_flag, p.status, ST_TIMEOUT_FULL, 12);
+                    ok = mbar_wait_warp(p_full(g), j & 1, abort_flag, p.status, ST_TIMEOUT_FULL, 12);
                     if (!ok) break;
                     tc_fence_after_sync();
-                    mma_pv<DVB>(tO(g), tS(g), sV, j > 0);
-                    umma_commit(o_full(g));
+                    if (elect_one()) { mma_pv<DVB>(tO(g), tS(g), sV, j > 0); }
+                    if (elect_one()) { umma_commit(o_full(g)); }
                     if (j + 1 < n_g) {
-                        ok = mbar_wait(k_full0 + 8 * s1, ((j + 1) >> 1) & 1, abort_flag, p.status, ST_TIMEOUT_FULL, 13);
+                        ok = mbar_wait_warp(k_full0 + 8 * s1, ((j + 1) >> 1) & 1, abort_flag, p.status, ST_TIMEOUT_FULL, 13);
                         if (!ok) break;
                         tc_fence_after_sync();
-                        mma_qk<DKB>(tS(g), sQ0 + g * C::QS, sK0 + s1 * C::QK, p.k_steps);
-                        umma_commit(s_full(g));
+                        if (elect_one()) { mma_qk<DKB>(tS(g), sQ0 + g * C::QS, sK0 + s1 * C::QK, p.k_steps); }
+                        if (elect_one()) { umma_commit(s_full(g)); }
                     }
                 }
                 if (!ok) break;
-                umma_commit(v_empty);
-                umma_commit(k_empty0 + 8 * s);
+                if (elect_one()) { umma_commit(v_empty); }
+                if (elect_one()) { umma_commit(k_empty0 + 8 * s); }
                 if (j + 1 < n_kv) {
-                    ok = mbar_wait(v_empty, j & 1, abort_flag, p.status, ST_TIMEOUT_EMPTY, 16);
+                    ok = mbar_wait_warp(v_empty, j & 1, abort_flag, p.status, ST_TIMEOUT_EMPTY, 16);
                     if (!ok) break;
-                    mbar_arrive_expect_tx(v_full, C::V);
-                    load_boxes<DVB>(sV, &tmV, v_full, hk, (j + 1) * kT, b);
+                    if (elect_one()) { mbar_arrive_expect_tx(v_full, C::V); }
+                    if (elect_one()) { load_boxes<DVB>(sV, &tmV, v_full, hk, (j + 1) * kT, b); }
                 }
                 if (j + 2 < n_kv) {
-                    ok = mbar_wait(k_empty0 + 8 * s, (j >> 1) & 1, abort_flag, p.status, ST_TIMEOUT_EMPTY, 14);
+                    ok = mbar_wait_warp(k_empty0 + 8 * s, (j >> 1) & 1, abort_flag, p.status, ST_TIMEOUT_EMPTY, 14);
                     if (!ok) break;
-                    mbar_arrive_expect_tx(k_full0 + 8 * s, C::QK);
-                    load_boxes2<DKB>(sK0 + s * C::QK, &tmK, &tmK2, p.k1_blocks, k_full0 + 8 * s, hk, 0, (j + 2) * kT, b);
+                    if (elect_one()) { mbar_arrive_expect_tx(k_full0 + 8 * s, C::QK); }
+                    if (elect_one()) { load_boxes2<DKB>(sK0 + s * C::QK, &tmK, &tmK2, p.k1_blocks, k_full0 + 8 * s, hk, 0, (j + 2) * kT, b); }
                 }
             }
         }

@@ -136,6 +136,12 @@ __device__ __forceinline__ bool mbar_wait_lean(uint32_t bar, uint32_t parity, vo
     return mbar_wait_slow(bar, parity, abort_flag, st, code, role);
 }
 
+// The lean wait by all lanes of a warp, with one answer for all.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile uint32_t* abort_flag, StatusWord* st,
+                                               uint32_t code, uint32_t role) {
+    return __all_sync(0xFFFFFFFFu, mbar_wait_lean(bar, parity, abort_flag, st, code, role));
+}
+
 // ---------------------------------------------------------------------------
 // proxies and fences
 // ---------------------------------------------------------------------------
