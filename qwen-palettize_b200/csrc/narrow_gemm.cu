@@ -13,7 +13,8 @@
 //             Shared memory and TMEM are kept to half of an SM's, so that two CTAs share one and hide each other's start and end.
 //   turned    (transposed) W is an activation matrix of any number of rows and x the few rows of a LoRA factor, t = s x A^T and dt = s dY B: the
 //             same launch with y stored [row of W][row of x], x from [M, K] or (x_mn) from [K, M].
-//             Rank 32, 1000 rows: K = 9728 33 -> 13 us, 2560 rows of B 12 -> 8 us; rank 16, 4096 rows: 9728 33 / 35 -> 24 us.
+//             Rank 32, 1000 rows: K = 9728 33 -> 12 us, 2560 rows of B 12 -> 8 us; rank 16, 4096 rows: 9728 33 / 35 -> 20 us; 16384 rows, where the rows
+//             alone fill the chip, 68 / 21 -> 79 / 23: the price of a split that does not depend on the rows.
 //   extra     an optional block of up to 64 more reduction elements (the LoRA up-projection: t [M, r] against B [N, r]).
 //
 // Accumulating into the tile the previous MMA still writes costs a TMEM round trip, so the four MMAs of a block go to several accumulators,
@@ -458,7 +459,9 @@ int launch_narrow_gemm(const NarrowArgs& a, cudaStream_t stream) {
         if ((rc = make_tmap_bf16(&tm[2], a.x2, a.M, a.r2, a.ldx2, 64, (uint32_t)p.npad))) return rc;
         if ((rc = make_tmap_bf16(&tm[3], a.w2, a.mat[0].N, a.r2, a.ldw2, 64, 128))) return rc;
     }
-    const int ranks = cluster_size(tiles, p.n_blocks, seq_sm_count(), 12);
+    // Transposed: by the reduction alone, so that a row's result does not depend on how many rows there are (a step over all tokens and the sum of
+    // steps over parts of them then agree); eight to twenty blocks per CTA.
+    const int ranks = a.transposed ? (p.n_blocks >= 64 ? 8 : p.n_blocks >= 32 ? 4 : p.n_blocks >= 16 ? 2 : 1) : cluster_size(tiles, p.n_blocks, seq_sm_count(), 12);
     return lut ? launch_ng<true>(p, tiles, ranks, tm, stream) : launch_ng<false>(p, tiles, ranks, tm, stream);
 }
 

@@ -86,3 +86,13 @@ def test_lora_factors(M, K, rank):
     w = ops.PackedWeight(ops.pack_indices(torch.zeros(64, K, dtype=torch.int8, device="cuda"), n_major=True), torch.zeros(64, 4, device="cuda", dtype=torch.bfloat16), 64, K, 1, K)
     t = ops.hard_forward(w, x, (a, rnd(64, rank), 0.5))[1]
     check(t, 0.5 * x.double() @ a.double().T, 0.5 * x.double().abs() @ a.double().abs().T, K)
+
+
+@pytest.mark.parametrize("K,rank", [(64, 8), (1088, 16), (2560, 32), (9728, 64)])
+def test_lora_rows_do_not_depend_on_their_number(K, rank):
+    g = torch.Generator(device="cuda").manual_seed(K)
+    x, b = torch.randn(20000, K, generator=g, device="cuda").bfloat16(), torch.randn(K, rank, generator=g, device="cuda").bfloat16()
+    a = torch.zeros(rank, K, device="cuda", dtype=torch.bfloat16)
+    t = ops.lora_dt((a, b, 1.0), x)
+    for lo, hi in ((0, 1), (100, 1100), (1100, 9000)):
+        assert torch.equal(ops.lora_dt((a, b, 1.0), x[lo:hi]), t[lo:hi])
