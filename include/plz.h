@@ -148,12 +148,16 @@ int32_t plz_hard_fwd_smallm(const plz_weight_t* w, const void* x, int64_t ldx, i
  * the palette grouping. A decode step is bound by launch latency, not bandwidth, at 7 MB per Linear. */
 int32_t plz_hard_fwd_smallm_multi(const plz_weight_t* const* ws, int32_t count, const void* x, int64_t ldx, int32_t M,
                                   void* const* ys, const int64_t* ldys, void* stream);
-/* on = 1: small-M launches (M <= 16) carry the programmatic-stream-serialization attribute, so a launch may start while the
+/* on = 1: the launches of a token step carry the programmatic-stream-serialization attribute, so a launch may start while the
  * previous kernel of the stream is still running: it issues the loads of its weights and builds its tables at once, and
- * waits for the previous kernel to finish (griddepcontrol.wait) only before it reads x or writes y. This hides the
- * launch latency between the Linears of a decode step. Only valid when the kernel that precedes a small-M call in its
- * stream does not write that call's packed indices or palettes (true in inference; not right after plz_soft_select or
- * plz_pack_indices). Process-wide, default 0. */
+ * waits for the previous kernel to finish (griddepcontrol.wait) only before it reads activations or writes results. This hides the
+ * launch latency between the kernels of a decode step. Read ahead of that wait, and so not to be written by the kernels right before
+ * the call in its stream (true in inference; not right after plz_soft_select or plz_pack_indices):
+ *   plz_hard_fwd_smallm, plz_hard_fwd_smallm_multi, plz_decode_hidden: packed indices and palettes;
+ *   plz_seq_linear with up to 128 rows and plz_head_linear: the matrix w;
+ *   plz_seq_embed, plz_seq_stream, plz_seq_rows_norm: norm weights and add_vec.
+ * All other entry points (plz_hard_fwd*, plz_dense_fwd, the backward ones) read nothing ahead, whatever their row count.
+ * Process-wide, default 0. */
 int32_t plz_set_smallm_overlap(int32_t on);
 
 /* One pass over the index logits: packed hard indices (argmax over the plain logits, first maximum

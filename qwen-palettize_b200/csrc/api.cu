@@ -1183,7 +1183,7 @@ int decode_linears(const plz_decode_linear_t* const* ws, int count, const void* 
     }
     if (alike && count > 1) {
         NarrowArgs n = {};
-        n.M = M; n.K = w[0].K; n.x = x; n.ldx = ldx; n.count = count; n.gs_n = w[0].gs_n; n.gs_k = w[0].gs_k; n.alpha = 1.0f;
+        n.M = M; n.K = w[0].K; n.x = x; n.ldx = ldx; n.count = count; n.gs_n = w[0].gs_n; n.gs_k = w[0].gs_k; n.alpha = 1.0f; n.early = 1;
         for (int i = 0; i < count; ++i) {
             n.mat[i].N = w[i].N; n.mat[i].packed = w[i].packed; n.mat[i].pitch = w[i].packed_pitch; n.mat[i].palette = w[i].palette;
             n.mat[i].y = ys[i]; n.mat[i].ldy = ldys[i];

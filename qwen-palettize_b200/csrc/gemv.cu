@@ -128,7 +128,7 @@ int launch_lut_gemv(const GemvArgs& a, cudaStream_t stream) {
     n.M = a.M; n.K = a.K; n.x = a.x; n.ldx = a.ldx; n.count = 1;
     n.mat[0].N = a.N; n.mat[0].packed = a.packed; n.mat[0].pitch = a.packed_pitch; n.mat[0].palette = a.palette;
     n.mat[0].y = a.out; n.mat[0].ldy = a.ld_out;
-    n.gs_n = a.gs_n; n.gs_k = a.gs_k; n.alpha = 1.0f;
+    n.gs_n = a.gs_n; n.gs_k = a.gs_k; n.alpha = 1.0f; n.early = 1;
     const int rc = launch_narrow_gemm(n, stream);
     if (rc == PLZ_ERR_UNSUPPORTED) { set_last_error("small-M forward: x rows must be multiples of 16 bytes, 16-byte aligned"); return PLZ_ERR_BAD_ALIGN; }
     return rc;

@@ -674,7 +674,7 @@ int launch_lut_gemm(const LutGemmArgs& a, cudaStream_t stream) {
         n.r2 = a.r2; n.x2 = a.A2; n.ldx2 = a.lda2; n.w2 = a.B2; n.ldw2 = a.ldb2;
         n.bias = a.fuse == 2 || a.fuse == 3 ? a.bias : nullptr;
         n.act = a.fuse == 4 ? 2 : a.fuse == 3 ? a.act : 0;
-        n.alpha = a.alpha;
+        n.alpha = a.alpha; n.early = a.early;
         const int rc = launch_narrow_gemm(n, stream);
         if (rc != PLZ_ERR_UNSUPPORTED) return rc;
     }

@@ -6,7 +6,7 @@
 //             leave most SMs idle (2560 rows are 20 tiles). Each CTA leaves its partial tile in its own shared memory and every CTA of the
 //             cluster adds up its share of the outputs over distributed shared memory, in rank order: no workspace, no atomics, the same
 //             bits on every run.
-//   operands  dense bf16 W by TMA (requested before the wait on the previous kernel of the stream), or packed 2-bit indices: a decode
+//   operands  dense bf16 W by TMA (requested before the wait on the previous kernel of the stream, for callers whose weights are constant), or packed 2-bit indices: a decode
 //             thread is one weight row, fetches the 16 bytes of a block of 64 columns several blocks ahead and writes the decoded row to
 //             TMEM, from where it is the A operand (lane = row: no shared memory, no swizzle, no proxy fence in between). x by TMA into a
 //             ring of its own, since TMEM has room for a few blocks of W only. A single issuing lane took 0.6 us a block (see there).
@@ -388,7 +388,7 @@ int cluster_size(int tiles, int blocks, int sms, int fixed) {
 }
 
 template <bool LUT>
-int launch_ng(const NarrowParams& p, int tiles, int ranks, const CUtensorMap (&tm)[4], cudaStream_t stream) {
+int launch_ng(const NarrowParams& p, int tiles, int ranks, bool early, const CUtensorMap (&tm)[4], cudaStream_t stream) {
     auto kern = narrow_gemm_kernel<LUT>;
     constexpr uint32_t smem = kNgRingBytes<LUT> + kNgBarBytes + 1024;
     static bool attr_set[64] = {};
@@ -405,7 +405,7 @@ int launch_ng(const NarrowParams& p, int tiles, int ranks, const CUtensorMap (&t
     attr[0].val.clusterDim.x = (unsigned)ranks; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[1].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr; cfg.numAttrs = g_smallm_overlap && !p.transposed ? 2 : 1;   // transposed: W is what the previous kernel wrote
+    cfg.attrs = attr; cfg.numAttrs = g_smallm_overlap && early ? 2 : 1;   // else W may be what the previous kernel writes: it is read ahead of the wait
     PLZ_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kern, tm[0], tm[1], tm[2], tm[3], p));
     ++g_launch_count;
     return PLZ_OK;
@@ -462,7 +462,8 @@ int launch_narrow_gemm(const NarrowArgs& a, cudaStream_t stream) {
     // Transposed: by the reduction alone, so that a row's result does not depend on how many rows there are (a step over all tokens and the sum of
     // steps over parts of them then agree); eight to twenty blocks per CTA.
     const int ranks = a.transposed ? (p.n_blocks >= 64 ? 8 : p.n_blocks >= 32 ? 4 : p.n_blocks >= 16 ? 2 : 1) : cluster_size(tiles, p.n_blocks, seq_sm_count(), 12);
-    return lut ? launch_ng<true>(p, tiles, ranks, tm, stream) : launch_ng<false>(p, tiles, ranks, tm, stream);
+    const bool early = a.early && !a.transposed;
+    return lut ? launch_ng<true>(p, tiles, ranks, early, tm, stream) : launch_ng<false>(p, tiles, ranks, early, tm, stream);
 }
 
 }  // namespace plz

@@ -27,6 +27,7 @@ struct LutGemmArgs {
     const void* bias;  // fuse == 2 or 3: optional bf16 [J], added in fp32 before the bf16 store
     int act;           // fuse == 3 (dense B, no LoRA block): 1 = square of relu after the bias
     int sm_limit;  // > 0: use at most this many CTAs (tests of the multi-tile schedule)
+    int early;     // NarrowArgs::early, where that kernel takes the call
     void* prof;  // optional device buffer of cycle counters, 8 x uint64 per CTA (diagnostics)
 };
 int launch_lut_gemm(const LutGemmArgs& a, cudaStream_t stream);
@@ -45,6 +46,7 @@ struct NarrowArgs {
     int M, K;
     const void* x; long long ldx;     // bf16 [M, K], or [K, M] with x_mn
     int x_mn, transposed;             // transposed: y [N, M]; W may be any previous kernel's output, any N
+    int early;                        // W, palettes and w2 are constant: with g_smallm_overlap they are read before the previous kernel has finished
     int count;                        // matrices sharing x (dense: 1)
     struct Mat {
         int N;

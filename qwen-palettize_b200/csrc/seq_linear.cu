@@ -321,7 +321,7 @@ int launch_seq_linear(int dtype, const void* x, long long ldx, int M, int K, con
         NarrowArgs n = {};
         n.M = M; n.K = K; n.x = x; n.ldx = ldx; n.count = 1;
         n.mat[0].N = N; n.mat[0].w = w; n.mat[0].ldw = ldw; n.mat[0].y = y; n.mat[0].ldy = ldy;
-        n.bias = bias; n.act = act; n.y_f32 = y_f32; n.alpha = 1.0f;
+        n.bias = bias; n.act = act; n.y_f32 = y_f32; n.alpha = 1.0f; n.early = 1;
         const int rc = launch_narrow_gemm(n, stream);
         if (rc != PLZ_ERR_UNSUPPORTED) return rc;
     }
@@ -336,7 +336,7 @@ int launch_seq_linear(int dtype, const void* x, long long ldx, int M, int K, con
         g.bmode = B_TMA_K; g.M = M; g.J = N; g.R = K;
         g.A = x; g.lda = ldx; g.Bdense = w; g.ldb = ldw;
         g.bias = bias; g.act = act; g.fuse = act == ACT_GLU_GELU ? 4 : ((bias || act) ? 3 : 0);
-        g.out = y; g.ld_out = ldy; g.alpha = 1.0f;
+        g.out = y; g.ld_out = ldy; g.alpha = 1.0f; g.early = 1;
         return launch_lut_gemm(g, stream);
     }
     if (dtype == 1) return launch_tile<float, float>(p, 1, stream);
