@@ -170,26 +170,18 @@ narrow_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
     const uint32_t tmem_w = tmem_base + (uint32_t)(p.n_acc * p.npad);      // LUT: 32 columns per stage
     pdl_launch_dependents();
 
+    // every wait below that x holds up starts after the previous kernel of the stream has finished: its time is not the wait's
+    int issued = pre;                      // stages the producing thread has filled
     if (warp == 0) {
         if (lane == 0) {
             pdl_wait();
             for (int it = 0; it < pre; ++it) load_x(it, it);
-            bool ok = true;
-            int issued = pre;
             for (int it = pre; it < nb; ++it) {
                 const int s = it % p.stages;
-                ok = mbar_wait(empty(s), ((it / p.stages) & 1) ^ 1u, abort_flag, p.status, ST_TIMEOUT_EMPTY, 0);
-                if (!ok) break;
+                if (!mbar_wait(empty(s), ((it / p.stages) & 1) ^ 1u, abort_flag, p.status, ST_TIMEOUT_EMPTY, 0)) break;
                 load_w(it, s);
                 load_x(it, s);
                 issued = it + 1;
-            }
-            if (!ok) {
-                // copies in flight get a bounded chance to land before the CTA exits
-                const uint64_t t0 = globaltimer_ns();
-                for (int it = issued > p.stages ? issued - p.stages : 0; it < issued; ++it)
-                    while (!mbar_try_wait(full(it % p.stages), (it / p.stages) & 1))
-                        if (globaltimer_ns() - t0 > 100000000ull) { report(p.status, ST_TIMEOUT_DRAIN, 0); break; }
             }
         }
     } else if (warp == 1) {
@@ -205,6 +197,7 @@ narrow_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
         bool ok = true;
         int s = 0, iw = 0;
         uint32_t ph = 0, phw = 0, lo = lo0;
+        pdl_wait();
         for (int it = 0; it < nb; ++it) {
             ok = mbar_wait(full(s), ph, abort_flag, p.status, ST_TIMEOUT_FULL, 1);
             if (LUT && ok) ok = mbar_wait(full_w(iw), phw, abort_flag, p.status, ST_TIMEOUT_FULL, 1);
@@ -247,6 +240,7 @@ narrow_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
                     const int it = it0 + 2 * j;
                     if (it >= nb || !ok) continue;
                     const int s = it % p.w_stages;       // an even number of blocks: a group always writes the same ones
+                    if (it >= p.w_stages) pdl_wait();
                     ok = mbar_wait(empty_w(s), ((it / p.w_stages) & 1) ^ 1u, abort_flag, p.status, ST_TIMEOUT_EMPTY, 3);
                     if (!ok) continue;
                     if (it < nw) {
@@ -269,6 +263,7 @@ narrow_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
         // ---------------------------------------------------------- this CTA's partial tile in the ring's space: [token][weight row], transposed
         // [weight row][npad tokens]
         if (warp < 6) {
+            pdl_wait();
             if (ok) ok = mbar_wait(acc_full, 0, abort_flag, p.status, ST_TIMEOUT_ACCUM, 4);
             if (ok) {
                 tc_fence_after_sync();

@@ -83,3 +83,17 @@ def test_matrix_of_the_kernel_before(M):
         got = run()
     P.device_status()
     assert all(torch.equal(p, q) for p, q in zip(want, got))
+
+
+def test_slow_kernel_before():
+    """A launch that starts early does not count the time of a kernel ahead of it, here one block that runs for two and a half seconds, against its
+    bounded waits (2 s)."""
+    slow = torch.ones(64, 40 << 20, device="cuda")
+    g = torch.Generator(device="cuda").manual_seed(6)
+    x, W = _rnd(g, 32, K), _rnd(g, 4096, K, scale=0.02)
+    want = S.linear(x, W)
+    with overlap():
+        S.linear(slow, slow)
+        got = S.linear(x, W)
+    P.device_status()
+    assert torch.equal(want, got)
