@@ -95,6 +95,7 @@ dense_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
         m0 = (band * kDpBand + in % rows) * 256;
     };
 
+    int issued = 0;        // stages the producing thread has filled
     if (warp == 0) {
         // ------------------------------------------------------------- TMA producer (one per CTA)
         if (lane == 0) {
@@ -134,6 +135,7 @@ dense_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
                             tma_load_2d_pair(sB, &tmB2, bar, 0, jr);
                         }
                     }
+                    ++issued;
                     if (++s == kDpStages) { s = 0; ph ^= 1u; }
                 }
             }
@@ -253,6 +255,13 @@ dense_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
     // neither CTA may leave while its partner can still touch its shared or tensor memory
     tc_fence_before_sync();
     __syncthreads();
+    if (threadIdx.x == 0 && rank == 0 && *abort_flag) {
+        // somebody gave up: the copies of both CTAs, which arrive on this CTA's barriers, get a bounded chance to land
+        const uint64_t t0 = globaltimer_ns();
+        for (int it = issued > kDpStages ? issued - kDpStages : 0; it < issued; ++it)
+            while (!mbar_try_wait(full(it % kDpStages), (it / kDpStages) & 1))
+                if (globaltimer_ns() - t0 > 100000000ull) { report(p.status, ST_TIMEOUT_DRAIN, 0); break; }
+    }
     cluster_sync_all();
     if (warp == 1) {
         tc_fence_after_sync();

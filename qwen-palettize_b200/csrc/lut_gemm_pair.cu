@@ -137,6 +137,7 @@ lut_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
         m0 = (tile / p.tiles_j) * 256;
     };
 
+    int issued = 0;        // stages the producing thread has filled
     if (warp == 0) {
         // ------------------------------------------------------------- TMA producer (one per CTA)
         if (lane == 0) {
@@ -169,6 +170,7 @@ lut_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
                             tma_load_2d_pair(sB, &tmB2, lead_full(s), 0, jr);
                         }
                     }
+                    ++issued;
                     if (++s == kStages) { s = 0; ph ^= 1u; }
                 }
             }
@@ -417,6 +419,13 @@ lut_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
     // barrier arrivals) or its tensor memory.
     tc_fence_before_sync();
     __syncthreads();
+    if (threadIdx.x == 0 && rank == 0 && *abort_flag) {
+        // somebody gave up: the copies of both CTAs, which arrive on this CTA's barriers, get a bounded chance to land
+        const uint64_t t0 = globaltimer_ns();
+        for (int it = issued > kStages ? issued - kStages : 0; it < issued; ++it)
+            while (!mbar_try_wait(full(it % kStages), (it / kStages) & 1))
+                if (globaltimer_ns() - t0 > 100000000ull) { report(p.status, ST_TIMEOUT_DRAIN, 0); break; }
+    }
     cluster_sync_all();
     if (warp == 1) {
         tc_fence_after_sync();

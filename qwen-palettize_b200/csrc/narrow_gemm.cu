@@ -293,6 +293,13 @@ narrow_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
     tc_fence_before_sync();
     __syncwarp();
     cluster_sync_all();        // every CTA's partial tile is complete and visible
+    if (threadIdx.x == 0 && *abort_flag) {
+        // somebody gave up: copies in flight get a bounded chance to land before the CTA exits
+        const uint64_t t0 = globaltimer_ns();
+        for (int it = issued > p.stages ? issued - p.stages : 0; it < issued; ++it)
+            while (!mbar_try_wait(full(it % p.stages), (it / p.stages) & 1))
+                if (globaltimer_ns() - t0 > 100000000ull) { report(p.status, ST_TIMEOUT_DRAIN, 0); break; }
+    }
     pdl_wait();                // outputs may be what the previous kernel still reads
     {
         uint32_t from[8];
