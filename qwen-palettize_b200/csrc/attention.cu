@@ -301,6 +301,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 // ---------------------------------------------------------------------------------------------------------------------
 // backward pre-pass: dsum[b, h, s] = sum_d dO * O   (one warp per (token, head) row)
 // ---------------------------------------------------------------------------------------------------------------------
+template <bool O16>      // o aligned to 16 bytes; else to 8
 __global__ void __launch_bounds__(256)
 attn_dsum_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ d_o, long long ld, int B, int S, int Hq,
                  float* __restrict__ dsum) {
@@ -315,7 +316,11 @@ attn_dsum_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __res
         a[i] = g[i] = make_uint4(0u, 0u, 0u, 0u);
         if (row < rows) {
             const long long at = row / Hq * ld + row % Hq * kD + l * 8;
-            a[i] = __ldcs(reinterpret_cast<const uint4*>(o + at));
+            if (O16) a[i] = __ldcs(reinterpret_cast<const uint4*>(o + at));
+            else {
+                const uint2 lo = __ldcs(reinterpret_cast<const uint2*>(o + at)), hi = __ldcs(reinterpret_cast<const uint2*>(o + at + 4));
+                a[i] = make_uint4(lo.x, lo.y, hi.x, hi.y);
+            }
             g[i] = *reinterpret_cast<const uint4*>(d_o + at);
         }
     }
@@ -654,6 +659,7 @@ int launch_attn_bwd(const AttnArgs& a, cudaStream_t stream) {
     int rc = check_attn(a);
     if (rc) return rc;
     if (!a.q || !a.k || !a.v || !a.o || !a.d_o || !a.dq || !a.dk || !a.dv || !a.lse || !a.dsum) { set_last_error("attention backward: null pointer"); return PLZ_ERR_NULL; }
+    if ((uintptr_t)a.o & 7) { set_last_error("attention backward: o must be 8-byte aligned"); return PLZ_ERR_BAD_ALIGN; }
     const uint64_t rows = (uint64_t)a.B * a.S;
     CUtensorMap tmQ, tmK, tmV, tmdO, tmdQ, tmdK, tmdV;
     if ((rc = make_tmap_bf16(&tmQ, a.q, rows, (uint64_t)a.Hq * kD, a.ldq, 64, kT))) return rc;
@@ -672,8 +678,8 @@ int launch_attn_bwd(const AttnArgs& a, cudaStream_t stream) {
         once = true;
     }
     const long long n_rows = (long long)a.B * a.S * a.Hq;
-    attn_dsum_kernel<<<(unsigned)((n_rows + 63) / 64), 256, 0, stream>>>((const __nv_bfloat16*)a.o, (const __nv_bfloat16*)a.d_o, a.ldo, a.B, a.S,
-                                                                       a.Hq, a.dsum);
+    const auto dsum = ((uintptr_t)a.o & 15) ? attn_dsum_kernel<false> : attn_dsum_kernel<true>;   // o passes no tensor map that would refuse it
+    dsum<<<(unsigned)((n_rows + 63) / 64), 256, 0, stream>>>((const __nv_bfloat16*)a.o, (const __nv_bfloat16*)a.d_o, a.ldo, a.B, a.S, a.Hq, a.dsum);
     PLZ_LAUNCH_CHECK();
     attn_bwd_dq_kernel<<<dim3(a.S / kT, a.Hq, a.B), kBwdThreads, kDqSmem, stream>>>(tmQ, tmK, tmV, tmdO, tmdQ, p);
     PLZ_LAUNCH_CHECK();

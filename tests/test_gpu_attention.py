@@ -74,3 +74,18 @@ def test_attention_argument_checks():
     k = torch.zeros(128, 2 * 128, dtype=torch.bfloat16, device="cuda")
     with pytest.raises(P.PlzError):
         ops.attention_forward(q, k, k, 1, 128, 3, 2)            # 3 query heads over 2 kv heads
+
+
+def test_backward_with_o_at_half_the_alignment():
+    """o is read by its row sums alone: 16 bytes at a time where it allows that, 8 where it starts at an odd multiple of 8 bytes, with the same results."""
+    import plz_ops as ops
+    B, S, H = 1, 256, 3
+    g = torch.Generator().manual_seed(11)
+    q, k, v, do = (torch.randn(B * S, H * 128, generator=g).to(torch.bfloat16).cuda() for _ in range(4))
+    o, lse = ops.attention_forward(q, k, v, B, S, H, H)
+    want = ops.attention_backward(q, k, v, o, do, lse, B, S, H, H)
+    for shift in (4, 8):                                      # elements
+        moved = torch.empty(o.numel() + 8, dtype=o.dtype, device="cuda")[shift:shift + o.numel()].view_as(o).copy_(o)
+        got = ops.attention_backward(q, k, v, moved, do, lse, B, S, H, H)
+        check_status()
+        assert all(torch.equal(a, b) for a, b in zip(want, got))
