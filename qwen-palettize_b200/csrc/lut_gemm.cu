@@ -654,6 +654,9 @@ int launch_lut_gemm(const LutGemmArgs& a, cudaStream_t stream) {
     if (a.J % 8) { set_last_error("lut_gemm: output width %d is not a multiple of 8", a.J); return PLZ_ERR_BAD_SHAPE; }
     if (a.r2 < 0 || a.r2 > 64 || (a.r2 % 8)) { set_last_error("lut_gemm: extra rank %d must be a multiple of 8 in [0, 64]", a.r2); return PLZ_ERR_BAD_SHAPE; }
     if (((uintptr_t)a.out & 15) || ((a.ld_out * 2) & 15)) { set_last_error("lut_gemm: output must be 16-byte aligned"); return PLZ_ERR_BAD_ALIGN; }
+    if (!a.out) { set_last_error("null matrix pointer"); return PLZ_ERR_NULL; }
+    const int out_cols = a.fuse == 1 || a.fuse == 4 ? a.J / 2 : a.J;
+    if (a.ld_out < out_cols) { set_last_error("row pitch %lld < columns %d", a.ld_out, out_cols); return PLZ_ERR_BAD_SHAPE; }
     const bool decode = (a.bmode == B_DECODE_K || a.bmode == B_DECODE_MN);
     if (decode) {
         if (!a.packed || !a.palette) { set_last_error("lut_gemm: null packed weights"); return PLZ_ERR_NULL; }

@@ -47,6 +47,10 @@ def test_argument_validation_without_gpu(built_lib):
     assert lib.plz_hard_fwd(C.byref(w), 0x10, 256, 8, C.byref(lo), 0x30, 0x20, 256, None) == 1
     lo = P.Lora(16, 1.0, 0x10, 256, 0x20, 16)
     assert lib.plz_hard_fwd(C.byref(w), 0x10, 256, 8, C.byref(lo), None, 0x20, 256, None) == 5  # no workspace
+    # rows of the result that overlap, at few rows and at many, from packed and dense weights
+    for M in (8, 100, 300):
+        assert lib.plz_hard_fwd(C.byref(w), 0x1000, 256, M, None, None, 0x2000, 248, None) == 1 and b"pitch" in lib.plz_last_error()
+        assert lib.plz_dense_fwd(0x1000, 256, 256, 256, 0x1000, 256, M, None, None, 0x2000, 248, None) == 1
     # attention backward: o must be aligned to 8 bytes (its row sums read it so)
     ptr = [0x1000] * 16
     assert lib.plz_attn_bwd(ptr[0], 128, ptr[1], 128, ptr[2], 128, 0x1004, ptr[3], 128, ptr[4], 1, 128, 1, 1, 128, 1.0, *ptr[5:9], None) == 2
