@@ -1203,8 +1203,10 @@ int64_t plz_decode_ws_bytes(int32_t B, int32_t T, int32_t hidden, int32_t interm
 
 int32_t plz_decode_hidden(const plz_decode_t* a, const plz_decode_layer_t* layers, void* stream) {
     if (!a || !layers) { set_last_error("null pointer"); return PLZ_ERR_NULL; }
-    if (a->B < 0 || a->B > 0x7FFFFFFF || a->T <= 0 || a->T > 0x7FFFFFFF || a->n_layers < 1 || a->hidden <= 0 || a->intermediate <= 0 || a->n_heads <= 0 ||
-        a->n_kv_heads <= 0 || a->head_dim != 128) {
+    const int64_t most = 0x7FFFFFFF;
+    if (a->B < 0 || a->B > 64) { set_last_error("decode_hidden handles 0 <= B <= 64 sequences (B=%lld)", (long long)a->B); return PLZ_ERR_BAD_SHAPE; }
+    if (a->T <= 0 || a->T > most || a->n_layers < 1 || a->hidden <= 0 || a->hidden > most || a->intermediate <= 0 || a->intermediate > most || a->n_heads <= 0 ||
+        a->n_heads > most / 128 || a->n_kv_heads <= 0 || a->n_kv_heads > most / 128 || a->head_dim != 128) {
         set_last_error("decode_hidden: bad shape"); return PLZ_ERR_BAD_SHAPE;
     }
     if (a->B == 0) return PLZ_OK;
@@ -1215,11 +1217,14 @@ int32_t plz_decode_hidden(const plz_decode_t* a, const plz_decode_layer_t* layer
             L.q.K != a->hidden || L.k.K != a->hidden || L.v.K != a->hidden || L.o.K != qd || L.gate.K != a->hidden || L.up.K != a->hidden || L.down.K != a->intermediate) {
             set_last_error("decode_hidden: the Linears of layer %lld do not fit the model's sizes", (long long)li); return PLZ_ERR_BAD_SHAPE;
         }
+        for (const plz_decode_linear_t* w : {&L.q, &L.k, &L.v, &L.o, &L.gate, &L.up, &L.down})
+            if (w->gs_n > most || w->gs_k > most) { set_last_error("decode_hidden: bad palette groups"); return PLZ_ERR_BAD_SHAPE; }
+        if (!L.k_cache || !L.v_cache) { set_last_error("decode_hidden: null cache pointer (layer %lld)", (long long)li); return PLZ_ERR_NULL; }
     }
     const int32_t B = (int32_t)a->B, T = (int32_t)a->T, H = (int32_t)a->hidden, F = (int32_t)a->intermediate, Hq = (int32_t)a->n_heads, Hkv = (int32_t)a->n_kv_heads;
     const float eps = (float)a->eps;
     const DecodeScratch d = decode_scratch(B, T, H, F, Hq, Hkv);
-    if (!a->ws || !a->h || !a->h1) { set_last_error("null pointer"); return PLZ_ERR_NULL; }
+    if (!a->ws || !a->h || !a->h1 || !a->embed || !a->ids || !a->cos_row || !a->sin_row) { set_last_error("null pointer"); return PLZ_ERR_NULL; }
     if (a->ws_bytes < d.total() || ((uintptr_t)a->ws & 15)) { set_last_error("decode_hidden: %lld bytes of 16-byte aligned scratch needed", (long long)d.total()); return PLZ_ERR_WORKSPACE; }
     uint8_t* at = (uint8_t*)a->ws;
     auto take = [&](int64_t cols) { uint8_t* p = at; at += d.bytes(cols); return (void*)p; };
@@ -1233,7 +1238,6 @@ int32_t plz_decode_hidden(const plz_decode_t* a, const plz_decode_layer_t* layer
         const plz_decode_layer_t& L = layers[li];
         const bool last = li + 1 == a->n_layers;
         __nv_bfloat16 *kc = (__nv_bfloat16*)L.k_cache, *vc = (__nv_bfloat16*)L.v_cache;
-        if (!kc || !vc) { set_last_error("null pointer"); return PLZ_ERR_NULL; }
         __nv_bfloat16 *k_new = kc + (int64_t)(T - 1) * a->tok_stride, *v_new = vc + (int64_t)(T - 1) * a->tok_stride;
         const plz_decode_linear_t *qkv[3] = {&L.q, &L.k, &L.v}, *gu[2] = {&L.gate, &L.up}, *ow = &L.o, *dw = &L.down;
         void *qkv_out[3] = {q_raw, k_raw, v_new}, *gu_out[2] = {gate, up};

@@ -563,7 +563,15 @@ def decode_hidden(ids: torch.Tensor, embed: torch.Tensor, layers, names, norms, 
     assert embed.dtype == torch.bfloat16 and embed.dim() == 2 and embed.stride(1) == 1 and ids.dtype == torch.int64
     ids = ids.reshape(-1).contiguous()
     B, hidden, dev = ids.numel(), embed.shape[1], embed.device
-    P._need_cuda(ids, embed, final_norm, cos, sin, k_cache, v_cache)
+    for t in (cos, sin):
+        assert t.dtype == torch.float32 and t.numel() == 64 and t.is_contiguous(), "cos / sin: 64 fp32 values of one position"
+
+    def vector(t, n):
+        assert t is None or (t.dtype == torch.bfloat16 and t.numel() == n and t.is_contiguous()), f"norm weights: bf16 [{n}]"
+        P._need_cuda(t)
+        return t.data_ptr() if t is not None else 0
+    last = vector(final_norm, hidden)
+    P._need_cuda(ids, embed, cos, sin, k_cache, v_cache)
     assert k_cache.dtype == v_cache.dtype == torch.bfloat16 and k_cache.shape == v_cache.shape and k_cache.stride() == v_cache.stride()
     n, st = len(layers), k_cache.stride()
     assert k_cache.dim() == 4 and k_cache.shape[0] >= n and k_cache.shape[1] == B and k_cache.shape[3] == n_kv_heads * 128 and st[3] == 1 and 0 < T <= k_cache.shape[2]
@@ -576,14 +584,14 @@ def decode_hidden(ids: torch.Tensor, embed: torch.Tensor, layers, names, norms, 
             assert packed.dtype == torch.uint8 and packed.dim() == 2 and packed.stride(1) == 1
             assert palette.dtype == torch.bfloat16 and palette.is_contiguous() and palette.numel() == (w.N // w.gs_n) * (w.K // w.gs_k) * 4, "palette size does not match the grouping"
             rows += (w.N, w.K, w.gs_n, w.gs_k, packed.data_ptr(), packed.stride(0), palette.data_ptr())
-        rows += [L[name].data_ptr() if L[name] is not None else 0 for name in norms]
+        rows += [vector(L[name], width) for name, width in zip(norms, (hidden, hidden, 128, 128))]
         rows += (k0 + 2 * i * st[0], v0 + 2 * i * st[0])
     lib = P.lib()
     out = torch.empty(2, B, hidden, dtype=torch.bfloat16, device=dev)
     nbytes = int(lib.plz_decode_ws_bytes(B, T, hidden, intermediate, n_heads, n_kv_heads))
     ws = torch.empty(nbytes, dtype=torch.uint8, device=dev)
     a = P.Decode(B, T, n, hidden, intermediate, n_heads, n_kv_heads, 128, st[1], st[2], embed.data_ptr(), embed.stride(0), embed.shape[0], ids.data_ptr(),
-                 cos.data_ptr(), sin.data_ptr(), final_norm.data_ptr() if final_norm is not None else None, out[0].data_ptr(), out[1].data_ptr(), ws.data_ptr(), nbytes, eps)
+                 cos.data_ptr(), sin.data_ptr(), last or None, out[0].data_ptr(), out[1].data_ptr(), ws.data_ptr(), nbytes, eps)
     P.check(lib.plz_decode_hidden(C.byref(a), (C.c_int64 * len(rows))(*rows), P.stream_ptr()), "plz_decode_hidden")
     return out[0], out[1]
 

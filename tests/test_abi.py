@@ -56,6 +56,38 @@ def test_argument_validation_without_gpu(built_lib):
     assert lib.plz_attn_bwd(ptr[0], 128, ptr[1], 128, ptr[2], 128, 0x1004, ptr[3], 128, ptr[4], 1, 128, 1, 1, 128, 1.0, *ptr[5:9], None) == 2
 
 
+def test_decode_step_is_checked_before_its_first_launch(built_lib):
+    import torch
+    import plz_native as P
+    import plz_ops as ops
+    lib, h, f = P.lib(), 256, 512
+    lin = lambda n, k: [n, k, 1, 256, 0x1000, k // 4, 0x2000]
+    layer = sum([lin(512, h), lin(128, h), lin(128, h), lin(h, 512), lin(f, h), lin(f, h), lin(h, f)], []) + [0x3000] * 6
+
+    def call(B=2, layers=(layer, layer), **kw):
+        rows = sum(layers, [])
+        a = dict(B=B, T=5, n_layers=len(layers), hidden=h, intermediate=f, n_heads=4, n_kv_heads=1, head_dim=128, batch_stride=1280, tok_stride=128, embed=0x4000, ld_embed=h, vocab=7,
+                 ids=0x5000, cos_row=0x6000, sin_row=0x7000, final_norm=0x8000, h=0x9000, h1=0xa000, ws=0xb000, ws_bytes=1 << 40, eps=1e-6)
+        return lib.plz_decode_hidden(C.byref(P.Decode(**{**a, **kw})), (C.c_int64 * len(rows))(*rows), None)
+    assert call(B=65) == 1 and b"64" in lib.plz_last_error()
+    assert call(layers=(layer, layer[:-1] + [0])) == 7 and b"cache" in lib.plz_last_error()      # of the second layer
+    assert call(layers=(layer[:2] + [1 << 32] + layer[3:], layer)) == 1
+    assert call(hidden=1 << 32) == 1 and call(n_heads=1 << 32) == 1
+    assert call(cos_row=None) == 7 and call(ids=None) == 7
+    assert call(B=0) == 0
+    # the binding: types and sizes of what it passes as bare pointers
+    bf, embed, cache = torch.bfloat16, torch.zeros(7, h, dtype=torch.bfloat16), torch.zeros(0, 2, 8, 128, dtype=torch.bfloat16)
+    tab, norm = torch.zeros(1, 64), torch.zeros(h, dtype=bf)
+
+    def bind(cos=tab, last=norm):
+        ops.decode_hidden(torch.zeros(2, dtype=torch.int64), embed, [], (), (), cache, cache, 1, last, cos, tab, 4, 1, f, 1e-6)
+    for kw in ({"cos": tab.double()}, {"cos": tab[:, :32]}, {"last": norm.float()}, {"last": norm[:8]}):
+        with pytest.raises(AssertionError):
+            bind(**kw)
+    with pytest.raises(P.PlzError):
+        bind()
+
+
 def test_ops_refuse_cpu_tensors(built_lib):
     import torch
     import fused_lut_linear_cuda as F
