@@ -138,7 +138,7 @@ static int lora_down(const plz_lora_t* l, const void* x, long long ldx, int M, i
     LutGemmArgs g = {};
     g.bmode = B_TMA_K; g.M = M; g.J = l->rank; g.R = K;
     g.A = x; g.lda = ldx; g.Bdense = l->A; g.ldb = l->lda;
-    g.out = t; g.ld_out = l->rank; g.alpha = l->scale;
+    g.out = t; g.ld_out = l->rank; g.alpha = l->scale; g.lora = 1;
     return launch_lut_gemm(g, s);
 }
 // dt = scale * dY B  (bf16 [M, rank]); reduction over N, B is [N, rank] -> MN-major operand
@@ -147,7 +147,7 @@ static int lora_up_bwd(const plz_lora_t* l, const void* dY, long long lddy, int 
     LutGemmArgs g = {};
     g.bmode = B_TMA_MN; g.M = M; g.J = l->rank; g.R = N;
     g.A = dY; g.lda = lddy; g.Bdense = l->B; g.ldb = l->ldb;
-    g.out = dt; g.ld_out = l->rank; g.alpha = l->scale;
+    g.out = dt; g.ld_out = l->rank; g.alpha = l->scale; g.lora = 1;
     return launch_lut_gemm(g, s);
 }
 

@@ -664,6 +664,17 @@ int launch_lut_gemm(const LutGemmArgs& a, cudaStream_t stream) {
         if ((uintptr_t)a.palette & 7) { set_last_error("lut_gemm: palette must be 8-byte aligned"); return PLZ_ERR_BAD_ALIGN; }
         if (a.gs_k % 64 || a.Wk % a.gs_k || a.Wk % 64) { set_last_error("lut_gemm: K group size %d must be a multiple of 64 dividing K=%d", a.gs_k, a.Wk); return PLZ_ERR_BAD_SHAPE; }
     }
+    // Outputs of at most 64 columns (the LoRA products x A^T and dY B): bound by streaming A. The turned kernels share a row tile among a cluster, or walk
+    // row tiles where those fill the chip. LoRA products go there at any number of rows, so that a row's result does not depend on that number.
+    if (!decode && a.J <= 64 && a.r2 == 0 && a.fuse == 0 && (a.lora || a.M > 128)) {
+        NarrowArgs n = {};
+        n.transposed = 1; n.x_mn = a.bmode == B_TMA_MN;
+        n.M = a.J; n.K = a.R; n.x = a.Bdense; n.ldx = a.ldb; n.count = 1;
+        n.mat[0].N = a.M; n.mat[0].w = a.A; n.mat[0].ldw = a.lda; n.mat[0].y = a.out; n.mat[0].ldy = a.ld_out; n.alpha = a.alpha;
+        int limit = a.sm_limit;
+        if (g_cta_limit > 0 && (limit <= 0 || g_cta_limit < limit)) limit = g_cta_limit;
+        return launch_turned_gemm(n, limit, stream);
+    }
     // Few rows: the swapped form with the reduction split over a cluster (narrow_gemm.cu). A 128 x 256 tile per CTA is as good only where the
     // tiles alone fill the chip (dense, wide outputs: 32768 x 2560 at 64 rows 31 against 36 us) or where the reduction is short and
     // the rows many (6144 x 1024 at 128 rows 11 / 13); else 64 rows of 9728 x 2560 / 2560 x 9728 / 1024 x 2560 take 20 / 58 / 18 us here
@@ -678,16 +689,6 @@ int launch_lut_gemm(const LutGemmArgs& a, cudaStream_t stream) {
         n.bias = a.fuse == 2 || a.fuse == 3 ? a.bias : nullptr;
         n.act = a.fuse == 4 ? 2 : a.fuse == 3 ? a.act : 0;
         n.alpha = a.alpha; n.early = a.early;
-        const int rc = launch_narrow_gemm(n, stream);
-        if (rc != PLZ_ERR_UNSUPPORTED) return rc;
-    }
-    // Outputs of at most 64 columns (the LoRA products x A^T and dY B): bound by streaming A, and 128 rows a CTA leave a launch of a few thousand
-    // rows with a few CTAs that stream one tile each. The narrow kernel turned round shares a tile among a cluster.
-    if (!decode && a.J <= 64 && a.r2 == 0 && a.fuse == 0 && a.sm_limit <= 0 && g_cta_limit <= 0) {
-        NarrowArgs n = {};
-        n.transposed = 1; n.x_mn = a.bmode == B_TMA_MN;
-        n.M = a.J; n.K = a.R; n.x = a.Bdense; n.ldx = a.ldb; n.count = 1;
-        n.mat[0].N = a.M; n.mat[0].w = a.A; n.mat[0].ldw = a.lda; n.mat[0].y = a.out; n.mat[0].ldy = a.ld_out; n.alpha = a.alpha;
         const int rc = launch_narrow_gemm(n, stream);
         if (rc != PLZ_ERR_UNSUPPORTED) return rc;
     }
@@ -715,10 +716,8 @@ int launch_lut_gemm(const LutGemmArgs& a, cudaStream_t stream) {
                 return big ? launch_t<2, B_TMA_K, false, 3>(a, stream) : launch_t<1, B_TMA_K, false, 3>(a, stream);
             }
             if (a.fuse == 4) return big ? launch_t<2, B_TMA_K, false, 4>(a, stream) : launch_t<1, B_TMA_K, false, 4>(a, stream);
-            if (narrow) return launch_t<1, B_TMA_K, true>(a, stream);
             return big ? launch_t<2, B_TMA_K, false>(a, stream) : launch_t<1, B_TMA_K, false>(a, stream);
         case B_TMA_MN:
-            if (narrow) return launch_t<1, B_TMA_MN, true>(a, stream);
             return big ? launch_t<2, B_TMA_MN, false>(a, stream) : launch_t<1, B_TMA_MN, false>(a, stream);
     }
     set_last_error("lut_gemm: unknown B mode %d", a.bmode);

@@ -12,9 +12,8 @@
 //             ring of its own, since TMEM has room for a few blocks of W only. A single issuing lane took 0.6 us a block (see there).
 //             Shared memory and TMEM are kept to half of an SM's, so that two CTAs share one and hide each other's start and end.
 //   turned    (transposed) W is an activation matrix of any number of rows and x the few rows of a LoRA factor, t = s x A^T and dt = s dY B: the
-//             same launch with y stored [row of W][row of x], x from [M, K] or (x_mn) from [K, M].
-//             Rank 32, 1000 rows: K = 9728 33 -> 12 us, 2560 rows of B 12 -> 8 us; rank 16, 4096 rows: 9728 33 / 35 -> 20 us; 16384 rows, where the rows
-//             alone fill the chip, 68 / 21 -> 79 / 23: the price of a split that does not depend on the rows.
+//             same launch with y stored [row of W][row of x], x from [M, K] or (x_mn) from [K, M]. Where the rows alone fill the chip a kernel of its
+//             own takes a row tile per CTA (turned_gemm_kernel).
 //   extra     an optional block of up to 64 more reduction elements (the LoRA up-projection: t [M, r] against B [N, r]).
 //
 // Accumulating into the tile the previous MMA still writes costs a TMEM round trip, so the four MMAs of a block go to several accumulators,
@@ -389,6 +388,10 @@ int cluster_size(int tiles, int blocks, int sms, int fixed) {
     return best;
 }
 
+// Parts of the reduction of a turned product: by the reduction alone, so that a row's result does not depend on how many rows there are (a step over
+// all tokens and the sum of steps over parts of them then agree); eight to twenty blocks per part.
+int turned_parts(int n_blocks) { return n_blocks >= 64 ? 8 : n_blocks >= 32 ? 4 : n_blocks >= 16 ? 2 : 1; }
+
 template <bool LUT>
 int launch_ng(const NarrowParams& p, int tiles, int ranks, bool early, const CUtensorMap (&tm)[4], cudaStream_t stream) {
     auto kern = narrow_gemm_kernel<LUT>;
@@ -461,11 +464,201 @@ int launch_narrow_gemm(const NarrowArgs& a, cudaStream_t stream) {
         if ((rc = make_tmap_bf16(&tm[2], a.x2, a.M, a.r2, a.ldx2, 64, (uint32_t)p.npad))) return rc;
         if ((rc = make_tmap_bf16(&tm[3], a.w2, a.mat[0].N, a.r2, a.ldw2, 64, 128))) return rc;
     }
-    // Transposed: by the reduction alone, so that a row's result does not depend on how many rows there are (a step over all tokens and the sum of
-    // steps over parts of them then agree); eight to twenty blocks per CTA.
-    const int ranks = a.transposed ? (p.n_blocks >= 64 ? 8 : p.n_blocks >= 32 ? 4 : p.n_blocks >= 16 ? 2 : 1) : cluster_size(tiles, p.n_blocks, seq_sm_count(), 12);
+    const int ranks = a.transposed ? turned_parts(p.n_blocks) : cluster_size(tiles, p.n_blocks, seq_sm_count(), 12);
     const bool early = a.early && !a.transposed;
     return lut ? launch_ng<true>(p, tiles, ranks, early, tm, stream) : launch_ng<false>(p, tiles, ranks, early, tm, stream);
+}
+
+namespace {
+// ---- turned round, a whole row tile per CTA ----------------------------------------------------------------------------------------------
+// Many row tiles, or a reduction of one part: no cluster. A CTA walks its tiles (grid: at most one CTA per SM, or the limit on CTAs) and of each the
+// parts of the reduction that the CTAs of a cluster would take; four output warps (thread = row) add up a part's accumulators and then the parts in
+// the same order, so that a row has the same bits either way. Two sets of accumulators, the next part's MMAs run under the sums of this one; the
+// ring takes the whole SM, with 16 KB of rows and the factor's tile (out of L2) per stage. Bound by streaming the rows: 16384 rows of 9728, rank 16, 62 -> 52 us
+// (6.1 TB/s) against clusters, rank 64 76 -> 53; of 2560 18 -> 14.5 and 23 -> 12.6; 1000 rows of 512, rank 64, 10.5 -> 5.1.
+constexpr int kTgThreads = 6 * 32;
+constexpr int kTgMaxStages = 11;
+constexpr uint32_t kTgRingBytes = 200 * 1024;
+struct TurnedParams {
+    int M, N, tiles, parts, n_blocks, x_mn, stages;
+    uint32_t x_bytes;
+    __nv_bfloat16* y; long long ldy;
+    float alpha;
+    StatusWord* status;
+};
+
+template <int NPAD>
+__global__ void __launch_bounds__(kTgThreads, 1)
+turned_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW, const TurnedParams p) {
+    constexpr int kAcc = 4;
+    extern __shared__ uint8_t smem_raw[];
+    const uint32_t raw = smem_u32(smem_raw);
+    const uint32_t base = (raw + 1023u) & ~1023u;
+    uint8_t* smem = smem_raw + (base - raw);
+    const uint32_t stage_bytes = kNgWBytes + p.x_bytes, bar = base + kTgRingBytes;
+    auto full = [&](int s) { return bar + 8u * s; };
+    auto empty = [&](int s) { return bar + 8u * (kTgMaxStages + s); };
+    auto acc_full = [&](int b) { return bar + 8u * (2 * kTgMaxStages + b); };
+    auto acc_empty = [&](int b) { return bar + 8u * (2 * kTgMaxStages + 2 + b); };
+    volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem + kTgRingBytes + 8 * (2 * kTgMaxStages + 4));
+    volatile uint32_t* abort_flag = tmem_slot + 1;
+    static_assert(8 * (2 * kTgMaxStages + 4) + 8 <= kNgBarBytes, "barriers");
+
+    const int warp = __shfl_sync(0xFFFFFFFFu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < kTgMaxStages; ++s) { mbar_init(full(s), 1); mbar_init(empty(s), 1); }
+        for (int b = 0; b < 2; ++b) { mbar_init(acc_full(b), 1); mbar_init(acc_empty(b), 4); }
+        *abort_flag = 0;
+        mbar_fence_init();
+        tma_prefetch_desc(&tmX);
+        tma_prefetch_desc(&tmW);
+    }
+    if (warp == 1) { tmem_alloc(smem_u32((const void*)tmem_slot), 2 * kAcc * NPAD); tmem_relinquish(); }
+    tc_fence_before_sync();
+    __syncthreads();
+    tc_fence_after_sync();
+    const uint32_t tmem_base = *tmem_slot;
+
+    int issued = 0;                        // stages the producing thread has filled
+    if (warp == 0) {
+        if (lane == 0) {
+            bool ok = true;
+            int s = 0;
+            uint32_t ph = 0;
+            for (int t = blockIdx.x; t < p.tiles && ok; t += gridDim.x) {
+                for (int b = 0; b < p.n_blocks; ++b) {
+                    ok = mbar_wait(empty(s), ph ^ 1u, abort_flag, p.status, ST_TIMEOUT_EMPTY, 0);
+                    if (!ok) break;
+                    const uint32_t at = base + s * stage_bytes;
+                    mbar_arrive_expect_tx(full(s), kNgWBytes + p.x_bytes);
+                    tma_load_2d(at, &tmW, full(s), b * 64, t * 128);
+                    tma_load_2d(at + kNgWBytes, &tmX, full(s), p.x_mn ? 0 : b * 64, p.x_mn ? b * 64 : 0);
+                    ++issued;
+                    if (++s == p.stages) { s = 0; ph ^= 1u; }
+                }
+            }
+        }
+    } else if (warp == 1) {
+        const uint32_t idesc = make_idesc(128, NPAD, 0, p.x_mn ? 1 : 0), x_step = p.x_mn ? 2048u >> 4 : 2u;
+        const uint64_t desc = make_sdesc(base, 16u, 1024u);
+        const uint32_t hi = (uint32_t)(desc >> 32), lo0 = (uint32_t)desc, slot = stage_bytes >> 4;
+        bool ok = true;
+        int s = 0, q = 0;
+        uint32_t ph = 0, lo = lo0;
+        for (int t = blockIdx.x; t < p.tiles && ok; t += gridDim.x) {
+            for (int part = 0; part < p.parts && ok; ++part, ++q) {
+                const int b0 = (int)((long long)part * p.n_blocks / p.parts), b1 = (int)((long long)(part + 1) * p.n_blocks / p.parts);
+                const uint32_t d = tmem_base + (uint32_t)(q & 1) * (kAcc * NPAD);
+                ok = mbar_wait_warp(acc_empty(q & 1), ((q >> 1) & 1) ^ 1u, abort_flag, p.status, ST_TIMEOUT_ACCUM, 1);
+                for (int b = b0; b < b1 && ok; ++b) {
+                    ok = mbar_wait_warp(full(s), ph, abort_flag, p.status, ST_TIMEOUT_FULL, 1);
+                    if (!ok) break;
+                    tc_fence_after_sync();
+                    const uint32_t xd = lo + (kNgWBytes >> 4), more = b > b0 ? 1u : 0u;
+                    if (elect_one()) {
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) umma_bf16_words<1>(d + i * NPAD, lo + 2u * i, hi, xd + x_step * i, hi, idesc, more);
+                        umma_commit(empty(s));
+                    }
+                    __syncwarp();
+                    lo += slot;
+                    if (++s == p.stages) { s = 0; ph ^= 1u; lo = lo0; }
+                }
+                if (ok && elect_one()) umma_commit(acc_full(q & 1));
+                __syncwarp();
+            }
+        }
+    } else {
+        const int lg = warp & 3;
+        const uint32_t lane_base = tmem_base + ((uint32_t)(lg * 32) << 16);
+        bool ok = true;
+        int q = 0;
+        for (int t = blockIdx.x; t < p.tiles && ok; t += gridDim.x) {
+            float tot[NPAD];
+#pragma unroll
+            for (int c = 0; c < NPAD; ++c) tot[c] = 0.f;
+            for (int part = 0; part < p.parts && ok; ++part, ++q) {
+                ok = mbar_wait(acc_full(q & 1), (q >> 1) & 1, abort_flag, p.status, ST_TIMEOUT_ACCUM, 4);
+                if (!__all_sync(0xFFFFFFFFu, ok)) { ok = false; break; }
+                tc_fence_after_sync();
+#pragma unroll
+                for (int c0 = 0; c0 < NPAD; c0 += 16) {
+                    float sum[16];
+#pragma unroll
+                    for (int a = 0; a < kAcc; ++a) {
+                        uint32_t v[16];
+                        tmem_ld_32x16(lane_base + (uint32_t)(((q & 1) * kAcc + a) * NPAD + c0), v);
+#pragma unroll
+                        for (int c = 0; c < 16; ++c) sum[c] = a == 0 ? __uint_as_float(v[c]) : sum[c] + __uint_as_float(v[c]);
+                    }
+#pragma unroll
+                    for (int c = 0; c < 16; ++c) tot[c0 + c] += sum[c];
+                }
+                tc_fence_before_sync();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(acc_empty(q & 1));
+            }
+            const int n = t * 128 + lg * 32 + lane;
+            if (ok && n < p.N) {
+                __nv_bfloat16* y = p.y + (long long)n * p.ldy;
+#pragma unroll
+                for (int c = 0; c < NPAD; c += 8)      // M is a multiple of 8, rows of y are aligned to 16 bytes
+                    if (c < p.M)
+                        *reinterpret_cast<uint4*>(y + c) = make_uint4(pack_bf16x2(tot[c] * p.alpha, tot[c + 1] * p.alpha), pack_bf16x2(tot[c + 2] * p.alpha, tot[c + 3] * p.alpha),
+                                                                      pack_bf16x2(tot[c + 4] * p.alpha, tot[c + 5] * p.alpha), pack_bf16x2(tot[c + 6] * p.alpha, tot[c + 7] * p.alpha));
+            }
+        }
+    }
+    tc_fence_before_sync();
+    __syncthreads();
+    if (threadIdx.x == 0 && *abort_flag) {
+        const uint64_t t0 = globaltimer_ns();
+        for (int it = issued > p.stages ? issued - p.stages : 0; it < issued; ++it)
+            while (!mbar_try_wait(full(it % p.stages), (it / p.stages) & 1))
+                if (globaltimer_ns() - t0 > 100000000ull) { report(p.status, ST_TIMEOUT_DRAIN, 0); break; }
+    }
+    __syncthreads();
+    if (warp == 1) { tc_fence_after_sync(); tmem_dealloc(tmem_base, 2 * kAcc * NPAD); }
+}
+
+template <int NPAD>
+int launch_tg(const NarrowArgs& a, const CUtensorMap& tmX, const CUtensorMap& tmW, int ctas, cudaStream_t stream) {
+    TurnedParams p = {};
+    p.M = a.M; p.N = a.mat[0].N; p.tiles = (p.N + 127) / 128; p.n_blocks = (a.K + 63) / 64; p.parts = turned_parts(p.n_blocks); p.x_mn = a.x_mn;
+    p.x_bytes = a.x_mn ? 64u * 128u : NPAD * 128u;
+    p.stages = (int)(kTgRingBytes / (kNgWBytes + p.x_bytes));
+    if (p.stages > kTgMaxStages) p.stages = kTgMaxStages;
+    p.y = (__nv_bfloat16*)a.mat[0].y; p.ldy = a.mat[0].ldy; p.alpha = a.alpha; p.status = device_status_ptr();
+    auto kern = turned_gemm_kernel<NPAD>;
+    constexpr uint32_t smem = kTgRingBytes + kNgBarBytes + 1024;
+    static bool attr_set[64] = {};
+    int dev = 0;
+    PLZ_CUDA_CHECK(cudaGetDevice(&dev));
+    if (!attr_set[dev & 63]) {
+        PLZ_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        attr_set[dev & 63] = true;
+    }
+    kern<<<p.tiles < ctas ? p.tiles : ctas, kTgThreads, smem, stream>>>(tmX, tmW, p);
+    PLZ_LAUNCH_CHECK();
+    return PLZ_OK;
+}
+
+}  // namespace
+
+// y [N, M] = alpha W x^T, M <= 64: x A^T and dY B of a LoRA branch. ctas > 0: a limit on the CTAs.
+int launch_turned_gemm(const NarrowArgs& a, int ctas, cudaStream_t stream) {
+    if (a.M < 8 || a.M > 64 || a.M % 8 || a.mat[0].N < 1 || a.K % 8) return PLZ_ERR_UNSUPPORTED;
+    const int sms = seq_sm_count(), tiles = (a.mat[0].N + 127) / 128, npad = a.M <= 16 ? 16 : a.M <= 32 ? 32 : 64, parts = turned_parts((a.K + 63) / 64);
+    CUtensorMap tmX, tmW;
+    int rc;
+    // A cluster per row tile while the rows leave SMs idle. us cluster / whole: 9728 columns, rank 16, 4096 rows 13.8 / 30, 6144 28 / 32, 8192 33 / 34, rank 64 35 / 34, 40 / 35 at the
+    // last two; 2560 columns, 6144 rows 9.0 / 11.2, 8192 9.9 / 11.7, 12288 16 / 13; 1024 columns, whatever the rows and the rank 6.3 to 9.3 / 5.9 to 6.8.
+    const bool few = (parts == 8 && tiles <= sms / 3) || (parts == 4 && tiles <= 9 * sms / 20);
+    if (ctas <= 0 && few && (rc = launch_narrow_gemm(a, stream)) != PLZ_ERR_UNSUPPORTED) return rc;   // which the maps below refuse
+    if ((rc = a.x_mn ? make_tmap_bf16(&tmX, a.x, a.K, a.M, a.ldx, 64, 64) : make_tmap_bf16(&tmX, a.x, a.M, a.K, a.ldx, 64, (uint32_t)npad))) return rc;
+    if ((rc = make_tmap_bf16(&tmW, a.mat[0].w, a.mat[0].N, a.K, a.mat[0].ldw, 64, 128))) return rc;
+    if (ctas <= 0 || ctas > sms) ctas = sms;
+    return npad == 16 ? launch_tg<16>(a, tmX, tmW, ctas, stream) : npad == 32 ? launch_tg<32>(a, tmX, tmW, ctas, stream) : launch_tg<64>(a, tmX, tmW, ctas, stream);
 }
 
 }  // namespace plz

@@ -28,6 +28,7 @@ struct LutGemmArgs {
     int act;           // fuse == 3 (dense B, no LoRA block): 1 = square of relu after the bias
     int sm_limit;  // > 0: use at most this many CTAs (tests of the multi-tile schedule)
     int early;     // NarrowArgs::early, where that kernel takes the call
+    int lora;      // a product with a LoRA factor (J <= 64): the order of its sums depends on R alone
     void* prof;  // optional device buffer of cycle counters, 8 x uint64 per CTA (diagnostics)
 };
 int launch_lut_gemm(const LutGemmArgs& a, cudaStream_t stream);
@@ -60,6 +61,7 @@ struct NarrowArgs {
     int y_f32; float alpha;           // y = act(alpha * sum + bias)
 };
 int launch_narrow_gemm(const NarrowArgs& a, cudaStream_t stream);   // PLZ_ERR_UNSUPPORTED: not a call for it
+int launch_turned_gemm(const NarrowArgs& a, int ctas, cudaStream_t stream);   // the same, transposed; ctas > 0: a limit on the CTAs
 
 // ---- tn_gemm.cu -------------------------------------------------------------------------------
 enum Epi { EPI_STORE = 0, EPI_SOFT = 1, EPI_HARD = 2 };

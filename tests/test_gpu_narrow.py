@@ -96,3 +96,27 @@ def test_lora_rows_do_not_depend_on_their_number(K, rank):
     t = ops.lora_dt((a, b, 1.0), x)
     for lo, hi in ((0, 1), (100, 1100), (1100, 9000)):
         assert torch.equal(ops.lora_dt((a, b, 1.0), x[lo:hi]), t[lo:hi])
+
+
+# the same for x A^T, at the row counts where other products change their kernel, at ones with more row tiles than SMs, and with a limit on the CTAs
+@pytest.mark.parametrize("K,rank", [(64, 64), (1088, 16), (2560, 24), (9728, 32), (4160, 64)])
+def test_lora_rows_and_cta_limit(K, rank):
+    import plz_native as P
+    g = torch.Generator(device="cuda").manual_seed(K + 1)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda").bfloat16()
+    x, a, b = rnd(20011, K), rnd(rank, K), rnd(K, rank)
+    w = ops.PackedWeight(ops.pack_indices(torch.zeros(64, K, dtype=torch.int8, device="cuda"), n_major=True), torch.zeros(64, 4, device="cuda", dtype=torch.bfloat16), 64, K, 1, K)
+    t = ops.hard_forward(w, x, (a, rnd(64, rank), 0.5))[1]
+    dt = ops.lora_dt((a, b, 0.5), x)
+    check(t, 0.5 * x.double() @ a.double().T, 0.5 * x.double().abs() @ a.double().abs().T, K)
+    check(dt, 0.5 * x.double() @ b.double(), 0.5 * x.double().abs() @ b.double().abs(), K)
+    for limit in (0, 5, 140):
+        P.lib().plz_set_cta_limit(limit)
+        try:
+            for rows in (1, 16, 17, 64, 65, 128, 129, 1000, 9000, 20011):
+                lo = 20011 - rows
+                assert torch.equal(ops.hard_forward(w, x[lo:], (a, b[:64], 0.5))[1], t[lo:]), (limit, rows)
+                assert torch.equal(ops.lora_dt((a, b, 0.5), x[lo:]), dt[lo:]), (limit, rows)
+        finally:
+            P.lib().plz_set_cta_limit(0)
+    P.device_status()
