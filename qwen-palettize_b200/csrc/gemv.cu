@@ -124,6 +124,12 @@ int launch_lut_gemv(const GemvArgs& a, cudaStream_t stream) {
         return launch_rows<4>(a, stream);
     }
     if (a.K % 64 || a.K > 16128) { set_last_error("small-M forward needs K %% 64 == 0 and K <= 16128 (K=%d)", a.K); return PLZ_ERR_BAD_SHAPE; }
+    if (g_cta_limit <= 0 && !((uintptr_t)a.out & 15) && a.ld_out % 8 == 0 && a.ld_out >= a.N) {       // a short reduction may do better elsewhere
+        LutGemmArgs g = {};
+        g.bmode = B_DECODE_K; g.M = a.M; g.J = a.N; g.R = a.K; g.A = a.x; g.lda = a.ldx; g.packed = a.packed; g.packed_pitch = a.packed_pitch; g.palette = a.palette;
+        g.gs_n = a.gs_n; g.gs_k = a.gs_k; g.Wn = a.N; g.Wk = a.K; g.out = a.out; g.ld_out = a.ld_out; g.alpha = 1.0f; g.early = 1;
+        return launch_lut_gemm(g, stream);
+    }
     NarrowArgs n = {};
     n.M = a.M; n.K = a.K; n.x = a.x; n.ldx = a.ldx; n.count = 1;
     n.mat[0].N = a.N; n.mat[0].packed = a.packed; n.mat[0].pitch = a.packed_pitch; n.mat[0].palette = a.palette;

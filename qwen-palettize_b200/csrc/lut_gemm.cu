@@ -647,6 +647,18 @@ static int launch_t(const LutGemmArgs& a, cudaStream_t stream) {
     return PLZ_OK;
 }
 
+// Products of at most 128 rows that a 128 x 256 tile per CTA serves as well as narrow_gemm.cu, whose start, sum over a cluster and end grow with the rows it
+// pads to (16, 32, 64, 128) and with the waves its 128-column tiles make: reductions of up to so many blocks of 64, by tiles that fill a quarter of the
+// chip / the chip / more. us here / there, 64 rows: dense 1024 x 256 5.9 / 7.6, x 512 6.9 / 6.8, x 2560 16 / 7.6; 9728 x 512 7.1 / 9.3, x 1536 11.7 / 11.2; packed 1024 x 128
+// 6.1 / 8.0, x 256 7.3 / 7.5, x 2560 31 / 8.5; 9728 x 512 10.4 / 10.9, x 1024 15.7 / 12.6; 128 rows: packed 24576 x 1536 22 / 25, x 2560 33 / 33. Up to 16 rows the kernels part at 128
+// columns. Dense: also where the tiles alone fill the chip (32 rows and more) and, beyond 64 rows, wider outputs of reductions below 2048.
+static bool few_rows_short(const LutGemmArgs& a, bool decode, int sms) {
+    static const int dense_line[3][4] = {{2, 4, 6, 8}, {4, 8, 16, 32}, {4, 8, 32, 32}}, packed_line[3][4] = {{2, 2, 4, 4}, {4, 4, 8, 8}, {6, 10, 16, 28}};
+    const int tiles = (a.J + 127) / 128, wide = 4 * tiles <= sms ? 0 : tiles <= sms ? 1 : 2, pad = a.M <= 16 ? 0 : a.M <= 32 ? 1 : a.M <= 64 ? 2 : 3;
+    if (!decode && ((a.M >= 32 && a.J >= 128 * sms) || (a.M > 64 && a.R < 2048 && a.J > 1024))) return true;
+    return (a.R + 63) / 64 <= (decode ? packed_line : dense_line)[wide][pad];
+}
+
 int launch_lut_gemm(const LutGemmArgs& a, cudaStream_t stream) {
     if (a.M <= 0 || a.J <= 0 || a.R <= 0) { set_last_error("lut_gemm: empty problem"); return PLZ_ERR_BAD_SHAPE; }
     const bool dense_k = a.bmode == B_TMA_K && a.r2 == 0;   // operands by TMA, reduction length padded with zeros by the copy
@@ -665,8 +677,9 @@ int launch_lut_gemm(const LutGemmArgs& a, cudaStream_t stream) {
         if (a.gs_k % 64 || a.Wk % a.gs_k || a.Wk % 64) { set_last_error("lut_gemm: K group size %d must be a multiple of 64 dividing K=%d", a.gs_k, a.Wk); return PLZ_ERR_BAD_SHAPE; }
     }
     // Outputs of at most 64 columns (the LoRA products x A^T and dY B): bound by streaming A. The turned kernels share a row tile among a cluster, or walk
-    // row tiles where those fill the chip. LoRA products go there at any number of rows, so that a row's result does not depend on that number.
-    if (!decode && a.J <= 64 && a.r2 == 0 && a.fuse == 0 && (a.lora || a.M > 128)) {
+    // row tiles where those fill the chip. LoRA products go there at any number of rows, so that a row's result does not depend on that number;
+    // so do others of up to 128 rows whose reduction is one part (64 x 512 at 64 rows 6.6 -> 4.9 us).
+    if (!decode && a.J <= 64 && a.r2 == 0 && a.fuse == 0 && (a.lora || a.M > 128 || a.R < 1024)) {
         NarrowArgs n = {};
         n.transposed = 1; n.x_mn = a.bmode == B_TMA_MN;
         n.M = a.J; n.K = a.R; n.x = a.Bdense; n.ldx = a.ldb; n.count = 1;
@@ -675,11 +688,8 @@ int launch_lut_gemm(const LutGemmArgs& a, cudaStream_t stream) {
         if (g_cta_limit > 0 && (limit <= 0 || g_cta_limit < limit)) limit = g_cta_limit;
         return launch_turned_gemm(n, limit, stream);
     }
-    // Few rows: the swapped form with the reduction split over a cluster (narrow_gemm.cu). A 128 x 256 tile per CTA is as good only where the
-    // tiles alone fill the chip (dense, wide outputs: 32768 x 2560 at 64 rows 31 against 36 us) or where the reduction is short and
-    // the rows many (6144 x 1024 at 128 rows 11 / 13); else 64 rows of 9728 x 2560 / 2560 x 9728 / 1024 x 2560 take 20 / 58 / 18 us here
-    // and 16 / 17 / 9 there, packed weights 32 / 122 / 30 and 18 / 22 / 9.
-    const bool own = !decode && ((a.M >= 32 && a.J >= 128 * 148) || (a.M > 64 && a.R < 2048 && a.J > 1024));
+    // Few rows: the swapped form with the reduction split over a cluster (narrow_gemm.cu), unless few_rows_short says that a 128 x 256 tile per CTA is as good
+    const bool own = a.M <= 128 && few_rows_short(a, decode, seq_sm_count());
     if (!own && a.M <= 128 && (a.bmode == B_TMA_K || a.bmode == B_DECODE_K) && a.fuse != 1 && !a.col_scale && !a.row_scale && a.sm_limit <= 0 && g_cta_limit <= 0) {
         NarrowArgs n = {};
         n.M = a.M; n.K = a.R; n.x = a.A; n.ldx = a.lda; n.count = 1;

@@ -42,6 +42,14 @@ int launch_dense_gemm_pair(const LutGemmArgs& a, cudaStream_t stream);
 extern int g_pair_gemm;  // 0: keep every product on the single-CTA kernel
 extern int g_cta_limit;
 
+inline int seq_sm_count() {
+    static int sms[64] = {};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (!sms[dev & 63]) cudaDeviceGetAttribute(&sms[dev & 63], cudaDevAttrMultiProcessorCount, dev);
+    return sms[dev & 63];
+}
+
 // ---- narrow_gemm.cu: M <= 128, operands swapped, reduction split over a cluster --------------------
 struct NarrowArgs {
     int M, K;

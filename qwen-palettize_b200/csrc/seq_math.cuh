@@ -55,12 +55,4 @@ __device__ __forceinline__ float block_sum(float v, float* part) {
     return s;
 }
 
-inline int seq_sm_count() {
-    static int sms[64] = {};
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (!sms[dev & 63]) cudaDeviceGetAttribute(&sms[dev & 63], cudaDevAttrMultiProcessorCount, dev);
-    return sms[dev & 63];
-}
-
 }  // namespace plz

@@ -120,3 +120,24 @@ def test_lora_rows_and_cta_limit(K, rank):
         finally:
             P.lib().plz_set_cta_limit(0)
     P.device_status()
+
+
+# reductions around the lines between this kernel and one CTA per 128 x 256 tile, at every padding of the rows and tiles that fill a part of the chip, most of it, and more
+@pytest.mark.parametrize("N,K", [(72, 128), (72, 192), (520, 256), (520, 320), (9728, 512), (9728, 576), (24576, 384), (24576, 640), (40, 960), (40, 1024)])
+def test_short_reductions(N, K):
+    g = torch.Generator(device="cuda").manual_seed(N + K)
+    idx = torch.randint(0, 4, (N, K), generator=g, device="cuda", dtype=torch.int8)
+    pal = torch.randn(N * (K // 64), 4, generator=g, device="cuda").bfloat16()
+    w = ops.PackedWeight(ops.pack_indices(idx, n_major=True), pal, N, K, 1, 64)
+    W = torch.gather(pal.view(N, K // 64, 1, 4).expand(-1, -1, 64, -1).reshape(N, K, 4), 2, idx.long()[:, :, None])[:, :, 0]
+    for M in (1, 16, 17, 33, 64, 65, 128):
+        x = torch.randn(M, K, generator=g, device="cuda").bfloat16()
+        ref, mag = x.double() @ W.double().T, x.double().abs() @ W.double().abs().T
+        check(ops.hard_forward(w, x)[0], ref, mag, K)
+        check(ops.dense_forward(W, x)[0], ref, mag, K)
+        if 16 < M <= 64:
+            check(ops.hard_forward_smallm(w, x), ref, mag, K)
+            out = torch.full((M, N + 8), 3.0, device="cuda", dtype=torch.bfloat16)
+            ops.hard_forward_smallm(w, x, out[:, 4:4 + N])           # not aligned to 16 bytes
+            check(out[:, 4:4 + N], ref, mag, K)
+            assert bool((out[:, :4] == 3).all()) and bool((out[:, 4 + N:] == 3).all())
