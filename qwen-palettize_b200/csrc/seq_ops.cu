@@ -177,7 +177,15 @@ rows_norm_kernel(const float* x, const long long* idx, const float* w, float w_o
     for (int c = threadIdx.x; c < W; c += 256) { const float v = x[r * W + c]; s = fmaf(v, v, s); }
     s = block_sum<8>(s, part);
     const float rs = 1.0f / sqrtf(s / (float)W + eps);
-    for (int c = threadIdx.x; c < W; c += 256) out[i * W + c] = from_f<T>(x[r * W + c] * rs * (w[c] + w_offset));
+    for (int c0 = threadIdx.x; c0 < W; c0 += 4 * 256) {      // loads ahead of the stores, which they would not pass by themselves
+        float a[4], g[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (c0 + u * 256 < W) { a[u] = x[r * W + c0 + u * 256]; g[u] = w[c0 + u * 256]; }
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (c0 + u * 256 < W) out[i * W + c0 + u * 256] = from_f<T>(a[u] * rs * (g[u] + w_offset));
+    }
 }
 
 // The embedding and the norm of picked rows for W % 4 == 0 and 16-byte aligned rows: one pass, the row kept in registers (W <= 1024 * NQ), weights
@@ -278,7 +286,15 @@ norm_gate_kernel(const float* o, const T* gate, long long ldg, const float* w, f
     s = BLOCK ? block_sum<8>(s, part) : warp_sum(s);
     const float rs = 1.0f / sqrtf(s / (float)L + eps);
     T* dst = out + r * W + (long long)g * L;
-    for (int c = t; c < L; c += team) dst[c] = from_f<T>(og[c] * rs * w[c] * sigmoid_f(to_f(gg[c])));
+    for (int c0 = t; c0 < L; c0 += 4 * team) {
+        float a[4], b[4], k[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (c0 + u * team < L) { a[u] = og[c0 + u * team]; b[u] = w[c0 + u * team]; k[u] = to_f(gg[c0 + u * team]); }
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (c0 + u * team < L) dst[c0 + u * team] = from_f<T>(a[u] * rs * b[u] * sigmoid_f(k[u]));
+    }
 }
 
 // the same four columns per access, everything of a group in registers (TEAM threads, L <= 4 TEAM NQ) and requested at once. 2048 x 2560 21 -> 13 us
