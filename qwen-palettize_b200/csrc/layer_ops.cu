@@ -434,7 +434,9 @@ int launch_qknorm_rope2(const void* x1, long long ldx1, const void* w1, int H1, 
     const QkSide b = {(const __nv_bfloat16*)x2, ldx2, (const __nv_bfloat16*)w2, (__nv_bfloat16*)out2, ldo2, H2};
     const bool wide = !(((uintptr_t)x1 | (uintptr_t)w1 | (uintptr_t)out1 | (uintptr_t)x2 | (uintptr_t)w2 | (uintptr_t)out2 | (uintptr_t)cs | (uintptr_t)sn) & 15) &&
                       !((ldx1 | ldo1 | ldx2 | ldo2) & 7);
-    if (wide) {
+    // With few rows the longer chain of the 16-byte form is the launch, and heads that leave a third of their quads empty waste it. us general / 16-byte:
+    // 32 + 8 heads, 1 token 2.2 / 2.7, 128 2.7 / 3.0, 256 3.9 / 3.5, 1000 9.3 / 7.0; 16 + 8 heads, 256 tokens 3.2 / 3.3, 512 4.2 / 3.5; 5 + 1 heads, 4096 tokens 6.4 / 8.0.
+    if (wide && rows >= 8192 && 8 * ((H1 + 3) / 4 + (H2 + 3) / 4) <= 3 * (H1 + H2)) {
         // quads of a token that a warp takes: as many as leave about 48 warps per SM
         const int quads = (H1 + 3) / 4 + (H2 + 3) / 4;
         long long per = tokens * quads / (48ll * sm_count_here());

@@ -62,3 +62,9 @@ def test_rmsnorm_backward(M, K, shift, weighted):
     assert bool(((dx.double() - want).abs() <= 2.0 ** -8 * want.abs() + 2.0 ** -18 * mag).all())
     if weighted:
         assert bool(((dg.double() - (d * v * r).sum(0)).abs() <= (M + 4) * 2.0 ** -23 * (d * v * r).abs().sum(0) + 1e-6).all())
+
+
+# the 16-byte forward takes 8192 rows (token, head) and more: quads of heads that are not full, and the sizes on either side of the line
+@pytest.mark.parametrize("tokens,S,Hq,Hk,shift", [(911, 7, 7, 2, 0), (1023, 1023, 6, 2, 0), (1024, 64, 6, 2, 0), (1400, 3, 6, 1, 0)])
+def test_qknorm_rope_many_rows(tokens, S, Hq, Hk, shift):
+    test_qknorm_rope(tokens, S, Hq, Hk, shift)
