@@ -2,14 +2,14 @@
 // opens a forward pass. Both are single passes that should be bound by HBM: a decode step reads every cached key and value once
 // (B * T * Hkv * 128 * 2 * 2 bytes per layer).
 //
-//   attn_decode_mma_kernel  bf16, head sizes above 64 and up to 128. With scores and sums on FMAs (the kernel below) a step of 64 sequences over 1025
+//   attn_decode_mma_kernel  bf16, head sizes above 64 and up to 128, long caches or many sequences. With scores and sums on FMAs (the kernel below) a step of 64 sequences over 1025
 //     tokens of 8 key / value heads issued about 1000 instructions per 16 tokens and warp and took 68 us for 268 MB, bound by issue. Here the
 //     scores are mma.sync m16n8k16 (A = the query heads of the group, 4 of 16 rows used; B = 8 keys straight from memory, the order of
 //     the dimensions permuted alike on both sides so that a lane's operands are whole 16-byte loads): products of bf16 are exact and sums
 //     are fp32 as before. The weights stay fp32: they pass through shared memory (16 tokens x 4 heads per warp and step) to the lanes that
 //     hold the values, and weight x value runs on packed fp32 pairs.
 //     Keys and values are requested one step ahead. 69 -> 51 us (5.3 TB/s); one sequence of 2049 tokens 6.2 -> 5.5 us.
-//   attn_decode_partial_kernel  the other types and sizes: grid (splits, Hkv, B), 4 warps. The sequence is cut into `splits` contiguous chunks so that
+//   attn_decode_partial_kernel  the other types and sizes, and few cached tokens: grid (splits, Hkv, B), 4 warps. The sequence is cut into `splits` contiguous chunks so that
 //     the launch has a few CTAs per SM whatever B is. Inside a CTA a warp takes 8 tokens per step: 16 lanes per token, each
 //     lane the 16 bytes (8 dims) of the key and of the value row that belong to it, so one load instruction of a warp covers
 //     two whole 256-byte rows, and four such loads for K and four for V are in flight per lane before anything is used. The
@@ -500,7 +500,11 @@ int launch_attn_decode(const AttnDecodeArgs& a, cudaStream_t stream) {
     p.ws_ml = p.ws_o ? p.ws_o + (long long)a.B * a.Hq * p.splits * 128 : nullptr;
     p.T = a.T; p.Hq = a.Hq; p.Hkv = a.Hkv; p.group = a.Hq / a.Hkv; p.passes = (p.group + 3) / 4;
     p.scale_log2e = a.scale * kLog2eDec;
-    PLZ_LAUNCH_CHAIN(attn_decode_mma_kernel<false>, dim3(p.splits, a.Hkv * p.passes, a.B), dim3(kDecWarps * 32), 0, stream, p);
+    // Few cached tokens in all: a step of half the size. us there / here: 1 x 16 tokens of 8 heads 3.0 / 3.2, 1 x 300 6.1 / 6.4, 64 x 16 4.0 / 4.6, 16 x 100 of one 6.3 / 6.6,
+    // 4 x 300 7.6 either way, 1 x 2049 9.3 / 8.8, 2 x 1000 7.8 / 7.5, 64 x 1025 67 / 46.
+    const dim3 grid(p.splits, a.Hkv * p.passes, a.B), block(kDecWarps * 32);
+    if ((long long)a.B * a.Hkv * a.T <= 8192) PLZ_LAUNCH_CHAIN((attn_decode_partial_kernel<__nv_bfloat16, 16, false>), grid, block, 0, stream, p);
+    else PLZ_LAUNCH_CHAIN(attn_decode_mma_kernel<false>, grid, block, 0, stream, p);
     if (p.splits > 1) {
         PLZ_LAUNCH_CHAIN(attn_decode_combine_kernel<__nv_bfloat16>, dim3(a.Hq, a.B), dim3(128), 0, stream, (const float*)p.ws_o, (const float*)p.ws_ml,
                          p.splits, a.Hq, 128, 0, (__nv_bfloat16*)p.out, p.ldo);

@@ -30,6 +30,12 @@ def test_decode_attention_matches_softmax(B, T, Hq, Hkv):
     assert_close(out, want, "decode attention", rel=1e-2, cos=0.9999)
 
 
+# both sides of the line between the two kernels (8192 cached tokens times key / value heads), and short caches of many sequences above it
+@pytest.mark.parametrize("B,T,Hq,Hkv", [(2, 4096, 2, 1), (2, 4097, 2, 1), (64, 17, 8, 8), (700, 1, 16, 16), (300, 33, 6, 1), (97, 65, 8, 2)])
+def test_decode_attention_on_both_kernels(B, T, Hq, Hkv):
+    test_decode_attention_matches_softmax(B, T, Hq, Hkv)
+
+
 def test_embed_gather():
     import plz_ops as ops
     dev = torch.device("cuda", 0)
