@@ -407,7 +407,8 @@ int launch_rmsnorm_bwd(const void* x, long long ldx, const void* dh, long long l
                        void* dx, long long lddx, float* dg, cudaStream_t stream) {
     if (M <= 0) return PLZ_OK;
     if (K > 512 * kNormPairsMax) { set_last_error("rmsnorm_bwd: K=%d exceeds %d", K, 512 * kNormPairsMax); return PLZ_ERR_TOO_LARGE; }
-    if (K % 8 == 0 && K <= kNorm8MaxK && !(((uintptr_t)x | (uintptr_t)dh | (uintptr_t)g | (uintptr_t)dx | (uintptr_t)dg) & 15) && !((ldx | lddh | lddx) & 7)) {
+    // from 64 rows or 4096 columns on: below, the chain of latencies of one row is the launch (7 rows of 2560 3.9 us in the kernel above, 4.2 here, of 8192 8.5 / 6.3)
+    if ((M >= 64 || K >= 4096) && K % 8 == 0 && K <= kNorm8MaxK && !(((uintptr_t)x | (uintptr_t)dh | (uintptr_t)g | (uintptr_t)dx | (uintptr_t)dg) & 15) && !((ldx | lddh | lddx) & 7)) {
         const int threads = (K / 8 + 31) / 32 * 32, per_sm = threads <= 320 ? 3 : threads <= 512 ? 2 : 1;
         int blocks = (M + 1) / 2;
         if (blocks > per_sm * sm_count_of_current_device()) blocks = per_sm * sm_count_of_current_device();

@@ -119,3 +119,10 @@ def test_overlapped_rows():
     finally:
         P.lib().plz_set_smallm_overlap(0)
     assert all(torch.equal(a, b) for a, b in zip(want, got))
+
+
+# the register forms start at 256 columns; beyond 4096 the update requests everything ahead for one row per SM only
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("rows,W", [(2, 252), (3, 256), (1, 260), (150, 8192), (140, 4100)])
+def test_rows_lines(rows, W, dtype):
+    test_rows(rows, W, dtype)

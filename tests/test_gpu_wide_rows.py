@@ -68,3 +68,9 @@ def test_rmsnorm_backward(M, K, shift, weighted):
 @pytest.mark.parametrize("tokens,S,Hq,Hk,shift", [(911, 7, 7, 2, 0), (1023, 1023, 6, 2, 0), (1024, 64, 6, 2, 0), (1400, 3, 6, 1, 0)])
 def test_qknorm_rope_many_rows(tokens, S, Hq, Hk, shift):
     test_qknorm_rope(tokens, S, Hq, Hk, shift)
+
+
+# the 16-byte kernel from 64 rows or 4096 columns on: threads beyond the columns, an odd last row
+@pytest.mark.parametrize("M,K,shift,weighted", [(64, 8, 0, True), (65, 264, 0, False), (63, 264, 0, True), (1, 4096, 0, True), (3, 4104, 0, True), (3, 4088, 0, True)])
+def test_rmsnorm_backward_lines(M, K, shift, weighted):
+    test_rmsnorm_backward(M, K, shift, weighted)
