@@ -589,8 +589,23 @@ tn_gemm_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant__ 
                 }
                 if (p.dpalette != nullptr) {
                     if (p.gs_n == 1) {
-                        // this thread's row has its own palette: the column parts add up in any order
-                        if (row_ok) {
+                        // this thread's row has its own palette. Two column parts add up in either order; of four, rounded differently in every
+                        // order, one thread adds the parts up in a fixed one
+                        if (EW > 8) {
+                            float4* parts = reinterpret_cast<float4*>(red);
+                            const int at = lane_group * 32 + lane;
+                            parts[col_part * 128 + at] = make_float4(acc[0], acc[1], acc[2], acc[3]);
+                            epi_bar_sync<EW>();
+                            if (col_part == 0) {
+#pragma unroll
+                                for (int i = 1; i < EW / 4; ++i) {
+                                    const float4 v = parts[i * 128 + at];
+                                    acc[0] += v.x; acc[1] += v.y; acc[2] += v.z; acc[3] += v.w;
+                                }
+                            }
+                            epi_bar_sync<EW>();
+                        }
+                        if (row_ok && (EW <= 8 || col_part == 0)) {
 #pragma unroll
                             for (int q = 0; q < 4; ++q) atomicAdd(p.dpalette + pg + q, acc[q]);
                         }

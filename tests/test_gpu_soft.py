@@ -113,3 +113,23 @@ def test_persistent_schedule_with_few_ctas(limit):
     want = _oracle(d, 1.0, True, noise=d["noise"])
     for k in ("y", "dx", "dlogits", "dpalette", "da", "db"):
         assert_close(got[k], want[k], k)
+
+
+def test_palette_gradient_of_planar_logits_repeats():
+    """Planar logits with a palette per row and 256 columns: the parts of a row's gradient are added up in one order, the same on every run."""
+    import plz_ops as ops
+    g = torch.Generator(device="cuda").manual_seed(3)
+    M, N, K = 300, 520, 768
+    x, dy = (torch.randn(M, n, generator=g, device="cuda").bfloat16() for n in (K, N))
+    logits, noise = torch.randn(4, K, N, generator=g, device="cuda").half(), torch.randn(4, K, N, generator=g, device="cuda")
+    pal = torch.randn(N * 3, 4, generator=g, device="cuda").bfloat16()
+    w = ops.PackedWeight(ops.empty_packed(N, K, "cuda"), pal, N, K, 1, 256)
+    dlog, dpal = ops.backward_dw_soft(w, x, dy, logits, "4kn", noise)
+    p = torch.softmax(logits.double() + noise.double(), 0).permute(2, 1, 0)                 # [N, K, 4]
+    dw = dy.double().T @ x.double()
+    want = torch.einsum("nkj,nkjp->nkp", dw.view(N, 3, 256), p.reshape(N, 3, 256, 4)).reshape(N * 3, 4)
+    mag = torch.einsum("nkj,nkjp->nkp", (dy.double().abs().T @ x.double().abs()).view(N, 3, 256), p.reshape(N, 3, 256, 4)).reshape(N * 3, 4)
+    assert bool(((dpal.double() - want).abs() <= (M + 256 + 32) * 2.0 ** -23 * mag).all())      # fp32 sums; softmax by the fast exponential
+    for _ in range(30):
+        a, b = ops.backward_dw_soft(w, x, dy, logits, "4kn", noise)
+        assert torch.equal(a, dlog) and torch.equal(b, dpal)
