@@ -86,12 +86,9 @@ def _mat(x: torch.Tensor, cols: int):
 
 
 def _zeros(shapes, device):
-    """Zeroed fp32 tensors of the given shapes (None: None), cleared by one launch; each starts at a multiple of 16 bytes."""
-    sizes = [0 if s is None else (s[0] * s[1] + 3) // 4 * 4 for s in shapes]
-    flat, at, out = torch.zeros(sum(sizes), dtype=torch.float32, device=device), 0, []
-    for s, n in zip(shapes, sizes):
-        out.append(None if s is None else flat[at:at + s[0] * s[1]].view(s))
-        at += n
+    """Zeroed fp32 tensors of the given shapes (None: None), each with a storage of its own, cleared by one launch."""
+    out = [None if s is None else torch.empty(s, dtype=torch.float32, device=device) for s in shapes]
+    torch._foreach_zero_([t for t in out if t is not None])
     return out
 
 

@@ -88,6 +88,15 @@ def test_decode_step_is_checked_before_its_first_launch(built_lib):
         bind()
 
 
+def test_gradients_share_no_storage(built_lib):
+    """dPalette, dA and dB of one call are cleared together but kept, saved and freed one by one."""
+    import torch
+    import plz_ops as ops
+    a, none, b, c = ops._zeros([(3, 4), None, (16, 7), (1, 1)], "cpu")
+    assert none is None and all(t.dtype == torch.float32 and not t.any() and t._base is None and t.untyped_storage().nbytes() == 4 * t.numel() for t in (a, b, c))
+    assert len({t.untyped_storage().data_ptr() for t in (a, b, c)}) == 3
+
+
 def test_ops_refuse_cpu_tensors(built_lib):
     import torch
     import fused_lut_linear_cuda as F
