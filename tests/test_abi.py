@@ -109,13 +109,17 @@ def test_ops_refuse_cpu_tensors(built_lib):
 
 def test_hot_kernels_do_not_spill():
     """Register spills in the pipelined GEMM kernels cost 15-20 % (measured once); keep them at zero.
-    (The eight-stage narrow variants for the rank-16/32 products may spill a few bytes in their epilogue.)"""
+    (The eight-stage narrow variant for outputs of up to 64 columns with a bias may spill a few bytes in its epilogue.)"""
     import build
     build.build(force=True)
     rep = build.spill_report()
-    # lut_gemm_kernel<MT, BMODE, NARROW=false, FUSE=0> mangles to ...ELb0ELi0EE...; tn_gemm / small-M kernels all count
-    hot = {k: v for k, v in rep.items()
-           if ("lut_gemm_kernel" in k and "ELb0ELi0EE" in k) or "tn_gemm_kernel" in k or "lut_gemv" in k or "lut_smallm_mma" in k}
-    assert len(hot) >= 12
+    # lut_gemm_kernel<MT, BMODE, NARROW=false, FUSE=0> mangles to ...ELb0ELi0EE...; the other product kernels all count
+    names = {"tn_gemm_kernel": 12, "lut_smallm_mma": 2, "lut_gemv_rows": 3, "lut_gemm_pair_kernel": 2, "dense_gemm_pair_kernel": 3, "narrow_gemm_kernel": 2, "turned_gemm_kernel": 3}
+    hot = {k: v for k, v in rep.items() if ("lut_gemm_kernel" in k and "ELb0ELi0EE" in k) or any(n in k for n in names)}
+    for n, least in names.items():
+        assert sum(n in k for k in hot) >= least, n
+    assert sum("lut_gemm_kernel" in k for k in hot) >= 7
+    # decode attention holds a step of keys and values in 128 registers, four CTAs per SM: a few words of addresses may spill, no more
+    assert all(v[0] <= 32 and v[1] <= 32 for k, v in rep.items() if "attn_decode_mma_kernel" in k)
     bad = {k: v for k, v in hot.items() if v[0] or v[1]}
     assert not bad, bad
