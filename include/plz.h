@@ -121,6 +121,11 @@ int32_t plz_dequantize(const plz_weight_t* w, void* dst, int64_t d_n, int64_t d_
 int32_t plz_hard_fwd(const plz_weight_t* w, const void* x, int64_t ldx, int32_t M, const plz_lora_t* lora,
                      void* t, void* y, int64_t ldy, void* stream);
 
+/* About the bits of a result: they repeat from run to run, but a row's do not stay the same when the number of rows changes what kernel takes the call or how it
+ * splits the reduction (at 16, 32, 64, 128 and 256 rows, and with plz_set_cta_limit): fp32 sums in another order, rounded once to bf16. The LoRA intermediates
+ * t = scale * x A^T and dt = scale * dY B are the exception: their sums follow the reduction length alone, so that a step over all tokens and steps over parts
+ * of them see the same t and dt. plz_hard_fwd_smallm* with up to 16 rows add partial sums with atomics: bits may differ between runs. */
+
 /* plz_hard_fwd with LoRA for callers that must not allocate. (No counterpart in the reference: its wrappers
  * allocate every intermediate through torch.)  Some hosts hand an operator its inputs and outputs and nothing
  * else: the host owns the whole device-memory pool, so a cudaMalloc inside the operator can fail or stall the
@@ -346,7 +351,7 @@ int32_t plz_weight_grad(const void* x, int64_t ldx, const void* dY, int64_t lddy
  * [B * S, Hkv * 128], o in the layout of q: exactly what the q/k/v projections write and o_proj reads. S % 128 == 0,
  * head_dim = 128, Hq % Hkv == 0. o = softmax(q k^T * scale + causal mask) v per (batch, head), fp32 softmax.
  * lse (fp32 [B, Hq, S], may be NULL in the forward) receives the natural-log sum-exp of the scaled scores; the backward
- * needs it, together with o, and a workspace dsum_ws of B * Hq * S floats. Gradients dq / dk / dv have the layouts and
+ * needs it, together with o (8-byte aligned here, all other matrices 16), and a workspace dsum_ws of B * Hq * S floats. Gradients dq / dk / dv have the layouts and
  * pitches of q / k / v and are WRITTEN (dk, dv already summed over the q heads of a group).
  * The reference has no attention code: it calls the HuggingFace decoder layer (scripts/train_qwen.py:1259-1266; SDPA
  * selected at scripts/qwen_model.py:454); semantics are those of transformers' Qwen3Attention after q/k norm and RoPE. */

@@ -651,7 +651,8 @@ tn_gemm_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant__ 
 // From this many tokens on the main loop of a tile (256 x 256, 0.33 us per 64 tokens) is longer than its soft epilogue with eight warps
 // (interleaved fp32 logits, 60 us), which then runs in its shadow. Measured at 9728 x 2560, noise tensor / sampled noise, eight against
 // sixteen warps: 512 tokens 320 / 336 against 288 / 260 us, 4096: 352 / 374 against 316 / 306, 8192: 435 / 443 against 417 / 410,
-// 10240: 493 / 491 against 488 / 483, 16384: 712 / 708 against 766 / -. Planar fp16 logits (4096 x 2560, 2048 tokens) take 125 us per
+// 10240: 493 / 491 against 488 / 483, 16384: 712 / 708 against 766 / -. The same line elsewhere, 8192 / 10240 tokens, noise tensor: 2560 x 9728 460 / 511 against 417 / 509, 4096 x 2560
+// 201 / 226 against 188 / 224, 1024 x 2560 93 / 101 against 82 / 89, 512 x 512 83 / 94 against 70 / 81. Planar fp16 logits (4096 x 2560, 2048 tokens) take 125 us per
 // tile with eight warps, longer than any main loop: 309 against 126 us, always sixteen. The hard epilogue has 45 against 40 us at
 // 512 tokens: always eight.
 constexpr int kTnLongLoop = 10241;
