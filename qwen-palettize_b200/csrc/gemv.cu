@@ -1,6 +1,6 @@
 // Small-M hard forward (token decode): y[M, N] = x[M, K] W^T for M <= 64 with packed 2-bit weights. launch_lut_gemv picks the kernel: mma.sync
-// fragments straight from registers (smallm_mma.cu) for up to 16 rows, the swapped tcgen05 form (narrow_gemm.cu) beyond and for
-// long reductions, and the CUDA-core kernel below where neither takes the shape.
+// fragments straight from registers (smallm_mma.cu) for up to 16 rows, the swapped tcgen05 form (narrow_gemm.cu; a tile per CTA for short
+// reductions) beyond and for long reductions, and the CUDA-core kernel below where none takes the shape.
 //
 // Replaces the reference's hard forward at decode batch sizes (scripts/qwen_model.py:164-192 dispatching to
 // fused_lut_linear_fwd_tc_kernel, scripts/fused_lut_kernel.cu:309, which reads 1 byte per weight).
