@@ -178,6 +178,9 @@ int32_t plz_soft_select(const plz_weight_t* w, const plz_logits_t* logits, const
 int32_t plz_dense_fwd(const void* Wd, int64_t ldw, int32_t N, int32_t K, const void* x, int64_t ldx, int32_t M,
                       const plz_lora_t* lora, void* t, void* y, int64_t ldy, void* stream);
 
+/* Clears up to 4 device buffers (gradients that the calls below accumulate into) by one launch. Addresses: multiples of 16 bytes; sizes: multiples of 4 bytes, 0 allowed. */
+int32_t plz_zero(void* const* ptrs, const int64_t* bytes, int32_t count, void* stream);
+
 /* ---- backward --------------------------------------------------------------------------------
  * dX[M, K] = dY[M, N] W (+ LoRA: dt = scale * dY B into the bf16 [M, rank] workspace `dt`, then
  * dX += dt A). fused_lut_linear_bwd_grad_x_tc_kernel (scripts/fused_lut_kernel.cu:551) and

@@ -364,6 +364,20 @@ int32_t plz_soft_select(const plz_weight_t* w, const plz_logits_t* logits, const
     return launch_soft_select(p, logits->dtype == 1, (cudaStream_t)stream);
 }
 
+int32_t plz_zero(void* const* ptrs, const int64_t* bytes, int32_t count, void* stream) {
+    if (count < 0 || count > 4) { set_last_error("zero: 0 to 4 buffers"); return PLZ_ERR_BAD_SHAPE; }
+    if (count == 0) return PLZ_OK;
+    if (!ptrs || !bytes) { set_last_error("null pointer"); return PLZ_ERR_NULL; }
+    long long n[4];
+    for (int i = 0; i < count; ++i) {
+        if (bytes[i] < 0 || bytes[i] % 4) { set_last_error("zero: %lld bytes", (long long)bytes[i]); return PLZ_ERR_BAD_SHAPE; }
+        if (bytes[i] && !ptrs[i]) { set_last_error("null pointer"); return PLZ_ERR_NULL; }
+        if ((uintptr_t)ptrs[i] & 15) { set_last_error("zero: buffers must be 16-byte aligned"); return PLZ_ERR_BAD_ALIGN; }
+        n[i] = bytes[i];
+    }
+    return launch_zero(ptrs, n, count, (cudaStream_t)stream);
+}
+
 int32_t plz_bwd_dx(const plz_weight_t* w, const void* dY, int64_t lddy, int32_t M, const plz_lora_t* lora, void* dt,
                    void* dX, int64_t lddx, void* stream) {
     int rc = check_weight(w, true);

@@ -50,6 +50,8 @@ inline int seq_sm_count() {
     return sms[dev & 63];
 }
 
+int launch_zero(void* const* ptrs, const long long* bytes, int count, cudaStream_t stream);   // train_ops.cu
+
 // ---- narrow_gemm.cu: M <= 128, operands swapped, reduction split over a cluster --------------------
 struct NarrowArgs {
     int M, K;

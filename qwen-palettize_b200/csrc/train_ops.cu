@@ -452,4 +452,37 @@ int launch_reduce_slots(const float* stage, int world, long long shard_elems, fl
     return PLZ_OK;
 }
 
+// ---- several buffers cleared by one launch -----------------------------------------------------------------------------------------------
+namespace {
+struct ZeroParams { uint4* p[4]; long long bytes[4]; };
+// bytes: multiples of 4, addresses multiples of 16. The gradients of a Linear (2 MB in three tensors): 1.8 us, one launch per tensor 1.6 each, torch's
+// multi-tensor form, 256 KB per block, 5.4.
+__global__ void __launch_bounds__(256)
+zero_kernel(const ZeroParams z) {
+    const long long first = (long long)blockIdx.x * 256 + threadIdx.x, step = (long long)gridDim.x * 256;
+#pragma unroll
+    for (int b = 0; b < 4; ++b) {
+        const long long units = z.bytes[b] >> 4;
+        for (long long i = first; i < units; i += step) z.p[b][i] = make_uint4(0u, 0u, 0u, 0u);
+        if (first < ((z.bytes[b] & 15) >> 2)) reinterpret_cast<uint32_t*>(z.p[b] + units)[first] = 0u;
+    }
+}
+}  // namespace
+
+int launch_zero(void* const* ptrs, const long long* bytes, int count, cudaStream_t stream) {
+    ZeroParams z = {};
+    long long most = 0;
+    for (int i = 0; i < count; ++i) {
+        z.p[i] = (uint4*)ptrs[i]; z.bytes[i] = bytes[i];
+        if (bytes[i] > most) most = bytes[i];
+    }
+    if (most == 0) return PLZ_OK;
+    long long blocks = (most / 16 + 255) / 256;
+    const long long cap = (long long)sm_count_of_current_device() * 8;
+    if (blocks < 1) blocks = 1;
+    zero_kernel<<<(unsigned)(blocks < cap ? blocks : cap), 256, 0, stream>>>(z);
+    PLZ_LAUNCH_CHECK();
+    return PLZ_OK;
+}
+
 }  // namespace plz

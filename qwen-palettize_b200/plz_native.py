@@ -163,6 +163,7 @@ SIGNATURES = {
     "plz_weight_grad": [_P, _I64, _P, _I64, _I32, _I32, _I32, _P, _I64, _I64, _P],
     "plz_attn_fwd": [_P, _I64, _P, _I64, _P, _I64, _I32, _I32, _I32, _I32, _I32, _F, _P, _I64, _P, _P],
     "plz_attn_bwd": [_P, _I64, _P, _I64, _P, _I64, _P, _P, _I64, _P, _I32, _I32, _I32, _I32, _I32, _F, _P, _P, _P, _P, _P],
+    "plz_zero": [_P, _P, _I32, _P],
     "plz_attn_decode_ws_bytes": [_I32, _I32, _I32, _I32],
     "plz_attn_decode": [_P, _I64, _P, _P, _I64, _I64, _I32, _I32, _I32, _I32, _I32, _F, _P, _I64, _P, _I64, _P],
     "plz_decode_ws_bytes": [_I32, _I32, _I32, _I32, _I32, _I32],

@@ -88,7 +88,9 @@ def _mat(x: torch.Tensor, cols: int):
 def _zeros(shapes, device):
     """Zeroed fp32 tensors of the given shapes (None: None), each with a storage of its own, cleared by one launch."""
     out = [None if s is None else torch.empty(s, dtype=torch.float32, device=device) for s in shapes]
-    torch._foreach_zero_([t for t in out if t is not None])
+    some = [t for t in out if t is not None]
+    P.check(P.lib().plz_zero((C.c_void_p * len(some))(*[t.data_ptr() for t in some]), (C.c_int64 * len(some))(*[4 * t.numel() for t in some]), len(some),
+                             P.stream_ptr()), "plz_zero")
     return out
 
 

@@ -77,3 +77,20 @@ def test_distill_loss_against_reference_vectors(golden):
     assert abs(out4[0].item() - float(golden["loss_vals"][0])) <= 1e-5
     assert abs(out4[1].item() - float(golden["loss_vals"][1])) <= 1e-5
     assert_close(ds.reshape(-1), torch.from_numpy(golden["loss_ds"]).reshape(-1), "dLoss/ds vs compute_loss autograd", rel=1e-3, cos=0.99999)
+
+
+@pytest.mark.parametrize("shapes", [[(3, 4)], [(3, 7), None, (16, 2560), (1, 1)], [(97280, 4), (16, 2560), (9728, 16)], [(1, 3), (1, 4), (1, 5), (257, 1023)]])
+def test_gradients_are_cleared_and_share_no_storage(shapes):
+    """dPalette, dA and dB of one call are cleared by one launch but kept, saved and freed one by one; nothing beside them is written."""
+    import ctypes as C
+    import plz_native as P
+    import plz_ops as ops
+    out = ops._zeros(shapes, "cuda")
+    assert [None if t is None else tuple(t.shape) for t in out] == shapes
+    some = [t for t in out if t is not None]
+    assert all(t.dtype == torch.float32 and not t.any() and t._base is None and t.untyped_storage().nbytes() == 4 * t.numel() for t in some)
+    assert len({t.untyped_storage().data_ptr() for t in some}) == len(some)
+    held = [torch.full((t.numel() + 8,), 5.0, device="cuda") for t in some]
+    n = len(held)
+    P.check(P.lib().plz_zero((C.c_void_p * n)(*[t.data_ptr() + 16 for t in held]), (C.c_int64 * n)(*[4 * t.numel() - 32 for t in held]), n, P.stream_ptr()), "plz_zero")
+    assert all(bool((t[:4] == 5).all()) and bool((t[-4:] == 5).all()) and not t[4:-4].any() for t in held)
