@@ -245,6 +245,38 @@ __global__ void __launch_bounds__(256) soft_select_nfast_kernel(const SelectPara
     }
 }
 
+// Indices alone of planar fp16 logits [4, K, N] (the reference's layout): a thread takes eight n of four k, 16 loads of 16 bytes at once where the kernel
+// above has one load of 2 bytes per logit. Bound by the logits' 8 bytes per weight. Block = 64 n x 32 bytes of k, the bytes transposed through shared memory.
+__global__ void __launch_bounds__(256) select_planar_half_kernel(const SelectParams p) {
+    __shared__ __align__(8) uint8_t tile[64][40];
+    const int tx = threadIdx.x & 7, ty = threadIdx.x >> 3;
+    const int n = blockIdx.x * 64 + tx * 8, kb = blockIdx.y * 32 + ty;
+    if (n < p.N && kb * 4 < p.K) {
+        const __half* src = reinterpret_cast<const __half*>(p.logits) + n + (long long)(kb * 4) * p.ls_k;
+        uint4 v[4][4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+            for (int q = 0; q < 4; ++q) v[j][q] = __ldcs(reinterpret_cast<const uint4*>(src + j * p.ls_k + q * p.ls_p));
+        uint32_t byte[8] = {};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const __half* h[4] = {reinterpret_cast<const __half*>(&v[j][0]), reinterpret_cast<const __half*>(&v[j][1]), reinterpret_cast<const __half*>(&v[j][2]),
+                                  reinterpret_cast<const __half*>(&v[j][3])};
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+                byte[i] |= (uint32_t)argmax4_first(__half2float(h[0][i]), __half2float(h[1][i]), __half2float(h[2][i]), __half2float(h[3][i])) << (2 * j);
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) tile[tx * 8 + i][ty] = (uint8_t)byte[i];
+    }
+    __syncthreads();
+    // K % 32 == 0: eight bytes of a row are all there or none
+    const int r = threadIdx.x >> 2, part = threadIdx.x & 3;
+    const int row = blockIdx.x * 64 + r, at = blockIdx.y * 32 + part * 8;
+    if (row < p.N && at * 4 < p.K) *reinterpret_cast<uint2*>(p.packed + (long long)row * p.pitch + at) = *reinterpret_cast<const uint2*>(&tile[r][part * 8]);
+}
+
 int launch_soft_select(const SelectParams& p, int logits_f16, cudaStream_t stream) {
     if (p.N <= 0 || p.K <= 0) return PLZ_OK;
     if (!p.logits) { set_last_error("soft_select: null logits"); return PLZ_ERR_NULL; }
@@ -257,7 +289,10 @@ int launch_soft_select(const SelectParams& p, int logits_f16, cudaStream_t strea
         set_last_error("soft_select: interleaved noise must be 16-byte aligned"); return PLZ_ERR_BAD_ALIGN;
     }
     const bool nfast = (p.ls_n == 1);
-    if (nfast) {
+    if (nfast && logits_f16 && p.packed && !p.w_soft && p.K % 32 == 0 && p.N % 8 == 0 && p.ls_k % 8 == 0 && p.ls_p % 8 == 0 && !((uintptr_t)p.logits & 15) &&
+        !((uintptr_t)p.packed & 7) && p.pitch % 8 == 0) {
+        select_planar_half_kernel<<<dim3((p.N + 63) / 64, (p.K / 4 + 31) / 32), 256, 0, stream>>>(p);
+    } else if (nfast) {
         dim3 grid((p.N + 31) / 32, ((p.K + 3) / 4 + 31) / 32);
         if (logits_f16) soft_select_nfast_kernel<__half><<<grid, 256, 0, stream>>>(p);
         else soft_select_nfast_kernel<float><<<grid, 256, 0, stream>>>(p);
