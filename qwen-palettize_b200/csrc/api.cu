@@ -355,7 +355,7 @@ int32_t plz_soft_select(const plz_weight_t* w, const plz_logits_t* logits, const
     SelectParams p = {};
     p.logits = logits->ptr; p.ls_n = logits->s_n; p.ls_k = logits->s_k; p.ls_p = logits->s_p;
     if (noise) { p.noise = noise->ptr; p.ns_n = noise->s_n; p.ns_k = noise->s_k; p.ns_p = noise->s_p; p.noise_mode = noise->mode; p.seed = noise->seed; }
-    p.inv_tau = 1.0f / tau;
+    p.scale = soft_scale(tau);
     p.palette = (const __nv_bfloat16*)w->palette; p.gs_n = w->gs_n; p.gs_k = w->gs_k; p.n_kgroups = w->K / w->gs_k;
     p.N = w->N; p.K = w->K;
     p.packed = want_packed ? (uint8_t*)const_cast<void*>(w->packed) : nullptr; p.pitch = w->packed_pitch;

@@ -168,10 +168,6 @@ __device__ __forceinline__ void select_one(const SelectParams& p, int n, int k, 
 #pragma unroll
                 for (int q = 0; q < 4; ++q) g[q] = __ldcs(p.noise + no + q * p.ns_p);
             }
-        } else if (p.noise_mode == NOISE_HASH) {
-            const uint32_t e = ((uint32_t)k * (uint32_t)p.N + (uint32_t)n) * 4u;
-#pragma unroll
-            for (int q = 0; q < 4; ++q) g[q] = gumbel_hash(p.seed, e + q);
         }
         const long long pg = ((long long)(n / p.gs_n) * p.n_kgroups + k / p.gs_k) * 4;
         const uint2 praw = __ldg(reinterpret_cast<const uint2*>(p.palette + pg));
@@ -180,7 +176,10 @@ __device__ __forceinline__ void select_one(const SelectParams& p, int n, int k, 
         c[1] = __uint_as_float(praw.x & 0xFFFF0000u);
         c[2] = __uint_as_float(praw.y << 16);
         c[3] = __uint_as_float(praw.y & 0xFFFF0000u);
-        const Soft4 s = soft4(l, g, c, p.inv_tau);
+        f32x2 z[2] = {pair2(l[0] + g[0], l[1] + g[1]), pair2(l[2] + g[2], l[3] + g[3])};
+        if (p.noise_mode == NOISE_HASH) add_gumbel_hash(z, p.seed, ((uint32_t)k * (uint32_t)p.N + (uint32_t)n) * 4u);
+        const f32x2 c2[2] = {pair2(c[0], c[1]), pair2(c[2], c[3])};
+        const Soft4 s = soft4(z, c2, p.scale);
         const __nv_bfloat16 b = __float2bfloat16_rn(s.w_soft);
         wsoft_bits = *reinterpret_cast<const uint16_t*>(&b);
     }

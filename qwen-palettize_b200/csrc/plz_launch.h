@@ -90,6 +90,7 @@ struct TnArgs {
     float tau;
     const void* palette; float* dpalette; int gs_n, gs_k, n_kgroups;
     const void* packed; long long packed_pitch;
+    void* pack_out;  // EPI_SOFT, rows_are_k: optional, receives the packed argmax indices of the logits (pitch packed_pitch)
     int sm_count;
     // optional side jobs appended to a dW launch: out[r, j] += sum_m S[m, r] * (q_is_p ? P : Q)[m, j]
     const void* side_S[2]; long long side_ld[2]; int side_rank; int side_q_is_p[2];
@@ -121,7 +122,7 @@ extern int g_debug_smallm_variant;  // 0 = automatic choice, 1 = never use the m
 struct SelectParams {
     const void* logits; long long ls_n, ls_k, ls_p;
     const float* noise; long long ns_n, ns_k, ns_p;
-    int noise_mode; uint32_t seed; float inv_tau;
+    int noise_mode; uint32_t seed; float scale;   // soft_scale(tau)
     const __nv_bfloat16* palette; int gs_n, gs_k, n_kgroups;
     int N, K;
     uint8_t* packed; long long pitch;             // may be null

@@ -73,6 +73,45 @@ __device__ __forceinline__ void palette4(const __nv_bfloat16* palette, long long
     c[3] = __uint_as_float(praw.y & 0xFFFF0000u);
 }
 
+// The tensors' own arithmetic, one rounding per step: the index taken from P (hard_from_noisy) depends on every one of them where two entries are close,
+// so soft_math.cuh's fused form would change it.
+__device__ __forceinline__ float gumbel_hash(uint32_t seed, uint32_t idx) {
+    uint32_t x = seed ^ (idx * 0x9E3779B9u);
+    x ^= x >> 13;
+    x = x * 1103515245u + 12345u;
+    x ^= x >> 17;
+    x = x * 1103515245u + 12345u;
+    float u = (float)(x & 0xFFFFFFu) * (1.0f / 16777216.0f);
+    u = fmaxf(u, 1e-7f);
+    return -__logf(-__logf(u));
+}
+struct SoftSteps {
+    float P[4];
+    float w_soft;
+};
+__device__ __forceinline__ SoftSteps soft_steps(const float (&l)[4], const float (&g)[4], const float (&c)[4], float inv_tau) {
+    float z[4];
+#pragma unroll
+    for (int p = 0; p < 4; ++p) z[p] = (l[p] + g[p]) * inv_tau;
+    const float mx = fmaxf(fmaxf(z[0], z[1]), fmaxf(z[2], z[3]));
+    float e[4];
+    float sum = 0.f;
+#pragma unroll
+    for (int p = 0; p < 4; ++p) {
+        e[p] = __expf(z[p] - mx);
+        sum += e[p];
+    }
+    const float inv = __fdividef(1.0f, sum);
+    SoftSteps r;
+    r.w_soft = 0.f;
+#pragma unroll
+    for (int p = 0; p < 4; ++p) {
+        r.P[p] = e[p] * inv;
+        r.w_soft += r.P[p] * c[p];
+    }
+    return r;
+}
+
 // One thread per weight. Consecutive threads walk the axis along which the logits are contiguous.
 __global__ void __launch_bounds__(256) soft_weights_kernel(const __grid_constant__ PwTable t) {
     int li = 0;
@@ -94,7 +133,7 @@ __global__ void __launch_bounds__(256) soft_weights_kernel(const __grid_constant
         for (int q = 0; q < 4; ++q) g[q] = gumbel_hash(d.seed, e + q);
     }
     palette4(d.palette, (long long)(n / d.gs_n) * d.n_kgroups + k / d.gs_k, c);
-    const Soft4 s = soft4(l, g, c, t.inv_tau);
+    const SoftSteps s = soft_steps(l, g, c, t.inv_tau);
     if (d.P) store4(d.P, 1, (long long)n * d.p_n + (long long)k * d.p_k, d.p_p, s.P);
     if (d.w_soft) d.w_soft[(long long)n * d.ws_n + (long long)k * d.ws_k] = __float2bfloat16_rn(s.w_soft);
     if (d.w_hard) {

@@ -28,7 +28,8 @@ namespace plz {
 
 struct TnParams {
     int M, I, J;       // P is [M, I], Q is [M, J], D is [I, J]
-    int n_whole, n_items;  // items [0, n_whole) are whole 128 x 256 tiles, the rest 128 x 128 halves (last round)
+    int n_whole, n_items;  // items [0, n_whole) are whole 128 x 256 tiles, the rest parts of them (last round)
+    int tail_shift;        // 1: parts are halves, 128 x 128; 2: quarters
     int splits;        // EPI_STORE only: the m range is cut into `splits` chunks, results atomically added
     int m_chunk;       // rows of m per split (multiple of 64)
     // EPI_STORE
@@ -38,10 +39,11 @@ struct TnParams {
     long long ls_row, ls_col, ls_p;          // strides of the logits for D row, D col, plane
     const float* noise; long long ns_row, ns_col, ns_p;
     int noise_mode; uint32_t seed; int hashN;  // hash noise index = (k * hashN + n) * 4 + p
-    float inv_tau;
+    float scale;   // soft_scale(tau)
     const __nv_bfloat16* palette; float* dpalette;
     int gs_n, gs_k, n_kgroups;
     const uint8_t* packed; long long packed_pitch;  // EPI_HARD
+    uint8_t* pack_out;  // EPI_SOFT, rows = k: when given, the argmax of the logits goes here (packed, the same pitch)
     // Side jobs (the LoRA factor gradients): extra work items appended to the list, D[r, j] = sum_m S[m, r] * Qs[m, j]
     // with S a skinny [M, rank] matrix and Qs one of the two main operands; results are atomically added to `out`.
     struct Side {
@@ -49,7 +51,7 @@ struct TnParams {
         float* out; long long out_si, out_sj;
     } side[2];
     int n_side_items;
-    // Tail of the persistent schedule. After the whole tiles come the half tiles (one per work unit, n_items - n_whole of
+    // Tail of the persistent schedule (halves or quarters). After the whole tiles come the half tiles (one per work unit, n_items - n_whole of
     // them) and then the side items, which are dealt only to the units that did not get a half tile: tail slots that fall on
     // a unit with a half tile stay empty, so that no unit carries a half tile AND a second side item while others idle.
     // tail_free = units without a half tile (0: the side items simply follow the halves); n_total = items including holes.
@@ -75,43 +77,75 @@ constexpr uint32_t kTnABytes = 128 * 64 * 2;  // 2 boxes of [64 m][64 i]
 constexpr uint32_t kTnBBytes = 256 * 64 * 2;  // 4 boxes of [64 m][64 j]
 constexpr uint32_t kTnStageBytes = kTnABytes + kTnBBytes;
 constexpr uint32_t kTnRedBytes = 4 * 256 * 4 * 4;  // per-warp palette-gradient partials
-constexpr uint32_t kTnSmemBytes = kTnStages * kTnStageBytes + kTnRedBytes + 1024 + 256;
 // CTA-pair form (cta_group::2, one 256 x 256 tile per pair): each CTA stages its own 128 i columns and HALF of the j
 // columns, 32 KB per 64 rows of m, so the ring holds six stages; every CTA reads 2/3 of the operand bytes of the one-CTA
 // form for the same work, which matters because this product is bound by the L2 -> SM operand feed.
 constexpr int kTnStagesPair = 6;
 constexpr uint32_t kTnBBytesPair = 128 * 64 * 2;
 constexpr uint32_t kTnStageBytesPair = kTnABytes + kTnBBytesPair;
-constexpr uint32_t kTnSmemBytesPair = kTnStagesPair * kTnStageBytesPair + kTnRedBytes + 1024 + 256;
+// The soft epilogue reads 16 to 32 bytes of logits and noise per weight, ten times what the tile's operands are. Read in batches by the warps that
+// use them, nothing is in flight while a batch is computed: 1000 tokens of 9728 x 2560 took 277 us with a noise tensor, 4.3 TB/s. So
+// the warps request them ahead, by asynchronous copies into a ring of their own, across the tiles' ends, and the ring takes the room of some stages: 215 us, 5.6 TB/s.
+// Planar fp16 logits, 2048 tokens of 4096 x 2560: 120 -> 82 us.
+//   STAGED_NONE    operands of the epilogue read when they are needed
+//   STAGED_LOGITS  logits through the ring; STAGED_NOISE: logits and noise
+// rows = k: a slot of 16 bytes per thread, column and tensor (a thread reads back what it requested: no barrier).
+// rows = n, planar fp16 logits: the 32 rows of a warp are 64 bytes of a plane, 128 of the noise; lanes request 16 bytes, the warp reads all.
+enum Staged { STAGED_NONE = 0, STAGED_LOGITS = 1, STAGED_NOISE = 2 };
+constexpr int kRingCols = 2;   // columns requested at a time
+constexpr uint32_t row_ring_bytes(int ew) { return 128u * 32u * (uint32_t)ew; }   // eight slots a thread
+constexpr uint32_t planar_group_bytes(int staged) { return kRingCols * 4 * (64u + (staged == STAGED_NOISE ? 128u : 0u)); }
+constexpr int planar_groups(int staged) { return staged == STAGED_NOISE ? 3 : 8; }
+template <bool ROWS_K, bool PAIR, int EW, int STAGED>
+struct TnLayout {
+    static constexpr int kStages = STAGED != STAGED_NONE ? (PAIR ? (ROWS_K && EW <= 8 ? 5 : 4) : 3) : (PAIR ? kTnStagesPair : kTnStages);
+    static constexpr uint32_t kStageBytes = PAIR ? kTnStageBytesPair : kTnStageBytes;
+    static constexpr int kGroups = ROWS_K ? (int)(row_ring_bytes(EW) / (32 * EW * 16) / (kRingCols * (STAGED ? STAGED : 1))) : planar_groups(STAGED);
+    static constexpr uint32_t kGroupStride = ROWS_K ? kRingCols * STAGED * 32u * EW * 16u : planar_group_bytes(STAGED);
+    static constexpr uint32_t kRingBytes = STAGED == STAGED_NONE ? 0u : ROWS_K ? row_ring_bytes(EW) : EW * planar_groups(STAGED) * planar_group_bytes(STAGED);
+    static constexpr uint32_t kSmemBytes = kStages * kStageBytes + kRingBytes + kTnRedBytes + 1024 + 256;
+    static_assert(kSmemBytes <= 232448, "shared memory of a CTA");
+};
 
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, o);
     return v;
 }
+// 16 bytes to shared memory, zeros where bytes = 0 (nothing is read then)
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, uint32_t bytes) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 template <int EW>
 __device__ __forceinline__ void epi_bar_sync() { asm volatile("bar.sync 1, %0;" ::"n"(32 * EW) : "memory"); }
 
-template <int EPI, typename LogitT, bool ROWS_K, bool PAIR, int EW>
+template <int EPI, typename LogitT, bool ROWS_K, bool PAIR, int EW, int STAGED>
 __global__ void __launch_bounds__(tn_threads(EW), 1)
 tn_gemm_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant__ CUtensorMap tmQ,
                const __grid_constant__ CUtensorMap tmS0, const __grid_constant__ CUtensorMap tmS1, const TnParams p) {
-    constexpr int kBatch = 64 / EW;   // columns an epilogue warp has in flight
-    constexpr int kStages = PAIR ? kTnStagesPair : kTnStages;
-    constexpr uint32_t kBBytes = PAIR ? kTnBBytesPair : kTnBBytes;
-    constexpr uint32_t kStageBytes = kTnABytes + kBBytes;
+    using Layout = TnLayout<ROWS_K, PAIR, EW, STAGED>;
+    static_assert(STAGED == STAGED_NONE || EPI == EPI_SOFT, "only the soft epilogue reads logits");
+    static_assert(EPI != EPI_SOFT || !ROWS_K || STAGED != STAGED_NONE, "rows = k: logits always through the ring");
+    static_assert(STAGED == STAGED_NONE || ROWS_K || sizeof(LogitT) == 2, "rows = n: staged for planar fp16 logits");
+    constexpr int kBatch = STAGED != STAGED_NONE ? 4 : 64 / EW;   // columns an epilogue warp works on at a time
+    constexpr int kStages = Layout::kStages;
+    constexpr uint32_t kStageBytes = Layout::kStageBytes;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
     const uint32_t base = (raw + 1023u) & ~1023u;
     uint8_t* smem = smem_raw + (base - raw);
-    float* red = reinterpret_cast<float*>(smem + kStages * kStageBytes);
-    const uint32_t bar_base = base + kStages * kStageBytes + kTnRedBytes;
+    constexpr uint32_t kRedAt = kStages * kStageBytes + Layout::kRingBytes;
+    float* red = reinterpret_cast<float*>(smem + kRedAt);
+    const uint32_t bar_base = base + kRedAt + kTnRedBytes;
     auto full = [&](int s) { return bar_base + 8u * s; };
     auto empty = [&](int s) { return bar_base + 8u * (kStages + s); };
     auto acc_full = [&](int b) { return bar_base + 8u * (2 * kStages + b); };
     auto acc_empty = [&](int b) { return bar_base + 8u * (2 * kStages + 2 + b); };
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(
-        smem + kStages * kStageBytes + kTnRedBytes + 8 * (2 * kStages + 4));
+        smem + kRedAt + kTnRedBytes + 8 * (2 * kStages + 4));
     volatile uint32_t* abort_flag = tmem_slot + 1;
 
     const int warp = __shfl_sync(0xFFFFFFFFu, (int)(threadIdx.x >> 5), 0);   // uniform to the compiler too
@@ -181,9 +215,9 @@ tn_gemm_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant__ 
         }
         int t = item;
         if (item >= p.n_whole) {
-            t = p.n_whole + ((item - p.n_whole) >> 1);
-            c_off = ((item - p.n_whole) & 1) * 128;
-            c_num = 128;
+            t = p.n_whole + ((item - p.n_whole) >> p.tail_shift);
+            c_num = 256 >> p.tail_shift;
+            c_off = ((item - p.n_whole) & ((1 << p.tail_shift) - 1)) * c_num;
         }
         ti = t % tiles_i;
         const int r = t / tiles_i;
@@ -224,7 +258,7 @@ tn_gemm_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant__ 
                     const uint32_t sB = sA + kTnABytes;
                     // PAIR: the leader announces the bytes of both CTAs; each CTA's copies complete on the leader's barrier
                     if (!PAIR) mbar_arrive_expect_tx(full(s), kTnABytes + (uint32_t)c_num * 128u);
-                    else if (rank == 0) mbar_arrive_expect_tx(full(s), 2u * (kTnABytes + (uint32_t)c_mine * 128u));
+                    else if (rank == 0) mbar_arrive_expect_tx(full(s), 2u * (kTnABytes + (uint32_t)(c_mine < 64 ? 64 : c_mine) * 128u));   // boxes are 64 wide
                     const int m = m_begin + it * 64;
                     const CUtensorMap* m_skinny = (job == 0) ? &tmS0 : &tmS1;
                     const CUtensorMap* m_big = (job >= 0 && p.side[job].q_is_p) ? &tmP : &tmQ;
@@ -323,12 +357,88 @@ tn_gemm_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant__ 
         const int ew = warp - 2;  // 0..EW - 1
         bool ok = true;
         int lt = 0;
+        // requests of the ring: the next kRingCols columns of this warp's part, on to the next tile behind the last one. They run ahead of the columns
+        // that are worked on by the groups of the ring.
+        constexpr int kGroups = Layout::kGroups;
+        const uint32_t own_ring = base + kStages * kStageBytes +
+                                  (ROWS_K ? (threadIdx.x - 64) * 16u : (uint32_t)(warp - 2) * (Layout::kRingBytes / EW));
+        constexpr uint32_t kGroupStride = Layout::kGroupStride;
+        int rq_item = unit - n_units, rq_left = 0, rq_col = 0, rq_row = 0, group = 0;
+        const LogitT* rq_l = nullptr;
+        const float* rq_g = nullptr;
+        auto request = [&](int g) {
+            if constexpr (STAGED != STAGED_NONE) {
+                while (rq_left == 0 && rq_item < n_tiles) {
+                    rq_item += n_units;
+                    if (rq_item >= n_tiles) break;
+                    int sp, ti, tj, c_off, c_num, job;
+                    tile_coords(rq_item, sp, ti, tj, c_off, c_num, job);
+                    if (job == -2) { rq_item = n_tiles; break; }
+                    if (job >= 0) continue;       // a side item reads no logits
+                    const int part = c_num / (EW / 4);
+                    rq_left = part;
+                    rq_col = tj * 256 + c_off + col_part * part;
+                    if (ROWS_K) {
+                        rq_row = ti * 128 + lane_group * 32 + lane;
+                        if (rq_row >= p.I) { rq_left = 0; continue; }   // none of this warp's rows are there (K % 32 == 0)
+                        rq_l = reinterpret_cast<const LogitT*>(p.logits) + (long long)rq_row * p.ls_row + (long long)rq_col * p.ls_col;
+                        if (STAGED == STAGED_NOISE) rq_g = p.noise + (long long)rq_row * p.ns_row + (long long)rq_col * p.ns_col;
+                    } else {
+                        // lane = (column, plane, quarter of the 32 rows) of the logits, (plane, eighth) of either column of the noise
+                        rq_row = ti * 128 + lane_group * 32;
+                        rq_l = reinterpret_cast<const LogitT*>(p.logits) + (rq_row + (lane & 3) * 8) + (long long)(rq_col + (lane >> 4)) * p.ls_col + ((lane >> 2) & 3) * p.ls_p;
+                        if (STAGED == STAGED_NOISE) rq_g = p.noise + (rq_row + (lane & 7) * 4) + (long long)rq_col * p.ns_col + (lane >> 3) * p.ns_p;
+                    }
+                }
+                if (rq_left > 0) {
+                    const uint32_t at = own_ring + g * kGroupStride;
+                    if (ROWS_K) {
+#pragma unroll
+                        for (int c = 0; c < kRingCols; ++c) {
+                            if (rq_col + c < p.J) {     // a column that is not there is worked on with what lies in the slot, and goes nowhere
+                                cp_async16(at + c * STAGED * (32u * EW * 16u), rq_l + c * p.ls_col, 16u);
+                                if (STAGED == STAGED_NOISE) cp_async16(at + (c * STAGED + 1) * (32u * EW * 16u), rq_g + c * p.ns_col, 16u);
+                            }
+                        }
+                    } else {
+                        const bool valid = rq_row + (lane & 3) * 8 < p.I && rq_col + (lane >> 4) < p.J;
+                        cp_async16(at + lane * 16u, valid ? (const void*)rq_l : p.logits, valid ? 16u : 0u);
+                        if (STAGED == STAGED_NOISE) {
+#pragma unroll
+                            for (int c = 0; c < kRingCols; ++c) {
+                                const bool in = rq_row + (lane & 7) * 4 < p.I && rq_col + c < p.J;
+                                cp_async16(at + kRingCols * 256u + c * 512u + lane * 16u, in ? (const void*)(rq_g + c * p.ns_col) : (const void*)p.noise, in ? 16u : 0u);
+                            }
+                        }
+                    }
+                    rq_left -= kRingCols;
+                    rq_col += kRingCols;
+                    rq_l += kRingCols * p.ls_col;
+                    if (STAGED == STAGED_NOISE) rq_g += kRingCols * p.ns_col;
+                }
+                cp_async_commit();   // also when nothing is left: the waits count groups
+            }
+        };
+        if constexpr (STAGED != STAGED_NONE) {
+            for (int g = 0; g < kGroups; ++g) request(g);
+        }
         for (int t = unit; t < n_tiles && ok; t += n_units, ++lt) {
             int sp, ti, tj, c_off, c_num, job, m_begin, nkb;
             tile_coords(t, sp, ti, tj, c_off, c_num, job);
             if (job == -2) break;
             m_range(sp, job, m_begin, nkb);
             const int buf = lt & 1;
+            if (EPI == EPI_SOFT && ROWS_K && job < 0) {
+                // the palettes of this warp's columns, in the places of `red` that their partial sums take later
+                const int part = c_num / (EW / 4), first = col_part * part, kgi = (ti * 128 < p.I ? ti * 128 : 0) / p.gs_k;
+                for (int c = lane; c < part; c += 32) {
+                    const int n = tj * 256 + c_off + first + c;
+                    const uint2 raw = n < p.J ? __ldg(reinterpret_cast<const uint2*>(p.palette + ((long long)n * p.n_kgroups + kgi) * 4)) : make_uint2(0u, 0u);
+                    *reinterpret_cast<float4*>(red + (lane_group * 256 + first + c) * 4) =
+                        make_float4(__uint_as_float(raw.x << 16), __uint_as_float(raw.x & 0xFFFF0000u), __uint_as_float(raw.y << 16), __uint_as_float(raw.y & 0xFFFF0000u));
+                }
+                __syncwarp();
+            }
             ok = mbar_wait(acc_full(buf), (lt >> 1) & 1, abort_flag, p.status, ST_TIMEOUT_ACCUM, 2);
             if (!ok) break;
             tc_fence_after_sync();
@@ -362,87 +472,95 @@ tn_gemm_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant__ 
                 // rows n, each with its own palette. The palette gradient of a column is a sum over lanes: the
                 // partials of a batch (kBatch columns x 4 entries) are reduced with a transposing butterfly.
                 const int k = row;
-                const int kgi = (row_ok ? k : 0) / p.gs_k;
-                // running addresses of the batch's first column
-                const float* lcol = reinterpret_cast<const float*>(p.logits) + (long long)k * p.ls_row + (long long)colbase * p.ls_col;
+                // running address of the batch's first column
                 float* dcol = p.dlogits ? reinterpret_cast<float*>(p.dlogits) + (long long)k * p.ls_row + (long long)colbase * p.ls_col : nullptr;
-                const float* ncol = p.noise ? p.noise + (long long)k * p.ns_row + (long long)colbase * p.ns_col : nullptr;
-                const long long pal_step = 4ll * p.n_kgroups;
-                const __nv_bfloat16* pcol = p.palette + (long long)colbase * pal_step + 4 * kgi;
+                if (EPI == EPI_SOFT && !row_ok) {     // all of a warp's rows are there or none
+                    for (int c = lane; c < wcols; c += 32) *reinterpret_cast<float4*>(red + (lane_group * 256 + col_part * wcols + c) * 4) = make_float4(0.f, 0.f, 0.f, 0.f);
+                }
 #pragma unroll 1
-                for (int c0 = 0; c0 < wcols; c0 += kBatch) {
+                for (int c0 = EPI == EPI_SOFT && !row_ok ? wcols : 0; c0 < wcols; c0 += kBatch) {
                     const int nb = colbase + c0;  // first n of the batch
-                    // fused reduce-scatter: the rows of a batch have one owner (rows_per_rank % 8 == 0); its buffer, this
-                    // rank's slot (or the accumulator) and this thread's k folded into one base pointer per batch
-                    float* sbase = nullptr;
-                    if (p.world > 1 && nb < p.J) {
-                        const int owner = nb / p.rows_per_rank;
-                        sbase = p.peer_stage[owner] + (p.scatter_add ? 0ll : (long long)p.rank * p.shard_elems) +
-                                ((long long)(nb - owner * p.rows_per_rank) * p.I + k) * 4;
-                    }
-                    float4 lv[kBatch], gv[kBatch];
-                    uint2 praw[kBatch];
-                    uint32_t hbyte[kBatch];
-                    // ---- phase 1: issue every load of the batch
+                    float part[4 * kBatch];
+                    if constexpr (EPI == EPI_SOFT) {
+                        // fused reduce-scatter: the rows of a batch have one owner (rows_per_rank % 8 == 0); its buffer, this
+                        // rank's slot (or the accumulator) and this thread's k folded into one base pointer per batch
+                        float* sbase = nullptr;
+                        if (p.world > 1 && nb < p.J) {
+                            const int owner = nb / p.rows_per_rank;
+                            sbase = p.peer_stage[owner] + (p.scatter_add ? 0ll : (long long)p.rank * p.shard_elems) +
+                                    ((long long)(nb - owner * p.rows_per_rank) * p.I + k) * 4;
+                        }
+                        uint32_t v[kBatch];
+                        tmem_ld_cols(trow + c0, v);
+                        uint2 picked = make_uint2(0u, 0u);   // lane c: the 32 indices of column c, packed
 #pragma unroll
-                    for (int c = 0; c < kBatch; ++c) {
-                        const bool valid = row_ok && nb + c < p.J;
-                        lv[c] = make_float4(0.f, 0.f, 0.f, 0.f);
-                        gv[c] = make_float4(0.f, 0.f, 0.f, 0.f);
-                        praw[c] = make_uint2(0u, 0u);
-                        hbyte[c] = 0;
-                        if (valid) {
-                            if (EPI == EPI_SOFT) {
-                                praw[c] = __ldg(reinterpret_cast<const uint2*>(pcol + c * pal_step));
-                                lv[c] = __ldcs(reinterpret_cast<const float4*>(lcol + c * p.ls_col));
-                                if (p.noise_mode == NOISE_TENSOR) gv[c] = __ldcs(reinterpret_cast<const float4*>(ncol + c * p.ns_col));
-                            } else {
-                                hbyte[c] = __ldg(p.packed + (long long)(nb + c) * p.packed_pitch + (k >> 2));
+                        for (int h = 0; h < kBatch / kRingCols; ++h) {
+                            cp_async_wait<kGroups - 1>();
+                            const uint8_t* slot = smem + (own_ring - base) + group * kGroupStride;
+                            ulonglong2 lv[kRingCols], gv[kRingCols];   // entries 0 1 | 2 3
+#pragma unroll
+                            for (int c = 0; c < kRingCols; ++c) {
+                                lv[c] = *reinterpret_cast<const ulonglong2*>(slot + c * STAGED * (32u * EW * 16u));
+                                if (STAGED == STAGED_NOISE) gv[c] = *reinterpret_cast<const ulonglong2*>(slot + (c * STAGED + 1) * (32u * EW * 16u));
+                            }
+                            request(group);
+                            group = group + 1 == kGroups ? 0 : group + 1;
+#pragma unroll
+                            for (int cc = 0; cc < kRingCols; ++cc) {
+                                const int c = h * kRingCols + cc, n = nb + c;
+                                const bool valid = n < p.J;
+                                // rows and columns beyond the operands came as zeros, so their sums are zero
+                                const f32x2 dw = pair2(__uint_as_float(v[c]), __uint_as_float(v[c]));
+                                const ulonglong2 praw = *reinterpret_cast<const ulonglong2*>(red + (lane_group * 256 + col_part * wcols + c0 + c) * 4);
+                                const f32x2 cp[2] = {praw.x, praw.y};
+                                if (p.pack_out != nullptr) {
+                                    float l[4];
+                                    split2(lv[cc].x, l[0], l[1]);
+                                    split2(lv[cc].y, l[2], l[3]);
+                                    const uint32_t idx = (uint32_t)argmax4_first(l[0], l[1], l[2], l[3]) << (2 * (lane & 15));
+                                    const uint32_t lo = __reduce_or_sync(0xFFFFFFFFu, lane < 16 ? idx : 0u), hi = __reduce_or_sync(0xFFFFFFFFu, lane < 16 ? 0u : idx);
+                                    if (lane == c) picked = make_uint2(lo, hi);
+                                }
+                                f32x2 z[2] = {lv[cc].x, lv[cc].y};
+                                if (STAGED == STAGED_NOISE) { z[0] = add2(z[0], gv[cc].x); z[1] = add2(z[1], gv[cc].y); }
+                                else if (p.noise_mode == NOISE_HASH) add_gumbel_hash(z, p.seed, ((uint32_t)k * (uint32_t)p.hashN + (uint32_t)n) * 4u);
+                                const Soft4 s4 = soft4(z, cp, p.scale);
+                                const f32x2 less = pair2(-s4.w_soft, -s4.w_soft);
+                                const f32x2 p0 = mul2(dw, s4.P[0]), p1 = mul2(dw, s4.P[1]);
+                                split2(p0, part[c * 4], part[c * 4 + 1]);
+                                split2(p1, part[c * 4 + 2], part[c * 4 + 3]);
+                                float dl[4];
+                                split2(mul2(p0, add2(cp[0], less)), dl[0], dl[1]);
+                                split2(mul2(p1, add2(cp[1], less)), dl[2], dl[3]);
+                                if (valid && p.world > 1) {
+                                    // plain (non-atomic) 16-byte store into the owner's staging slot of this rank: the 32 lanes
+                                    // of the warp cover 512 contiguous bytes there, peer or local alike
+                                    float* dst = sbase + (long long)c * p.I * 4;
+                                    if (p.scatter_add) {
+                                        asm volatile("red.relaxed.sys.global.add.v4.f32 [%0], {%1, %2, %3, %4};"
+                                                     :: "l"(dst), "f"(dl[0]), "f"(dl[1]), "f"(dl[2]), "f"(dl[3]) : "memory");
+                                    } else {
+                                        *reinterpret_cast<float4*>(dst) = make_float4(dl[0], dl[1], dl[2], dl[3]);
+                                    }
+                                } else if (valid && dcol != nullptr)
+                                    __stcs(reinterpret_cast<float4*>(dcol + c * p.ls_col), make_float4(dl[0], dl[1], dl[2], dl[3]));
                             }
                         }
-                    }
-                    uint32_t v[kBatch];
-                    tmem_ld_cols(trow + c0, v);
-                    // ---- phase 2: arithmetic and stores
-                    float part[4 * kBatch];
+                        if (p.pack_out != nullptr) {
+                            const int k0 = ti * 128 + lane_group * 32;
+                            if (lane < kBatch && nb + lane < p.J)
+                                *reinterpret_cast<uint2*>(p.pack_out + (long long)(nb + lane) * p.packed_pitch + (k0 >> 2)) = picked;
+                        }
+                    } else {
+                        uint32_t hbyte[kBatch];
 #pragma unroll
-                    for (int c = 0; c < kBatch; ++c) {
-                        const int n = nb + c;
-                        const bool valid = row_ok && n < p.J;
-                        const float dw = valid ? __uint_as_float(v[c]) : 0.f;
-                        if (EPI == EPI_SOFT) {
-                            float cp[4], l[4], g[4];
-                            cp[0] = __uint_as_float(praw[c].x << 16);
-                            cp[1] = __uint_as_float(praw[c].x & 0xFFFF0000u);
-                            cp[2] = __uint_as_float(praw[c].y << 16);
-                            cp[3] = __uint_as_float(praw[c].y & 0xFFFF0000u);
-                            l[0] = lv[c].x; l[1] = lv[c].y; l[2] = lv[c].z; l[3] = lv[c].w;
-                            g[0] = gv[c].x; g[1] = gv[c].y; g[2] = gv[c].z; g[3] = gv[c].w;
-                            if (p.noise_mode == NOISE_HASH) {
-                                const uint32_t e = ((uint32_t)k * (uint32_t)p.hashN + (uint32_t)n) * 4u;
+                        for (int c = 0; c < kBatch; ++c)
+                            hbyte[c] = row_ok && nb + c < p.J ? __ldg(p.packed + (long long)(nb + c) * p.packed_pitch + (k >> 2)) : 0u;
+                        uint32_t v[kBatch];
+                        tmem_ld_cols(trow + c0, v);
 #pragma unroll
-                                for (int q = 0; q < 4; ++q) g[q] = gumbel_hash(p.seed, e + q);
-                            }
-                            const Soft4 s4 = soft4(l, g, cp, p.inv_tau);
-                            float dl[4];
-#pragma unroll
-                            for (int q = 0; q < 4; ++q) {
-                                part[c * 4 + q] = dw * s4.P[q];
-                                dl[q] = part[c * 4 + q] * (cp[q] - s4.w_soft);
-                            }
-                            if (valid && p.world > 1) {
-                                // plain (non-atomic) 16-byte store into the owner's staging slot of this rank: the 32 lanes
-                                // of the warp cover 512 contiguous bytes there, peer or local alike
-                                float* dst = sbase + (long long)c * p.I * 4;
-                                if (p.scatter_add) {
-                                    asm volatile("red.relaxed.sys.global.add.v4.f32 [%0], {%1, %2, %3, %4};"
-                                                 :: "l"(dst), "f"(dl[0]), "f"(dl[1]), "f"(dl[2]), "f"(dl[3]) : "memory");
-                                } else {
-                                    *reinterpret_cast<float4*>(dst) = make_float4(dl[0], dl[1], dl[2], dl[3]);
-                                }
-                            } else if (valid && dcol != nullptr)
-                                __stcs(reinterpret_cast<float4*>(dcol + c * p.ls_col), make_float4(dl[0], dl[1], dl[2], dl[3]));
-                        } else {
+                        for (int c = 0; c < kBatch; ++c) {
+                            const float dw = row_ok && nb + c < p.J ? __uint_as_float(v[c]) : 0.f;
                             const int idx = (hbyte[c] >> (2 * (k & 3))) & 3;
 #pragma unroll
                             for (int q = 0; q < 4; ++q) part[c * 4 + q] = (q == idx) ? dw : 0.f;
@@ -456,19 +574,19 @@ tn_gemm_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant__ 
                         for (int s = 16, h = kVals / 2; s >= 1; s >>= 1, h >>= 1) {
                             const bool up = (lane & s) != 0;
                             if (h == 0) part[0] += __shfl_xor_sync(0xFFFFFFFFu, part[0], s);
+                            float got[kVals / 2];
 #pragma unroll
                             for (int j = 0; j < h; ++j) {
-                                const float send = up ? part[j] : part[j + h];
-                                const float keep = up ? part[j + h] : part[j];
-                                part[j] = keep + __shfl_xor_sync(0xFFFFFFFFu, send, s);
+                                got[j] = __shfl_xor_sync(0xFFFFFFFFu, up ? part[j] : part[j + h], s);
+                                part[j] = up ? part[j + h] : part[j];
                             }
+#pragma unroll
+                            for (int j = 0; j + 1 < h; j += 2) split2(add2(pair2(part[j], part[j + 1]), pair2(got[j], got[j + 1])), part[j], part[j + 1]);
+                            if (h == 1) part[0] += got[0];
                         }
                         if (lane % (32 / kVals) == 0) red[(lane_group * 256 + col_part * wcols + c0) * 4 + lane / (32 / kVals)] = part[0];
                     }
-                    lcol += kBatch * p.ls_col;
-                    pcol += kBatch * pal_step;
                     if (dcol != nullptr) dcol += kBatch * p.ls_col;
-                    if (ncol != nullptr) ncol += kBatch * p.ns_col;
                 }
                 if (p.dpalette != nullptr) {
                     epi_bar_sync<EW>();
@@ -497,20 +615,82 @@ tn_gemm_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant__ 
                 const int n = row;
                 const int k_tile0 = tj * 256 + c_off;
                 const long long pg = ((long long)((row_ok ? n : 0) / p.gs_n) * p.n_kgroups + k_tile0 / p.gs_k) * 4;
-                float cpal[4] = {0.f, 0.f, 0.f, 0.f};
+                f32x2 cpal[2] = {0ull, 0ull};
                 if (EPI == EPI_SOFT) {
                     const uint2 praw = __ldg(reinterpret_cast<const uint2*>(p.palette + pg));
-                    cpal[0] = __uint_as_float(praw.x << 16);
-                    cpal[1] = __uint_as_float(praw.x & 0xFFFF0000u);
-                    cpal[2] = __uint_as_float(praw.y << 16);
-                    cpal[3] = __uint_as_float(praw.y & 0xFFFF0000u);
+                    cpal[0] = pair2(__uint_as_float(praw.x << 16), __uint_as_float(praw.x & 0xFFFF0000u));
+                    cpal[1] = pair2(__uint_as_float(praw.y << 16), __uint_as_float(praw.y & 0xFFFF0000u));
                 }
+                float acc[4] = {0.f, 0.f, 0.f, 0.f};
+                f32x2 acc2[2] = {0ull, 0ull};
+                if constexpr (STAGED != STAGED_NONE) {
+                    // planar fp16: odd and even lanes exchange halves, so that each stores two planes of the pair of rows, 4 bytes at a time
+                    const bool odd = (lane & 1) != 0;
+                    __half* dcol = p.dlogits ? reinterpret_cast<__half*>(p.dlogits) + (n - (odd ? 1 : 0)) + (long long)colbase * p.ls_col + (odd ? 2 : 0) * p.ls_p : nullptr;
+#pragma unroll 1
+                    for (int c0 = 0; c0 < wcols; c0 += kBatch) {
+                        uint32_t v[kBatch];
+                        tmem_ld_cols(trow + c0, v);
+#pragma unroll
+                        for (int h = 0; h < kBatch / kRingCols; ++h) {
+                            cp_async_wait<kGroups - 1>();
+                            __syncwarp();
+                            const uint8_t* slot = smem + (own_ring - base) + group * kGroupStride;
+                            f32x2 z[kRingCols][2];
+#pragma unroll
+                            for (int c = 0; c < kRingCols; ++c) {
+                                float l[4], g[4];
+#pragma unroll
+                                for (int q = 0; q < 4; ++q) {
+                                    l[q] = __half2float(*reinterpret_cast<const __half*>(slot + (c * 4 + q) * 64 + lane * 2));
+                                    g[q] = STAGED == STAGED_NOISE ? *reinterpret_cast<const float*>(slot + kRingCols * 256 + (c * 4 + q) * 128 + lane * 4) : 0.f;
+                                }
+                                z[c][0] = pair2(l[0], l[1]);
+                                z[c][1] = pair2(l[2], l[3]);
+                                if (STAGED == STAGED_NOISE) { z[c][0] = add2(z[c][0], pair2(g[0], g[1])); z[c][1] = add2(z[c][1], pair2(g[2], g[3])); }
+                            }
+                            __syncwarp();
+                            request(group);
+                            group = group + 1 == kGroups ? 0 : group + 1;
+#pragma unroll
+                            for (int c = 0; c < kRingCols; ++c) {
+                                const int k = colbase + c0 + h * kRingCols + c;
+                                const bool valid = row_ok && k < p.J;
+                                const float dwv = valid ? __uint_as_float(v[h * kRingCols + c]) : 0.f;
+                                const f32x2 dw = pair2(dwv, dwv);
+                                if (STAGED == STAGED_LOGITS && p.noise_mode == NOISE_HASH)
+                                    add_gumbel_hash(z[c], p.seed, ((uint32_t)k * (uint32_t)p.hashN + (uint32_t)n) * 4u);
+                                const Soft4 s4 = soft4(z[c], cpal, p.scale);
+                                const f32x2 less = pair2(-s4.w_soft, -s4.w_soft);
+                                const f32x2 p0 = mul2(dw, s4.P[0]), p1 = mul2(dw, s4.P[1]);
+                                acc2[0] = add2(acc2[0], p0);
+                                acc2[1] = add2(acc2[1], p1);
+                                float dl[4];
+                                split2(mul2(p0, add2(cpal[0], less)), dl[0], dl[1]);
+                                split2(mul2(p1, add2(cpal[1], less)), dl[2], dl[3]);
+                                if (p.dlogits != nullptr) {
+                                    const __half2 ab = __floats2half2_rn(dl[0], dl[1]), cd = __floats2half2_rn(dl[2], dl[3]);
+                                    const uint32_t lo = *reinterpret_cast<const uint32_t*>(&ab), hi = *reinterpret_cast<const uint32_t*>(&cd);
+                                    const uint32_t got = __shfl_xor_sync(0xFFFFFFFFu, odd ? lo : hi, 1);
+                                    const uint32_t a = odd ? got : lo, b = odd ? hi : got;   // the even row's and the odd row's two planes
+                                    if (valid) {
+                                        __half* d = dcol + (long long)(h * kRingCols + c) * p.ls_col;
+                                        __stcs(reinterpret_cast<unsigned int*>(d), prmt_raw(a, b, 0x5410u));
+                                        __stcs(reinterpret_cast<unsigned int*>(d + p.ls_p), prmt_raw(a, b, 0x7632u));
+                                    }
+                                }
+                            }
+                        }
+                        if (dcol != nullptr) dcol += kBatch * p.ls_col;
+                    }
+                    split2(acc2[0], acc[0], acc[1]);
+                    split2(acc2[1], acc[2], acc[3]);
+                } else {
                 // running addresses of the batch's first column
                 const LogitT* lcol = reinterpret_cast<const LogitT*>(p.logits) + (long long)n * p.ls_row + (long long)colbase * p.ls_col;
                 LogitT* dcol = p.dlogits ? reinterpret_cast<LogitT*>(p.dlogits) + (long long)n * p.ls_row + (long long)colbase * p.ls_col : nullptr;
                 const float* ncol = p.noise ? p.noise + (long long)n * p.ns_row + (long long)colbase * p.ns_col : nullptr;
                 const uint8_t* prow = p.packed ? p.packed + (long long)n * p.packed_pitch : nullptr;
-                float acc[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll 1
                 for (int c0 = 0; c0 < wcols; c0 += kBatch) {
                     const int kb = colbase + c0;  // first k of the batch
@@ -555,20 +735,16 @@ tn_gemm_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant__ 
                         const bool valid = row_ok && (kb + c) < p.J;
                         const float dw = valid ? __uint_as_float(v[c]) : 0.f;
                         if (EPI == EPI_SOFT) {
-                            if (p.noise_mode == NOISE_HASH) {
-                                const uint32_t e = ((uint32_t)(kb + c) * (uint32_t)p.hashN + (uint32_t)n) * 4u;
-#pragma unroll
-                                for (int q = 0; q < 4; ++q) g[c][q] = gumbel_hash(p.seed, e + q);
-                            }
-                            const float lf[4] = {to_f32(l[c][0]), to_f32(l[c][1]), to_f32(l[c][2]), to_f32(l[c][3])};
-                            const Soft4 s4 = soft4(lf, g[c], cpal, p.inv_tau);
+                            f32x2 z[2] = {pair2(to_f32(l[c][0]) + g[c][0], to_f32(l[c][1]) + g[c][1]), pair2(to_f32(l[c][2]) + g[c][2], to_f32(l[c][3]) + g[c][3])};
+                            if (p.noise_mode == NOISE_HASH) add_gumbel_hash(z, p.seed, ((uint32_t)(kb + c) * (uint32_t)p.hashN + (uint32_t)n) * 4u);
+                            const Soft4 s4 = soft4(z, cpal, p.scale);
+                            const f32x2 w2 = pair2(dw, dw), less = pair2(-s4.w_soft, -s4.w_soft);
+                            const f32x2 p0 = mul2(w2, s4.P[0]), p1 = mul2(w2, s4.P[1]);
+                            acc2[0] = add2(acc2[0], p0);
+                            acc2[1] = add2(acc2[1], p1);
                             float dl[4];
-#pragma unroll
-                            for (int q = 0; q < 4; ++q) {
-                                const float cq = dw * s4.P[q];
-                                acc[q] += cq;
-                                dl[q] = cq * (cpal[q] - s4.w_soft);
-                            }
+                            split2(mul2(p0, add2(cpal[0], less)), dl[0], dl[1]);
+                            split2(mul2(p1, add2(cpal[1], less)), dl[2], dl[3]);
                             if (valid && dcol != nullptr) {
                                 if (vec_l) {
                                     __stcs(reinterpret_cast<float4*>(reinterpret_cast<float*>(dcol + c * p.ls_col)), make_float4(dl[0], dl[1], dl[2], dl[3]));
@@ -586,6 +762,8 @@ tn_gemm_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant__ 
                     lcol += kBatch * p.ls_col;
                     if (dcol != nullptr) dcol += kBatch * p.ls_col;
                     if (ncol != nullptr) ncol += kBatch * p.ns_col;
+                }
+                if (EPI == EPI_SOFT) { split2(acc2[0], acc[0], acc[1]); split2(acc2[1], acc[2], acc[3]); }
                 }
                 if (p.dpalette != nullptr) {
                     if (p.gs_n == 1) {
@@ -632,6 +810,7 @@ tn_gemm_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant__ 
             __syncwarp();
             if (lane == 0) { if (PAIR) mbar_arrive_cluster(lead_acc_empty(buf)); else mbar_arrive(acc_empty(buf)); }
         }
+        if (STAGED != STAGED_NONE) cp_async_wait<0>();   // also after a give-up: nothing may still be on its way into this shared memory
     }
     tc_fence_before_sync();
     __syncthreads();
@@ -648,20 +827,18 @@ tn_gemm_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant__ 
 // host side
 // ---------------------------------------------------------------------------------------------
 
-// From this many tokens on the main loop of a tile (256 x 256, 0.33 us per 64 tokens) is longer than its soft epilogue with eight warps
-// (interleaved fp32 logits, 60 us), which then runs in its shadow. Measured at 9728 x 2560, noise tensor / sampled noise, eight against
-// sixteen warps: 512 tokens 320 / 336 against 288 / 260 us, 4096: 352 / 374 against 316 / 306, 8192: 435 / 443 against 417 / 410,
-// 10240: 493 / 491 against 488 / 483, 16384: 712 / 708 against 766 / -. The same line elsewhere, 8192 / 10240 tokens, noise tensor: 2560 x 9728 460 / 511 against 417 / 509, 4096 x 2560
-// 201 / 226 against 188 / 224, 1024 x 2560 93 / 101 against 82 / 89, 512 x 512 83 / 94 against 70 / 81. Planar fp16 logits (4096 x 2560, 2048 tokens) take 125 us per
-// tile with eight warps, longer than any main loop: 309 against 126 us, always sixteen. The hard epilogue has 45 against 40 us at
-// 512 tokens: always eight.
-constexpr int kTnLongLoop = 10241;
+// Epilogue warps of the interleaved soft epilogue: sixteen, or eight and a stage more for the main loop where that is what takes the time, in a launch of more
+// than one wave. us at 9728 x 2560, sixteen / eight warps (before the ring of requests: sixteen below 10241 tokens, else eight), noise tensor: 1000 tokens 215 (277),
+// 4096 tokens 273 / 295 (310), 6144 348 / 351 (355), 8192 422 / 391 (405), 10240 499 / 463 (483), 16384 - / 691 (738); sampled noise: 1000 tokens 183 (248), 4096 262 / 325 (294),
+// 8192 390 / 416 (402), 10240 474 / 468 (488), 16384 - / 694 (732). One wave (1024 x 2560), 10240 tokens: 107 / 109 (109) and 115 / 121 (114).
+// Planar fp16 logits: always sixteen. The hard epilogue has 45 us with sixteen against 40 at 512 tokens: always eight.
+constexpr int kTnLongLoopNoise = 7168, kTnLongLoop = 10241;
 
-template <int EPI, typename LogitT, bool ROWS_K, bool PAIR, int EW>
+template <int EPI, typename LogitT, bool ROWS_K, bool PAIR, int EW, int STAGED = STAGED_NONE>
 static int launch_tn_t(const TnArgs& a, const TnParams& p, const CUtensorMap& tmP, const CUtensorMap& tmQ,
                        const CUtensorMap& tmS0, const CUtensorMap& tmS1, int grid, cudaStream_t stream) {
-    auto kern = tn_gemm_kernel<EPI, LogitT, ROWS_K, PAIR, EW>;
-    constexpr uint32_t smem = PAIR ? kTnSmemBytesPair : kTnSmemBytes;
+    auto kern = tn_gemm_kernel<EPI, LogitT, ROWS_K, PAIR, EW, STAGED>;
+    constexpr uint32_t smem = TnLayout<ROWS_K, PAIR, EW, STAGED>::kSmemBytes;
     static bool attr_set[64] = {};
     int dev = 0;
     PLZ_CUDA_CHECK(cudaGetDevice(&dev));
@@ -693,7 +870,7 @@ int launch_tn_gemm(const TnArgs& a, cudaStream_t stream) {
     if ((rc = make_tmap_bf16(&tmQ, a.Q, a.M, a.J, a.ldq, 64, 64))) return rc;
     TnParams p = {};
     p.M = a.M; p.I = a.I; p.J = a.J;
-    p.splits = 1; p.m_chunk = ((a.M + 63) / 64) * 64;
+    p.splits = 1; p.m_chunk = ((a.M + 63) / 64) * 64; p.tail_shift = 1;
     if (a.epi == EPI_STORE) {
         if (!a.out) { set_last_error("tn_gemm: null output"); return PLZ_ERR_NULL; }
         int s = a.splits > 0 ? a.splits : 1;
@@ -726,10 +903,14 @@ int launch_tn_gemm(const TnArgs& a, cudaStream_t stream) {
         p.ls_row = a.ls_row; p.ls_col = a.ls_col; p.ls_p = a.ls_p;
         p.noise = a.noise; p.ns_row = a.ns_row; p.ns_col = a.ns_col; p.ns_p = a.ns_p;
         p.noise_mode = a.noise_mode; p.seed = a.seed; p.hashN = a.hashN;
-        p.inv_tau = 1.0f / a.tau;
+        p.scale = soft_scale(a.tau);
         p.palette = (const __nv_bfloat16*)a.palette; p.dpalette = a.dpalette;
         p.gs_n = a.gs_n; p.gs_k = a.gs_k; p.n_kgroups = a.n_kgroups;
         p.packed = (const uint8_t*)a.packed; p.packed_pitch = a.packed_pitch;
+        p.pack_out = (uint8_t*)a.pack_out;
+        if (a.pack_out && (a.epi != EPI_SOFT || !a.rows_are_k || a.I % 32 || ((uintptr_t)a.pack_out & 7) || (a.packed_pitch & 7))) {
+            set_last_error("tn_gemm: indices are written for interleaved fp32 logits, 8-byte aligned rows"); return PLZ_ERR_UNSUPPORTED;
+        }
         if (a.epi == EPI_SOFT) {
             if (!a.logits) { set_last_error("tn_gemm: null logits"); return PLZ_ERR_NULL; }
             if (a.noise_mode == NOISE_TENSOR && !a.noise) { set_last_error("tn_gemm: null noise"); return PLZ_ERR_NULL; }
@@ -798,9 +979,14 @@ int launch_tn_gemm(const TnArgs& a, cudaStream_t stream) {
         }
     }
     if (a.epi != EPI_STORE) {
-        // the last, partially filled round of the persistent schedule is cut into half tiles
+        // the last, partially filled round of the persistent schedule is cut into parts of tiles
         const int rem = tiles % grid;
-        if (tiles > grid && rem > 0 && 2 * rem <= grid) { p.n_whole = tiles - rem; p.n_items = p.n_whole + 2 * rem; }
+        if (tiles > grid && rem > 0 && 2 * rem <= grid) {
+            // quarters where the soft epilogue is the longer part (1000 tokens of 2560 x 9728 218 -> 209 us): a product of 64 columns feeds on as many bytes of P as
+            // one of 256, so a long main loop would not gain
+            p.tail_shift = a.epi == EPI_SOFT && a.M < kTnLongLoop && 4 * rem <= grid ? 2 : 1;
+            p.n_whole = tiles - rem; p.n_items = p.n_whole + (rem << p.tail_shift);
+        }
     }
     {
         int next = 0;      // side items are numbered from 0
@@ -824,14 +1010,24 @@ int launch_tn_gemm(const TnArgs& a, cudaStream_t stream) {
         }
     }
     const int ctas = pair ? 2 * grid : grid;
-#define PLZ_TN(EPI, T, ROWS_K, EW) \
-    return pair ? launch_tn_t<EPI, T, ROWS_K, true, EW>(a, p, tmP, tmQ, tmS0, tmS1, ctas, stream) : launch_tn_t<EPI, T, ROWS_K, false, EW>(a, p, tmP, tmQ, tmS0, tmS1, ctas, stream)
+#define PLZ_TN(EPI, T, ROWS_K, EW, STAGED) \
+    return pair ? launch_tn_t<EPI, T, ROWS_K, true, EW, STAGED>(a, p, tmP, tmQ, tmS0, tmS1, ctas, stream) : launch_tn_t<EPI, T, ROWS_K, false, EW, STAGED>(a, p, tmP, tmQ, tmS0, tmS1, ctas, stream)
     if (a.epi == EPI_STORE) return launch_tn_t<EPI_STORE, float, false, false, 8>(a, p, tmP, tmQ, tmS0, tmS1, ctas, stream);
-    if (a.epi == EPI_HARD) { if (a.rows_are_k) PLZ_TN(EPI_HARD, float, true, 8); else PLZ_TN(EPI_HARD, float, false, 8); }
+    if (a.epi == EPI_HARD) { if (a.rows_are_k) PLZ_TN(EPI_HARD, float, true, 8, STAGED_NONE); else PLZ_TN(EPI_HARD, float, false, 8, STAGED_NONE); }
     if (a.epi == EPI_SOFT) {
-        const bool long_loop = a.M >= kTnLongLoop;
-        if (!a.rows_are_k) { if (a.logits_f16) PLZ_TN(EPI_SOFT, __half, false, 16); else PLZ_TN(EPI_SOFT, float, false, 16); }
-        if (long_loop) PLZ_TN(EPI_SOFT, float, true, 8); else PLZ_TN(EPI_SOFT, float, true, 16);
+        const bool tensor = a.noise_mode == NOISE_TENSOR;
+        if (!a.rows_are_k) {
+            if (!a.logits_f16) PLZ_TN(EPI_SOFT, float, false, 16, STAGED_NONE);
+            // requests of 16 bytes along n: rows of the planes next to each other, every stride and address a multiple of 16 bytes
+            const bool lined = pair && a.ls_row == 1 && a.ls_col % 8 == 0 && a.ls_p % 8 == 0 && !((uintptr_t)a.logits & 15) && !((uintptr_t)a.dlogits & 15) && a.I % 8 == 0 &&
+                               (!tensor || (a.ns_row == 1 && a.ns_col % 4 == 0 && a.ns_p % 4 == 0 && !((uintptr_t)a.noise & 15)));
+            if (lined && tensor) return launch_tn_t<EPI_SOFT, __half, false, true, 16, STAGED_NOISE>(a, p, tmP, tmQ, tmS0, tmS1, ctas, stream);
+            if (lined) return launch_tn_t<EPI_SOFT, __half, false, true, 16, STAGED_LOGITS>(a, p, tmP, tmQ, tmS0, tmS1, ctas, stream);
+            PLZ_TN(EPI_SOFT, __half, false, 16, STAGED_NONE);
+        }
+        const bool long_loop = tiles > units && a.M >= (tensor ? kTnLongLoopNoise : kTnLongLoop);
+        if (tensor) { if (long_loop) PLZ_TN(EPI_SOFT, float, true, 8, STAGED_NOISE); else PLZ_TN(EPI_SOFT, float, true, 16, STAGED_NOISE); }
+        if (long_loop) PLZ_TN(EPI_SOFT, float, true, 8, STAGED_LOGITS); else PLZ_TN(EPI_SOFT, float, true, 16, STAGED_LOGITS);
     }
 #undef PLZ_TN
     set_last_error("tn_gemm: unknown epilogue %d", a.epi);
