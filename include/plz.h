@@ -121,6 +121,12 @@ int32_t plz_dequantize(const plz_weight_t* w, void* dst, int64_t d_n, int64_t d_
 int32_t plz_hard_fwd(const plz_weight_t* w, const void* x, int64_t ldx, int32_t M, const plz_lora_t* lora,
                      void* t, void* y, int64_t ldy, void* stream);
 
+/* The two halves of plz_hard_fwd for callers that want t early (plz_bwd_dw_soft_select needs it before the indices are there):
+ * plz_lora_down: t[M, rank] = scale * x A^T;  plz_hard_fwd_with_t: y = x W^T + t B^T with t as given (lora may be NULL). */
+int32_t plz_lora_down(const plz_lora_t* lora, const void* x, int64_t ldx, int32_t M, int32_t K, void* t, void* stream);
+int32_t plz_hard_fwd_with_t(const plz_weight_t* w, const void* x, int64_t ldx, int32_t M, const plz_lora_t* lora, const void* t,
+                            void* y, int64_t ldy, void* stream);
+
 /* About the bits of a result: they repeat from run to run, but a row's do not stay the same when the number of rows changes what kernel takes the call or how it
  * splits the reduction (at 16, 32, 64, 128 and 256 rows, and with plz_set_cta_limit): fp32 sums in another order, rounded once to bf16. The LoRA intermediates
  * t = scale * x A^T and dt = scale * dY B are the exception: their sums follow the reduction length alone, so that a step over all tokens and steps over parts
@@ -212,6 +218,12 @@ int32_t plz_bwd_dw_soft(const plz_weight_t* w, const void* x, int64_t ldx, const
 int32_t plz_bwd_dw_soft_lora(const plz_weight_t* w, const void* x, int64_t ldx, const void* dY, int64_t lddy, int32_t M,
                              const plz_logits_t* logits, const plz_noise_t* noise, float tau, void* dlogits, float* dpalette,
                              const void* t, const void* dt, int32_t rank, float* dA, float* dB, void* stream);
+/* plz_bwd_dw_soft_lora (rank = 0: without LoRA) that also writes the packed hard indices, argmax of the logits, into w->packed, as plz_soft_select with
+ * want_packed does: the gradient of a straight-through step does not depend on them, so a caller that has dY at hand reads the logits
+ * once instead of twice. In the layout of plz_bwd_dw_soft_scatter the launch itself writes them, in others a pass ahead of it. */
+int32_t plz_bwd_dw_soft_select(const plz_weight_t* w, const void* x, int64_t ldx, const void* dY, int64_t lddy, int32_t M,
+                               const plz_logits_t* logits, const plz_noise_t* noise, float tau, void* dlogits, float* dpalette,
+                               const void* t, const void* dt, int32_t rank, float* dA, float* dB, void* stream);
 /* Hard-mode palette gradient dPalette[group][idx[n,k]] += dW[n,k] (fp32, accumulated):
  * fused_lut_linear_bwd_grad_palette_kernel (scripts/fused_lut_kernel.cu:902-1127). */
 int32_t plz_bwd_dw_hard(const plz_weight_t* w, const void* x, int64_t ldx, const void* dY, int64_t lddy,

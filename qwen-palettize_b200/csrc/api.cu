@@ -230,6 +230,27 @@ int32_t plz_hard_fwd(const plz_weight_t* w, const void* x, int64_t ldx, int32_t 
     if ((rc = check_lora(lora, t))) return rc;
     cudaStream_t s = (cudaStream_t)stream;
     if (lora && (rc = lora_down(lora, x, ldx, M, w->K, t, s))) return rc;
+    return plz_hard_fwd_with_t(w, x, ldx, M, lora, t, y, ldy, stream);
+}
+
+int32_t plz_lora_down(const plz_lora_t* lora, const void* x, int64_t ldx, int32_t M, int32_t K, void* t, void* stream) {
+    if (!lora) { set_last_error("null LoRA descriptor"); return PLZ_ERR_NULL; }
+    if (M < 0 || K <= 0) { set_last_error("lora_down: bad shape"); return PLZ_ERR_BAD_SHAPE; }
+    if (M == 0) return PLZ_OK;
+    if (!x) { set_last_error("null activation pointer"); return PLZ_ERR_NULL; }
+    int rc = check_lora(lora, t);
+    if (rc) return rc;
+    return lora_down(lora, x, ldx, M, K, t, (cudaStream_t)stream);
+}
+
+int32_t plz_hard_fwd_with_t(const plz_weight_t* w, const void* x, int64_t ldx, int32_t M, const plz_lora_t* lora, const void* t,
+                            void* y, int64_t ldy, void* stream) {
+    int rc = check_weight(w, true);
+    if (rc) return rc;
+    if (M < 0) { set_last_error("negative M"); return PLZ_ERR_BAD_SHAPE; }
+    if (M == 0) return PLZ_OK;
+    if (!x || !y) { set_last_error("null activation pointer"); return PLZ_ERR_NULL; }
+    if ((rc = check_lora(lora, t))) return rc;
     LutGemmArgs g = {};
     g.bmode = B_DECODE_K; g.M = M; g.J = w->N; g.R = w->K;
     g.A = x; g.lda = ldx;
@@ -237,7 +258,7 @@ int32_t plz_hard_fwd(const plz_weight_t* w, const void* x, int64_t ldx, int32_t 
     g.gs_n = w->gs_n; g.gs_k = w->gs_k; g.Wn = w->N; g.Wk = w->K;
     if (lora) { g.r2 = lora->rank; g.A2 = t; g.lda2 = lora->rank; g.B2 = lora->B; g.ldb2 = lora->ldb; }
     g.out = y; g.ld_out = ldy; g.alpha = 1.0f; g.prof = g_prof_buffer;
-    return launch_lut_gemm(g, s);
+    return launch_lut_gemm(g, (cudaStream_t)stream);
 }
 
 // ---- allocation-free LoRA forward ---------------------------------------------------------------
@@ -449,10 +470,11 @@ static int bwd_dw_common(int epi, const plz_weight_t* w, const void* x, int64_t 
                          int32_t M, const plz_logits_t* logits, const plz_noise_t* noise, float tau, void* dlogits,
                          float* dpalette, void* stream, const void* t = nullptr, const void* dt = nullptr, int rank = 0,
                          float* dA = nullptr, float* dB = nullptr, float* const* peer_stage = nullptr, int world = 1,
-                         int my_rank = 0, int scatter_add = 0) {
-    int rc = check_weight(w, epi == EPI_HARD);
+                         int my_rank = 0, int scatter_add = 0, bool select = false) {
+    int rc = check_weight(w, epi == EPI_HARD || select);
     if (rc) return rc;
     if (M < 0) { set_last_error("negative M"); return PLZ_ERR_BAD_SHAPE; }
+    if (select && M == 0) return plz_soft_select(w, logits, nullptr, tau, 1, nullptr, 0, 0, stream);
     if (M == 0) {
         // A rank without tokens contributes zeros. In the slot form of the fused reduce-scatter its slots would otherwise
         // keep the previous step's partials, which the owners' slot reduction would add again: clear them.
@@ -478,6 +500,9 @@ static int bwd_dw_common(int epi, const plz_weight_t* w, const void* x, int64_t 
                      (!noise || noise->mode != 1 || (noise->s_p == 1 && noise->s_k < noise->s_n));
     }
     a.rows_are_k = rows_are_k ? 1 : 0;
+    // the indices come out of the epilogue where its warps walk k (w->K % 64 == 0: a warp's 32 rows are 8 whole bytes), elsewhere from a pass of their own
+    if (select && rows_are_k) a.pack_out = const_cast<void*>(w->packed);
+    else if (select && (rc = plz_soft_select(w, logits, nullptr, tau, 1, nullptr, 0, 0, stream))) return rc;
     if (rows_are_k) { a.I = w->K; a.J = w->N; a.P = x; a.ldp = ldx; a.Q = dY; a.ldq = lddy; }
     else { a.I = w->N; a.J = w->K; a.P = dY; a.ldp = lddy; a.Q = x; a.ldq = ldx; }
     if (epi == EPI_SOFT) {
@@ -532,6 +557,15 @@ int32_t plz_bwd_dw_soft_lora(const plz_weight_t* w, const void* x, int64_t ldx, 
     if (rank <= 0 || rank > 64 || rank % 8) { set_last_error("LoRA rank %d must be a multiple of 8 in [8, 64]", rank); return PLZ_ERR_BAD_SHAPE; }
     if ((dA && !dt) || (dB && !t)) { set_last_error("bwd_dw_soft_lora: dA needs dt and dB needs t"); return PLZ_ERR_NULL; }
     return bwd_dw_common(EPI_SOFT, w, x, ldx, dY, lddy, M, logits, noise, tau, dlogits, dpalette, stream, t, dt, rank, dA, dB);
+}
+
+int32_t plz_bwd_dw_soft_select(const plz_weight_t* w, const void* x, int64_t ldx, const void* dY, int64_t lddy, int32_t M,
+                               const plz_logits_t* logits, const plz_noise_t* noise, float tau, void* dlogits, float* dpalette,
+                               const void* t, const void* dt, int32_t rank, float* dA, float* dB, void* stream) {
+    if (!(tau > 0.f)) { set_last_error("tau must be positive"); return PLZ_ERR_BAD_SHAPE; }
+    if (rank < 0 || rank > 64 || rank % 8) { set_last_error("LoRA rank %d must be 0 or a multiple of 8 in [8, 64]", rank); return PLZ_ERR_BAD_SHAPE; }
+    if ((dA && !dt) || (dB && !t)) { set_last_error("bwd_dw_soft_select: dA needs dt and dB needs t"); return PLZ_ERR_NULL; }
+    return bwd_dw_common(EPI_SOFT, w, x, ldx, dY, lddy, M, logits, noise, tau, dlogits, dpalette, stream, t, dt, rank, dA, dB, nullptr, 1, 0, 0, true);
 }
 
 int32_t plz_bwd_dw_soft_scatter(const plz_weight_t* w, const void* x, int64_t ldx, const void* dY, int64_t lddy, int32_t M,

@@ -4,11 +4,14 @@ output row and 256 input columns, index logits fp32 [N, K, 4]) with the LoRA bra
 `linear_step` is the hot path as one call -- soft forward (straight-through or pure soft) plus the full
 backward -- exactly the sequence of library calls a training step makes per Linear:
 
-    soft_select   logits -> packed argmax indices (or W_soft)          one pass over the logits
-    hard_fwd      y  = x W^T + (s x A^T) B^T                           tcgen05, weights decoded in-kernel
-    bwd_dx        dX = dY W + (s dY B) A                               tcgen05, weights decoded in-kernel
-    bwd_dw_soft   dW = x^T dY on tcgen05, epilogue -> dLogits, dPalette (dW never stored)
-    lora_bwd      dA, dB
+    lora_t, lora_dt    t = s x A^T, dt = s dY B
+    bwd_dw_soft_select dW = x^T dY on tcgen05, epilogue -> dLogits, dPalette, packed argmax indices; dA, dB as extra tiles (dW never
+                       stored, one pass over the logits)
+    hard_fwd           y  = x W^T + t B^T                                 tcgen05, weights decoded in-kernel
+    bwd_dx             dX = dY W + dt A                                   tcgen05, weights decoded in-kernel
+
+The straight-through gradient of the logits does not depend on the hard indices, so it can come first. A forward without dY, a pure soft
+step and a data-parallel one begin with soft_select instead.
 
 Module counterpart of the reference's PalettizedLinear + QwenLoRA (scripts/qwen_model.py:65-304).
 """
@@ -42,6 +45,18 @@ def linear_step(x, dy, palette, logits, noise, tau, lora=None, ste=True, packed=
         packed = ops.empty_packed(N, K, x.device)
     w = ops.PackedWeight(packed, palette, N, K, gs_n, gs_k)
     out = {"packed": packed}
+    if ste and dy is not None and ("dlogits" in want or "dpalette" in want) and (dp_scatter is None or dp_scatter.world <= 1):
+        grads = lora is not None and ("da" in want or "db" in want)
+        t = ops.lora_t(lora, x) if lora is not None else None
+        dt = ops.lora_dt(lora, dy) if lora is not None and (grads or "dx" in want) else None
+        dlog, dpal, da, db = ops.backward_dw_soft_select(w, x, dy, logits, "nk4", noise=noise, tau=tau, seed=seed, want_dlogits="dlogits" in want,
+                                                         want_dpalette="dpalette" in want, lora_ws=(t, dt) if grads else None)
+        out.update(y=ops.hard_forward_with_t(w, x, lora, t), dlogits=dlog, dpalette=dpal)
+        if grads:
+            out.update(da=da, db=db)
+        if "dx" in want:
+            out["dx"] = ops.backward_dx_with_dt(w, dy, lora, dt) if lora is not None else ops.backward_dx(w, dy)[0]
+        return out
     w_soft = ops.soft_select(w, logits, "nk4", noise=noise, tau=tau, seed=seed, want_packed=True, want_soft=not ste)
     if ste:
         y, t = ops.hard_forward(w, x, lora)
@@ -51,22 +66,13 @@ def linear_step(x, dy, palette, logits, noise, tau, lora=None, ste=True, packed=
     if dy is None:
         return out
     fused_lora = ste and lora is not None and ("da" in want or "db" in want) and ("dlogits" in want or "dpalette" in want)
-    if fused_lora and dp_scatter is not None and dp_scatter.world > 1:
+    if fused_lora and dp_scatter is not None and dp_scatter.world > 1:   # the only straight-through steps with these gradients that come here
         dt = ops.lora_dt(lora, dy)
         dpal, da, db = dp_scatter.dw(w, x, dy, logits, noise, tau, seed=seed, lora_ws=(t, dt))
         handle = dp_scatter.start([dpal, da, db])
         if "dx" in want:
             out["dx"] = ops.backward_dx_with_dt(w, dy, lora, dt)
         out.update(dlogits=dp_scatter.finish(handle), dpalette=dpal, da=da, db=db)
-        return out
-    if fused_lora:
-        # dt first, then the weight-gradient launch also produces dA and dB, then dX with the dt already there
-        dt = ops.lora_dt(lora, dy)
-        dlog, dpal, da, db = ops.backward_dw_soft(w, x, dy, logits, "nk4", noise=noise, tau=tau, seed=seed,
-                                                  want_dlogits="dlogits" in want, want_dpalette="dpalette" in want, lora_ws=(t, dt))
-        out.update(dlogits=dlog, dpalette=dpal, da=da, db=db)
-        if "dx" in want:
-            out["dx"] = ops.backward_dx_with_dt(w, dy, lora, dt)
         return out
     if "dx" in want:
         dx, dt = ops.backward_dx(w, dy, lora) if ste else ops.dense_backward_dx(w_soft, dy, lora)

@@ -126,6 +126,8 @@ SIGNATURES = {
     "plz_unpack_indices": [_P, _I64, _I32, _I32, _P, _I64, _I64, _P],
     "plz_dequantize": [_WP, _P, _I64, _I64, _P],
     "plz_hard_fwd": [_WP, _P, _I64, _I32, _LP, _P, _P, _I64, _P],
+    "plz_lora_down": [_LP, _P, _I64, _I32, _I32, _P, _P],
+    "plz_hard_fwd_with_t": [_WP, _P, _I64, _I32, _LP, _P, _P, _I64, _P],
     "plz_hard_fwd_lora_static": [_WP, _P, _I64, _I32, _LP, _P, _I64, _P],
     "plz_hard_fwd_smallm": [_WP, _P, _I64, _I32, _P, _I64, _P],
     "plz_hard_fwd_smallm_multi": [C.POINTER(_WP), _I32, _P, _I64, _I32, C.POINTER(C.c_void_p), C.POINTER(C.c_int64), _P],
@@ -138,6 +140,7 @@ SIGNATURES = {
     "plz_dense_bwd_dx": [_P, _I64, _I32, _I32, _P, _I64, _I32, _LP, _P, _P, _I64, _P],
     "plz_bwd_dw_soft": [_WP, _P, _I64, _P, _I64, _I32, _GP, _NP, _F, _P, _P, _P],
     "plz_bwd_dw_soft_lora": [_WP, _P, _I64, _P, _I64, _I32, _GP, _NP, _F, _P, _P, _P, _P, _I32, _P, _P, _P],
+    "plz_bwd_dw_soft_select": [_WP, _P, _I64, _P, _I64, _I32, _GP, _NP, _F, _P, _P, _P, _P, _I32, _P, _P, _P],
     "plz_bwd_dw_soft_scatter": [_WP, _P, _I64, _P, _I64, _I32, _GP, _NP, _F, C.POINTER(C.c_void_p), _I32, _I32, _I32, _P, _P, _P, _I32,
                                 _P, _P, _P],
     "plz_peer_alloc": [_I64, C.POINTER(C.c_void_p), C.c_char_p],

@@ -106,6 +106,27 @@ def hard_forward(w: PackedWeight, x: torch.Tensor, lora=None):
     return y, t
 
 
+def lora_t(lora, x: torch.Tensor) -> torch.Tensor:
+    """t = scale * x A^T, bf16 [M, rank]."""
+    a, b, scale = lora
+    _mat(x, x.shape[1])
+    d = P.lora_desc(a, b, scale)
+    t = torch.empty(x.shape[0], a.shape[0], dtype=torch.bfloat16, device=x.device)
+    P.check(P.lib().plz_lora_down(C.byref(d), x.data_ptr(), x.stride(0), x.shape[0], x.shape[1], t.data_ptr(), P.stream_ptr()), "plz_lora_down")
+    return t
+
+
+def hard_forward_with_t(w: PackedWeight, x: torch.Tensor, lora=None, t: torch.Tensor | None = None) -> torch.Tensor:
+    """y = x W^T + t B^T with a precomputed t."""
+    _mat(x, w.K)
+    y = torch.empty(x.shape[0], w.N, dtype=torch.bfloat16, device=x.device)
+    ld = P.lora_desc(*lora) if lora is not None else None
+    d = w.desc()
+    P.check(P.lib().plz_hard_fwd_with_t(C.byref(d), x.data_ptr(), x.stride(0), x.shape[0], C.byref(ld) if ld is not None else None,
+                                        t.data_ptr() if t is not None else None, y.data_ptr(), y.stride(0), P.stream_ptr()), "plz_hard_fwd_with_t")
+    return y
+
+
 def hard_forward_smallm(w: PackedWeight, x: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
     _mat(x, w.K)
     M = x.shape[0]
@@ -233,6 +254,24 @@ def backward_dw_soft(w: PackedWeight, x: torch.Tensor, dy: torch.Tensor, logits:
                                     C.byref(nd), float(tau), dlog.data_ptr() if dlog is not None else None,
                                     dpal.data_ptr() if dpal is not None else None, P.stream_ptr()), "plz_bwd_dw_soft")
     return dlog, dpal
+
+
+def backward_dw_soft_select(w: PackedWeight, x: torch.Tensor, dy: torch.Tensor, logits: torch.Tensor, layout: str, noise=None, tau: float = 1.0,
+                            seed: int = 0, want_dlogits: bool = True, want_dpalette: bool = True, lora_ws=None):
+    """backward_dw_soft that also writes the argmax of the logits into w.packed. Returns (dLogits, dPalette, dA, dB), the last two None without
+    lora_ws."""
+    _mat(x, w.K), _mat(dy, w.N)
+    ld, nd = P.logits_desc(logits, layout), P.noise_desc(noise, layout, seed)
+    dlog = torch.empty_like(logits) if want_dlogits else None
+    assert dlog is None or dlog.stride() == logits.stride()
+    t, dt = lora_ws if lora_ws is not None else (None, None)
+    r = t.shape[1] if t is not None else 0
+    dpal, da, db = _zeros([(w.palette.numel() // 4, 4) if want_dpalette else None, (r, w.K) if r else None, (w.N, r) if r else None], x.device)
+    d = w.desc()
+    ptr = lambda z: z.data_ptr() if z is not None else None
+    P.check(P.lib().plz_bwd_dw_soft_select(C.byref(d), x.data_ptr(), x.stride(0), dy.data_ptr(), dy.stride(0), x.shape[0], C.byref(ld), C.byref(nd),
+                                           float(tau), ptr(dlog), ptr(dpal), ptr(t), ptr(dt), r, ptr(da), ptr(db), P.stream_ptr()), "plz_bwd_dw_soft_select")
+    return dlog, dpal, da, db
 
 
 def backward_dw_soft_scatter(w: PackedWeight, x: torch.Tensor, dy: torch.Tensor, logits: torch.Tensor, stage_ptrs, world: int,
