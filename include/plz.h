@@ -595,6 +595,9 @@ typedef struct plz_latent_attn {
 } plz_latent_attn_t;
 int64_t plz_latent_attn_ws_bytes(int32_t dtype, int32_t B, int32_t n, int32_t H, int32_t R, int32_t dr, int32_t cap);
 int32_t plz_latent_attn(int32_t dtype, const plz_latent_attn_t* args, void* ws, int64_t ws_bytes, void* stream);
+/* dst[0 .. n) = values[0 .. n) with values in HOST memory, read before the call returns (token ids, row numbers; n <= 4096): the numbers travel as kernel
+ * arguments, 256 to a launch, so the call waits for nothing, where a copy from pageable memory waits for all that its stream has queued. */
+int32_t plz_put_words(int64_t* dst, const int64_t* values, int32_t n, void* stream);
 /* *pos += n, at the end of a step */
 int32_t plz_advance(int32_t* pos, int32_t n, void* stream);
 /* Next token of every row of fp32 logits [rows, V]: temperature 0: the largest (first of equals); else a draw from

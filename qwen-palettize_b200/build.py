@@ -3,9 +3,11 @@
 Usage: python build.py [--force] [--verbose]
 The library lands next to this file so that it travels with the source tree.
 """
+import importlib.util
 import os
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
@@ -15,6 +17,8 @@ SOURCES = ["api.cu", "lut_gemm.cu", "lut_gemm_pair.cu", "dense_gemm_pair.cu", "n
 PRECISE = {"narrow_gemm.cu", "seq_linear.cu", "seq_ops.cu", "seq_recurrent.cu", "seq_chunk.cu", "seq_scan.cu", "attention_bias.cu", "latent_ops.cu", "latent_attention.cu"}   # compiled without --use_fast_math
 HEADERS = ["plz_sm100.cuh", "plz_host.h", "plz_launch.h", "soft_math.cuh", "seq_math.cuh", "seq_chunk.cuh", "latent_attention.cuh", "attention_tiles.cuh", os.path.join("..", "..", "include", "plz.h")]
 LIB = os.path.join(HERE, "libplz.so")
+CALLS_SRC = os.path.join(CSRC, "torch_calls.cpp")
+CALLS = os.path.join(HERE, "_plz_torch.so")   # Python module over libplz.so for torch tensors
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
          "-Xcompiler", "-fPIC", "--use_fast_math", "-Xptxas", "-v"]
@@ -22,17 +26,37 @@ if os.environ.get("PLZ_DIAGNOSTICS") == "1":   # cycle counters inside the kerne
     FLAGS.append("-DPLZ_DIAGNOSTICS")
 
 
-def _stale():
-    if not os.path.exists(LIB):
+def _older(target, deps):
+    if not os.path.exists(target):
         return True
-    t = os.path.getmtime(LIB)
-    deps = [os.path.join(CSRC, s) for s in SOURCES + HEADERS] + [os.path.abspath(__file__)]
-    return any(os.path.exists(d) and os.path.getmtime(d) > t for d in deps)
+    t = os.path.getmtime(target)
+    return any(os.path.exists(d) and os.path.getmtime(d) > t for d in deps + [os.path.abspath(__file__)])
+
+
+def _stale():
+    return _older(LIB, [os.path.join(CSRC, s) for s in SOURCES + HEADERS])
+
+
+def _build_calls(force):
+    """The Python module, compiled against the installed torch (host code only)."""
+    if not force and not _older(CALLS, [CALLS_SRC, os.path.join(HERE, "..", "include", "plz.h")]):
+        return
+    root = os.path.dirname(importlib.util.find_spec("torch").origin)
+    inc, lib = os.path.join(root, "include"), os.path.join(root, "lib")
+    cuda = os.path.dirname(os.path.dirname(NVCC))
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", CALLS_SRC, "-o", CALLS, "-I" + inc,
+           "-I" + os.path.join(inc, "torch", "csrc", "api", "include"), "-I" + sysconfig.get_paths()["include"], "-I" + os.path.join(cuda, "include"),
+           "-L" + lib, "-ltorch_python", "-ltorch_cpu", "-lc10_cuda", "-lc10", "-L" + HERE, "-l:libplz.so", "-Wl,-rpath,$ORIGIN"]
+    r = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+    if r.returncode != 0:
+        sys.stderr.write(r.stdout)
+        raise RuntimeError("g++ failed on torch_calls.cpp")
 
 
 def build(force=False, verbose=False):
-    """Compile every .cu into an object (in parallel) and link the shared library."""
+    """Compile every .cu into an object (in parallel), link the shared library, and compile the Python module over it."""
     if not force and not _stale():
+        _build_calls(force)
         return LIB
     objdir = os.path.join(HERE, "build")
     os.makedirs(objdir, exist_ok=True)
@@ -63,6 +87,7 @@ def build(force=False, verbose=False):
     if r.returncode != 0:
         sys.stderr.write(r.stdout)
         raise RuntimeError("link failed")
+    _build_calls(force)
     return LIB
 
 

@@ -1188,6 +1188,14 @@ int32_t plz_latent_attn(int32_t dtype, const plz_latent_attn_t* a, void* ws, int
     return launch_latent_attn(dtype, *a, ws, ws ? ws_bytes : 0, (cudaStream_t)stream);
 }
 
+int32_t plz_put_words(int64_t* dst, const int64_t* values, int32_t n, void* stream) {
+    if (n < 0 || n > 4096) { set_last_error("put_words: 0 to 4096 numbers"); return PLZ_ERR_BAD_SHAPE; }
+    if (n && (!dst || !values)) { set_last_error("null pointer"); return PLZ_ERR_NULL; }
+    if ((uintptr_t)dst & 7) { set_last_error("put_words: misaligned destination"); return PLZ_ERR_BAD_ALIGN; }
+    static_assert(sizeof(long long) == sizeof(int64_t), "64-bit numbers");
+    return launch_put_words((long long*)dst, (const long long*)values, n, (cudaStream_t)stream);
+}
+
 int32_t plz_advance(int32_t* pos, int32_t n, void* stream) {
     if (!pos) { set_last_error("null pointer"); return PLZ_ERR_NULL; }
     return launch_advance(pos, n, (cudaStream_t)stream);

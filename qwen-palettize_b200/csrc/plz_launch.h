@@ -243,6 +243,7 @@ using LatentAttnArgs = plz_latent_attn_t;
 long long latent_attn_ws_bytes(int dtype, int B, int n, int H, int R, int dr, int cap);
 int launch_latent_attn(int dtype, const LatentAttnArgs& a, void* ws, long long ws_bytes, cudaStream_t stream);
 int launch_advance(int* pos, int n, cudaStream_t stream);
+int launch_put_words(long long* dst, const long long* values, int n, cudaStream_t stream);
 int launch_sample(const float* logits, long long ld, int rows, int V, float temperature, int top_k, uint32_t seed, const int* pos, long long* out,
                   cudaStream_t stream);
 

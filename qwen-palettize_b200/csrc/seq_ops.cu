@@ -815,6 +815,23 @@ int launch_attn_prep(int dtype, const AttnPrepArgs& a, cudaStream_t stream) {
     return PLZ_OK;
 }
 
+// Few numbers from the host, as arguments of the launch.
+constexpr int kPutWords = 256;
+struct PutWords { long long v[kPutWords]; };
+__global__ void __launch_bounds__(kPutWords) put_words_kernel(long long* dst, const __grid_constant__ PutWords w, int n) {
+    if ((int)threadIdx.x < n) dst[threadIdx.x] = w.v[threadIdx.x];
+}
+int launch_put_words(long long* dst, const long long* values, int n, cudaStream_t stream) {
+    for (int at = 0; at < n; at += kPutWords) {
+        PutWords w;
+        const int part = n - at < kPutWords ? n - at : kPutWords;
+        for (int i = 0; i < part; ++i) w.v[i] = values[at + i];
+        put_words_kernel<<<1, kPutWords, 0, stream>>>(dst + at, w, part);
+        PLZ_LAUNCH_CHECK();
+    }
+    return PLZ_OK;
+}
+
 int launch_advance(int* pos, int n, cudaStream_t stream) {
     PLZ_LAUNCH_CHAIN(advance_kernel, dim3(1), dim3(1), 0, stream, pos, n);
     return PLZ_OK;

@@ -266,13 +266,13 @@ class HybridModel:
             cache.length += 1
             if want is None or len(want) == 0:
                 return None
-            return out.clone() if list(want) == list(range(B)) else out[torch.as_tensor(want, device=self.device)]
-        ids = ids.to(self.device).contiguous()
+            return out.clone() if list(want) == list(range(B)) else out[S.on_device(torch.as_tensor(want), self.device)]
+        ids = S.on_device(ids, self.device).contiguous()
         x = self.hidden(ids, cache, cache.length)
         cache.length += n
         if want is None or len(want) == 0:
             return None
-        return self.logits(x, torch.as_tensor(want, dtype=torch.int64, device=self.device))
+        return self.logits(x, S.on_device(torch.as_tensor(want, dtype=torch.int64), self.device))
 
     def _token(self, ids: torch.Tensor, cache: SequenceState) -> torch.Tensor:
         """One token per sequence. The first such step of a state runs eagerly, the second is captured (capturing runs nothing) and from
@@ -280,7 +280,7 @@ class HybridModel:
         g = cache.step_graph
         if g is None:
             cache.step_graph = (None, torch.empty(cache.B, 1, dtype=torch.int64, device=self.device), None)
-            cache.step_graph[1].copy_(ids)
+            S.put(cache.step_graph[1], ids)
             return self._token_chain(cache.step_graph[1], cache)
         graph, buf, out = g
         if graph is None:
@@ -289,7 +289,7 @@ class HybridModel:
             with torch.cuda.graph(graph):
                 out = self._token_chain(buf, cache)
             cache.step_graph = (graph, buf, out)
-        buf.copy_(ids)
+        S.put(buf, ids)
         graph.replay()
         return out
 

@@ -165,6 +165,9 @@ class PalettizedLinear(nn.Module):
             self.step_seed = (self.step_seed + 1) & 0xFFFFFFFF
             cfg = (float(self.tau), self.lora_scale, self.ste, self.step_seed, 1, self.group_k)
             return _PalettizedLoraFn.apply(x, self.palette, self.index_logits, self.lora_A, self.lora_B, self.noise, cfg)
+        y = ops.eval_linear(self.packed, self.palette, N, K, 1, self.group_k, x, self.lora_A, self.lora_B, self.lora_scale)
+        if y is not None:
+            return y
         x2 = x.reshape(-1, K).contiguous()
         w = ops.PackedWeight(self.packed, self.palette.detach(), N, K, 1, self.group_k)
         lora = (self.lora_A.detach(), self.lora_B.detach(), self.lora_scale) if self.lora_A is not None else None

@@ -27,6 +27,10 @@ class PackedWeight:
         return P.weight_desc(self.packed, self.palette, self.N, self.K, self.gs_n, self.gs_k)
 
 
+def _weight_args(w: PackedWeight):
+    return w.packed, w.palette, w.N, w.K, w.gs_n, w.gs_k
+
+
 def _pitch(K: int) -> int:
     return (K // 4 + 15) // 16 * 16
 
@@ -96,6 +100,10 @@ def _zeros(shapes, device):
 
 def hard_forward(w: PackedWeight, x: torch.Tensor, lora=None):
     """y = x W^T (+ LoRA).  Returns (y, t) where t = scale * x A^T (None without LoRA)."""
+    if lora is None:
+        y = P.calls().hard_forward(*_weight_args(w), x)
+        if y is not None:
+            return y, None
     _mat(x, w.K)
     M = x.shape[0]
     y = torch.empty(M, w.N, dtype=torch.bfloat16, device=x.device)
@@ -104,6 +112,11 @@ def hard_forward(w: PackedWeight, x: torch.Tensor, lora=None):
     P.check(P.lib().plz_hard_fwd(C.byref(d), x.data_ptr(), x.stride(0), M, lp, t.data_ptr() if t is not None else None,
                                  y.data_ptr(), y.stride(0), P.stream_ptr()), "plz_hard_fwd")
     return y, t
+
+
+def eval_linear(packed, palette, N: int, K: int, gs_n: int, gs_k: int, x: torch.Tensor, a, b, scale: float):
+    """What a Linear in eval mode does with x [..., K], as one native call; None where x or the weights are not what that call takes."""
+    return P.calls().eval_linear(packed, palette, N, K, gs_n, gs_k, x, a, b, scale)
 
 
 def lora_t(lora, x: torch.Tensor) -> torch.Tensor:
@@ -128,6 +141,10 @@ def hard_forward_with_t(w: PackedWeight, x: torch.Tensor, lora=None, t: torch.Te
 
 
 def hard_forward_smallm(w: PackedWeight, x: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
+    if out is None:
+        y = P.calls().hard_forward_smallm(*_weight_args(w), x)
+        if y is not None:
+            return y
     _mat(x, w.K)
     M = x.shape[0]
     y = out if out is not None else torch.empty(M, w.N, dtype=torch.bfloat16, device=x.device)
@@ -158,6 +175,8 @@ def hard_forward_smallm_multi(ws, x: torch.Tensor, outs=None):
 def soft_select(w: PackedWeight, logits: torch.Tensor, layout: str, noise=None, tau: float = 1.0, seed: int = 0,
                 want_packed: bool = True, want_soft: bool = False):
     """Writes argmax indices into w.packed (if want_packed) and returns W_soft bf16 [N, K] (if want_soft)."""
+    if want_packed and not want_soft and P.calls().select_indices(*_weight_args(w), logits, layout == "4kn", noise, tau):
+        return None
     ld, nd = P.logits_desc(logits, layout), P.noise_desc(noise, layout, seed)
     w_soft = torch.empty(w.N, w.K, dtype=torch.bfloat16, device=logits.device) if want_soft else None
     d = w.desc()
@@ -180,6 +199,10 @@ def dense_forward(wd: torch.Tensor, x: torch.Tensor, lora=None):
 
 def backward_dx(w: PackedWeight, dy: torch.Tensor, lora=None):
     """dX = dY W (+ LoRA).  Returns (dX, dt) with dt = scale * dY B."""
+    if lora is None:
+        dx = P.calls().backward_dx(*_weight_args(w), dy)
+        if dx is not None:
+            return dx, None
     _mat(dy, w.N)
     M = dy.shape[0]
     dx = torch.empty(M, w.K, dtype=torch.bfloat16, device=dy.device)
@@ -233,6 +256,10 @@ def backward_dw_soft(w: PackedWeight, x: torch.Tensor, dy: torch.Tensor, logits:
                      tau: float = 1.0, seed: int = 0, want_dlogits: bool = True, want_dpalette: bool = True, lora_ws=None):
     """Returns (dLogits with the dtype/shape of `logits`, dPalette fp32 [groups, 4]); with lora_ws = (t, dt), the workspaces
     left by the forward and by backward_dx, also (dA fp32 [r, K], dB fp32 [N, r]) computed in the same launch."""
+    if lora_ws is None:
+        out = P.calls().backward_dw_soft(*_weight_args(w), x, dy, logits, layout == "4kn", noise, tau, seed, want_dlogits, want_dpalette)
+        if out is not None:
+            return out
     _mat(x, w.K), _mat(dy, w.N)
     M = x.shape[0]
     ld, nd = P.logits_desc(logits, layout), P.noise_desc(noise, layout, seed)
@@ -312,6 +339,9 @@ def reduce_slots(stage_ptr: int, world: int, out: torch.Tensor, scale: float = 1
 
 
 def backward_dw_hard(w: PackedWeight, x: torch.Tensor, dy: torch.Tensor) -> torch.Tensor:
+    dpal = P.calls().backward_dw_hard(*_weight_args(w), x, dy)
+    if dpal is not None:
+        return dpal
     _mat(x, w.K), _mat(dy, w.N)
     dpal = torch.zeros(w.palette.numel() // 4, 4, dtype=torch.float32, device=x.device)
     d = w.desc()
@@ -453,6 +483,9 @@ def mlp_front_backward(w_gate: PackedWeight, w_up: PackedWeight, x: torch.Tensor
 
 def hard_forward_bias(w: PackedWeight, x: torch.Tensor, bias: torch.Tensor | None) -> torch.Tensor:
     """y = x W^T + bias, the bias (bf16 [N]) added in fp32 inside the GEMM epilogue."""
+    y = P.calls().hard_forward_bias(*_weight_args(w), x, bias)
+    if y is not None:
+        return y
     _mat(x, w.K)
     M = x.shape[0]
     y = torch.empty(M, w.N, dtype=torch.bfloat16, device=x.device)
@@ -467,6 +500,9 @@ def hard_forward_bias(w: PackedWeight, x: torch.Tensor, bias: torch.Tensor | Non
 
 def col_sum(dy: torch.Tensor) -> torch.Tensor:
     """fp32 [N]: sum over the rows of a bf16 [M, N] matrix (the bias gradient)."""
+    out = P.calls().col_sum(dy)
+    if out is not None:
+        return out
     _mat(dy, dy.shape[1])
     out = torch.zeros(dy.shape[1], dtype=torch.float32, device=dy.device)
     P.check(P.lib().plz_col_sum(dy.data_ptr(), dy.stride(0), dy.shape[0], dy.shape[1], out.data_ptr(), P.stream_ptr()), "plz_col_sum")

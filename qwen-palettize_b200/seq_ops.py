@@ -232,6 +232,24 @@ def latent_attention(q: torch.Tensor, c: torch.Tensor, kr, sinks, pos: torch.Ten
     return o
 
 
+def put(dst: torch.Tensor, values: torch.Tensor):
+    """dst.copy_(values), for the few int64 numbers in host memory that a step starts with without waiting for the work before it."""
+    if values.device.type == "cpu" and values.dtype == dst.dtype == torch.int64 and values.shape == dst.shape and 0 < values.numel() <= 4096 and dst.is_contiguous():
+        values = values.contiguous()
+        P.check(P.lib().plz_put_words(dst.data_ptr(), values.data_ptr(), values.numel(), P.stream_ptr()), "plz_put_words")
+    else:
+        dst.copy_(values)
+
+
+def on_device(t: torch.Tensor, device) -> torch.Tensor:
+    """t.to(device), by `put` where t is such a tensor."""
+    if t.device.type != "cpu" or t.dtype != torch.int64 or not 0 < t.numel() <= 4096:
+        return t.to(device)
+    out = torch.empty(t.shape, dtype=torch.int64, device=device)
+    put(out, t)
+    return out
+
+
 def advance(pos: torch.Tensor, n: int):
     P.check(P.lib().plz_advance(pos.data_ptr(), n, P.stream_ptr()), "plz_advance")
 
