@@ -5,11 +5,13 @@
 //                        weights are requested before the wait on the previous kernel of the stream.
 //   linear_skinny_kernel 2 .. 16 rows, bf16: the same streaming with mma.sync fragments loaded straight from memory.
 //                        Both also serve one small product per head (grid y = head, z = group of 16 rows).
+//   linear_stream_kernel one row, bf16, matrices of some size: a CTA per SM, the matrix by bulk copies into a ring of shared memory.
 //   linear_tile_kernel   any shape and both types on the CUDA cores, fp32 products and sums: the 32-bit mode, and bf16 shapes
 //                        that the tensor-core path's 16-byte rows exclude.
 //   launch_seq_linear    picks one of them, the swapped tcgen05 form (narrow_gemm.cu) or the tcgen05 GEMM (lut_gemm.cu, dense B, bias and
 //                        activation in its epilogue).
 #include "seq_math.cuh"
+#include "plz_sm100.cuh"
 
 namespace plz {
 namespace {
@@ -210,6 +212,137 @@ linear_skinny_kernel(const LinParams p, int ks) {
     }
 }
 
+// One row of x, bf16. Bound by streaming W once. linear_rows_kernel holds 128 bytes per lane of W in registers and waits for them before it asks for more, in
+// blocks that come in 2.05 waves for 19456 rows, 1.08 for 2560. Here a CTA per SM takes an even share of the row pairs and cuts it into pieces of two
+// rows by kStreamCols columns; a warp takes an even, contiguous run of them and keeps kStreamDepth pieces in flight by bulk copies into a
+// ring of its own, 160 KB per SM, filled ahead of the wait on the previous kernel. Sums stay in registers over a run, are written down where it leaves
+// a row pair, and are added in the order of the warps. The ring is more than half of an SM's shared memory on purpose: with 96 KB two CTAs of a launch
+// that starts early met on the SMs that happened to be free, and the launch took twice as long (32768 x 2560 in a served request 30 -> 68 us).
+constexpr int kStreamWarps = 16, kStreamDepth = 5, kStreamCols = 512;
+constexpr uint32_t kStreamPiece = 2 * kStreamCols * 2, kStreamRing = kStreamWarps * kStreamDepth * kStreamPiece, kStreamHeader = 1024;
+
+template <typename TO>
+__global__ void __launch_bounds__(kStreamWarps * 32, 2)
+linear_stream_kernel(const LinParams p, int units, int max_pairs, StatusWord* status) {
+    extern __shared__ __align__(128) uint8_t smem[];
+    const int warp = __shfl_sync(0xFFFFFFFFu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+    const uint32_t bars = smem_u32(smem) + kStreamRing + warp * kStreamDepth * 8;
+    volatile uint32_t* abort_flag = reinterpret_cast<volatile uint32_t*>(smem + kStreamRing + kStreamHeader - 16);
+    uint8_t* xs = smem + kStreamRing + kStreamHeader;
+    float2* part = reinterpret_cast<float2*>(xs + ((p.K * 2 + 15) & ~15));
+    const int all = (p.N + 1) / 2, grid = (int)gridDim.x, b = (int)blockIdx.x;
+    const int pair0 = (int)((long long)all * b / grid), pairs = (int)((long long)all * (b + 1) / grid) - pair0;
+    const int total = pairs * units;
+    auto start = [&](int w) { return (int)((long long)total * w / kStreamWarps); };
+    const int first = start(warp), last = start(warp + 1);
+    const uint32_t ring = smem_u32(smem) + warp * kStreamDepth * kStreamPiece;
+    const __nv_bfloat16* w = (const __nv_bfloat16*)p.w;
+
+    int rq = first, rq_pair = first / units, rq_unit = first - rq_pair * units, rq_slot = 0;
+    auto request = [&]() {          // the next piece of the run into the next slot; one lane
+        const int n = (pair0 + rq_pair) * 2, k = rq_unit * kStreamCols;
+        const uint32_t bytes = (uint32_t)min(kStreamCols, p.K - k) * 2u, bar = bars + rq_slot * 8, dst = ring + rq_slot * kStreamPiece;
+        const __nv_bfloat16* src = w + (long long)n * p.ldw + k;
+        const bool two = n + 1 < p.N;
+        mbar_arrive_expect_tx(bar, two ? 2 * bytes : bytes);
+        bulk_load(dst, src, bytes, bar);
+        if (two) bulk_load(dst + kStreamCols * 2, src + p.ldw, bytes, bar);
+    };
+    auto requested = [&]() {
+        ++rq;
+        if (++rq_unit == units) { rq_unit = 0; ++rq_pair; }
+        if (++rq_slot == kStreamDepth) rq_slot = 0;
+    };
+    if (threadIdx.x == 0) *abort_flag = 0;
+    if (lane == 0) {
+        for (int s = 0; s < kStreamDepth; ++s) mbar_init(bars + s * 8, 1);
+        mbar_fence_init();
+    }
+    __syncwarp();
+    for (int s = 0; s < kStreamDepth && rq < last; ++s) {      // weights do not depend on the previous kernel
+        if (lane == 0) request();
+        requested();
+    }
+    pdl_launch_dependents();
+    pdl_wait();
+    for (int c = threadIdx.x; c < p.K / 8; c += kStreamWarps * 32) reinterpret_cast<uint4*>(xs)[c] = *reinterpret_cast<const uint4*>((const __nv_bfloat16*)p.x + c * 8);
+    __syncthreads();
+    bool ok = true;
+    int at = first, pair = first / units, unit = first - pair * units, slot = 0;
+    uint32_t phase = 0;
+    const int pair_first = pair;
+    uint64_t s0 = 0ull, s1 = 0ull;         // two partial sums of either row
+    auto fma2 = [](uint64_t a, uint64_t c, uint64_t d) { uint64_t r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(c), "l"(d)); return r; };
+    auto widen = [](uint32_t v) { uint64_t r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(v << 16), "r"(v & 0xFFFF0000u)); return r; };
+    while (at < last) {
+        ok = mbar_wait_warp(bars + slot * 8, phase, abort_flag, status, ST_TIMEOUT_FULL, 1);
+        if (!ok) break;
+        const uint8_t* wp = smem + warp * kStreamDepth * kStreamPiece + slot * kStreamPiece;
+        const int k0 = unit * kStreamCols;
+#pragma unroll
+        for (int j = 0; j < kStreamCols / 256; ++j) {
+            const int k = (lane + 32 * j) * 8;
+            if (k0 + k < p.K) {
+                const uint4 xv = *reinterpret_cast<const uint4*>(xs + (k0 + k) * 2), a = *reinterpret_cast<const uint4*>(wp + k * 2);
+                const uint4 c = *reinterpret_cast<const uint4*>(wp + kStreamCols * 2 + k * 2);   // of a row that is not there: goes nowhere
+                const uint64_t x2[4] = {widen(xv.x), widen(xv.y), widen(xv.z), widen(xv.w)};
+                s0 = fma2(widen(a.x), x2[0], s0); s1 = fma2(widen(c.x), x2[0], s1);
+                s0 = fma2(widen(a.y), x2[1], s0); s1 = fma2(widen(c.y), x2[1], s1);
+                s0 = fma2(widen(a.z), x2[2], s0); s1 = fma2(widen(c.z), x2[2], s1);
+                s0 = fma2(widen(a.w), x2[3], s0); s1 = fma2(widen(c.w), x2[3], s1);
+            }
+        }
+        __syncwarp();                      // the slot has been read
+        if (rq < last) {
+            if (lane == 0) request();
+            requested();
+        }
+        if (++slot == kStreamDepth) { slot = 0; phase ^= 1u; }
+        ++at;
+        if (++unit == units || at == last) {
+            float v0, v1, t;
+            asm("mov.b64 {%0, %1}, %2;" : "=f"(v0), "=f"(t) : "l"(s0));
+            v0 += t;
+            asm("mov.b64 {%0, %1}, %2;" : "=f"(v1), "=f"(t) : "l"(s1));
+            v1 += t;
+            // lanes below 16 end up with the sum of the first row, the others with that of the second
+            v0 = (lane < 16 ? v0 : v1) + __shfl_xor_sync(0xFFFFFFFFu, lane < 16 ? v1 : v0, 16);
+#pragma unroll
+            for (int o = 8; o > 0; o >>= 1) v0 += __shfl_xor_sync(0xFFFFFFFFu, v0, o);
+            if ((lane & 15) == 0) reinterpret_cast<float*>(part + warp * max_pairs + pair - pair_first)[lane >> 4] = v0;
+            s0 = s1 = 0ull;
+            if (unit == units) { unit = 0; ++pair; }
+        }
+    }
+    if (!ok) {                             // copies in flight get a bounded chance to land before the CTA leaves
+        const uint64_t t0 = globaltimer_ns();
+        for (; at < rq; ++at) {
+            while (!mbar_try_wait(bars + slot * 8, phase))
+                if (globaltimer_ns() - t0 > 100000000ull) { report(status, ST_TIMEOUT_DRAIN, 1); break; }
+            if (++slot == kStreamDepth) { slot = 0; phase ^= 1u; }
+        }
+    }
+    __syncthreads();
+    if (*abort_flag) return;
+    for (int q = threadIdx.x; q < pairs; q += kStreamWarps * 32) {
+        const int from = q * units, to = from + units;
+        int wi = (int)((long long)from * kStreamWarps / total);
+        while (start(wi + 1) <= from) ++wi;
+        float v[2] = {0.f, 0.f};
+        for (; wi < kStreamWarps && start(wi) < to; ++wi) {
+            if (start(wi + 1) == start(wi)) continue;
+            const float2 t = part[wi * max_pairs + q - start(wi) / units];
+            v[0] += t.x; v[1] += t.y;
+        }
+        const int n = (pair0 + q) * 2;
+        if (p.act == ACT_GLU_GELU) { put<__nv_bfloat16, TO>(p, 0, 0, n >> 1, gelu_tanh_f(v[0]) * v[1]); continue; }
+        for (int r = 0; r < 2 && n + r < p.N; ++r) {
+            if (p.bias) v[r] += to_f(((const __nv_bfloat16*)p.bias)[n + r]);
+            put<__nv_bfloat16, TO>(p, 0, 0, n + r, activate(v[r], p.act));
+        }
+    }
+}
+
 template <typename T, typename TO>
 __global__ void __launch_bounds__(256)
 linear_tile_kernel(const LinParams p) {
@@ -276,6 +409,25 @@ int launch_rows(const LinParams& p, int heads, cudaStream_t stream) {
     else PLZ_LAUNCH_CHAIN((linear_rows_kernel<T, TO, 8>), grid, dim3(256), 0, stream, p, ks);
     return PLZ_OK;
 }
+// PLZ_ERR_UNSUPPORTED: more shared memory than there is
+template <typename TO>
+int launch_stream(const LinParams& p, cudaStream_t stream) {
+    const int all = (p.N + 1) / 2, sms = seq_sm_count(), grid = all < sms ? all : sms, units = (p.K + kStreamCols - 1) / kStreamCols;
+    const long long most = (long long)((all + grid - 1) / grid) * units;
+    const int max_pairs = (int)((most / kStreamWarps + 1) / units + 2);
+    const long long bytes = (long long)kStreamRing + kStreamHeader + ((p.K * 2ll + 15) & ~15ll) + (long long)kStreamWarps * max_pairs * 8;
+    constexpr int kRoom = 227 * 1024;
+    if (bytes > kRoom || most > (1 << 26)) return PLZ_ERR_UNSUPPORTED;
+    static bool attr_set[64] = {};
+    int dev = 0;
+    PLZ_CUDA_CHECK(cudaGetDevice(&dev));
+    if (!attr_set[dev & 63]) {
+        PLZ_CUDA_CHECK(cudaFuncSetAttribute(linear_stream_kernel<TO>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRoom));
+        attr_set[dev & 63] = true;
+    }
+    PLZ_LAUNCH_CHAIN(linear_stream_kernel<TO>, dim3(grid), dim3(kStreamWarps * 32), (size_t)bytes, stream, p, units, max_pairs, device_status_ptr());
+    return PLZ_OK;
+}
 template <typename TO>
 int launch_skinny(const LinParams& p, int heads, cudaStream_t stream) {
     const int tiles = (p.N + 15) / 16;
@@ -294,6 +446,12 @@ int launch_tile(const LinParams& p, int heads, cudaStream_t stream) {
     PLZ_LAUNCH_CHAIN((linear_tile_kernel<T, TO>), dim3((p.N + 63) / 64, (unsigned)my, heads), dim3(256), 0, stream, p);
     return PLZ_OK;
 }
+
+// Weights from which one row streams through shared memory. A decode step of one sequence with the line at 4.2 / 16.8 million weights (before: linear_rows_kernel throughout), us:
+// Gopunex of width 2560 195 / 201 (224), Latodra 190 / 192 (212), Gopunex of width 1024, whose 4096 x 1024 projections lie at the lower line, 103.4 / 102.8 (102.2). By sizes, one after the other,
+// here / linear_rows: 32768 x 2560 26.7 / 29.4, 19456 x 2560 17.0 / 20.1, 2560 x 9728 11.0 / 13.8, 9728 x 2560 10.1 / 12.6, 5632 x 2560 7.6 / 8.6, 1024 x 3072 4.1 / 2.4. Two rows and more are faster in
+// the kernels below (two rows, 9728 x 2560: 11.9 / 10.6).
+constexpr long long kStreamFrom = 5 << 20;
 
 // 2 to 16 rows: narrow_gemm.cu streams large weights faster (its time hardly grows with the rows), but starts and ends later than the
 // register kernels here. us here / there in a decode chain: 8 rows 9728 x 2560 17.8 / 12.7, 4096 x 2560 8.3 / 9.7, 32768 x 2560
@@ -326,6 +484,10 @@ int launch_seq_linear(int dtype, const void* x, long long ldx, int M, int K, con
         if (rc != PLZ_ERR_UNSUPPORTED) return rc;
     }
     if (dtype == 0 && M > 1 && M <= 16 && vec) return y_f32 ? launch_skinny<float>(p, 1, stream) : launch_skinny<__nv_bfloat16>(p, 1, stream);
+    if (dtype == 0 && M == 1 && vec && (long long)N * K >= kStreamFrom && p.K <= 16384) {
+        const int rc = y_f32 ? launch_stream<float>(p, stream) : launch_stream<__nv_bfloat16>(p, stream);
+        if (rc != PLZ_ERR_UNSUPPORTED) return rc;
+    }
     if (M <= 8 && vec) {
         if (dtype == 1) return launch_rows<float, float>(p, 1, stream);
         return y_f32 ? launch_rows<__nv_bfloat16, float>(p, 1, stream) : launch_rows<__nv_bfloat16, __nv_bfloat16>(p, 1, stream);

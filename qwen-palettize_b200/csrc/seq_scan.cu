@@ -21,9 +21,6 @@ namespace {
 
 constexpr int kScanThreads = 320;   // warps 0-7 epilogue (two per 32 value columns, half of the TMEM columns each), 8 MMA, 9 copies
 
-__device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
-}
 
 template <int KB, bool HASW>
 struct ScanCfg {

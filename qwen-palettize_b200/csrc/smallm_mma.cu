@@ -78,11 +78,6 @@ __device__ __forceinline__ void mma_bf16_16816(float (&d)[4], const uint32_t (&a
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
-__device__ __forceinline__ void bulk_load(uint32_t dst_smem, const void* src, uint32_t bytes, uint32_t bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                 :: "r"(dst_smem), "l"(src), "r"(bytes), "r"(bar) : "memory");
-}
-
 template <int MT>  // MT m8 tiles: M <= 8 * MT
 __global__ void __launch_bounds__(SmallmCfg<MT>::kThreads, 1)
 lut_smallm_mma_kernel(const SmallmParams p) {

@@ -26,6 +26,7 @@ if _HERE not in sys.path:
 
 import plz_native as P  # noqa: E402
 import plz_ops as ops  # noqa: E402
+import seq_ops as S  # noqa: E402
 from decoder_layer import LINEARS, LayerConfig  # noqa: E402
 
 
@@ -147,6 +148,8 @@ class PalettizedQwen:
 
     def head(self, hn: torch.Tensor) -> torch.Tensor:
         """Logits bf16 [rows, vocab] of already normalised hidden states (tied embedding table)."""
+        if self.embed.shape[0] % 8 == 0 and self.embed.shape[1] % 64 == 0 and hn.shape[0] > 0:
+            return S.linear(hn, self.embed)      # in a decode step its reads of the table may start early
         return ops.dense_forward(self.embed, hn)[0]
 
     def decode_logits(self, ids: torch.Tensor, cache: KVCache, pos: int | None = None) -> torch.Tensor:
