@@ -46,7 +46,7 @@ template <bool BMN, bool GLU>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kDpThreads, 1)
 dense_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmBh,
                        const __grid_constant__ CUtensorMap tmA2, const __grid_constant__ CUtensorMap tmB2, const __grid_constant__ CUtensorMap tmD,
-                       const __grid_constant__ CUtensorMap tmD32, const DpParams p) {
+                       const __grid_constant__ CUtensorMap tmD16, const DpParams p) {
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
     const uint32_t base = (raw + 1023u) & ~1023u;
@@ -185,7 +185,7 @@ dense_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
             }
         }
     } else {
-        // ------------------------------------------------------------- epilogue warps: TMEM lanes 32 * (warp % 4), boxes of 64 (the last: 32) outputs
+        // ------------------------------------------------------------- epilogue warps: TMEM lanes 32 * (warp % 4), boxes of 64 outputs (of 16 where the tile ends sooner)
         const int lane_group = warp & 3;
         uint8_t* stage = smem + kDpEpiOff + (warp - 2) * kDpEpiBytes;
         const uint32_t stage_u32 = base + kDpEpiOff + (warp - 2) * kDpEpiBytes;
@@ -202,14 +202,15 @@ dense_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
             tc_fence_after_sync();
 #pragma unroll 1
             for (int col = 0; col < w_out; col += 64) {
-                const bool wide = col + 32 < w_out;
+                const int left = w_out - col;
+                const bool wide = left >= 64;
                 if (lane == 0) tma_store_wait_read();       // the previous box must have been read out of the staging buffer
                 __syncwarp();
                 // 32 accumulator columns: 32 outputs, or 16 gated ones
                 constexpr int kChunks = GLU ? 4 : 2, kOut = GLU ? 16 : 32;
 #pragma unroll
                 for (int c = 0; c < kChunks; ++c) {
-                    if (c * kOut >= 32 && !wide) break;
+                    if (c * kOut >= left) break;
                     uint32_t v[32];
                     const int at = (GLU ? 2 * col : col) + c * 32;
                     tmem_ld_32x32(lane_base + buf * 256u + at, v);
@@ -238,14 +239,16 @@ dense_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
                             }
                         }
                         const int chunk = c * (kOut / 8) + g;
-                        const uint32_t to = wide ? swz128(lane, chunk) : (uint32_t)(lane * 64 + ((chunk ^ ((lane >> 1) & 3)) << 4));
+                        const uint32_t to = wide ? swz128(lane, chunk) : (uint32_t)((chunk >> 1) * 1024 + lane * 32 + ((chunk & 1) << 4));
                         *reinterpret_cast<uint4*>(stage + to) = make_uint4(pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]), pack_bf16x2(f[4], f[5]), pack_bf16x2(f[6], f[7]));
                     }
                 }
                 fence_proxy_async_smem();
                 __syncwarp();
                 if (lane == 0 && o0 + col < p.out_cols && mrow < p.M) {
-                    tma_store_2d(wide ? &tmD : &tmD32, stage_u32, o0 + col, mrow);
+                    if (wide) tma_store_2d(&tmD, stage_u32, o0 + col, mrow);
+                    else
+                        for (int b = 0; b * 16 < left && o0 + col + b * 16 < p.out_cols; ++b) tma_store_2d(&tmD16, stage_u32 + b * 1024u, o0 + col + b * 16, mrow);
                     tma_store_commit();
                 }
             }
@@ -276,10 +279,11 @@ int launch_dp(const LutGemmArgs& a, int sms, cudaStream_t stream) {
     p.alpha = a.alpha; p.bias = (const __nv_bfloat16*)a.bias; p.relu2 = a.fuse == 3 && a.act == 1;
     p.status = device_status_ptr();
     int pairs = sms / 2;
-    const PairTiles pt = plan_pair_tiles(a.M, a.J, pairs, GLU ? 64 : 32);
+    // columns of a row-major B come in boxes of 64, so there other widths would read what they do not use
+    const PairTiles pt = GLU ? plan_pair_tiles(a.M, a.J, pairs, 64) : BMN ? plan_pair_tiles(a.M, a.J, pairs, 32) : plan_pair_waves(a.M, a.J, pairs, 16);
     p.tiles_m = (a.M + 255) / 256; p.tiles_j = pt.tiles_j; p.tile_w = pt.tile_w; p.n_whole = pt.n_whole; p.n_items = pt.n_items;
     if (pairs > p.n_items) pairs = p.n_items;
-    CUtensorMap tmA, tmB, tmBh, tmA2, tmB2, tmD, tmD32;
+    CUtensorMap tmA, tmB, tmBh, tmA2, tmB2, tmD, tmD16;
     int rc;
     if ((rc = make_tmap_bf16(&tmA, a.A, a.M, a.R, a.lda, 64, 128))) return rc;
     if (BMN) {
@@ -299,7 +303,7 @@ int launch_dp(const LutGemmArgs& a, int sms, cudaStream_t stream) {
         }
     }
     if ((rc = make_tmap_bf16(&tmD, a.out, a.M, p.out_cols, a.ld_out, 64, 32))) return rc;
-    if ((rc = make_tmap_bf16(&tmD32, a.out, a.M, p.out_cols, a.ld_out, 32, 32))) return rc;
+    if ((rc = make_tmap_bf16(&tmD16, a.out, a.M, p.out_cols, a.ld_out, 16, 32))) return rc;
     auto kern = dense_gemm_pair_kernel<BMN, GLU>;
     static bool attr_set[64] = {};
     int dev = 0;
@@ -308,7 +312,7 @@ int launch_dp(const LutGemmArgs& a, int sms, cudaStream_t stream) {
         PLZ_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kDpSmemBytes));
         attr_set[dev & 63] = true;
     }
-    kern<<<2 * pairs, kDpThreads, kDpSmemBytes, stream>>>(tmA, tmB, tmBh, tmA2, tmB2, tmD, tmD32, p);
+    kern<<<2 * pairs, kDpThreads, kDpSmemBytes, stream>>>(tmA, tmB, tmBh, tmA2, tmB2, tmD, tmD16, p);
     PLZ_LAUNCH_CHECK();
     return PLZ_OK;
 }

@@ -513,6 +513,27 @@ PairTiles plan_pair_tiles(int M, int J, int pairs, int step) {
     return t;
 }
 
+// One or two waves of narrower tiles where they are fewer columns in all: 2048 x 2560 outputs are 80 tiles of 256 on 74 pairs, a wave and one of halves, 384
+// columns; or 144 tiles of 144, two nearly full waves, 288. For the dense kernel (packed weights are decoded in chains that cost 160 columns at least).
+// us plan_pair_tiles / here: 2048 rows, 2560 x 2560 26.5 / 22.4, 2560 x 9728 87.6 / 84.8, 2560 x 4096 40.8 / 38.9; 1000 rows, 7680 x 2560 34.0 / 31.7; 512 rows, 9728 x 2560
+// 30.0 / 28.2. More waves or more rows do not pay, as narrow tiles read more of both operands: 1536 rows, 9728 x 2560 in four waves of 208 columns 57.6 / 62.5, 4096 rows,
+// 2560 x 9728 in four of 144 151 / 178; nor do gated outputs (512 rows, 19456 x 2560 44.2 / 45.4).
+PairTiles plan_pair_waves(int M, int J, int pairs, int step) {
+    PairTiles best = plan_pair_tiles(M, J, pairs, 32);
+    const int tiles_m = (M + 255) / 256;
+    if (tiles_m > 8) return best;
+    auto waves = [&](int tiles) { return (tiles + pairs - 1) / pairs; };
+    int cost = best.n_items > best.n_whole ? waves(best.n_whole) * 256 + 128 : waves(best.n_whole) * best.tile_w;
+    for (int w = 256 - step; w >= 128; w -= step) {
+        const int tj = (J + w - 1) / w, n = waves(tiles_m * tj);
+        if (n <= 2 && n * w * 100 < cost * 97) {
+            cost = n * w;
+            best.tile_w = w; best.tiles_j = tj; best.n_whole = best.n_items = tiles_m * tj;
+        }
+    }
+    return best;
+}
+
 // PLZ_ERR_UNSUPPORTED: not a shape for this kernel, the caller falls back to the single-CTA kernel.
 int launch_lut_gemm_pair(const LutGemmArgs& a, cudaStream_t stream) {
     if (!g_pair_gemm) return PLZ_ERR_UNSUPPORTED;

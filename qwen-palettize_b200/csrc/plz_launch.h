@@ -36,7 +36,8 @@ int launch_lut_gemm(const LutGemmArgs& a, cudaStream_t stream);
 int launch_lut_gemm_pair(const LutGemmArgs& a, cudaStream_t stream);
 // tiles of 256 x tile_w outputs for CTA pairs: items [0, n_whole) whole, the others halves (128 columns) of the tiles behind them
 struct PairTiles { int tile_w, tiles_j, n_whole, n_items; };
-PairTiles plan_pair_tiles(int M, int J, int pairs, int step = 32);   // step: tile widths are multiples of it
+PairTiles plan_pair_tiles(int M, int J, int pairs, int step);   // step: tile widths are multiples of it
+PairTiles plan_pair_waves(int M, int J, int pairs, int step);   // the same with other widths where one or two waves of them are fewer columns in all
 // dense_gemm_pair.cu: the dense modes on CTA pairs; PLZ_ERR_UNSUPPORTED = not a shape for it
 int launch_dense_gemm_pair(const LutGemmArgs& a, cudaStream_t stream);
 extern int g_pair_gemm;  // 0: keep every product on the single-CTA kernel
