@@ -170,8 +170,9 @@ lut_smallm_mma_kernel(const SmallmParams p) {
         // 8-byte unit. Up to eight loads (one per row) per thread in flight together. Only the M real rows are staged: a
         // column n >= M of an mma only ever reaches the same column of D, which is never written out, so the lanes of those
         // columns simply read row 0
+        // Warp 0 last: it is still issuing copies, and what it would load comes behind all of them.
         const int chunks_per_row = p.K >> 3;
-        for (int c = threadIdx.x; c < chunks_per_row; c += kThreads) {
+        for (int c = (threadIdx.x - 32) & (kThreads - 1); c < chunks_per_row; c += kThreads) {
             const int k = c << 3;
             const int kg = k >> 8, r = k & 255, tq = r >> 6, wi = (r & 63) >> 4, hh = (r >> 3) & 1;
             uint8_t* dst = xs + (size_t)(((kg * 16 + wi * 4) * 4 + tq) * 8 + hh * 4);
