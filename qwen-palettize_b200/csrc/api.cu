@@ -344,7 +344,7 @@ int32_t plz_hard_fwd_smallm_multi(const plz_weight_t* const* ws, int32_t count, 
     }
     if (M == 0) return PLZ_OK;
     if (!x) { set_last_error("null activation pointer"); return PLZ_ERR_NULL; }
-    int rc = launch_lut_smallm_mma_multi(g, count, (cudaStream_t)stream);
+    int rc = launch_lut_smallm_mma_multi(g, count, (cudaStream_t)stream, false);
     if (rc == PLZ_ERR_UNSUPPORTED)
         set_last_error("smallm_multi: needs K %% 256 == 0, palette groups of a multiple of 256 columns, 16-byte aligned x rows "
                        "and M * K small enough for shared memory; call plz_hard_fwd_smallm per matrix instead");
@@ -1251,6 +1251,24 @@ int decode_linears(const plz_decode_linear_t* const* ws, int count, const void* 
         if ((rc = plz_hard_fwd_smallm(wp[i], x, ldx, M, ys[i], ldys[i], stream))) return rc;
     return PLZ_OK;
 }
+// act = silu(x Wg^T) * (x Wu^T) by one launch, or PLZ_ERR_UNSUPPORTED: the products and the activation apart
+int decode_gate_up(const plz_decode_linear_t& gate, const plz_decode_linear_t& up, const void* x, int64_t ldx, int32_t M, void* act, int64_t ld, void* stream) {
+    if (gate.N != up.N || gate.K != up.K || gate.gs_n != up.gs_n || gate.gs_k != up.gs_k || M > 64) return PLZ_ERR_UNSUPPORTED;
+    int rc;
+    NarrowArgs n = {};
+    GemvArgs g[2] = {};
+    for (int i = 0; i < 2; ++i) {
+        const plz_decode_linear_t& w = i ? up : gate;
+        const plz_weight_t d = {(int32_t)w.N, (int32_t)w.K, (int32_t)w.gs_n, (int32_t)w.gs_k, w.packed, w.packed_pitch, w.palette};
+        if ((rc = check_weight(&d, true))) return rc;
+        n.mat[i].N = d.N; n.mat[i].packed = d.packed; n.mat[i].pitch = d.packed_pitch; n.mat[i].palette = d.palette; n.mat[i].y = act; n.mat[i].ldy = ld;
+        g[i].M = M; g[i].N = d.N; g[i].K = d.K; g[i].x = x; g[i].ldx = ldx; g[i].packed = d.packed; g[i].packed_pitch = d.packed_pitch; g[i].palette = d.palette;
+        g[i].gs_n = d.gs_n; g[i].gs_k = d.gs_k; g[i].out = act; g[i].ld_out = ld; g[i].sm_count = seq_sm_count();
+    }
+    if (M <= 16) return launch_lut_smallm_mma_multi(g, 2, (cudaStream_t)stream, true);
+    n.M = M; n.K = g[0].K; n.x = x; n.ldx = ldx; n.count = 2; n.gs_n = g[0].gs_n; n.gs_k = g[0].gs_k; n.alpha = 1.0f; n.early = 1; n.glu = 1;
+    return launch_narrow_gemm(n, (cudaStream_t)stream);
+}
 }  // namespace
 
 int64_t plz_decode_ws_bytes(int32_t B, int32_t T, int32_t hidden, int32_t intermediate, int32_t n_heads, int32_t n_kv_heads) {
@@ -1304,8 +1322,11 @@ int32_t plz_decode_hidden(const plz_decode_t* a, const plz_decode_layer_t* layer
         if ((rc = plz_attn_decode(q, d.qd, kc, vc, a->batch_stride, a->tok_stride, B, T, Hq, Hkv, 128, (float)(1.0 / sqrt(128.0)), att, d.qd, ws, d.attn, stream))) return rc;
         if ((rc = decode_linears(&ow, 1, att, d.qd, B, &lin, &h_ld, stream))) return rc;
         if ((rc = plz_add_rmsnorm_fwd(h, H, lin, H, x2, H, L.post_ln, B, H, eps, norm, H, nullptr, stream))) return rc;
-        if ((rc = decode_linears(gu, 2, norm, H, B, gu_out, gu_ld, stream))) return rc;
-        if ((rc = plz_swiglu_fwd(gate, F, up, F, B, F, act, F, stream))) return rc;
+        if ((rc = decode_gate_up(L.gate, L.up, norm, H, B, act, F, stream)) == PLZ_ERR_UNSUPPORTED) {
+            if ((rc = decode_linears(gu, 2, norm, H, B, gu_out, gu_ld, stream))) return rc;
+            rc = plz_swiglu_fwd(gate, F, up, F, B, F, act, F, stream);
+        }
+        if (rc) return rc;
         if ((rc = decode_linears(&dw, 1, act, F, B, &lin, &h_ld, stream))) return rc;
         // the residual add closes the layer and the same pass applies the next layer's (or the final) norm
         void* h_next = last ? a->h : h_a;

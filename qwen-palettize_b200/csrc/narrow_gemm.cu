@@ -49,6 +49,7 @@ struct NarrowParams {
     int nkb, n_blocks;             // blocks of 64 columns of W; the same plus the extra block
     int count; NarrowMat mat[kNgMaxMats];
     int gs_n, gs_k, n_kgroups;
+    int glu;                       // a tile is 64 rows of mat[0] and the same rows of mat[1]
     const __nv_bfloat16* bias; int act, y_f32; float alpha;
     StatusWord* status;
 };
@@ -103,7 +104,8 @@ narrow_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
     for (int i = 1; i < kNgMaxMats; ++i)
         if (i < p.count && tile >= p.mat[i].first_tile) mi = i;
     const NarrowMat& mat = p.mat[mi];
-    const int n0 = (tile - mat.first_tile) * 128;
+    const bool glu = LUT && p.glu;
+    const int n0 = (tile - mat.first_tile) * (glu ? 64 : 128);
     const int b_begin = (int)((long long)rank * p.n_blocks / n_ranks), b_end = (int)((long long)(rank + 1) * p.n_blocks / n_ranks);
     const int nb = b_end - b_begin;        // at least one: the cluster is no larger than the number of blocks
 
@@ -127,9 +129,11 @@ narrow_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
     const int row = (warp & 3) * 32 + lane;                         // decode: thread = one weight row = its TMEM lane
     const int grp = LUT && warp >= 6 ? 1 : 0;
     const int nw = b_end < p.nkb ? nb : p.nkb - b_begin;            // blocks of W in this CTA's range
-    const bool row_ok = n0 + row < mat.N;
-    const uint8_t* prow = LUT ? mat.packed + (row_ok ? (long long)(n0 + row) * mat.pitch : 0ll) + (long long)b_begin * 16 : nullptr;
-    const __nv_bfloat16* pal = LUT ? mat.palette + (row_ok ? (long long)((n0 + row) / p.gs_n) * p.n_kgroups * 4 : 0ll) : nullptr;
+    const NarrowMat& own = glu && row >= 64 ? p.mat[1] : mat;
+    const int wrow = n0 + (glu ? row & 63 : row);
+    const bool row_ok = wrow < mat.N;
+    const uint8_t* prow = LUT ? own.packed + (row_ok ? (long long)wrow * own.pitch : 0ll) + (long long)b_begin * 16 : nullptr;
+    const __nv_bfloat16* pal = LUT ? own.palette + (row_ok ? (long long)(wrow / p.gs_n) * p.n_kgroups * 4 : 0ll) : nullptr;
     uint4 w[kAhead];
     uint2 pr[kAhead];
     auto fetch = [&](int it, int j) {
@@ -305,7 +309,31 @@ narrow_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
 #pragma unroll
         for (int i = 0; i < 8; ++i) from[i] = map_rank(base, i < n_ranks ? i : 0);
         const bool turned = !LUT && p.transposed;
-        const int quads = p.npad / 4, units = turned ? 128 * quads : p.M * 32;       // (token, 4 weight rows); turned: (weight row, 4 tokens)
+        if (glu) {       // (token, 4 outputs): gate rows from lanes below 64, up rows from the others
+            const int units = p.M * 16, u1 = (int)((long long)(rank + 1) * units / n_ranks);
+            for (int u = (int)((long long)rank * units / n_ranks) + threadIdx.x; u < u1; u += kNgThreads<LUT>) {
+                const int m = u >> 4, r = (u & 15) * 4, n = n0 + r;
+                float v[8] = {};
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    float4 f[8];
+#pragma unroll
+                    for (int i = 0; i < 8; ++i)
+                        if (i < n_ranks) f[i] = ld_cluster_f4(from[i] + (uint32_t)(m * 128 + h * 64 + r) * 4u);
+#pragma unroll
+                    for (int i = 0; i < 8; ++i)
+                        if (i < n_ranks) { v[h * 4] += f[i].x; v[h * 4 + 1] += f[i].y; v[h * 4 + 2] += f[i].z; v[h * 4 + 3] += f[i].w; }
+                }
+#pragma unroll
+                for (int e = 0; e < 4; ++e) v[e] = swiglu_of_sums(v[e], v[4 + e]);
+                __nv_bfloat16* y = (__nv_bfloat16*)mat.y + (long long)m * mat.ldy + n;
+                if (n + 3 < mat.N && !((uintptr_t)y & 7)) { *reinterpret_cast<uint2*>(y) = make_uint2(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3])); continue; }
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    if (n + e < mat.N) y[e] = __float2bfloat16_rn(v[e]);
+            }
+        }
+        const int quads = p.npad / 4, units = glu ? 0 : turned ? 128 * quads : p.M * 32;       // (token, 4 weight rows); turned: (weight row, 4 tokens)
         const int u1 = (int)((long long)(rank + 1) * units / n_ranks);
         for (int u = (int)((long long)rank * units / n_ranks) + threadIdx.x; u < u1; u += kNgThreads<LUT>) {
             const int m = turned ? u % quads * 4 : u >> 5, r = turned ? u / quads : (u & 31) * 4, n = n0 + r;
@@ -447,6 +475,8 @@ int launch_narrow_gemm(const NarrowArgs& a, cudaStream_t stream) {
     p.nkb = (a.K + 63) / 64; p.n_blocks = p.nkb + (a.r2 > 0 ? 1 : 0);
     p.count = a.count;
     p.gs_n = a.gs_n; p.gs_k = a.gs_k; p.n_kgroups = lut ? a.K / a.gs_k : 0;
+    if (a.glu && (!lut || a.count != 2 || a.mat[0].N != a.mat[1].N || a.r2 || a.bias || a.act || a.y_f32 || a.alpha != 1.0f)) return PLZ_ERR_UNSUPPORTED;
+    p.glu = a.glu;
     p.bias = (const __nv_bfloat16*)a.bias; p.act = a.act; p.y_f32 = a.y_f32; p.alpha = a.alpha;
     p.status = device_status_ptr();
     int tiles = 0, rc;
@@ -455,6 +485,10 @@ int launch_narrow_gemm(const NarrowArgs& a, cudaStream_t stream) {
         if (s.N < 1 || (a.act == ACT_GLU_GELU && s.N % 2) || (lut && (((uintptr_t)s.packed & 15) || s.pitch % 16 || ((uintptr_t)s.palette & 7)))) return PLZ_ERR_UNSUPPORTED;
         p.mat[i] = NarrowMat{s.N, tiles, (const uint8_t*)s.packed, s.pitch, (const __nv_bfloat16*)s.palette, s.y, s.ldy};
         tiles += (s.N + 127) / 128;
+    }
+    if (a.glu) {
+        tiles = (a.mat[0].N + 63) / 64;
+        p.mat[1].first_tile = 0x7FFFFFFF;        // every tile belongs to the first
     }
     CUtensorMap tm[4];
     if ((rc = a.x_mn ? make_tmap_bf16(&tm[0], a.x, a.K, a.M, a.ldx, 64, 64) : make_tmap_bf16(&tm[0], a.x, a.M, a.K, a.ldx, 64, (uint32_t)p.npad))) return rc;

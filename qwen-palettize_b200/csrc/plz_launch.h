@@ -68,6 +68,7 @@ struct NarrowArgs {
     } mat[4];
     int gs_n, gs_k;
     int r2; const void* x2; long long ldx2; const void* w2; long long ldw2;   // extra block: x2 [M, r2], w2 [N, r2]
+    int glu;                          // packed, two matrices of the same size: mat[0].y = silu(x W0^T) * (x W1^T)
     const void* bias; int act;        // bf16 [N], SeqAct
     int y_f32; float alpha;           // y = act(alpha * sum + bias)
 };
@@ -115,7 +116,8 @@ struct GemvArgs {
 int launch_lut_gemv(const GemvArgs& a, cudaStream_t stream);
 // smallm_mma.cu: M <= 16 on mma.sync fragments; PLZ_ERR_UNSUPPORTED = shape outside its domain, use launch_lut_gemv's kernels
 int launch_lut_smallm_mma(const GemvArgs& a, cudaStream_t stream);
-int launch_lut_smallm_mma_multi(const GemvArgs* mats, int count, cudaStream_t stream);  // 1..4 matrices sharing x
+// 1..4 matrices sharing x; glu: two of the same size, mats[0].out = silu(x W0^T) * (x W1^T)
+int launch_lut_smallm_mma_multi(const GemvArgs* mats, int count, cudaStream_t stream, bool glu);
 extern int g_smallm_overlap;        // 1: launch the mma.sync small-M kernel with programmatic stream serialization
 extern int g_debug_smallm_variant;  // 0 = automatic choice, 1 = never use the mma.sync kernel (comparisons)
 

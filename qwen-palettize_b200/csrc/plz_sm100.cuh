@@ -410,6 +410,13 @@ __device__ __forceinline__ void decode16(uint32_t w, const PalRegs& pal, uint32_
     out[7] = prmt_raw(pal.lo, pal.hi, cd1 >> 16);
 }
 
+// silu(gate) * up of two products' sums, rounded where the products, the activation and the multiplication as kernels of their own round to bf16
+// (the last rounding is the caller's)
+__device__ __forceinline__ float swiglu_of_sums(float gate, float up) {
+    const float g = __bfloat162float(__float2bfloat16_rn(gate)), u = __bfloat162float(__float2bfloat16_rn(up));
+    return __bfloat162float(__float2bfloat16_rn(__fdividef(g, 1.0f + __expf(-g)))) * u;
+}
+
 __device__ __forceinline__ uint32_t pack_bf16x2(float a, float b) {
     __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
     return *reinterpret_cast<uint32_t*>(&v);

@@ -78,7 +78,8 @@ __device__ __forceinline__ void mma_bf16_16816(float (&d)[4], const uint32_t (&a
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
-template <int MT>  // MT m8 tiles: M <= 8 * MT
+// MT m8 tiles: M <= 8 * MT. GLU: two matrices of N rows, a gate and an up projection; a CTA takes the same rows of both and writes silu(gate) * up
+template <int MT, bool GLU>
 __global__ void __launch_bounds__(SmallmCfg<MT>::kThreads, 1)
 lut_smallm_mma_kernel(const SmallmParams p) {
     constexpr int kThreads = SmallmCfg<MT>::kThreads, kWarps = SmallmCfg<MT>::kWarps, kBatch = SmallmCfg<MT>::kBatch;
@@ -89,8 +90,8 @@ lut_smallm_mma_kernel(const SmallmParams p) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int g = lane >> 2, t = lane & 3;
     const int r0 = blockIdx.x * p.rows_per_cta;
-    const int r1 = min(p.N, r0 + p.rows_per_cta);
-    const int rows = r1 - r0;
+    const int mine = min(p.N, r0 + p.rows_per_cta) - r0;
+    const int rows = GLU ? 2 * mine : mine;
     const int strips = (rows + 15) >> 4;
     const int kgs = p.K >> 8;               // 256-column groups along K
     const int n_items = strips * kgs;
@@ -100,6 +101,12 @@ lut_smallm_mma_kernel(const SmallmParams p) {
     uint8_t* pal_sm = wsm + (size_t)p.rows_alloc * row_bytes;
     uint8_t* xs = pal_sm + (size_t)p.rows_alloc * p.pal_bytes;
     float* acc_s = reinterpret_cast<float*>(xs + (size_t)p.M * p.x_pitch);
+
+    // row r of the CTA: its matrix and row there
+    auto locate = [&](int r, int& mi, int& lr) {
+        mi = GLU ? (r >= mine ? 1 : 0) : mat_of(p, r0 + r);
+        lr = GLU ? r0 + r - mi * mine : r0 + r - p.row_start[mi];
+    };
 
     const long long t_entry = PLZ_PROF_ON(p.prof) ? clock64() : 0;
     // ---- the CTA's packed rows: one bulk copy per 16-row strip (rows of a matrix are contiguous when its pitch is the
@@ -116,10 +123,11 @@ lut_smallm_mma_kernel(const SmallmParams p) {
             mbar_arrive_expect_tx(bar0 + 8u * s, (uint32_t)(b - a) * (row_bytes + p.pal_bytes));
             int r = a;
             while (r < b) {
-                const int mi = mat_of(p, r0 + r), lr = r0 + r - p.row_start[mi];
+                int mi, lr;
+                locate(r, mi, lr);
                 const long long pitch = p.pitch[mi];
                 int n = 1;  // rows of this piece
-                if (pitch == (long long)row_bytes) n = min(b - r, p.row_start[mi + 1] - (r0 + r));
+                if (pitch == (long long)row_bytes) n = min(b - r, GLU ? (mi + 1) * mine - r : p.row_start[mi + 1] - (r0 + r));
                 bulk_load(smem_u32(wsm) + (uint32_t)r * row_bytes, p.packed[mi] + (long long)lr * pitch, (uint32_t)n * row_bytes,
                           bar0 + 8u * s);
                 if (p.pal_bytes)
@@ -140,8 +148,9 @@ lut_smallm_mma_kernel(const SmallmParams p) {
         kg += kWarps;
         while (kg >= kgs) { kg -= kgs; ++s; }
     };
-    auto palette_of = [&](int v, int kg) -> uint2 {
-        const int mi = mat_of(p, v), lr = v - p.row_start[mi];
+    auto palette_of = [&](int r, int kg) -> uint2 {
+        int mi, lr;
+        locate(r, mi, lr);
         const int ng = p.gs_n_shift >= 0 ? (lr >> p.gs_n_shift) : (lr / p.gs_n);
         const int pg = p.gs_k_shift >= 0 ? ((kg << 8) >> p.gs_k_shift) : ((kg << 8) / p.gs_k);
         return __ldg(reinterpret_cast<const uint2*>(p.palette[mi] + ((long long)ng * p.n_kgroups + pg) * 4));
@@ -152,9 +161,9 @@ lut_smallm_mma_kernel(const SmallmParams p) {
             const int item = first_item + q * kWarps;
             pa[q] = make_uint2(0u, 0u); pb[q] = pa[q];
             if (item < n_items) {
-                const int ra = r0 + s * 16 + g, rb = ra + 8;
-                if (ra < r1) pa[q] = palette_of(ra, kg);
-                if (rb < r1) pb[q] = palette_of(rb, kg);
+                const int ra = s * 16 + g, rb = ra + 8;
+                if (ra < rows) pa[q] = palette_of(ra, kg);
+                if (rb < rows) pb[q] = palette_of(rb, kg);
             }
             advance(s, kg);
         }
@@ -287,7 +296,13 @@ lut_smallm_mma_kernel(const SmallmParams p) {
     __syncthreads();
     ok = (abort_flag[0] == 0u) && (abort_flag[1] == 0u);
     // ---- write the tile: consecutive threads walk the weight rows of one token (contiguous in y)
-    for (int i = threadIdx.x; ok && i < p.M * rows; i += kThreads) {
+    if (GLU) {
+        for (int i = threadIdx.x; ok && i < p.M * mine; i += kThreads) {
+            const int m = i / mine, r = i - m * mine;
+            p.out[0][(long long)m * p.ld_out[0] + r0 + r] = __float2bfloat16_rn(swiglu_of_sums(acc_s[(size_t)r * (8 * MT) + m], acc_s[(size_t)(mine + r) * (8 * MT) + m]));
+        }
+    }
+    for (int i = threadIdx.x; ok && !GLU && i < p.M * rows; i += kThreads) {
         const int m = i / rows, r = i - m * rows;
         const int mi = mat_of(p, r0 + r), lr = r0 + r - p.row_start[mi];
         p.out[mi][(long long)m * p.ld_out[mi] + lr] = __float2bfloat16_rn(acc_s[(size_t)r * (8 * MT) + m]);
@@ -305,7 +320,8 @@ int g_smallm_overlap = 0;  // plz_set_smallm_overlap
 
 // Returns PLZ_OK, or PLZ_ERR_UNSUPPORTED (without setting the error text) when the shape is outside this kernel's
 // domain and the caller should use another small-M kernel. `mats` matrices (1..4) share x, K and the palette grouping.
-int launch_lut_smallm_mma_multi(const GemvArgs* mats, int count, cudaStream_t stream) {
+int launch_lut_smallm_mma_multi(const GemvArgs* mats, int count, cudaStream_t stream, bool glu) {
+    if (glu && (count != 2 || mats[0].N != mats[1].N)) return PLZ_ERR_UNSUPPORTED;
     if (count < 1 || count > kMaxMats) return PLZ_ERR_UNSUPPORTED;
     const GemvArgs& a = mats[0];
     if (a.M < 1 || a.M > 16 || a.K % 256 || a.gs_k % 256 || ((uintptr_t)a.x & 15) || (a.ldx & 7)) return PLZ_ERR_UNSUPPORTED;
@@ -327,12 +343,14 @@ int launch_lut_smallm_mma_multi(const GemvArgs* mats, int count, cudaStream_t st
     const int sms = a.sm_count > 0 ? a.sm_count : 1;
     int grid = sms;
     if (grid > (total + 15) / 16) grid = (total + 15) / 16;
-    int rows_per_cta = (total + grid - 1) / grid;
-    grid = (total + rows_per_cta - 1) / rows_per_cta;
+    if (glu) total = a.N;                 // rows of either matrix
+    const int share = (total + grid - 1) / grid;
+    grid = (total + share - 1) / share;
+    const int rows_per_cta = glu ? 2 * share : share;
     const int rows_pad = ((rows_per_cta + 15) / 16) * 16;
     p.x = (const __nv_bfloat16*)a.x; p.ldx = a.ldx;
     p.M = a.M; p.N = total; p.K = a.K; p.gs_n = a.gs_n; p.gs_k = a.gs_k; p.n_kgroups = a.K / a.gs_k;
-    p.rows_per_cta = rows_per_cta;
+    p.rows_per_cta = share;
     p.gs_n_shift = p.gs_k_shift = -1;
     for (int sh = 0; sh < 31; ++sh) {
         if ((1 << sh) == a.gs_n) p.gs_n_shift = sh;
@@ -374,18 +392,20 @@ int launch_lut_smallm_mma_multi(const GemvArgs* mats, int count, cudaStream_t st
                 half[i].x = (const __nv_bfloat16*)mats[i].x + (long long)m0 * mats[i].ldx;
                 half[i].out = (__nv_bfloat16*)mats[i].out + (long long)m0 * mats[i].ld_out;
             }
-            const int rc = launch_lut_smallm_mma_multi(half, count, stream);
+            const int rc = launch_lut_smallm_mma_multi(half, count, stream, glu);
             if (rc != PLZ_OK) return rc;
         }
         return PLZ_OK;
     }
-    static int attr_smem[2][64] = {};
+    void (*const kern)(const SmallmParams) = mt == 1 ? (glu ? lut_smallm_mma_kernel<1, true> : lut_smallm_mma_kernel<1, false>)
+                                                     : (glu ? lut_smallm_mma_kernel<2, true> : lut_smallm_mma_kernel<2, false>);
+    static bool attr_set[4][64] = {};
     int dev = 0;
     PLZ_CUDA_CHECK(cudaGetDevice(&dev));
-    if (attr_smem[mt - 1][dev & 63] < (int)smem) {
-        if (mt == 1) PLZ_CUDA_CHECK(cudaFuncSetAttribute(lut_smallm_mma_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
-        else PLZ_CUDA_CHECK(cudaFuncSetAttribute(lut_smallm_mma_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
-        attr_smem[mt - 1][dev & 63] = 227 * 1024;
+    bool& set = attr_set[2 * (mt - 1) + (glu ? 1 : 0)][dev & 63];
+    if (!set) {
+        PLZ_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+        set = true;
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid); cfg.blockDim = dim3(mt == 1 ? SmallmCfg<1>::kThreads : SmallmCfg<2>::kThreads); cfg.dynamicSmemBytes = smem; cfg.stream = stream;
@@ -393,12 +413,11 @@ int launch_lut_smallm_mma_multi(const GemvArgs* mats, int count, cudaStream_t st
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr; cfg.numAttrs = g_smallm_overlap ? 1 : 0;
-    if (mt == 1) PLZ_CUDA_CHECK(cudaLaunchKernelEx(&cfg, lut_smallm_mma_kernel<1>, p));
-    else PLZ_CUDA_CHECK(cudaLaunchKernelEx(&cfg, lut_smallm_mma_kernel<2>, p));
+    PLZ_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kern, p));
     ++g_launch_count;
     return PLZ_OK;
 }
 
-int launch_lut_smallm_mma(const GemvArgs& a, cudaStream_t stream) { return launch_lut_smallm_mma_multi(&a, 1, stream); }
+int launch_lut_smallm_mma(const GemvArgs& a, cudaStream_t stream) { return launch_lut_smallm_mma_multi(&a, 1, stream, false); }
 
 }  // namespace plz
