@@ -50,6 +50,7 @@ struct PairParams {
     int n_whole, n_items;    // items [0, n_whole) are whole tiles, the others halves of 128 columns of the tiles behind (tile_w = 256 then)
     const uint8_t* packed; long long packed_pitch;
     const __nv_bfloat16* palette;
+    const uint8_t* packed2; const __nv_bfloat16* palette2;   // GLU: the up projection
     int gs_n, gs_k, n_kgroups, gs_n_shift;
     int gs_k_shift;          // log2(gs_k / 64) or -1
     int Wn, Wk;
@@ -74,7 +75,9 @@ constexpr uint32_t kEpiOff = kStages * kStageBytes;
 constexpr uint32_t kBarOff = kEpiOff + kEpiWarps * kEpiStageBytes;
 constexpr uint32_t kSmemBytes = kBarOff + 1024 + 256;
 
-template <int BMODE>
+// GLU (forward): the tile's columns are the same outputs of a gate and of an up projection, half and half, one decoded by either CTA, and the
+// epilogue writes silu(gate) * up: of a feed-forward's 4096 x 9728 outputs 80 MB reach memory, where the products apart and an element-wise pass move 400.
+template <int BMODE, bool GLU>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 lut_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmA2,
                      const __grid_constant__ CUtensorMap tmB2, const __grid_constant__ CUtensorMap tmD, const __grid_constant__ CUtensorMap tmD32,
@@ -133,7 +136,7 @@ lut_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
     auto item_origin = [&](int t, int& m0, int& j0) {
         const int cut = t - p.n_whole;                       // >= 0: a half tile
         const int tile = cut < 0 ? t : p.n_whole + (cut >> 1);
-        j0 = (tile % p.tiles_j) * p.tile_w + (cut < 0 ? 0 : (cut & 1) * 128);
+        j0 = ((tile % p.tiles_j) * p.tile_w + (cut < 0 ? 0 : (cut & 1) * 128)) >> (GLU ? 1 : 0);
         m0 = (tile / p.tiles_j) * 256;
     };
 
@@ -269,11 +272,11 @@ lut_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
                 q.ip = p.packed + (long long)rr * p.packed_pitch + (k >> 2);
                 q.pp = p.palette;
             } else {
-                const int n = jr + rr;
+                const int n = (GLU ? j0 : jr) + rr;
                 q.ok0 = q.ok1 = n < p.Wn && rr < half;
-                q.ip = p.packed + (long long)n * p.packed_pitch + h * 8;
+                q.ip = (GLU && rank ? p.packed2 : p.packed) + (long long)n * p.packed_pitch + h * 8;
                 const int ng = q.ok0 ? ((p.gs_n_shift >= 0) ? (n >> p.gs_n_shift) : (n / p.gs_n)) : 0;
-                q.pp = p.palette + (long long)ng * p.n_kgroups * 4;
+                q.pp = (GLU && rank ? p.palette2 : p.palette) + (long long)ng * p.n_kgroups * 4;
             }
         };
         auto normalise = [&](int& tile, int& it) {          // true: another tile
@@ -367,7 +370,7 @@ lut_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
         for (int t = pair; t < p.n_items && ok; t += n_pairs, ++lt) {
             int m0, j0;
             item_origin(t, m0, j0);
-            const int w = item_width(t);
+            const int w = GLU ? item_width(t) >> 1 : item_width(t);     // outputs
             const int buf = lt & 1;
             const int mrow = m0 + 128 * (int)rank + lane_group * 32;
             ok = mbar_wait(acc_full(buf), (lt >> 1) & 1, abort_flag, p.status, ST_TIMEOUT_ACCUM, 4);
@@ -378,8 +381,30 @@ lut_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
                 const bool wide = col + 32 < w;            // a box of 64 columns, or the last 32 of a tile
                 if (lane == 0) tma_store_wait_read();
                 __syncwarp();
+                if (GLU) {
+                    const uint32_t at = tmem_base + ((uint32_t)(lane_group * 32) << 16) + buf * 256u + col;
 #pragma unroll
-                for (int c = 0; c < 2; ++c) {
+                    for (int c = 0; c < 8; ++c) {
+                        if (c == 4 && !wide) break;
+                        uint32_t vg[8], vu[8], o[4];
+                        tmem_ld_32x8(at + c * 8, vg);
+                        tmem_ld_32x8(at + w + c * 8, vu);
+                        if (col + 8 * (c + 1) >= w) {
+                            tc_fence_before_sync();
+                            __syncwarp();
+                            if (lane == 0) mbar_arrive_cluster(lead_acc_empty(buf));
+                        }
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            const float a0 = __uint_as_float(vg[2 * i]), a1 = __uint_as_float(vg[2 * i + 1]);
+                            o[i] = pack_bf16x2(__fdividef(a0, 1.0f + __expf(-a0)) * __uint_as_float(vu[2 * i]), __fdividef(a1, 1.0f + __expf(-a1)) * __uint_as_float(vu[2 * i + 1]));
+                        }
+                        const uint32_t to = wide ? swz128(lane, c) : (uint32_t)(lane * 64 + ((c ^ ((lane >> 1) & 3)) << 4));
+                        *reinterpret_cast<uint4*>(stage + to) = make_uint4(o[0], o[1], o[2], o[3]);
+                    }
+                }
+#pragma unroll
+                for (int c = 0; c < (GLU ? 0 : 2); ++c) {
                     if (c == 1 && !wide) break;
                     uint32_t v[32];
                     tmem_ld_32x32(tmem_base + ((uint32_t)(lane_group * 32) << 16) + buf * 256u + col + c * 32, v);
@@ -433,8 +458,9 @@ lut_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
     }
 }
 
-template <int BMODE>
+template <int BMODE, bool GLU = false>
 int launch_pair_t(const LutGemmArgs& a, cudaStream_t stream) {
+    const int J = GLU ? a.J / 2 : a.J;     // columns of the result
     CUtensorMap tmA, tmA2, tmB2, tmD, tmD32;
     int rc;
     if ((rc = make_tmap_bf16(&tmA, a.A, a.M, a.R, a.lda, 64, 128))) return rc;
@@ -447,12 +473,13 @@ int launch_pair_t(const LutGemmArgs& a, cudaStream_t stream) {
             if ((rc = make_tmap_bf16(&tmB2, a.B2, a.J, a.r2, a.ldb2, 64, 128))) return rc;
         }
     }
-    if ((rc = make_tmap_bf16(&tmD, a.out, a.M, a.J, a.ld_out, 64, 32))) return rc;
-    if ((rc = make_tmap_bf16(&tmD32, a.out, a.M, a.J, a.ld_out, 32, 32))) return rc;
+    if ((rc = make_tmap_bf16(&tmD, a.out, a.M, J, a.ld_out, 64, 32))) return rc;
+    if ((rc = make_tmap_bf16(&tmD32, a.out, a.M, J, a.ld_out, 32, 32))) return rc;
     PairParams p = {};
-    p.M = a.M; p.J = a.J; p.R = a.R; p.n_extra = a.r2 > 0 ? 1 : 0;
+    p.M = a.M; p.J = J; p.R = a.R; p.n_extra = a.r2 > 0 ? 1 : 0;
     p.packed = (const uint8_t*)a.packed; p.packed_pitch = a.packed_pitch;
     p.palette = (const __nv_bfloat16*)a.palette;
+    p.packed2 = (const uint8_t*)a.packed2; p.palette2 = (const __nv_bfloat16*)a.palette2;
     p.gs_n = a.gs_n > 0 ? a.gs_n : 1; p.gs_k = a.gs_k > 0 ? a.gs_k : kBK;
     p.n_kgroups = a.gs_k > 0 ? (a.Wk / a.gs_k) : 1;
     p.gs_n_shift = -1;
@@ -463,7 +490,7 @@ int launch_pair_t(const LutGemmArgs& a, cudaStream_t stream) {
     p.alpha = a.alpha; p.bias = (const __nv_bfloat16*)a.bias;
     p.status = device_status_ptr();
     p.prof = (unsigned long long*)a.prof;
-    auto kern = lut_gemm_pair_kernel<BMODE>;
+    auto kern = lut_gemm_pair_kernel<BMODE, GLU>;
     static bool attr_set[64] = {};
     int dev = 0, sms = 0;
     PLZ_CUDA_CHECK(cudaGetDevice(&dev));
@@ -477,7 +504,8 @@ int launch_pair_t(const LutGemmArgs& a, cudaStream_t stream) {
     int pairs = sms / 2;
     if (pairs < 1) return PLZ_ERR_UNSUPPORTED;
     // backward product: a decode thread's 32 columns start at a multiple of 32 (8-byte loads of indices, one palette group)
-    const PairTiles pt = plan_pair_tiles(a.M, a.J, pairs, BMODE == B_DECODE_MN ? 64 : 32);
+    // gated: half of a tile's columns is a multiple of 32 outputs
+    const PairTiles pt = plan_pair_tiles(a.M, a.J, pairs, BMODE == B_DECODE_MN || GLU ? 64 : 32);
     p.tiles_j = pt.tiles_j; p.tile_w = pt.tile_w; p.n_whole = pt.n_whole; p.n_items = pt.n_items;
     if (pairs > p.n_items) pairs = p.n_items;
     cudaLaunchConfig_t cfg = {};
@@ -538,7 +566,11 @@ PairTiles plan_pair_waves(int M, int J, int pairs, int step) {
 int launch_lut_gemm_pair(const LutGemmArgs& a, cudaStream_t stream) {
     if (!g_pair_gemm) return PLZ_ERR_UNSUPPORTED;
     if (a.bmode != B_DECODE_K && a.bmode != B_DECODE_MN) return PLZ_ERR_UNSUPPORTED;
-    const bool plain = a.fuse == 0 || (a.fuse == 2 && !a.col_scale && !a.row_scale);   // fuse 2 without norm factors: at most a bias
+    const bool factors = a.col_scale || a.row_scale;
+    if (a.fuse == 1 && !factors && !a.gate_out && !a.up_out && a.r2 == 0 && a.alpha == 1.0f && a.M >= 256 && a.J >= 512 && a.Wk % 16 == 0 && a.bmode == B_DECODE_K &&
+        !((uintptr_t)a.packed2 & 15) && !((uintptr_t)a.palette2 & 7))
+        return launch_pair_t<B_DECODE_K, true>(a, stream);
+    const bool plain = a.fuse == 0 || (a.fuse == 2 && !factors);   // fuse 2 without norm factors: at most a bias
     if (!plain || a.M < 256 || a.J < 256) return PLZ_ERR_UNSUPPORTED;
     if ((uintptr_t)a.bias & 15) return PLZ_ERR_UNSUPPORTED;
     if (a.bmode == B_DECODE_MN && (a.J % 16)) return PLZ_ERR_UNSUPPORTED;

@@ -188,7 +188,11 @@ class PalettizedQwen:
                 act = ops.mlp_gate_up_forward(L["gate"], L["up"], x2, ops.rms_rstd(x2, c.eps), L["post_ln"])
             else:
                 x2, h2 = ops.add_rmsnorm_forward(h, o, L["post_ln"], c.eps)
-                act = ops.swiglu_forward(ops.hard_forward(L["gate"], h2)[0], ops.hard_forward(L["up"], h2)[0])
+                g, u = L["gate"], L["up"]
+                if B * S >= 256 and g.N % 128 == 0 and (u.N, u.K, u.gs_n, u.gs_k, u.packed.stride(0)) == (g.N, g.K, g.gs_n, g.gs_k, g.packed.stride(0)):
+                    act = ops.mlp_gate_up_forward(g, u, h2)      # on CTA pairs too, act is all that is written
+                else:
+                    act = ops.swiglu_forward(ops.hard_forward(g, h2)[0], ops.hard_forward(u, h2)[0])
             d = ops.hard_forward(L["down"], act)[0]
             # the residual add closes the layer and the same pass applies the next layer's (or the final) norm
             h, h1 = ops.add_rmsnorm_forward(x2, d, self.layers[li + 1]["input_ln"] if li + 1 < n else self.final_norm, c.eps)
