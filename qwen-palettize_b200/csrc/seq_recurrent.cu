@@ -6,7 +6,7 @@
 // This form serves token decode (bound by streaming the state), short portions and the 32-bit mode. A warp holds 8 value columns
 // x dk key rows in registers: lane = 8 * (key row group) + column, row group g owning rows g, g + 4, g + 8, ..., so a warp's access
 // to the state is whole 32-byte sectors, a token's key and query are conflict-free broadcasts from shared memory, and the sums
-// over the key dimension take two shuffles.
+// over the key dimension take two shuffles. A single token moves the state through 16-byte accesses instead (recurrent_step_kernel).
 #include "seq_math.cuh"
 
 namespace plz {
@@ -105,6 +105,97 @@ recurrent_kernel(const RecParams p) {
     }
 }
 
+// One token, dk a multiple of 16 up to 128: bound by reading and writing the state once. A warp of the kernel above moves it 4 bytes per lane, 32 bytes of a row at a
+// time; here a lane holds four columns of eight rows, a warp access is 128 bytes of four rows, and the four warps of a block share the key rows of 32 columns, so the
+// sums over keys meet in shared memory. 64 sequences, 20 heads of 128 x 128 (168 MB), in a decode chain: decayed 41 -> 30 us, delta 42 -> 25.
+constexpr int kStepRows = 8;       // key rows of a lane
+__device__ __forceinline__ float4 load4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float4 load4(const __nv_bfloat16* p) {
+    const uint2 r = *reinterpret_cast<const uint2*>(p);
+    return make_float4(__uint_as_float(r.x << 16), __uint_as_float(r.x & 0xFFFF0000u), __uint_as_float(r.y << 16), __uint_as_float(r.y & 0xFFFF0000u));
+}
+__device__ __forceinline__ void fma4(float4& d, float a, const float4& b) { d.x = fmaf(a, b.x, d.x); d.y = fmaf(a, b.y, d.y); d.z = fmaf(a, b.z, d.z); d.w = fmaf(a, b.w, d.w); }
+// over the four row groups of a warp
+__device__ __forceinline__ float4 sum_groups(float4 v) {
+#pragma unroll
+    for (int o = 8; o <= 16; o <<= 1) {
+        v.x += __shfl_xor_sync(0xFFFFFFFFu, v.x, o); v.y += __shfl_xor_sync(0xFFFFFFFFu, v.y, o);
+        v.z += __shfl_xor_sync(0xFFFFFFFFu, v.z, o); v.w += __shfl_xor_sync(0xFFFFFFFFu, v.w, o);
+    }
+    return v;
+}
+__device__ __forceinline__ float4 sum_warps(const float4 (&part)[4][8], int c) {
+    float4 v = part[0][c];
+#pragma unroll
+    for (int w = 1; w < 4; ++w) { v.x += part[w][c].x; v.y += part[w][c].y; v.z += part[w][c].z; v.w += part[w][c].w; }
+    return v;
+}
+
+template <typename T, bool DELTA>
+__global__ void __launch_bounds__(128)
+recurrent_step_kernel(const RecParams p) {
+    __shared__ float sq[128], sk[128], sg[128];
+    __shared__ float4 part[2][4][8];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, kg = lane >> 3, c = lane & 7;
+    const int col = (int)blockIdx.x * 32 + c * 4, h = blockIdx.y;
+    const long long b = blockIdx.z;
+    const int hk = DELTA ? h / (p.H / p.G) : h;
+    const bool live = col < p.dv;
+    const int row0 = warp * (p.dk >> 2) + kg, rows = p.dk >> 4;      // key rows of this lane: row0 + 4 i, i < rows
+    float* Sp = p.S + ((b * p.H + h) * p.dk + row0) * (long long)p.dv + col;
+    const long long step = 4ll * p.dv;
+    pdl_launch_dependents();
+    pdl_wait();
+    float4 s[kStepRows];
+#pragma unroll
+    for (int i = 0; i < kStepRows; ++i) s[i] = live && i < rows ? __ldcs(reinterpret_cast<const float4*>(Sp + i * step)) : make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 v = live ? load4((const T*)p.v + b * p.ldv + (long long)h * p.dv + col) : make_float4(0.f, 0.f, 0.f, 0.f);
+    if ((int)threadIdx.x < p.dk) {
+        float q = to_f(((const T*)p.q)[b * p.ldq + (long long)hk * p.dk + threadIdx.x]), k = to_f(((const T*)p.k)[b * p.ldk + (long long)hk * p.dk + threadIdx.x]);
+        if (DELTA) sg[threadIdx.x] = expf(p.logg[(b * p.H + h) * p.dk + threadIdx.x]);
+        else { q = silu_f(q); k = silu_f(k); }
+        sq[threadIdx.x] = q;
+        sk[threadIdx.x] = k;
+    }
+    const float lam = DELTA ? p.beta[b * p.H + h] : p.decay[h];
+    __syncthreads();
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f), u = v;
+    if (DELTA) {
+        float4 pred = acc;
+#pragma unroll
+        for (int i = 0; i < kStepRows; ++i) {
+            if (i >= rows) break;
+            const float g = sg[row0 + 4 * i];
+            s[i] = make_float4(s[i].x * g, s[i].y * g, s[i].z * g, s[i].w * g);
+            fma4(pred, sk[row0 + 4 * i], s[i]);
+        }
+        pred = sum_groups(pred);
+        if (kg == 0) part[0][warp][c] = pred;
+        __syncthreads();
+        pred = sum_warps(part[0], c);
+        u = make_float4(lam * (v.x - pred.x), lam * (v.y - pred.y), lam * (v.z - pred.z), lam * (v.w - pred.w));
+    } else {
+        u = make_float4(silu_f(v.x), silu_f(v.y), silu_f(v.z), silu_f(v.w));
+    }
+#pragma unroll
+    for (int i = 0; i < kStepRows; ++i) {
+        if (i >= rows) break;
+        if (!DELTA) s[i] = make_float4(lam * s[i].x, lam * s[i].y, lam * s[i].z, lam * s[i].w);
+        fma4(s[i], sk[row0 + 4 * i], u);
+        fma4(acc, sq[row0 + 4 * i], s[i]);
+        if (live) __stcs(reinterpret_cast<float4*>(Sp + i * step), s[i]);
+    }
+    acc = sum_groups(acc);
+    if (kg == 0) part[1][warp][c] = acc;
+    __syncthreads();
+    if (threadIdx.x < 8 && live) *reinterpret_cast<float4*>(p.o + (b * p.H + h) * (long long)p.dv + col) = sum_warps(part[1], c);
+}
+
+template <typename T, bool DELTA>
+bool step_form(const RecParams& p) {
+    return p.n == 1 && p.dk <= 128 && p.dk % 16 == 0 && p.dv % 4 == 0 && !(((uintptr_t)p.S | (uintptr_t)p.o) & 15) && !((uintptr_t)p.v & (4 * sizeof(T) - 1)) && p.ldv % 4 == 0;
+}
+
 template <typename T, bool DELTA, int RK>
 int launch_rk(const RecParams& p, int B, cudaStream_t stream) {
     const size_t smem = (size_t)(DELTA ? 3 : 2) * kTok * 4 * RK * sizeof(float);
@@ -113,6 +204,10 @@ int launch_rk(const RecParams& p, int B, cudaStream_t stream) {
 }
 template <typename T, bool DELTA>
 int launch_any(const RecParams& p, int B, cudaStream_t stream) {
+    if (step_form<T, DELTA>(p)) {
+        PLZ_LAUNCH_CHAIN((recurrent_step_kernel<T, DELTA>), dim3((p.dv + 31) / 32, p.H, B), dim3(128), 0, stream, p);
+        return PLZ_OK;
+    }
     if (p.dk <= 32) return launch_rk<T, DELTA, 8>(p, B, stream);
     if (p.dk <= 64) return launch_rk<T, DELTA, 16>(p, B, stream);
     if (p.dk <= 128) return launch_rk<T, DELTA, 32>(p, B, stream);
