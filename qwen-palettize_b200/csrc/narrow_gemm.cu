@@ -18,6 +18,8 @@
 //
 // Accumulating into the tile the previous MMA still writes costs a TMEM round trip, so the four MMAs of a block go to several accumulators,
 // as many as fit, which the epilogue adds.
+#include <type_traits>
+
 #include "attention_tiles.cuh"
 #include "seq_math.cuh"
 
@@ -70,8 +72,9 @@ __device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr) {
     return v;
 }
 
+// dense: four warps read the accumulators, two more help with the cluster's sums
 template <bool LUT>
-constexpr int kNgThreads = 64 + 32 * (LUT ? kNgDecodeWarps : 4);
+constexpr int kNgThreads = 64 + 32 * (LUT ? kNgDecodeWarps : 6);
 
 template <bool LUT>
 __global__ void __launch_bounds__(kNgThreads<LUT>, 2)
@@ -265,20 +268,36 @@ narrow_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
         }
         // ---------------------------------------------------------- this CTA's partial tile in the ring's space: [token][weight row], transposed
         // [weight row][npad tokens]
-        if (warp < 6) {
+        // The accumulators of 16 columns are read behind one wait, packed by both groups of decode warps in turn. Read one after the other, they and the
+        // sums below were half of what a launch costs beside its blocks. 64 rows, microseconds in a row of launches: dense 2560 x 2560 8.1 -> 7.6,
+        // 9728 x 2560 13.7 -> 13.0; packed 2560 x 2560 8.6 -> 8.1, 19456 x 2560 24.7 -> 23.7. Pushing the shares to their owner with bulk copies
+        // instead of fetching them behind the cluster's barrier is slower by 0.8 - 1.4 (dense 2560 x 2560 8.7, packed 9.4).
+        if (LUT || warp < 6) {
             pdl_wait();
             if (ok) ok = mbar_wait(acc_full, 0, abort_flag, p.status, ST_TIMEOUT_ACCUM, 4);
             if (ok) {
                 tc_fence_after_sync();
                 const int lg = warp & 3;
                 float* part = reinterpret_cast<float*>(smem) + lg * 32 + lane;
-                for (int c0 = 0; c0 < p.npad && c0 < p.M; c0 += 16) {
+                constexpr int kGroups = LUT ? 2 : 1;
+                for (int c0 = LUT && warp >= 6 ? 16 : 0; c0 < p.npad && c0 < p.M; c0 += 16 * kGroups) {
+                    const uint32_t at = tmem_base + ((uint32_t)(lg * 32) << 16) + c0;
                     float sum[16];
-                    for (int a = 0; a < p.n_acc; ++a) {
-                        uint32_t v[16];
-                        tmem_ld_32x16(tmem_base + ((uint32_t)(lg * 32) << 16) + a * p.npad + c0, v);
+                    if (p.n_acc == 4) {
+                        uint32_t v[4][16];
+                        tmem_ld_sets(at, (uint32_t)p.npad, v);
 #pragma unroll
-                        for (int c = 0; c < 16; ++c) sum[c] = a == 0 ? __uint_as_float(v[c]) : sum[c] + __uint_as_float(v[c]);
+                        for (int c = 0; c < 16; ++c) sum[c] = __uint_as_float(v[0][c]) + __uint_as_float(v[1][c]) + __uint_as_float(v[2][c]) + __uint_as_float(v[3][c]);
+                    } else if (p.n_acc == 2) {
+                        uint32_t v[2][16];
+                        tmem_ld_sets(at, (uint32_t)p.npad, v);
+#pragma unroll
+                        for (int c = 0; c < 16; ++c) sum[c] = __uint_as_float(v[0][c]) + __uint_as_float(v[1][c]);
+                    } else {
+                        uint32_t v[16];
+                        tmem_ld_32x16(at, v);
+#pragma unroll
+                        for (int c = 0; c < 16; ++c) sum[c] = __uint_as_float(v[c]);
                     }
                     if (!LUT && p.transposed) {
                         float4* to = reinterpret_cast<float4*>(smem) + ((lg * 32 + lane) * p.npad + c0) / 4;
@@ -309,43 +328,11 @@ narrow_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
 #pragma unroll
         for (int i = 0; i < 8; ++i) from[i] = map_rank(base, i < n_ranks ? i : 0);
         const bool turned = !LUT && p.transposed;
-        if (glu) {       // (token, 4 outputs): gate rows from lanes below 64, up rows from the others
-            const int units = p.M * 16, u1 = (int)((long long)(rank + 1) * units / n_ranks);
-            for (int u = (int)((long long)rank * units / n_ranks) + threadIdx.x; u < u1; u += kNgThreads<LUT>) {
-                const int m = u >> 4, r = (u & 15) * 4, n = n0 + r;
-                float v[8] = {};
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    float4 f[8];
-#pragma unroll
-                    for (int i = 0; i < 8; ++i)
-                        if (i < n_ranks) f[i] = ld_cluster_f4(from[i] + (uint32_t)(m * 128 + h * 64 + r) * 4u);
-#pragma unroll
-                    for (int i = 0; i < 8; ++i)
-                        if (i < n_ranks) { v[h * 4] += f[i].x; v[h * 4 + 1] += f[i].y; v[h * 4 + 2] += f[i].z; v[h * 4 + 3] += f[i].w; }
-                }
-#pragma unroll
-                for (int e = 0; e < 4; ++e) v[e] = swiglu_of_sums(v[e], v[4 + e]);
-                __nv_bfloat16* y = (__nv_bfloat16*)mat.y + (long long)m * mat.ldy + n;
-                if (n + 3 < mat.N && !((uintptr_t)y & 7)) { *reinterpret_cast<uint2*>(y) = make_uint2(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3])); continue; }
-#pragma unroll
-                for (int e = 0; e < 4; ++e)
-                    if (n + e < mat.N) y[e] = __float2bfloat16_rn(v[e]);
-            }
-        }
-        const int quads = p.npad / 4, units = glu ? 0 : turned ? 128 * quads : p.M * 32;       // (token, 4 weight rows); turned: (weight row, 4 tokens)
-        const int u1 = (int)((long long)(rank + 1) * units / n_ranks);
-        for (int u = (int)((long long)rank * units / n_ranks) + threadIdx.x; u < u1; u += kNgThreads<LUT>) {
+        const int quads = p.npad / 4;
+        // one unit of the results with its sums: (token, 4 weight rows), turned: (weight row, 4 tokens), glu: (token, 4 outputs), gate sums behind up sums
+        auto finish = [&](int u, float (&v)[4]) {
             const int m = turned ? u % quads * 4 : u >> 5, r = turned ? u / quads : (u & 31) * 4, n = n0 + r;
-            float v[4] = {0.f, 0.f, 0.f, 0.f};
-            float4 f[8];
-#pragma unroll
-            for (int i = 0; i < 8; ++i)
-                if (i < n_ranks) f[i] = ld_cluster_f4(from[i] + (uint32_t)u * 16u);
-#pragma unroll
-            for (int i = 0; i < 8; ++i)
-                if (i < n_ranks) { v[0] += f[i].x; v[1] += f[i].y; v[2] += f[i].z; v[3] += f[i].w; }
-            if (n >= mat.N) continue;
+            if (n >= mat.N) return;
             if (turned) {
                 __nv_bfloat16* y = (__nv_bfloat16*)mat.y + (long long)n * mat.ldy + m;
 #pragma unroll
@@ -356,7 +343,7 @@ narrow_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
                     for (int e = 0; e < 4; ++e)
                         if (m + e < p.M) y[e] = __float2bfloat16_rn(v[e]);
                 }
-                continue;
+                return;
             }
             if (p.act == ACT_GLU_GELU) {      // N is even
                 const long long o = (long long)m * mat.ldy + (n >> 1);
@@ -370,7 +357,7 @@ narrow_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
                     y[0] = __float2bfloat16_rn(a);
                     if (n + 2 < mat.N) y[1] = __float2bfloat16_rn(b);
                 }
-                continue;
+                return;
             }
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
@@ -381,18 +368,69 @@ narrow_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
             const long long o = (long long)m * mat.ldy + n;
             if (p.y_f32) {
                 float* y = (float*)mat.y + o;
-                if (n + 3 < mat.N && !((uintptr_t)y & 15)) { *reinterpret_cast<float4*>(y) = make_float4(v[0], v[1], v[2], v[3]); continue; }
+                if (n + 3 < mat.N && !((uintptr_t)y & 15)) { *reinterpret_cast<float4*>(y) = make_float4(v[0], v[1], v[2], v[3]); return; }
 #pragma unroll
                 for (int e = 0; e < 4; ++e)
                     if (n + e < mat.N) y[e] = v[e];
             } else {
                 __nv_bfloat16* y = (__nv_bfloat16*)mat.y + o;
-                if (n + 3 < mat.N && !((uintptr_t)y & 7)) { *reinterpret_cast<uint2*>(y) = make_uint2(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3])); continue; }
+                if (n + 3 < mat.N && !((uintptr_t)y & 7)) { *reinterpret_cast<uint2*>(y) = make_uint2(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3])); return; }
 #pragma unroll
                 for (int e = 0; e < 4; ++e)
                     if (n + e < mat.N) y[e] = __float2bfloat16_rn(v[e]);
             }
-        }
+        };
+        auto finish_glu = [&](int u, const float (&g)[4], const float (&h)[4]) {
+            const int m = u >> 4, n = n0 + (u & 15) * 4;
+            float v[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) v[e] = swiglu_of_sums(g[e], h[e]);
+            __nv_bfloat16* y = (__nv_bfloat16*)mat.y + (long long)m * mat.ldy + n;
+            if (n + 3 < mat.N && !((uintptr_t)y & 7)) { *reinterpret_cast<uint2*>(y) = make_uint2(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3])); return; }
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                if (n + e < mat.N) y[e] = __float2bfloat16_rn(v[e]);
+        };
+        const int units = glu ? p.M * 16 : turned ? 128 * quads : p.M * 32;
+        const int u0 = (int)((long long)rank * units / n_ranks), u1 = (int)((long long)(rank + 1) * units / n_ranks);
+        // packed: two units at a time in a cluster of two, whose trips to the partner's shared memory would come one after the other; no gain where W is dense
+        auto gather = [&](auto ranks_at_most) {
+            constexpr int kRanks = decltype(ranks_at_most)::value, kUnits = LUT && kRanks < 4 ? 4 / kRanks : 1;
+            for (int at = u0 + (int)threadIdx.x; at < u1; at += kNgThreads<LUT> * kUnits) {
+                float v[kUnits][4] = {};
+                auto sums = [&](int half, float (&to)[kUnits][4]) {
+                    float4 f[kUnits][kRanks];
+#pragma unroll
+                    for (int b = 0; b < kUnits; ++b) {
+                        const int u = at + b * kNgThreads<LUT>;
+                        const uint32_t off = (uint32_t)(glu ? (u >> 4) * 32 + half * 16 + (u & 15) : u) * 16u;
+#pragma unroll
+                        for (int i = 0; i < kRanks; ++i)
+                            if (u < u1 && i < n_ranks) f[b][i] = ld_cluster_f4(from[i] + off);
+                    }
+#pragma unroll
+                    for (int b = 0; b < kUnits; ++b)
+#pragma unroll
+                        for (int i = 0; i < kRanks; ++i)
+                            if (i < n_ranks) { to[b][0] += f[b][i].x; to[b][1] += f[b][i].y; to[b][2] += f[b][i].z; to[b][3] += f[b][i].w; }
+                };
+                sums(0, v);
+                if (glu) {
+                    float h[kUnits][4] = {};
+                    sums(1, h);
+#pragma unroll
+                    for (int b = 0; b < kUnits; ++b)
+                        if (at + b * kNgThreads<LUT> < u1) finish_glu(at + b * kNgThreads<LUT>, v[b], h[b]);
+                } else {
+#pragma unroll
+                    for (int b = 0; b < kUnits; ++b)
+                        if (at + b * kNgThreads<LUT> < u1) finish(at + b * kNgThreads<LUT>, v[b]);
+                }
+            }
+        };
+        if (n_ranks <= 2) gather(std::integral_constant<int, 2>());
+        else if (n_ranks <= 4) gather(std::integral_constant<int, 4>());
+        else gather(std::integral_constant<int, 8>());
     }
     cluster_sync_all();        // nobody leaves while its partial tile may still be read
     if (warp == 1) { tc_fence_after_sync(); tmem_dealloc(tmem_base, p.tmem_cols); }
