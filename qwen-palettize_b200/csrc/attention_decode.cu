@@ -441,6 +441,81 @@ attn_decode_combine_kernel(const float* ws_o, const float* ws_ml, int splits, in
     }
 }
 
+// The same with a chain of one trip to memory instead of two: a warp takes every `parts`-th split and four dimensions per lane, requests its partial sums together with the
+// maxima of all splits, of which every warp works out the weights for itself. dv a multiple of 4 up to 128. 2048 keys, 32 heads: 4.5 -> 2.05 us, of a step of one sequence 242 -> 232 us.
+template <typename T>
+__global__ void __launch_bounds__(512)
+attn_decode_combine4_kernel(const float* ws_o, const float* ws_ml, int splits, int Hq, int dv, int sink, T* out, long long ldo) {
+    __shared__ float4 red[16][32];
+    const int head = blockIdx.x, b = blockIdx.y, lane = threadIdx.x & 31, part = threadIdx.x >> 5, parts = blockDim.x >> 5;
+    const long long slot0 = ((long long)b * Hq + head) * splits;
+    const bool live = lane * 4 < dv;
+    pdl_launch_dependents();
+    pdl_wait();
+    constexpr int kEach = kMaxSplits / 16, kMl = kMaxSplits / 32;
+    float4 o[kEach];
+#pragma unroll
+    for (int j = 0; j < kEach; ++j) {
+        const int s = part + j * parts;
+        o[j] = live && s < splits ? __ldcs(reinterpret_cast<const float4*>(ws_o + (slot0 + s) * dv) + lane) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    float m[kMl], l[kMl], M = sink ? 0.f : kNegBig;
+#pragma unroll
+    for (int i = 0; i < kMl; ++i) {
+        const int s = lane + 32 * i;
+        const float2 ml = s < splits ? *reinterpret_cast<const float2*>(ws_ml + (slot0 + s) * 2) : make_float2(kNegBig, 0.f);
+        m[i] = ml.x;
+        l[i] = ml.y;
+        M = fmaxf(M, ml.x);
+    }
+#pragma unroll
+    for (int i = 16; i > 0; i >>= 1) M = fmaxf(M, __shfl_xor_sync(0xFFFFFFFFu, M, i));
+    float L = 0.f;
+#pragma unroll
+    for (int i = 0; i < kMl; ++i) {
+        m[i] = ex2(m[i] - M);
+        L = fmaf(m[i], l[i], L);
+    }
+#pragma unroll
+    for (int i = 16; i > 0; i >>= 1) L += __shfl_xor_sync(0xFFFFFFFFu, L, i);
+    if (sink) L += ex2(-M);
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int j = 0; j < kEach; ++j) {
+        const int s = part + j * parts;             // the same in all lanes
+        if (s >= splits) break;
+        const float w = s < 32 ? m[0] : s < 64 ? m[1] : s < 96 ? m[2] : m[3];
+        const float c = __shfl_sync(0xFFFFFFFFu, w, s & 31);
+        acc.x = fmaf(c, o[j].x, acc.x); acc.y = fmaf(c, o[j].y, acc.y); acc.z = fmaf(c, o[j].z, acc.z); acc.w = fmaf(c, o[j].w, acc.w);
+    }
+    red[part][lane] = acc;
+    __syncthreads();
+    if (part == 0 && live) {
+        for (int i = 1; i < parts; ++i) {
+            const float4 v = red[i][lane];
+            acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
+        }
+        T* to = out + (long long)b * ldo + (long long)head * dv + lane * 4;
+        const float v[4] = {acc.x, acc.y, acc.z, acc.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) store_elem(to + e, L > 0.f ? v[e] / L : 0.f);
+    }
+}
+
+template <typename T>
+int launch_combine(const DecParams& p, int B, int dv, int sink, cudaStream_t stream) {
+    if (dv % 4 == 0 && dv <= 128 && !((uintptr_t)p.ws_o & 15) && !((uintptr_t)p.ws_ml & 7)) {
+        int parts = 1;
+        while (parts < p.splits && parts < 16) parts *= 2;
+        PLZ_LAUNCH_CHAIN(attn_decode_combine4_kernel<T>, dim3(p.Hq, B), dim3(32 * parts), 0, stream, (const float*)p.ws_o, (const float*)p.ws_ml, p.splits, p.Hq, dv, sink,
+                         (T*)p.out, p.ldo);
+    } else {
+        PLZ_LAUNCH_CHAIN(attn_decode_combine_kernel<T>, dim3(p.Hq, B), dim3(128), 0, stream, (const float*)p.ws_o, (const float*)p.ws_ml, p.splits, p.Hq, dv, sink, (T*)p.out,
+                         p.ldo);
+    }
+    return PLZ_OK;
+}
+
 // out[i, :] = table[ids[i], :] (bf16 rows of `width`, width % 8 == 0); an id outside [0, vocab) gives a zero row and sets *bad
 __global__ void __launch_bounds__(256)
 embed_gather_kernel(const __nv_bfloat16* __restrict__ table, long long ldt, const long long* __restrict__ ids, long long n, int width,
@@ -505,11 +580,7 @@ int launch_attn_decode(const AttnDecodeArgs& a, cudaStream_t stream) {
     const dim3 grid(p.splits, a.Hkv * p.passes, a.B), block(kDecWarps * 32);
     if ((long long)a.B * a.Hkv * a.T <= 8192) PLZ_LAUNCH_CHAIN((attn_decode_partial_kernel<__nv_bfloat16, 16, false>), grid, block, 0, stream, p);
     else PLZ_LAUNCH_CHAIN(attn_decode_mma_kernel<false>, grid, block, 0, stream, p);
-    if (p.splits > 1) {
-        PLZ_LAUNCH_CHAIN(attn_decode_combine_kernel<__nv_bfloat16>, dim3(a.Hq, a.B), dim3(128), 0, stream, (const float*)p.ws_o, (const float*)p.ws_ml,
-                         p.splits, a.Hq, 128, 0, (__nv_bfloat16*)p.out, p.ldo);
-    }
-    return PLZ_OK;
+    return p.splits > 1 ? launch_combine<__nv_bfloat16>(p, a.B, 128, 0, stream) : PLZ_OK;
 }
 
 // splits for a cache of `cap` positions whose length is known on the device only
@@ -538,11 +609,7 @@ static int launch_attn_bias_decode_t(const AttnBiasArgs& a, int cap, float* ws, 
     else if (d <= 128 && sizeof(T) == 2) PLZ_LAUNCH_CHAIN(attn_decode_mma_kernel<true>, grid, block, 0, stream, p);
     else if (d <= 128) PLZ_LAUNCH_CHAIN((attn_decode_partial_kernel<float, 16, true>), grid, block, 0, stream, p);
     else PLZ_LAUNCH_CHAIN((attn_decode_partial_kernel<T, 32, true>), grid, block, 0, stream, p);
-    if (p.splits > 1) {
-        PLZ_LAUNCH_CHAIN(attn_decode_combine_kernel<T>, dim3(a.H, a.B), dim3(128), 0, stream, (const float*)p.ws_o, (const float*)p.ws_ml, p.splits, a.H,
-                         a.dv, a.sink, (T*)p.out, p.ldo);
-    }
-    return PLZ_OK;
+    return p.splits > 1 ? launch_combine<T>(p, a.B, a.dv, a.sink, stream) : PLZ_OK;
 }
 int launch_attn_bias_decode(int dtype, const AttnBiasArgs& a, int cap, void* ws, long long ws_bytes, cudaStream_t stream) {
     if (a.B <= 0) return PLZ_OK;
