@@ -9,13 +9,15 @@
 // All products run on the 5th-generation tensor cores (tcgen05.mma, 128 x 128 x 16, accumulators in TMEM), operands
 // staged by TMA in 128-byte-swizzled tiles. One CTA handles one (batch, head) and one or two 128-token tiles:
 //   forward        two neighbouring query tiles per CTA: S = Q K^T -> online softmax by 128 threads per tile (one row each,
-//                  TMEM -> registers) -> P (bf16) to shared memory -> O += P V, O rescaled in TMEM when a row maximum grows;
+//                  TMEM -> registers) -> P (bf16) to shared memory -> O += P V, O rescaled in TMEM when a row maximum has outgrown its reference;
 //                  the softmax of one tile runs under the MMAs of the other; also writes the row log-sum-exp.
 //   backward dQ    per q tile: S, dP = dO V^T -> dS = P (dP - D) / sqrt(d) -> dQ += dS K
 //   backward dKdV  per kv tile and kv head, over the q heads of the group and the q tiles at or after it:
 //                  S, dP -> P, dS to shared memory -> dV += P^T dO, dK += dS^T Q  (P^T / dS^T are the same bytes read
 //                  through an MN-major operand descriptor)
 // D[row] = sum_d dO O is a small pre-pass. Every barrier wait is bounded (status word, as in the GEMM kernels).
+#include <type_traits>
+
 #include "attention_tiles.cuh"
 
 namespace plz {
@@ -61,15 +63,24 @@ __device__ __forceinline__ void load_tile(uint32_t dst, const CUtensorMap* map, 
 // ---------------------------------------------------------------------------------------------------------------------
 // One CTA takes TWO neighbouring 128-query tiles (A = tile 2i, B = tile 2i + 1) of one head and walks the key / value tiles
 // they share once. Warps 0-3 are the softmax group of A, warps 4-7 of B (thread = query row = TMEM lane), warp 8 issues the
-// TMA copies and the MMAs. S_A, S_B, O_A, O_B fill the 512 TMEM columns; Q_A, Q_B, two K stages, one V stage and one P tile
-// per group (7 x 32 KB) fill the shared memory. While one group runs its softmax on S(j), the tensor core runs the other group's O += P V(j - 1... j)
-// and S(j + 1): the exponentials (MUFU, 16 per clock) and the MMAs cost about the same per tile, so each hides the other.
-constexpr int kFwdThreads = 288;   // warps 0..3 / 4..7: softmax of tile A / B, warp 8: TMA + MMA
-constexpr uint32_t kFwdSmem = 7 * kTile + 1024 + 256;   // Q x 2, K x 2, V, P x 2
+// MMAs, warp 9 the TMA copies. S_A, S_B, O_A, O_B fill the 512 TMEM columns; Q_A, Q_B, a ring of three key or value tiles and one P tile
+// per group (7 x 32 KB) fill the shared memory. A group takes its scores S(j) into registers at once, and S(j + 1) is computed
+// while it works on them, so that it waits for neither product: the exponentials (MUFU, 16 per clock) and the MMAs cost about the same per tile
+// and each hides the other. The ring takes the tiles in the order of their use, K_0 K_1 V_0 K_2 V_1 .., each requested a whole step ahead.
+constexpr int kFwdThreads = 320;   // warps 0..3 / 4..7: softmax of tile A / B, warp 8: MMA, warp 9: TMA
+constexpr uint32_t kFwdSmem = 7 * kTile + 1024 + 256;   // Q x 2, K / V x 3, P x 2
+
+__device__ __forceinline__ uint64_t pair_f32(float a, float b) { uint64_t d; asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(a), "f"(b)); return d; }
+__device__ __forceinline__ void split_f32(uint64_t v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c) { uint64_t d; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c)); return d; }
+__device__ __forceinline__ uint64_t mul_f32x2(uint64_t a, uint64_t b) { uint64_t d; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
+__device__ __forceinline__ uint64_t add_f32x2(uint64_t a, uint64_t b) { uint64_t d; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
+
+__device__ __forceinline__ float ex2(float x) { float y; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
 
 struct FwdGroup {          // what one softmax group works on
     uint32_t tS, tO;       // TMEM columns of its score and output accumulators
-    uint32_t s_full, p_full, o_full;
+    uint32_t s_full, s_free, p_full, o_full;
     uint8_t* pP; uint32_t sP;
     int qt;                // its query tile; it attends key tiles 0 .. qt
 };
@@ -80,77 +91,102 @@ __device__ __forceinline__ void fwd_softmax_group(const FwdGroup& G, const AttnP
     const uint32_t lane_off = (uint32_t)(warp_in_group * 32) << 16;
     const float c = p.scale * kLog2e;
     const int n_kv = G.qt + 1;
-    float m_run = -INFINITY, l_run = 0.f;
+    // m_run: the reference of the exponentials, moved only when the maximum has outgrown it by 2^8: O is then rescaled in the first tiles of a row and hardly again.
+    // The scores of a row stay in registers between the maximum and the exponentials (128 of them, one read of TMEM instead of two), maximum and sum run in
+    // four chains each, and only the tile on the diagonal is compared with the row. 4 x 1024 tokens, 32 heads: 84 -> 67 us, and 53 us with S(j + 1) computed meanwhile (8 x 512: 53 -> 43,
+    // 1 x 4096: 255 -> 120); the exponentials alone are 17 us.
+    float m_run = -INFINITY;
+    uint64_t l_run[2] = {0ull, 0ull};
     bool ok = true;
     for (int j = 0; j < n_kv && ok; ++j) {
         ok = mbar_wait(G.s_full, j & 1, abort_flag, p.status, ST_TIMEOUT_ACCUM, 20);
         if (!ok) break;
         tc_fence_after_sync();
+        uint32_t v[128];
+        tmem_ld_32x128(G.tS + lane_off, v);
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(G.s_free);
         const bool diag = (j == G.qt);
-        // pass 1: row maximum of this tile
-        float m_tile = -INFINITY;
-#pragma unroll 1
-        for (int cb = 0; cb < 4; ++cb) {
-            uint32_t v[32];
-            tmem_ld_32x32(G.tS + lane_off + cb * 32, v);
+        if (diag) {
 #pragma unroll
-            for (int i = 0; i < 32; ++i) {
-                const float sc = __uint_as_float(v[i]);
-                if (!diag || cb * 32 + i <= r) m_tile = fmaxf(m_tile, sc);
-            }
+            for (int i = 0; i < 128; ++i)
+                if (i > r) v[i] = 0xFF800000u;                 // -inf
         }
-        const float m_new = fmaxf(m_run, m_tile);
-        const float alpha = (m_run == -INFINITY) ? 0.f : exp2f((m_run - m_new) * c);
+        float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+        for (int i = 0; i < 128; i += 8)
+#pragma unroll
+            for (int k = 0; k < 4; ++k) m4[k] = fmaxf(fmaxf(m4[k], __uint_as_float(v[i + k])), __uint_as_float(v[i + 4 + k]));
+        const float m_tile = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3]));
+        const bool moved = m_run == -INFINITY || (m_tile - m_run) * c > kLazyGrowth;
+        const float alpha = !moved ? 1.f : m_run == -INFINITY ? 0.f : exp2f((m_run - m_tile) * c);
+        if (moved) m_run = m_tile;
         // the previous P V product must have landed before O is rescaled and before P is overwritten
         if (j > 0) {
             ok = mbar_wait(G.o_full, (j - 1) & 1, abort_flag, p.status, ST_TIMEOUT_ACCUM, 21);
             if (!ok) break;
             tc_fence_after_sync();
-            if (__any_sync(0xFFFFFFFFu, m_new > m_run)) {
+            if (__any_sync(0xFFFFFFFFu, moved)) {
+                const uint64_t a2 = pair_f32(alpha, alpha);
+                l_run[0] = mul_f32x2(l_run[0], a2);
+                l_run[1] = mul_f32x2(l_run[1], a2);
 #pragma unroll 1
-                for (int cb = 0; cb < 4; ++cb) {
-                    uint32_t v[32];
-                    tmem_ld_32x32(G.tO + lane_off + cb * 32, v);
+                for (int cb = 0; cb < 16; ++cb) {
+                    uint32_t o[8];
+                    tmem_ld_32x8(G.tO + lane_off + cb * 8, o);
 #pragma unroll
-                    for (int i = 0; i < 32; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) * alpha);
-                    tmem_st_32x32(G.tO + lane_off + cb * 32, v);
+                    for (int i = 0; i < 8; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+                    tmem_st_32x8(G.tO + lane_off + cb * 8, o);
                 }
+                tmem_wait_st();
             }
         }
-        // pass 2: P = exp2(s c - m c), row sum, bf16 row into the swizzled P tile
-        const float mc = m_new * c;
-        float l_tile = 0.f;
-#pragma unroll 1
-        for (int cb = 0; cb < 4; ++cb) {
-            uint32_t v[32];
-            tmem_ld_32x32(G.tS + lane_off + cb * 32, v);
+        // P = exp2(s c - m c), row sum, bf16 row into the swizzled P tile; of the diagonal tile only the 32-column blocks that some row of this warp attends
+        const uint64_t c2 = pair_f32(c, c), mc2 = pair_f32(-m_run * c, -m_run * c);
+        auto weights = [&](auto on_diagonal) {
+            constexpr bool kDiag = decltype(on_diagonal)::value;
 #pragma unroll
-            for (int g = 0; g < 4; ++g) {
-                uint32_t o[4];
+            for (int cb = 0; cb < 4; ++cb) {
+                if (!kDiag || cb <= warp_in_group) {
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const int c0 = cb * 32 + g * 8 + 2 * i;
-                    float p0 = exp2f(fmaf(__uint_as_float(v[g * 8 + 2 * i]), c, -mc));
-                    float p1 = exp2f(fmaf(__uint_as_float(v[g * 8 + 2 * i + 1]), c, -mc));
-                    if (diag) { if (c0 > r) p0 = 0.f; if (c0 + 1 > r) p1 = 0.f; }
-                    l_tile += p0 + p1;
-                    o[i] = pack_bf16x2(p0, p1);
+                    for (int g = 0; g < 4; ++g) {
+                        uint32_t o[4];
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            const int c0 = cb * 32 + g * 8 + 2 * i;
+                            float p0, p1;
+                            split_f32(fma_f32x2(pair_f32(__uint_as_float(v[c0]), __uint_as_float(v[c0 + 1])), c2, mc2), p0, p1);
+                            p0 = ex2(p0);
+                            p1 = ex2(p1);
+                            if (kDiag) { if (c0 > r) p0 = 0.f; if (c0 + 1 > r) p1 = 0.f; }
+                            l_run[i & 1] = add_f32x2(l_run[i & 1], pair_f32(p0, p1));
+                            o[i] = pack_bf16x2(p0, p1);
+                        }
+                        *reinterpret_cast<uint4*>(tile_chunk(G.pP, r, cb * 4 + g)) = make_uint4(o[0], o[1], o[2], o[3]);
+                    }
+                } else {
+#pragma unroll
+                    for (int g = 0; g < 4; ++g) *reinterpret_cast<uint4*>(tile_chunk(G.pP, r, cb * 4 + g)) = make_uint4(0u, 0u, 0u, 0u);
                 }
-                *reinterpret_cast<uint4*>(tile_chunk(G.pP, r, cb * 4 + g)) = make_uint4(o[0], o[1], o[2], o[3]);
             }
-        }
-        l_run = l_run * alpha + l_tile;
-        m_run = m_new;
+        };
+        if (diag) weights(std::true_type());
+        else weights(std::false_type());
         tc_fence_before_sync();
         fence_proxy_async_smem();
         __syncwarp();
         if (lane == 0) mbar_arrive(G.p_full);
     }
+    float l0, l1, l2, l3;
+    split_f32(l_run[0], l0, l1);
+    split_f32(l_run[1], l2, l3);
+    const float l_sum = (l0 + l1) + (l2 + l3);
     // epilogue: O / l -> bf16 -> the P tile as staging -> TMA store; log-sum-exp for the backward
     if (ok) ok = mbar_wait(G.o_full, (n_kv - 1) & 1, abort_flag, p.status, ST_TIMEOUT_ACCUM, 22);
     if (ok) {
         tc_fence_after_sync();
-        const float inv_l = 1.0f / l_run;
+        const float inv_l = 1.0f / l_sum;
 #pragma unroll 1
         for (int cb = 0; cb < 4; ++cb) {
             uint32_t v[32];
@@ -164,7 +200,7 @@ __device__ __forceinline__ void fwd_softmax_group(const FwdGroup& G, const AttnP
                 *reinterpret_cast<uint4*>(tile_chunk(G.pP, r, cb * 4 + g)) = make_uint4(o[0], o[1], o[2], o[3]);
             }
         }
-        if (p.lse) p.lse[((long long)b * p.Hq + h) * p.S + G.qt * kT + r] = m_run * p.scale + logf(l_run);
+        if (p.lse) p.lse[((long long)b * p.Hq + h) * p.S + G.qt * kT + r] = m_run * p.scale + logf(l_sum);
         fence_proxy_async_smem();
         asm volatile("bar.sync %0, 128;" ::"r"(bar_id) : "memory");
         if (r == 0) {
@@ -183,33 +219,34 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     const uint32_t raw = smem_u32(smem_raw);
     const uint32_t base = (raw + 1023u) & ~1023u;
     uint8_t* smem = smem_raw + (base - raw);
-    const uint32_t sQ0 = base, sK0 = base + 2 * kTile, sV = base + 4 * kTile, sP0 = base + 5 * kTile;
+    const uint32_t sQ0 = base, sKV = base + 2 * kTile, sP0 = base + 5 * kTile;
     const uint32_t bar = base + 7 * kTile;
-    const uint32_t q_full = bar, k_full0 = bar + 8, k_empty0 = bar + 24, v_full = bar + 40, v_empty = bar + 48;
+    const uint32_t q_full = bar;
+    auto full = [&](int i) { return bar + 8u + 8u * i; };
+    auto empty = [&](int i) { return bar + 32u + 8u * i; };
     auto s_full = [&](int g) { return bar + 56u + 8u * g; };
     auto p_full = [&](int g) { return bar + 72u + 8u * g; };
     auto o_full = [&](int g) { return bar + 88u + 8u * g; };
-    volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem + 7 * kTile + 112);
+    auto s_free = [&](int g) { return bar + 104u + 8u * g; };
+    volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem + 7 * kTile + 120);
     volatile uint32_t* abort_flag = tmem_slot + 1;
 
     const int warp = __shfl_sync(0xFFFFFFFFu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;   // uniform to the compiler too
     const int n_qt = p.S / kT;
     const int n_pairs = (n_qt + 1) / 2;
-    const int pi = n_pairs - 1 - (int)blockIdx.x;   // heavy pairs first
+    const int pi = n_pairs - 1 - (int)blockIdx.y;   // heavy pairs first, over all heads
     const int qtA = 2 * pi, qtB = 2 * pi + 1;
     const bool hasB = qtB < n_qt;
-    const int h = blockIdx.y, b = blockIdx.z;
+    const int h = blockIdx.x % p.Hq, b = blockIdx.x / p.Hq;
     const int hk = h / (p.Hq / p.Hkv);
     const int n_kvA = qtA + 1;
     const int n_kv = hasB ? qtB + 1 : n_kvA;
     const int row0 = b * p.S;
 
     if (threadIdx.x == 0) {
-        mbar_init(q_full, 1); mbar_init(v_full, 1); mbar_init(v_empty, 1);
-        for (int i = 0; i < 2; ++i) {
-            mbar_init(k_full0 + 8 * i, 1); mbar_init(k_empty0 + 8 * i, 1);
-            mbar_init(s_full(i), 1); mbar_init(p_full(i), 4); mbar_init(o_full(i), 1);
-        }
+        mbar_init(q_full, 1);
+        for (int i = 0; i < 3; ++i) { mbar_init(full(i), 1); mbar_init(empty(i), 1); }
+        for (int i = 0; i < 2; ++i) { mbar_init(s_full(i), 1); mbar_init(s_free(i), 4); mbar_init(p_full(i), 4); mbar_init(o_full(i), 1); }
         *abort_flag = 0;
         mbar_fence_init();
     }
@@ -221,74 +258,68 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     auto tS = [&](int g) { return tmem + 128u * g; };
     auto tO = [&](int g) { return tmem + 256u + 128u * g; };
 
-    if (warp == 8) {
+    // the ring's items: K_0, then K_{j + 1} and V_j in turns (the last V_j without a K_{j + 1})
+    const int last = 2 * n_kv;
+    auto k_item = [](int j) { return j == 0 ? 0 : 2 * j - 1; };
+    auto v_item = [](int j) { return 2 * j + 2; };
+    if (warp == 9) {
+        if (elect_one()) { tma_prefetch_desc(&tmQ); tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmV); }
+        if (elect_one()) { mbar_arrive_expect_tx(q_full, hasB ? 2 * kTile : kTile); }
+        if (elect_one()) { load_tile(sQ0, &tmQ, q_full, h * kD, row0 + qtA * kT); }
+        bool ok = true;
+        for (int i = 0, s = 0; i <= last && ok; ++i, s = s == 2 ? 0 : s + 1) {
+            if (i == 1 && hasB && elect_one()) load_tile(sQ0 + kTile, &tmQ, q_full, h * kD, row0 + qtB * kT);
+            if (i == last - 1) continue;
+            if (i >= 3) ok = mbar_wait_warp(empty(s), (i / 3 - 1) & 1, abort_flag, p.status, ST_TIMEOUT_EMPTY, 14);
+            if (!ok) break;
+            const bool is_k = i == 0 || (i & 1);
+            const int row = row0 + (i == 0 ? 0 : is_k ? (i + 1) / 2 : i / 2 - 1) * kT;
+            if (elect_one()) { mbar_arrive_expect_tx(full(s), kTile); }
+            if (elect_one()) { load_tile(sKV + s * kTile, is_k ? &tmK : &tmV, full(s), hk * kD, row); }
+        }
+    } else if (warp == 8) {
         // the whole warp walks the tiles and one elected lane issues (narrow_gemm.cu: operands stay in uniform registers):
         // 4 x 1024 tokens, 32 heads 87 -> 82 us; backward of 8 x 512: dK and dV 106 -> 101, dQ 71 -> 68
-        {
-            if (elect_one()) { tma_prefetch_desc(&tmQ); tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmV); }
-            if (elect_one()) { mbar_arrive_expect_tx(q_full, hasB ? 2 * kTile : kTile); }
-            if (elect_one()) { load_tile(sQ0, &tmQ, q_full, h * kD, row0 + qtA * kT); }
-            if (hasB && elect_one()) load_tile(sQ0 + kTile, &tmQ, q_full, h * kD, row0 + qtB * kT);
-            bool ok = true;
-            for (int j = 0; j < 2 && j < n_kv; ++j) {
-                if (elect_one()) { mbar_arrive_expect_tx(k_full0 + 8 * j, kTile); }
-                if (elect_one()) { load_tile(sK0 + j * kTile, &tmK, k_full0 + 8 * j, hk * kD, row0 + j * kT); }
-            }
-            if (elect_one()) { mbar_arrive_expect_tx(v_full, kTile); }
-            if (elect_one()) { load_tile(sV, &tmV, v_full, hk * kD, row0); }
-            ok = mbar_wait_warp(q_full, 0, abort_flag, p.status, ST_TIMEOUT_FULL, 10);
-            if (ok) ok = mbar_wait_warp(k_full0, 0, abort_flag, p.status, ST_TIMEOUT_FULL, 11);
-            if (ok) {
-                tc_fence_after_sync();
-                if (elect_one()) { mma_128(tS(0), sQ0, false, sK0, false, false); } // S_A(0) = Q_A K_0^T
-                if (elect_one()) { umma_commit(s_full(0)); }
-                if (hasB && elect_one()) { mma_128(tS(1), sQ0 + kTile, false, sK0, false, false); umma_commit(s_full(1)); }
-            }
-            for (int j = 0; j < n_kv && ok; ++j) {
-                const int s = j & 1, s1 = (j + 1) & 1;
-                ok = mbar_wait_warp(v_full, j & 1, abort_flag, p.status, ST_TIMEOUT_FULL, 15);
-                if (!ok) break;
+        auto ready = [&](int item) { return mbar_wait_warp(full(item % 3), (item / 3) & 1, abort_flag, p.status, ST_TIMEOUT_FULL, 11); };
+        auto done = [&](int item) { if (item + 3 <= last && elect_one()) umma_commit(empty(item % 3)); };
+        bool ok = mbar_wait_warp(q_full, 0, abort_flag, p.status, ST_TIMEOUT_FULL, 10);
+        for (int j = -1; j < n_kv && ok; ++j) {
+            if (j + 1 < n_kv) {                     // S_g(j + 1) = Q_g K_{j + 1}^T once S_g(j) is in registers
+                const int item = k_item(j + 1);
+                ok = ready(item);
 #pragma unroll
-                for (int g = 0; g < 2; ++g) {
-                    const int n_g = g == 0 ? n_kvA : n_kv;
-                    if ((g == 1 && !hasB) || j >= n_g) continue;
-                    // P_g(j) is ready (and S_g(j) has been read): O_g += P_g V_j, then S_g(j + 1) while the other group's softmax runs
-                    ok = mbar_wait_warp(p_full(g), j & 1, abort_flag, p.status, ST_TIMEOUT_FULL, 12);
+                for (int g = 0; g < 2 && ok; ++g) {
+                    if ((g == 1 && !hasB) || j + 1 >= (g == 0 ? n_kvA : n_kv)) continue;
+                    if (j >= 0) ok = mbar_wait_warp(s_free(g), j & 1, abort_flag, p.status, ST_TIMEOUT_ACCUM, 12);
                     if (!ok) break;
                     tc_fence_after_sync();
-                    if (elect_one()) { mma_128(tO(g), sP0 + g * kTile, false, sV, true, j > 0); } // V: rows = kv = reduction index
-                    if (elect_one()) { umma_commit(o_full(g)); }
-                    if (j + 1 < n_g) {
-                        ok = mbar_wait_warp(k_full0 + 8 * s1, ((j + 1) >> 1) & 1, abort_flag, p.status, ST_TIMEOUT_FULL, 13);
-                        if (!ok) break;
-                        tc_fence_after_sync();
-                        if (elect_one()) { mma_128(tS(g), sQ0 + g * kTile, false, sK0 + s1 * kTile, false, false); }
-                        if (elect_one()) { umma_commit(s_full(g)); }
-                    }
+                    if (elect_one()) { mma_128(tS(g), sQ0 + g * kTile, false, sKV + item % 3 * kTile, false, false); }
+                    if (elect_one()) { umma_commit(s_full(g)); }
                 }
                 if (!ok) break;
-                // every product that reads V_j and K_j has been issued: the two buffers are free once those have completed
-                if (elect_one()) { umma_commit(v_empty); }
-                if (elect_one()) { umma_commit(k_empty0 + 8 * s); }
-                if (j + 1 < n_kv) {
-                    ok = mbar_wait_warp(v_empty, j & 1, abort_flag, p.status, ST_TIMEOUT_EMPTY, 16);
+                done(item);
+            }
+            if (j >= 0) {                           // O_g += P_g V_j
+                const int item = v_item(j);
+                ok = ready(item);
+#pragma unroll
+                for (int g = 0; g < 2 && ok; ++g) {
+                    if ((g == 1 && !hasB) || j >= (g == 0 ? n_kvA : n_kv)) continue;
+                    ok = mbar_wait_warp(p_full(g), j & 1, abort_flag, p.status, ST_TIMEOUT_FULL, 13);
                     if (!ok) break;
-                    if (elect_one()) { mbar_arrive_expect_tx(v_full, kTile); }
-                    if (elect_one()) { load_tile(sV, &tmV, v_full, hk * kD, row0 + (j + 1) * kT); }
+                    tc_fence_after_sync();
+                    if (elect_one()) { mma_128(tO(g), sP0 + g * kTile, false, sKV + item % 3 * kTile, true, j > 0); } // V: rows = kv = reduction index
+                    if (elect_one()) { umma_commit(o_full(g)); }
                 }
-                if (j + 2 < n_kv) {
-                    ok = mbar_wait_warp(k_empty0 + 8 * s, (j >> 1) & 1, abort_flag, p.status, ST_TIMEOUT_EMPTY, 14);
-                    if (!ok) break;
-                    if (elect_one()) { mbar_arrive_expect_tx(k_full0 + 8 * s, kTile); }
-                    if (elect_one()) { load_tile(sK0 + s * kTile, &tmK, k_full0 + 8 * s, hk * kD, row0 + (j + 2) * kT); }
-                }
+                if (!ok) break;
+                done(item);
             }
         }
     } else {
         const int g = warp >> 2;
         if (g == 0 || hasB) {
             FwdGroup G;
-            G.tS = tS(g); G.tO = tO(g); G.s_full = s_full(g); G.p_full = p_full(g); G.o_full = o_full(g);
+            G.tS = tS(g); G.tO = tO(g); G.s_full = s_full(g); G.s_free = s_free(g); G.p_full = p_full(g); G.o_full = o_full(g);
             G.pP = smem + 5 * kTile + g * kTile; G.sP = sP0 + g * kTile; G.qt = g == 0 ? qtA : qtB;
             fwd_softmax_group(G, p, &tmO, h, b, row0, warp & 3, lane, 1 + g, abort_flag);
         }
@@ -650,7 +681,7 @@ int launch_attn_fwd(const AttnArgs& a, cudaStream_t stream) {
     p.B = a.B; p.S = a.S; p.Hq = a.Hq; p.Hkv = a.Hkv; p.scale = a.scale; p.lse = a.lse; p.status = device_status_ptr();
     static bool once = false;
     if (!once) { if ((rc = set_smem(attn_fwd_kernel, kFwdSmem))) return rc; once = true; }
-    attn_fwd_kernel<<<dim3((a.S / kT + 1) / 2, a.Hq, a.B), kFwdThreads, kFwdSmem, stream>>>(tmQ, tmK, tmV, tmO, p);
+    attn_fwd_kernel<<<dim3(a.Hq * a.B, (a.S / kT + 1) / 2), kFwdThreads, kFwdSmem, stream>>>(tmQ, tmK, tmV, tmO, p);
     PLZ_LAUNCH_CHECK();
     return PLZ_OK;
 }

@@ -1,0 +1,51 @@
+"""Attention where its sums are put together: the merge of a decode step's splits over head sizes, split counts and empty splits, and the
+prompt kernel's running maximum when scores grow along the sequence.  Checked against softmax in 64 bits (32 bits for the prompt)."""
+import pytest
+import torch
+
+from helpers import assert_close, check_status
+
+pytestmark = pytest.mark.gpu
+
+
+# positions: fewer keys than a split takes, splits without keys (few keys in a long cache), all of them at work
+@pytest.mark.parametrize("B,H,G,dk,dv,cap,pos", [(1, 2, 1, 16, 8, 4096, 0), (1, 4, 2, 64, 40, 4096, 70), (2, 3, 3, 128, 120, 900, 899), (1, 1, 1, 128, 128, 20000, 17777),
+                                                 (1, 4, 1, 64, 128, 300, 299), (1, 2, 2, 128, 136, 2048, 1500)])
+@pytest.mark.parametrize("dtype,sink", [(torch.float32, True), (torch.bfloat16, False)])
+def test_splits_of_a_decode_step(B, H, G, dk, dv, cap, pos, dtype, sink):
+    import seq_ops as S
+    g = torch.Generator().manual_seed(cap + pos)
+    q = torch.randn(B, H * dk, generator=g).to(dtype).cuda()
+    kc = torch.randn(B, cap, G * dk, generator=g).to(dtype).cuda()
+    vc = torch.randn(B, cap, G * dv, generator=g).to(dtype).cuda()
+    got = S.attention_bias(q, kc, vc, None, torch.tensor([pos], dtype=torch.int32, device="cuda"), -1, B, 1, H, G, dk, dv, dk ** -0.5, sink)
+    check_status()
+    qf = q.double().view(B, G, H // G, dk)
+    kf, vf = (t[:, :pos + 1].double().view(B, pos + 1, G, -1).transpose(1, 2) for t in (kc, vc))
+    s = qf @ kf.transpose(-1, -2) * dk ** -0.5
+    if sink: s = torch.cat([s, torch.zeros_like(s[..., :1])], -1)
+    want = (torch.softmax(s, -1)[..., :pos + 1] @ vf).reshape(B, H * dv)
+    if dtype == torch.float32:
+        # scores of size < 8 with a relative error of about dk 2^-24: weights within 1e-4, values below 6
+        assert (got.double() - want).abs().max() < 6e-4
+    else:
+        assert_close(got, want.float(), "decode", rel=1e-2, cos=0.9999)
+
+
+@pytest.mark.parametrize("S", [128, 384, 1024])
+@pytest.mark.parametrize("growth", [0.0, 0.5, 3.0, -3.0])       # by tile of 128 keys, in units of the score's spread
+def test_scores_that_grow_along_the_sequence(S, growth):
+    import plz_ops as ops
+    B, Hq, Hkv, D = 1, 2, 1, 128
+    g = torch.Generator().manual_seed(S)
+    q, do = (torch.randn(B * S, Hq * D, generator=g) for _ in range(2))
+    k, v = (torch.randn(B * S, Hkv * D, generator=g) for _ in range(2))
+    q[:, ::D] = 4.0
+    k[:, 0] = growth * (torch.arange(S) // 128 + torch.arange(S) / 512) * D ** 0.5 / 4
+    q, k, v, do = (t.to(torch.bfloat16).cuda() for t in (q, k, v, do))
+    o, lse = ops.attention_forward(q, k, v, B, S, Hq, Hkv)
+    check_status()
+    s = (q.double().view(S, Hq, D).transpose(0, 1) @ k.double().t()) * D ** -0.5
+    s = s.masked_fill(~torch.ones(S, S, dtype=torch.bool, device="cuda").tril(), float("-inf"))
+    assert_close(o, (torch.softmax(s, -1) @ v.double()).transpose(0, 1).reshape(S, Hq * D).float(), "o")
+    assert_close(lse, torch.logsumexp(s, -1).float().view(B, Hq, S), "log-sum-exp", rel=1e-3)
