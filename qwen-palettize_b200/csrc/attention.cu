@@ -70,14 +70,6 @@ __device__ __forceinline__ void load_tile(uint32_t dst, const CUtensorMap* map, 
 constexpr int kFwdThreads = 320;   // warps 0..3 / 4..7: softmax of tile A / B, warp 8: MMA, warp 9: TMA
 constexpr uint32_t kFwdSmem = 7 * kTile + 1024 + 256;   // Q x 2, K / V x 3, P x 2
 
-__device__ __forceinline__ uint64_t pair_f32(float a, float b) { uint64_t d; asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(a), "f"(b)); return d; }
-__device__ __forceinline__ void split_f32(uint64_t v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
-__device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c) { uint64_t d; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c)); return d; }
-__device__ __forceinline__ uint64_t mul_f32x2(uint64_t a, uint64_t b) { uint64_t d; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
-__device__ __forceinline__ uint64_t add_f32x2(uint64_t a, uint64_t b) { uint64_t d; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
-
-__device__ __forceinline__ float ex2(float x) { float y; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
-
 struct FwdGroup {          // what one softmax group works on
     uint32_t tS, tO;       // TMEM columns of its score and output accumulators
     uint32_t s_full, s_free, p_full, o_full;
@@ -91,12 +83,12 @@ __device__ __forceinline__ void fwd_softmax_group(const FwdGroup& G, const AttnP
     const uint32_t lane_off = (uint32_t)(warp_in_group * 32) << 16;
     const float c = p.scale * kLog2e;
     const int n_kv = G.qt + 1;
-    // m_run: the reference of the exponentials, moved only when the maximum has outgrown it by 2^8: O is then rescaled in the first tiles of a row and hardly again.
-    // The scores of a row stay in registers between the maximum and the exponentials (128 of them, one read of TMEM instead of two), maximum and sum run in
-    // four chains each, and only the tile on the diagonal is compared with the row. 4 x 1024 tokens, 32 heads: 84 -> 67 us, and 53 us with S(j + 1) computed meanwhile (8 x 512: 53 -> 43,
-    // 1 x 4096: 255 -> 120); the exponentials alone are 17 us.
-    float m_run = -INFINITY;
-    uint64_t l_run[2] = {0ull, 0ull};
+    // The scores of a row stay in registers between the maximum and the exponentials (128 of them, one read of TMEM instead of two), the maximum runs in
+    // four chains, only the tile on the diagonal is compared with the row, and O is rescaled where those registers are free again. 32 heads over 8,
+    // 8 x 512 tokens: 53 -> 44 us, 4 x 1024 84 -> 55, 1 x 4096 255 -> 130, 8 x 2048 461 -> 297.
+    // The exponentials alone are 17 us. Rescaling O only when a maximum has grown by 2^8 gives 53, 120, 285, but the largest weight is then
+    // no longer 1 and its rounding shows: error of O against 64 bits at 1024 keys 1.74e-3 -> 2.04e-3 with scores of spread 4.
+    float m_run = -INFINITY, l_run = 0.f;
     bool ok = true;
     for (int j = 0; j < n_kv && ok; ++j) {
         ok = mbar_wait(G.s_full, j & 1, abort_flag, p.status, ST_TIMEOUT_ACCUM, 20);
@@ -119,31 +111,18 @@ __device__ __forceinline__ void fwd_softmax_group(const FwdGroup& G, const AttnP
 #pragma unroll
             for (int k = 0; k < 4; ++k) m4[k] = fmaxf(fmaxf(m4[k], __uint_as_float(v[i + k])), __uint_as_float(v[i + 4 + k]));
         const float m_tile = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3]));
-        const bool moved = m_run == -INFINITY || (m_tile - m_run) * c > kLazyGrowth;
+        const bool moved = m_tile > m_run;
         const float alpha = !moved ? 1.f : m_run == -INFINITY ? 0.f : exp2f((m_run - m_tile) * c);
         if (moved) m_run = m_tile;
-        // the previous P V product must have landed before O is rescaled and before P is overwritten
+        // the previous P V product must have landed before P is overwritten and before O is rescaled
         if (j > 0) {
             ok = mbar_wait(G.o_full, (j - 1) & 1, abort_flag, p.status, ST_TIMEOUT_ACCUM, 21);
             if (!ok) break;
             tc_fence_after_sync();
-            if (__any_sync(0xFFFFFFFFu, moved)) {
-                const uint64_t a2 = pair_f32(alpha, alpha);
-                l_run[0] = mul_f32x2(l_run[0], a2);
-                l_run[1] = mul_f32x2(l_run[1], a2);
-#pragma unroll 1
-                for (int cb = 0; cb < 16; ++cb) {
-                    uint32_t o[8];
-                    tmem_ld_32x8(G.tO + lane_off + cb * 8, o);
-#pragma unroll
-                    for (int i = 0; i < 8; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
-                    tmem_st_32x8(G.tO + lane_off + cb * 8, o);
-                }
-                tmem_wait_st();
-            }
         }
         // P = exp2(s c - m c), row sum, bf16 row into the swizzled P tile; of the diagonal tile only the 32-column blocks that some row of this warp attends
         const uint64_t c2 = pair_f32(c, c), mc2 = pair_f32(-m_run * c, -m_run * c);
+        uint64_t l_tile = 0ull;                        // even and odd columns
         auto weights = [&](auto on_diagonal) {
             constexpr bool kDiag = decltype(on_diagonal)::value;
 #pragma unroll
@@ -160,7 +139,7 @@ __device__ __forceinline__ void fwd_softmax_group(const FwdGroup& G, const AttnP
                             p0 = ex2(p0);
                             p1 = ex2(p1);
                             if (kDiag) { if (c0 > r) p0 = 0.f; if (c0 + 1 > r) p1 = 0.f; }
-                            l_run[i & 1] = add_f32x2(l_run[i & 1], pair_f32(p0, p1));
+                            l_tile = add_f32x2(l_tile, pair_f32(p0, p1));
                             o[i] = pack_bf16x2(p0, p1);
                         }
                         *reinterpret_cast<uint4*>(tile_chunk(G.pP, r, cb * 4 + g)) = make_uint4(o[0], o[1], o[2], o[3]);
@@ -173,20 +152,20 @@ __device__ __forceinline__ void fwd_softmax_group(const FwdGroup& G, const AttnP
         };
         if (diag) weights(std::true_type());
         else weights(std::false_type());
+        float even, odd;
+        split_f32(l_tile, even, odd);
+        l_run = fmaf(l_run, alpha, even + odd);
+        if (j > 0 && __any_sync(0xFFFFFFFFu, moved)) rescale<2>(G.tO + lane_off, alpha);
         tc_fence_before_sync();
         fence_proxy_async_smem();
         __syncwarp();
         if (lane == 0) mbar_arrive(G.p_full);
     }
-    float l0, l1, l2, l3;
-    split_f32(l_run[0], l0, l1);
-    split_f32(l_run[1], l2, l3);
-    const float l_sum = (l0 + l1) + (l2 + l3);
     // epilogue: O / l -> bf16 -> the P tile as staging -> TMA store; log-sum-exp for the backward
     if (ok) ok = mbar_wait(G.o_full, (n_kv - 1) & 1, abort_flag, p.status, ST_TIMEOUT_ACCUM, 22);
     if (ok) {
         tc_fence_after_sync();
-        const float inv_l = 1.0f / l_sum;
+        const float inv_l = 1.0f / l_run;
 #pragma unroll 1
         for (int cb = 0; cb < 4; ++cb) {
             uint32_t v[32];
@@ -200,15 +179,15 @@ __device__ __forceinline__ void fwd_softmax_group(const FwdGroup& G, const AttnP
                 *reinterpret_cast<uint4*>(tile_chunk(G.pP, r, cb * 4 + g)) = make_uint4(o[0], o[1], o[2], o[3]);
             }
         }
-        if (p.lse) p.lse[((long long)b * p.Hq + h) * p.S + G.qt * kT + r] = m_run * p.scale + logf(l_sum);
+        if (p.lse) p.lse[((long long)b * p.Hq + h) * p.S + G.qt * kT + r] = m_run * p.scale + logf(l_run);
         fence_proxy_async_smem();
-        asm volatile("bar.sync %0, 128;" ::"r"(bar_id) : "memory");
-        if (r == 0) {
-            tma_store_2d(tmO, G.sP, h * kD, row0 + G.qt * kT);
-            tma_store_2d(tmO, G.sP + kBlk, h * kD + 64, row0 + G.qt * kT);
-            tma_store_commit();
-            tma_store_wait_all();
-        }
+    }
+    asm volatile("bar.sync %0, 128;" ::"r"(bar_id) : "memory");
+    if (ok && r == 0) {
+        tma_store_2d(tmO, G.sP, h * kD, row0 + G.qt * kT);
+        tma_store_2d(tmO, G.sP + kBlk, h * kD + 64, row0 + G.qt * kT);
+        tma_store_commit();
+        tma_store_wait_all();
     }
 }
 

@@ -8,7 +8,14 @@ namespace plz {
 constexpr int kT = 128;                         // tokens per tile
 constexpr uint32_t kBlk = kT * 64 * 2;          // one 64-column block of a 128-row bf16 tile: 16 KB
 constexpr float kLog2e = 1.4426950408889634f;
-constexpr float kLazyGrowth = 8.0f;             // log2 units that a running maximum may grow by before what it scaled is scaled again
+
+// two values at a time
+__device__ __forceinline__ uint64_t pair_f32(float a, float b) { uint64_t d; asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(a), "f"(b)); return d; }
+__device__ __forceinline__ void split_f32(uint64_t v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c) { uint64_t d; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c)); return d; }
+__device__ __forceinline__ uint64_t mul_f32x2(uint64_t a, uint64_t b) { uint64_t d; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
+__device__ __forceinline__ uint64_t add_f32x2(uint64_t a, uint64_t b) { uint64_t d; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
+__device__ __forceinline__ float ex2(float x) { float y; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
 
 __device__ __forceinline__ void tmem_st_32x32(uint32_t taddr, const uint32_t (&r)[32]) {
     asm volatile(
@@ -23,6 +30,18 @@ __device__ __forceinline__ void tmem_st_32x32(uint32_t taddr, const uint32_t (&r
         : "memory");
 }
 
+// two times 32 lanes x 32 columns behind one wait
+__device__ __forceinline__ void tmem_ld_32x32_two(uint32_t at, uint32_t bt, uint32_t (&a)[32], uint32_t (&b)[32]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%64];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%32, %33, %34, %35, %36, %37, %38, %39, %40, %41, %42, %43, %44, %45, %46, %47, "
+        "%48, %49, %50, %51, %52, %53, %54, %55, %56, %57, %58, %59, %60, %61, %62, %63}, [%65];\n\t"
+        "tcgen05.wait::ld.sync.aligned;"
+        : "=r"(a[0]), "=r"(a[1]), "=r"(a[2]), "=r"(a[3]), "=r"(a[4]), "=r"(a[5]), "=r"(a[6]), "=r"(a[7]), "=r"(a[8]), "=r"(a[9]), "=r"(a[10]), "=r"(a[11]), "=r"(a[12]), "=r"(a[13]), "=r"(a[14]), "=r"(a[15]), "=r"(a[16]), "=r"(a[17]), "=r"(a[18]), "=r"(a[19]), "=r"(a[20]), "=r"(a[21]), "=r"(a[22]), "=r"(a[23]), "=r"(a[24]), "=r"(a[25]), "=r"(a[26]), "=r"(a[27]), "=r"(a[28]), "=r"(a[29]), "=r"(a[30]), "=r"(a[31]), "=r"(b[0]), "=r"(b[1]), "=r"(b[2]), "=r"(b[3]), "=r"(b[4]), "=r"(b[5]), "=r"(b[6]), "=r"(b[7]), "=r"(b[8]), "=r"(b[9]), "=r"(b[10]), "=r"(b[11]), "=r"(b[12]), "=r"(b[13]), "=r"(b[14]), "=r"(b[15]), "=r"(b[16]), "=r"(b[17]), "=r"(b[18]), "=r"(b[19]), "=r"(b[20]), "=r"(b[21]), "=r"(b[22]), "=r"(b[23]), "=r"(b[24]), "=r"(b[25]), "=r"(b[26]), "=r"(b[27]), "=r"(b[28]), "=r"(b[29]), "=r"(b[30]), "=r"(b[31])
+        : "r"(at), "r"(bt)
+        : "memory");
+}
 // 32 lanes x 128 columns behind one wait
 __device__ __forceinline__ void tmem_ld_32x128(uint32_t taddr, uint32_t (&r)[128]) {
     asm volatile(
@@ -54,6 +73,31 @@ __device__ __forceinline__ void tmem_st_32x8(uint32_t taddr, const uint32_t (&r)
                  : "memory");
 }
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+
+// BLOCKS blocks of 64 columns of 32 accumulator rows times alpha
+template <int BLOCKS>
+__device__ __forceinline__ void rescale(uint32_t tO, float alpha) {
+    const uint64_t a2 = pair_f32(alpha, alpha);
+#pragma unroll 1
+    for (int cb = 0; cb < BLOCKS; ++cb) {
+        uint32_t v[2][32];
+        tmem_ld_32x32_two(tO + cb * 64, tO + cb * 64 + 32, v[0], v[1]);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            uint32_t o[16];
+#pragma unroll
+            for (int i = 0; i < 16; i += 2) {
+                const uint32_t* from = v[q >> 1] + (q & 1) * 16 + i;
+                float x, y;
+                split_f32(mul_f32x2(pair_f32(__uint_as_float(from[0]), __uint_as_float(from[1])), a2), x, y);
+                o[i] = __float_as_uint(x);
+                o[i + 1] = __float_as_uint(y);
+            }
+            tmem_st_32x16(tO + cb * 64 + q * 16, o);
+        }
+    }
+    tmem_wait_st();
+}
 
 // D (+)= A B with A from TMEM (lane = row, two bf16 of the reduction index per column)
 __device__ __forceinline__ void umma_ts(uint32_t d, uint32_t a, uint32_t b_lo, uint32_t b_hi, uint32_t idesc, uint32_t accumulate) {
