@@ -13,8 +13,7 @@
 //                  the softmax of one tile runs under the MMAs of the other; also writes the row log-sum-exp.
 //   backward dQ    per q tile: S, dP = dO V^T -> dS = P (dP - D) / sqrt(d) -> dQ += dS K
 //   backward dKdV  per kv tile and kv head, over the q heads of the group and the q tiles at or after it:
-//                  S, dP -> P, dS to shared memory -> dV += P^T dO, dK += dS^T Q  (P^T / dS^T are the same bytes read
-//                  through an MN-major operand descriptor)
+//                  S^T = K Q^T, dP^T = V dO^T -> P^T, dS^T in TMEM -> dV += P^T dO, dK += dS^T Q
 // D[row] = sum_d dO O is a small pre-pass. Every barrier wait is bounded (status word, as in the GEMM kernels).
 #include <type_traits>
 
@@ -33,8 +32,6 @@ struct AttnParams {
     const float* dsum;    // [B, Hq, S] sum_d dO * O (backward)
     StatusWord* status;
 };
-
-__device__ __forceinline__ void bar_sync_128() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
 
 // eight MMAs of one 128 x 128 x 128 product. A / B tiles are 128-row bf16 tiles of two 64-column blocks.
 //   K-major operand (rows = M or N index, reduction along the 128-byte row):  step ks -> block ks / 4, 32 bytes * (ks % 4)
@@ -351,284 +348,243 @@ attn_dsum_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __res
     }
 }
 
-// The element-wise middle of both backward kernels: thread r (row = query r of the q tile) turns the score row in tS and
-// the dP row in tdP into P (optional) and dS = P (dP - D) scale, written as bf16 rows of swizzled K-major tiles.
-__device__ __forceinline__ void bwd_rows(uint32_t tS, uint32_t tdP, uint32_t lane_off, int r, bool diag, float c, float lse_l2, float dsum_r,
-                                         float scale, uint8_t* pP, uint8_t* pdS) {
-#pragma unroll 1
-    for (int cb = 0; cb < 4; ++cb) {
-        uint32_t vs[32], vd[32];
-        tmem_ld_32x32(tS + lane_off + cb * 32, vs);
-        tmem_ld_32x32(tdP + lane_off + cb * 32, vd);
+// ---------------------------------------------------------------------------------------------------------------------
+// backward: dK and dV (KV: one CTA per kv tile and kv head, walking the q heads of the group and the q tiles), or dQ (one CTA per
+// q tile and q head, walking the kv tiles)
+// ---------------------------------------------------------------------------------------------------------------------
+// Either way two tiles X1, X2 stay (K, V or Q, dO) and pairs Y1, Y2 walk by (Q, dO or K, V) in halves of 64 tokens, one half to each of two groups of four warps:
+//   S = X1 Y1^T, dP = X2 Y2^T        X's tokens are the accumulators' rows, so with KV both come out transposed
+//   P, dS = P (dP - D) scale         in registers, written over S and dP in TMEM as bf16
+//   dV += P Y2 (KV), dX1 += dS Y1    P and dS as operands in TMEM
+// P and dS never go through shared memory, which leaves room for a second pair Y; while one group works on its half, the tensor core runs the products of the
+// other's. Before, four warps and the tensor core took turns and every pair was loaded when the last one was done with. 32 heads over 8, all three
+// backward launches: 8 x 512 tokens 191 -> 126 us, 4 x 1024 298 -> 167, 1 x 4096 902 -> 444.
+constexpr int kBwdThreads = 320;   // warps 0..3 / 4..7: halves 0 / 1, warp 8: MMA, warp 9: TMA
+constexpr uint32_t kBwdSmem = 6 * kTile + 1024 + 256 + 8 * 2 * 128 * 4;   // X1, X2, (Y1, Y2) x 2, [warp][parity][lse, dsum of its 64 queries]
+
+// eight MMAs S_half = X Y_half^T: 128 rows, 64 tokens, 128 head columns
+__device__ __forceinline__ void mma_half(uint32_t d_tmem, uint32_t sX, uint32_t sY, int half) {
+    const uint32_t idesc = make_idesc(128, 64, 0, 0);
+    const uint64_t ad = make_sdesc(sX, 16u, 1024u), bd = make_sdesc(sY + (uint32_t)half * 8192u, 16u, 1024u);
 #pragma unroll
-        for (int g = 0; g < 4; ++g) {
-            uint32_t op[4], od[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const int c0 = cb * 32 + g * 8 + 2 * i;
-                float p0 = exp2f(__uint_as_float(vs[g * 8 + 2 * i]) * c - lse_l2);
-                float p1 = exp2f(__uint_as_float(vs[g * 8 + 2 * i + 1]) * c - lse_l2);
-                if (diag) { if (c0 > r) p0 = 0.f; if (c0 + 1 > r) p1 = 0.f; }
-                const float d0 = p0 * (__uint_as_float(vd[g * 8 + 2 * i]) - dsum_r) * scale;
-                const float d1 = p1 * (__uint_as_float(vd[g * 8 + 2 * i + 1]) - dsum_r) * scale;
-                op[i] = pack_bf16x2(p0, p1);
-                od[i] = pack_bf16x2(d0, d1);
-            }
-            if (pP) *reinterpret_cast<uint4*>(tile_chunk(pP, r, cb * 4 + g)) = make_uint4(op[0], op[1], op[2], op[3]);
-            *reinterpret_cast<uint4*>(tile_chunk(pdS, r, cb * 4 + g)) = make_uint4(od[0], od[1], od[2], od[3]);
-        }
+    for (int ks = 0; ks < 8; ++ks) {
+        const uint32_t off = (uint32_t)((ks >> 2) * (kBlk >> 4) + (ks & 3) * 2);
+        umma_bf16_words<1>(d_tmem, (uint32_t)ad + off, (uint32_t)(ad >> 32), (uint32_t)bd + off, (uint32_t)(bd >> 32), idesc, ks > 0 ? 1u : 0u);
     }
 }
+// four MMAs acc += A Y_half with A (128 rows, 64 tokens) in TMEM: 128 rows, 128 head columns
+__device__ __forceinline__ void mma_grad(uint32_t acc, uint32_t tA, uint32_t sY, int half, bool accumulate) {
+    const uint32_t idesc = make_idesc(128, 128, 0, 1);
+    const uint64_t bd = make_sdesc(sY + (uint32_t)half * 8192u, kBlk, 1024u);
+#pragma unroll
+    for (int ks = 0; ks < 4; ++ks)
+        umma_ts(acc, tA + ks * 8u, (uint32_t)bd + (uint32_t)(ks * 128), (uint32_t)(bd >> 32), idesc, (ks > 0 || accumulate) ? 1u : 0u);
+}
 
-// write a finished 128 x 128 fp32 accumulator (TMEM) as bf16 through a staging tile and two TMA boxes
-__device__ __forceinline__ void store_acc_tile(uint32_t tacc, uint32_t lane_off, int r, uint8_t* stage, uint32_t stage_u32,
-                                               const CUtensorMap* map, int col0, int row0) {
+// One half's rows, 32 columns at a time: thread r (row r) turns its scores and dP into bf16 P (KV) and dS over them. nl, nd: -lse (log2 units) and -dsum of the
+// row, or with KV of the 64 columns in shared memory. masked: of the tile on the diagonal.
+template <bool KV>
+__device__ __forceinline__ void bwd_rows(uint32_t tS, uint32_t tdP, int half, int r, bool diag, float c, float scale, float nl, float nd, const float* col_stats) {
+    const uint64_t c2 = pair_f32(c, c), scale2 = pair_f32(scale, scale);
+#pragma unroll
+    for (int cb = 0; cb < 2; ++cb) {
+        uint32_t vs[32], vd[32], op[16], od[16];
+        tmem_ld_32x32_two(tS + cb * 32, tdP + cb * 32, vs, vd);
+#pragma unroll
+        for (int i = 0; i < 32; i += 4) {
+            float4 l4 = make_float4(nl, nl, nl, nl), d4 = make_float4(nd, nd, nd, nd);
+            if (KV) {
+                l4 = *reinterpret_cast<const float4*>(col_stats + cb * 32 + i);
+                d4 = *reinterpret_cast<const float4*>(col_stats + 64 + cb * 32 + i);
+            }
+#pragma unroll
+            for (int e = 0; e < 4; e += 2) {
+                const uint64_t l2 = e == 0 ? pair_f32(l4.x, l4.y) : pair_f32(l4.z, l4.w), n2 = e == 0 ? pair_f32(d4.x, d4.y) : pair_f32(d4.z, d4.w);
+                float p0, p1, d0, d1;
+                split_f32(fma_f32x2(pair_f32(__uint_as_float(vs[i + e]), __uint_as_float(vs[i + e + 1])), c2, l2), p0, p1);
+                p0 = ex2(p0);
+                p1 = ex2(p1);
+                if (diag) {
+                    const int t = half * 64 + cb * 32 + i + e;      // a key comes no later than its query
+                    if (KV ? t < r : t > r) p0 = 0.f;
+                    if (KV ? t + 1 < r : t + 1 > r) p1 = 0.f;
+                }
+                split_f32(mul_f32x2(mul_f32x2(pair_f32(p0, p1), add_f32x2(pair_f32(__uint_as_float(vd[i + e]), __uint_as_float(vd[i + e + 1])), n2)), scale2), d0, d1);
+                op[(i + e) / 2] = pack_bf16x2(p0, p1);
+                od[(i + e) / 2] = pack_bf16x2(d0, d1);
+            }
+        }
+        if (KV) tmem_st_32x16(tS + cb * 16, op);
+        tmem_st_32x16(tdP + cb * 16, od);
+    }
+    tmem_wait_st();
+}
+
+// 64 columns of a finished fp32 accumulator as one swizzled bf16 block
+__device__ __forceinline__ void stage_block(uint32_t tacc, int r, uint8_t* block) {
 #pragma unroll 1
-    for (int cb = 0; cb < 4; ++cb) {
+    for (int cb = 0; cb < 2; ++cb) {
         uint32_t v[32];
-        tmem_ld_32x32(tacc + lane_off + cb * 32, v);
+        tmem_ld_32x32(tacc + cb * 32, v);
 #pragma unroll
         for (int g = 0; g < 4; ++g) {
             uint32_t o[4];
 #pragma unroll
             for (int i = 0; i < 4; ++i) o[i] = pack_bf16x2(__uint_as_float(v[g * 8 + 2 * i]), __uint_as_float(v[g * 8 + 2 * i + 1]));
-            *reinterpret_cast<uint4*>(tile_chunk(stage, r, cb * 4 + g)) = make_uint4(o[0], o[1], o[2], o[3]);
+            *reinterpret_cast<uint4*>(tile_chunk(block, r, cb * 4 + g)) = make_uint4(o[0], o[1], o[2], o[3]);
         }
     }
-    fence_proxy_async_smem();
-    bar_sync_128();
-    if (threadIdx.x == 0) {
-        tma_store_2d(map, stage_u32, col0, row0);
-        tma_store_2d(map, stage_u32 + kBlk, col0 + 64, row0);
-        tma_store_commit();
-        tma_store_wait_all();
-    }
-    bar_sync_128();
 }
 
-// ---------------------------------------------------------------------------------------------------------------------
-// backward, dQ: one CTA per (q tile, q head, batch)
-// ---------------------------------------------------------------------------------------------------------------------
-constexpr int kBwdThreads = 160;
-constexpr uint32_t kDqSmem = 7 * kTile + 1024 + 256;   // Q, dO, K x 2, V x 2, dS
-
+// the maps of X1, X2, Y1, Y2 and of the gradients of X1 and (KV) X2
+template <bool KV>
 __global__ void __launch_bounds__(kBwdThreads, 1)
-attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
-                   const __grid_constant__ CUtensorMap tmdO, const __grid_constant__ CUtensorMap tmdQ, const AttnParams p) {
+attn_bwd_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_constant__ CUtensorMap tmX2, const __grid_constant__ CUtensorMap tmY1,
+                const __grid_constant__ CUtensorMap tmY2, const __grid_constant__ CUtensorMap tmG1, const __grid_constant__ CUtensorMap tmG2, const AttnParams p) {
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
     const uint32_t base = (raw + 1023u) & ~1023u;
     uint8_t* smem = smem_raw + (base - raw);
-    const uint32_t sQ = base, sdO = base + kTile, sK0 = base + 2 * kTile, sV0 = base + 4 * kTile, sdS = base + 6 * kTile;
-    uint8_t* pdS = smem + 6 * kTile;
-    const uint32_t bar = base + 7 * kTile;
-    const uint32_t q_full = bar, kv_full0 = bar + 8, kv_empty0 = bar + 24, sd_full = bar + 40, ds_full = bar + 48, dq_full = bar + 56;
-    volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem + 7 * kTile + 64);
+    const uint32_t sX1 = base, sX2 = base + kTile, bar = base + 6 * kTile;
+    auto sY1 = [&](int s) { return base + (2 + 2 * s) * kTile; };
+    auto sY2 = [&](int s) { return base + (3 + 2 * s) * kTile; };
+    const uint32_t x_full = bar, acc_full = bar + 8;
+    auto full = [&](int s) { return bar + 16u + 8u * s; };
+    auto empty = [&](int s) { return bar + 32u + 8u * s; };
+    auto sd_full = [&](int g) { return bar + 48u + 8u * g; };
+    auto ds_full = [&](int g) { return bar + 64u + 8u * g; };
+    auto done = [&](int g) { return bar + 80u + 8u * g; };
+    volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem + 6 * kTile + 96);
     volatile uint32_t* abort_flag = tmem_slot + 1;
+    float* stats = reinterpret_cast<float*>(smem + 6 * kTile + 256);
 
     const int warp = __shfl_sync(0xFFFFFFFFu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;   // uniform to the compiler too
+    const int heads = KV ? p.Hkv : p.Hq, group = p.Hq / p.Hkv;
+    const int head = blockIdx.x % heads, b = blockIdx.x / heads;
     const int n_qt = p.S / kT;
-    const int qt = n_qt - 1 - (int)blockIdx.x;
-    const int h = blockIdx.y, b = blockIdx.z;
-    const int hk = h / (p.Hq / p.Hkv);
-    const int n_kv = qt + 1;
+    const int xt = KV ? (int)blockIdx.y : n_qt - 1 - (int)blockIdx.y;      // the tile that stays; those with the most work first
+    const int n_i = KV ? n_qt - xt : xt + 1;                                // pairs per walk
+    const int n_it = KV ? group * n_i : n_i;
     const int row0 = b * p.S;
 
     if (threadIdx.x == 0) {
-        mbar_init(q_full, 1);
-        for (int i = 0; i < 2; ++i) { mbar_init(kv_full0 + 8 * i, 1); mbar_init(kv_empty0 + 8 * i, 1); }
-        mbar_init(sd_full, 1); mbar_init(ds_full, 4); mbar_init(dq_full, 1);
+        mbar_init(x_full, 1); mbar_init(acc_full, 1);
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(full(i), 1); mbar_init(empty(i), 1);
+            mbar_init(sd_full(i), 1); mbar_init(ds_full(i), 4); mbar_init(done(i), 1);
+        }
         *abort_flag = 0;
         mbar_fence_init();
     }
-    if (warp == 4) { tmem_alloc(smem_u32((const void*)tmem_slot), 512); tmem_relinquish(); }
+    if (warp == 8) { tmem_alloc(smem_u32((const void*)tmem_slot), 512); tmem_relinquish(); }
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem = *tmem_slot;
-    const uint32_t tS = tmem, tdP = tmem + 128, tdQ = tmem + 256;
+    auto tS = [&](int g) { return tmem + 128u * g; };
+    auto tdP = [&](int g) { return tmem + 128u * g + 64u; };
+    const uint32_t tG1 = tmem + 256, tG2 = tmem + 384;
 
-    if (warp == 4) {
-        // the whole warp walks the tiles and one elected lane issues (narrow_gemm.cu: operands stay in uniform registers)
-        {
-            if (elect_one()) { mbar_arrive_expect_tx(q_full, 2 * kTile); }
-            if (elect_one()) { load_tile(sQ, &tmQ, q_full, h * kD, row0 + qt * kT); }
-            if (elect_one()) { load_tile(sdO, &tmdO, q_full, h * kD, row0 + qt * kT); }
-            for (int j = 0; j < 2 && j < n_kv; ++j) {
-                if (elect_one()) { mbar_arrive_expect_tx(kv_full0 + 8 * j, 2 * kTile); }
-                if (elect_one()) { load_tile(sK0 + j * kTile, &tmK, kv_full0 + 8 * j, hk * kD, row0 + j * kT); }
-                if (elect_one()) { load_tile(sV0 + j * kTile, &tmV, kv_full0 + 8 * j, hk * kD, row0 + j * kT); }
-            }
-            bool ok = mbar_wait_warp(q_full, 0, abort_flag, p.status, ST_TIMEOUT_FULL, 30);
-            for (int j = 0; j < n_kv && ok; ++j) {
-                const int s = j & 1;
-                ok = mbar_wait_warp(kv_full0 + 8 * s, (j >> 1) & 1, abort_flag, p.status, ST_TIMEOUT_FULL, 31);
-                if (!ok) break;
-                if (j > 0) {
-                    // the threads have read S / dP of the previous tile (they arrived on ds_full) before these are overwritten
-                    ok = mbar_wait_warp(ds_full, (j - 1) & 1, abort_flag, p.status, ST_TIMEOUT_FULL, 32);
-                    if (!ok) break;
-                }
-                tc_fence_after_sync();
-                if (j > 0) {
-                    if (elect_one()) { mma_128(tdQ, sdS, false, sK0 + ((j - 1) & 1) * kTile, true, j > 1); } // dQ += dS_{j-1} K_{j-1}
-                    if (elect_one()) { umma_commit(kv_empty0 + 8 * ((j - 1) & 1)); }
-                }
-                if (elect_one()) { mma_128(tS, sQ, false, sK0 + s * kTile, false, false); } // S  = Q K_j^T
-                if (elect_one()) { mma_128(tdP, sdO, false, sV0 + s * kTile, false, false); } // dP = dO V_j^T
-                if (elect_one()) { umma_commit(sd_full); }
-                if (j >= 1 && j + 1 < n_kv) {
-                    // stage (j - 1) & 1 == (j + 1) & 1 is free once dQ += dS_{j-1} K_{j-1} has completed
-                    const int s1 = (j + 1) & 1;
-                    ok = mbar_wait_warp(kv_empty0 + 8 * s1, ((j - 1) >> 1) & 1, abort_flag, p.status, ST_TIMEOUT_EMPTY, 33);
-                    if (!ok) break;
-                    if (elect_one()) { mbar_arrive_expect_tx(kv_full0 + 8 * s1, 2 * kTile); }
-                    if (elect_one()) { load_tile(sK0 + s1 * kTile, &tmK, kv_full0 + 8 * s1, hk * kD, row0 + (j + 1) * kT); }
-                    if (elect_one()) { load_tile(sV0 + s1 * kTile, &tmV, kv_full0 + 8 * s1, hk * kD, row0 + (j + 1) * kT); }
-                }
-            }
-            if (ok) ok = mbar_wait_warp(ds_full, (n_kv - 1) & 1, abort_flag, p.status, ST_TIMEOUT_FULL, 34);
-            if (ok) {
-                tc_fence_after_sync();
-                if (elect_one()) { mma_128(tdQ, sdS, false, sK0 + ((n_kv - 1) & 1) * kTile, true, n_kv > 1); }
-                if (elect_one()) { umma_commit(dq_full); }
-            }
-        }
-    } else {
-        const int r = threadIdx.x;
-        const uint32_t lane_off = (uint32_t)(warp * 32) << 16;
-        const float c = p.scale * kLog2e;
-        const long long stat = ((long long)b * p.Hq + h) * p.S + qt * kT + r;
-        const float lse_l2 = p.lse[stat] * kLog2e, dsum_r = p.dsum[stat];
+    if (warp == 9) {
+        if (elect_one()) { mbar_arrive_expect_tx(x_full, 2 * kTile); }
+        if (elect_one()) { load_tile(sX1, &tmX1, x_full, head * kD, row0 + xt * kT); }
+        if (elect_one()) { load_tile(sX2, &tmX2, x_full, head * kD, row0 + xt * kT); }
         bool ok = true;
-        for (int j = 0; j < n_kv && ok; ++j) {
-            ok = mbar_wait(sd_full, j & 1, abort_flag, p.status, ST_TIMEOUT_ACCUM, 40);
+        int yh = KV ? head * group : head / group, yt = KV ? xt : 0;
+        for (int it = 0; it < n_it; ++it) {
+            const int s = it & 1;
+            if (it >= 2) ok = mbar_wait_warp(empty(s), ((it >> 1) - 1) & 1, abort_flag, p.status, ST_TIMEOUT_EMPTY, 30);
             if (!ok) break;
-            tc_fence_after_sync();
-            // dS_{j-1} must have been consumed (dQ product issued AND completed) before the dS tile is rewritten: the
-            // S / dP products of this tile were issued after it in the same thread, so sd_full implies it
-            bwd_rows(tS, tdP, lane_off, r, j == qt, c, lse_l2, dsum_r, p.scale, nullptr, pdS);
-            tc_fence_before_sync();
-            fence_proxy_async_smem();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(ds_full);
+            if (elect_one()) { mbar_arrive_expect_tx(full(s), 2 * kTile); }
+            if (elect_one()) { load_tile(sY1(s), &tmY1, full(s), yh * kD, row0 + yt * kT); }
+            if (elect_one()) { load_tile(sY2(s), &tmY2, full(s), yh * kD, row0 + yt * kT); }
+            if (++yt == (KV ? n_qt : n_it)) { yt = KV ? xt : 0; ++yh; }
         }
-        if (ok) ok = mbar_wait(dq_full, 0, abort_flag, p.status, ST_TIMEOUT_ACCUM, 41);
-        if (ok) {
-            tc_fence_after_sync();
-            store_acc_tile(tdQ, lane_off, r, pdS, sdS, &tmdQ, h * kD, row0 + qt * kT);
-        }
-    }
-    tc_fence_before_sync();
-    __syncthreads();
-    if (warp == 4) { tc_fence_after_sync(); tmem_dealloc(tmem, 512); }
-}
-
-// ---------------------------------------------------------------------------------------------------------------------
-// backward, dK and dV: one CTA per (kv tile, kv head, batch); inner loop over the q heads of the group and the q tiles
-// ---------------------------------------------------------------------------------------------------------------------
-constexpr uint32_t kDkvSmem = 6 * kTile + 1024 + 256;   // K, V, Q, dO, P, dS
-
-__global__ void __launch_bounds__(kBwdThreads, 1)
-attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
-                    const __grid_constant__ CUtensorMap tmdO, const __grid_constant__ CUtensorMap tmdK, const __grid_constant__ CUtensorMap tmdV,
-                    const AttnParams p) {
-    extern __shared__ uint8_t smem_raw[];
-    const uint32_t raw = smem_u32(smem_raw);
-    const uint32_t base = (raw + 1023u) & ~1023u;
-    uint8_t* smem = smem_raw + (base - raw);
-    const uint32_t sK = base, sV = base + kTile, sQ = base + 2 * kTile, sdO = base + 3 * kTile, sP = base + 4 * kTile, sdS = base + 5 * kTile;
-    uint8_t* pP = smem + 4 * kTile;
-    uint8_t* pdS = smem + 5 * kTile;
-    const uint32_t bar = base + 6 * kTile;
-    const uint32_t kv_full = bar, q_full = bar + 8, q_empty = bar + 16, sd_full = bar + 24, ds_full = bar + 32, acc_full = bar + 40;
-    volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem + 6 * kTile + 64);
-    volatile uint32_t* abort_flag = tmem_slot + 1;
-
-    const int warp = __shfl_sync(0xFFFFFFFFu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;   // uniform to the compiler too
-    const int n_qt = p.S / kT;
-    const int jt = blockIdx.x;                    // kv tile (the first ones have the most q tiles)
-    const int hk = blockIdx.y, b = blockIdx.z;
-    const int group = p.Hq / p.Hkv;
-    const int n_i = n_qt - jt;                    // q tiles at or after the kv tile
-    const int n_it = group * n_i;                 // inner iterations: (q head of the group) x (q tile)
-    const int row0 = b * p.S;
-
-    if (threadIdx.x == 0) {
-        mbar_init(kv_full, 1); mbar_init(q_full, 1); mbar_init(q_empty, 1);
-        mbar_init(sd_full, 1); mbar_init(ds_full, 4); mbar_init(acc_full, 1);
-        *abort_flag = 0;
-        mbar_fence_init();
-    }
-    if (warp == 4) { tmem_alloc(smem_u32((const void*)tmem_slot), 512); tmem_relinquish(); }
-    tc_fence_before_sync();
-    __syncthreads();
-    tc_fence_after_sync();
-    const uint32_t tmem = *tmem_slot;
-    const uint32_t tS = tmem, tdP = tmem + 128, tdV = tmem + 256, tdK = tmem + 384;
-
-    if (warp == 4) {
+    } else if (warp == 8) {
         // the whole warp walks the tiles and one elected lane issues (narrow_gemm.cu: operands stay in uniform registers)
-        {
-            if (elect_one()) { mbar_arrive_expect_tx(kv_full, 2 * kTile); }
-            if (elect_one()) { load_tile(sK, &tmK, kv_full, hk * kD, row0 + jt * kT); }
-            if (elect_one()) { load_tile(sV, &tmV, kv_full, hk * kD, row0 + jt * kT); }
-            bool ok = mbar_wait_warp(kv_full, 0, abort_flag, p.status, ST_TIMEOUT_FULL, 50);
-            for (int it = 0; it < n_it && ok; ++it) {
-                const int h = hk * group + it / n_i, qi = jt + it % n_i;
-                // Q / dO of the previous iteration are free once its dV / dK products have completed
-                if (it > 0) {
-                    ok = mbar_wait_warp(q_empty, (it - 1) & 1, abort_flag, p.status, ST_TIMEOUT_EMPTY, 51);
-                    if (!ok) break;
-                }
-                if (elect_one()) { mbar_arrive_expect_tx(q_full, 2 * kTile); }
-                if (elect_one()) { load_tile(sQ, &tmQ, q_full, h * kD, row0 + qi * kT); }
-                if (elect_one()) { load_tile(sdO, &tmdO, q_full, h * kD, row0 + qi * kT); }
-                ok = mbar_wait_warp(q_full, it & 1, abort_flag, p.status, ST_TIMEOUT_FULL, 52);
-                if (!ok) break;
-                tc_fence_after_sync();
-                if (elect_one()) { mma_128(tS, sQ, false, sK, false, false); } // S  = Q K^T      (rows = queries)
-                if (elect_one()) { mma_128(tdP, sdO, false, sV, false, false); } // dP = dO V^T
-                if (elect_one()) { umma_commit(sd_full); }
-                ok = mbar_wait_warp(ds_full, it & 1, abort_flag, p.status, ST_TIMEOUT_FULL, 53);
-                if (!ok) break;
-                tc_fence_after_sync();
-                if (elect_one()) { mma_128(tdV, sP, true, sdO, true, it > 0); } // dV += P^T dO    (P^T: the P tile read MN-major)
-                if (elect_one()) { mma_128(tdK, sdS, true, sQ, true, it > 0); } // dK += dS^T Q
-                if (elect_one()) { umma_commit(q_empty); }
-                if (it == n_it - 1 && elect_one()) umma_commit(acc_full);
-            }
-        }
-    } else {
-        const int r = threadIdx.x;
-        const uint32_t lane_off = (uint32_t)(warp * 32) << 16;
-        const float c = p.scale * kLog2e;
-        bool ok = true;
+        bool ok = mbar_wait_warp(x_full, 0, abort_flag, p.status, ST_TIMEOUT_FULL, 31);
+        auto scores = [&](int it, int g) {          // over P and dS of the half before, whose products must be done
+            if (g == 0) ok = mbar_wait_warp(full(it & 1), (it >> 1) & 1, abort_flag, p.status, ST_TIMEOUT_FULL, 32);
+            if (ok && it > 0) ok = mbar_wait_warp(done(g), (it - 1) & 1, abort_flag, p.status, ST_TIMEOUT_ACCUM, 33);
+            if (!ok) return;
+            tc_fence_after_sync();
+            if (elect_one()) { mma_half(tS(g), sX1, sY1(it & 1), g); }
+            if (elect_one()) { mma_half(tdP(g), sX2, sY2(it & 1), g); }
+            if (elect_one()) { umma_commit(sd_full(g)); }
+        };
+        if (ok) scores(0, 0);
+        if (ok) scores(0, 1);
         for (int it = 0; it < n_it && ok; ++it) {
-            const int h = hk * group + it / n_i, qi = jt + it % n_i;
-            const long long stat = ((long long)b * p.Hq + h) * p.S + qi * kT + r;
-            const float lse_l2 = p.lse[stat] * kLog2e, dsum_r = p.dsum[stat];
-            ok = mbar_wait(sd_full, it & 1, abort_flag, p.status, ST_TIMEOUT_ACCUM, 60);
+#pragma unroll
+            for (int g = 0; g < 2 && ok; ++g) {
+                ok = mbar_wait_warp(ds_full(g), it & 1, abort_flag, p.status, ST_TIMEOUT_FULL, 34);
+                if (!ok) break;
+                tc_fence_after_sync();
+                if (KV && elect_one()) mma_grad(tG2, tS(g), sY2(it & 1), g, it > 0 || g > 0);
+                if (elect_one()) { mma_grad(tG1, tdP(g), sY1(it & 1), g, it > 0 || g > 0); }
+                if (elect_one()) { umma_commit(done(g)); }
+                if (g == 1 && it + 2 < n_it && elect_one()) umma_commit(empty(it & 1));
+                if (it + 1 < n_it) scores(it + 1, g);
+                else if (g == 1 && elect_one()) umma_commit(acc_full);
+            }
+        }
+    } else {
+        const int g = warp >> 2, t = threadIdx.x & 127;
+        const uint32_t lane_off = (uint32_t)((warp & 3) * 32) << 16;
+        const float c = p.scale * kLog2e;
+        float nl = 0.f, nd = 0.f;
+        int yh = head * group, yt = xt;             // KV: the queries whose statistics are requested next
+        float st[4] = {};
+        auto request = [&]() {
+            const long long at = ((long long)b * p.Hq + yh) * p.S + yt * kT + g * 64 + lane;
+            st[0] = p.lse[at]; st[1] = p.lse[at + 32]; st[2] = p.dsum[at]; st[3] = p.dsum[at + 32];
+            if (++yt == n_qt) { yt = xt; ++yh; }
+        };
+        if (KV) {
+            request();
+        } else {
+            const long long at = ((long long)b * p.Hq + head) * p.S + xt * kT + t;
+            nl = -p.lse[at] * kLog2e;
+            nd = -p.dsum[at];
+        }
+        bool ok = true;
+        for (int it = 0, i = 0; it < n_it; ++it) {
+            float* mine = stats + (warp * 2 + (it & 1)) * 128;
+            if (KV) {
+                mine[lane] = -st[0] * kLog2e; mine[lane + 32] = -st[1] * kLog2e; mine[lane + 64] = -st[2]; mine[lane + 96] = -st[3];
+                __syncwarp();
+                if (it + 1 < n_it) request();
+            }
+            ok = mbar_wait_warp(sd_full(g), it & 1, abort_flag, p.status, ST_TIMEOUT_ACCUM, 40);
             if (!ok) break;
             tc_fence_after_sync();
-            // the P / dS tiles of the previous iteration have been consumed: S / dP of this one were issued after the
-            // previous dV / dK products by the same thread and have completed
-            bwd_rows(tS, tdP, lane_off, r, qi == jt, c, lse_l2, dsum_r, p.scale, pP, pdS);
+            bwd_rows<KV>(tS(g) + lane_off, tdP(g) + lane_off, g, t, KV ? i == 0 : it == n_it - 1, c, p.scale, nl, nd, mine);
+            if (++i == n_i) i = 0;
             tc_fence_before_sync();
-            fence_proxy_async_smem();
             __syncwarp();
-            if (lane == 0) mbar_arrive(ds_full);
+            if (lane == 0) mbar_arrive(ds_full(g));
         }
-        if (ok) ok = mbar_wait(acc_full, 0, abort_flag, p.status, ST_TIMEOUT_ACCUM, 61);
+        if (ok) ok = mbar_wait_warp(acc_full, 0, abort_flag, p.status, ST_TIMEOUT_ACCUM, 41);
+        // KV: the first group stores dK, the second dV; else each half the columns of dQ. The walk is over: its tiles serve as staging.
+        const uint32_t stage = (KV ? 2 + g : 2) * kTile + (KV ? 0 : g * kBlk), acc = (KV && g ? tG2 : tG1) + lane_off + (KV ? 0 : 64 * g);
         if (ok) {
             tc_fence_after_sync();
-            store_acc_tile(tdV, lane_off, r, pP, sP, &tmdV, hk * kD, row0 + jt * kT);
-            store_acc_tile(tdK, lane_off, r, pdS, sdS, &tmdK, hk * kD, row0 + jt * kT);
+            stage_block(acc, t, smem + stage);
+            if (KV) stage_block(acc + 64, t, smem + stage + kBlk);
+            fence_proxy_async_smem();
+        }
+        asm volatile("bar.sync %0, 128;" ::"r"(1 + g) : "memory");
+        if (ok && t == 0) {
+            const CUtensorMap* map = KV && g ? &tmG2 : &tmG1;
+            tma_store_2d(map, base + stage, head * kD + (KV ? 0 : 64 * g), row0 + xt * kT);
+            if (KV) tma_store_2d(map, base + stage + kBlk, head * kD + 64, row0 + xt * kT);
+            tma_store_commit();
+            tma_store_wait_all();
         }
     }
     tc_fence_before_sync();
     __syncthreads();
-    if (warp == 4) { tc_fence_after_sync(); tmem_dealloc(tmem, 512); }
+    if (warp == 8) { tc_fence_after_sync(); tmem_dealloc(tmem, 512); }
 }
 
 int check_attn(const AttnArgs& a) {
@@ -683,17 +639,17 @@ int launch_attn_bwd(const AttnArgs& a, cudaStream_t stream) {
     p.B = a.B; p.S = a.S; p.Hq = a.Hq; p.Hkv = a.Hkv; p.scale = a.scale; p.lse = a.lse; p.dsum = a.dsum; p.status = device_status_ptr();
     static bool once = false;
     if (!once) {
-        if ((rc = set_smem(attn_bwd_dq_kernel, kDqSmem))) return rc;
-        if ((rc = set_smem(attn_bwd_dkv_kernel, kDkvSmem))) return rc;
+        if ((rc = set_smem(attn_bwd_kernel<false>, kBwdSmem))) return rc;
+        if ((rc = set_smem(attn_bwd_kernel<true>, kBwdSmem))) return rc;
         once = true;
     }
     const long long n_rows = (long long)a.B * a.S * a.Hq;
     const auto dsum = ((uintptr_t)a.o & 15) ? attn_dsum_kernel<false> : attn_dsum_kernel<true>;   // o passes no tensor map that would refuse it
     dsum<<<(unsigned)((n_rows + 63) / 64), 256, 0, stream>>>((const __nv_bfloat16*)a.o, (const __nv_bfloat16*)a.d_o, a.ldo, a.B, a.S, a.Hq, a.dsum);
     PLZ_LAUNCH_CHECK();
-    attn_bwd_dq_kernel<<<dim3(a.S / kT, a.Hq, a.B), kBwdThreads, kDqSmem, stream>>>(tmQ, tmK, tmV, tmdO, tmdQ, p);
+    attn_bwd_kernel<false><<<dim3(a.Hq * a.B, a.S / kT), kBwdThreads, kBwdSmem, stream>>>(tmQ, tmdO, tmK, tmV, tmdQ, tmdQ, p);
     PLZ_LAUNCH_CHECK();
-    attn_bwd_dkv_kernel<<<dim3(a.S / kT, a.Hkv, a.B), kBwdThreads, kDkvSmem, stream>>>(tmQ, tmK, tmV, tmdO, tmdK, tmdV, p);
+    attn_bwd_kernel<true><<<dim3(a.Hkv * a.B, a.S / kT), kBwdThreads, kBwdSmem, stream>>>(tmK, tmV, tmQ, tmdO, tmdK, tmdV, p);
     PLZ_LAUNCH_CHECK();
     return PLZ_OK;
 }
