@@ -231,6 +231,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem = *tmem_slot;
+    pdl_wait();
+    pdl_launch_dependents();
     auto tS = [&](int g) { return tmem + 128u * g; };
     auto tO = [&](int g) { return tmem + 256u + 128u * g; };
 
@@ -310,13 +312,14 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 // ---------------------------------------------------------------------------------------------------------------------
 template <bool O16>      // o aligned to 16 bytes; else to 8
 __global__ void __launch_bounds__(256)
-attn_dsum_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ d_o, long long ld, int B, int S, int Hq,
-                 float* __restrict__ dsum) {
+attn_dsum_kernel(const __nv_bfloat16* o, const __nv_bfloat16* d_o, long long ld, int B, int S, int Hq, float* dsum) {
     // sixteen lanes per (token, head) row, eight rows of a warp at once: four 16-byte loads of each operand in flight per lane (4096 tokens x 32
     // heads 23 -> 18 us against one row per warp)
     const int lane = threadIdx.x & 31, l = lane & 15;
     const long long rows = (long long)B * S * Hq, row0 = ((long long)blockIdx.x * 8 + (threadIdx.x >> 5)) * 8 + (lane >> 4);
     uint4 a[4], g[4];
+    pdl_wait();
+    pdl_launch_dependents();
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         const long long row = row0 + 2 * i;
@@ -481,6 +484,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_constant_
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem = *tmem_slot;
+    pdl_wait();
+    pdl_launch_dependents();
     auto tS = [&](int g) { return tmem + 128u * g; };
     auto tdP = [&](int g) { return tmem + 128u * g + 64u; };
     const uint32_t tG1 = tmem + 256, tG2 = tmem + 384;
@@ -616,8 +621,7 @@ int launch_attn_fwd(const AttnArgs& a, cudaStream_t stream) {
     p.B = a.B; p.S = a.S; p.Hq = a.Hq; p.Hkv = a.Hkv; p.scale = a.scale; p.lse = a.lse; p.status = device_status_ptr();
     static bool once = false;
     if (!once) { if ((rc = set_smem(attn_fwd_kernel, kFwdSmem))) return rc; once = true; }
-    attn_fwd_kernel<<<dim3(a.Hq * a.B, (a.S / kT + 1) / 2), kFwdThreads, kFwdSmem, stream>>>(tmQ, tmK, tmV, tmO, p);
-    PLZ_LAUNCH_CHECK();
+    PLZ_LAUNCH_BEHIND(attn_fwd_kernel, dim3(a.Hq * a.B, (a.S / kT + 1) / 2), dim3(kFwdThreads), kFwdSmem, stream, tmQ, tmK, tmV, tmO, p);
     return PLZ_OK;
 }
 
@@ -645,12 +649,9 @@ int launch_attn_bwd(const AttnArgs& a, cudaStream_t stream) {
     }
     const long long n_rows = (long long)a.B * a.S * a.Hq;
     const auto dsum = ((uintptr_t)a.o & 15) ? attn_dsum_kernel<false> : attn_dsum_kernel<true>;   // o passes no tensor map that would refuse it
-    dsum<<<(unsigned)((n_rows + 63) / 64), 256, 0, stream>>>((const __nv_bfloat16*)a.o, (const __nv_bfloat16*)a.d_o, a.ldo, a.B, a.S, a.Hq, a.dsum);
-    PLZ_LAUNCH_CHECK();
-    attn_bwd_kernel<false><<<dim3(a.Hq * a.B, a.S / kT), kBwdThreads, kBwdSmem, stream>>>(tmQ, tmdO, tmK, tmV, tmdQ, tmdQ, p);
-    PLZ_LAUNCH_CHECK();
-    attn_bwd_kernel<true><<<dim3(a.Hkv * a.B, a.S / kT), kBwdThreads, kBwdSmem, stream>>>(tmK, tmV, tmQ, tmdO, tmdK, tmdV, p);
-    PLZ_LAUNCH_CHECK();
+    PLZ_LAUNCH_BEHIND(dsum, dim3((unsigned)((n_rows + 63) / 64)), dim3(256), 0, stream, (const __nv_bfloat16*)a.o, (const __nv_bfloat16*)a.d_o, a.ldo, a.B, a.S, a.Hq, a.dsum);
+    PLZ_LAUNCH_BEHIND(attn_bwd_kernel<false>, dim3(a.Hq * a.B, a.S / kT), dim3(kBwdThreads), kBwdSmem, stream, tmQ, tmdO, tmK, tmV, tmdQ, tmdQ, p);
+    PLZ_LAUNCH_BEHIND(attn_bwd_kernel<true>, dim3(a.Hkv * a.B, a.S / kT), dim3(kBwdThreads), kBwdSmem, stream, tmK, tmV, tmQ, tmdO, tmdK, tmdV, p);
     return PLZ_OK;
 }
 

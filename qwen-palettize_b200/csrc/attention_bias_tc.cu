@@ -191,7 +191,7 @@ __device__ __forceinline__ void softmax_group(const Group& G, const TcParams& p,
 #pragma unroll
                 for (int i = 0; i < 8; ++i) f[i] = __uint_as_float(v[g * 8 + i]) * inv_l;
                 if (gate && cb * 32 + g * 8 < p.dv) {
-                    const uint4 q = __ldg(reinterpret_cast<const uint4*>(gate + cb * 32 + g * 8));
+                    const uint4 q = *reinterpret_cast<const uint4*>(gate + cb * 32 + g * 8);
                     const uint32_t w[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
                     for (int i = 0; i < 4; ++i) {
@@ -260,6 +260,8 @@ attn_bias_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem = *tmem_slot;
+    pdl_wait();
+    pdl_launch_dependents();
     auto tS = [&](int g) { return tmem + 128u * g; };
     auto tO = [&](int g) { return tmem + 256u + 128u * g; };
 
@@ -370,8 +372,7 @@ int launch_t(const AttnBiasArgs& a, cudaStream_t stream) {
     PLZ_CUDA_CHECK(cudaGetDevice(&dev));
     if (!once[dev & 63]) { PLZ_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM)); once[dev & 63] = true; }
     const int n_qt = (a.n + kT - 1) / kT;
-    kern<<<dim3((n_qt + 1) / 2, a.H, a.B), kThreads, C::SMEM, stream>>>(tmQ, tmK, tmV, tmO, tmQ2, tmK2, p);
-    PLZ_LAUNCH_CHECK();
+    PLZ_LAUNCH_BEHIND(kern, dim3((n_qt + 1) / 2, a.H, a.B), dim3(kThreads), C::SMEM, stream, tmQ, tmK, tmV, tmO, tmQ2, tmK2, p);
     return PLZ_OK;
 }
 

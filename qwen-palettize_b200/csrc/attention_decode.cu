@@ -520,6 +520,7 @@ int launch_combine(const DecParams& p, int B, int dv, int sink, cudaStream_t str
 __global__ void __launch_bounds__(256)
 embed_gather_kernel(const __nv_bfloat16* __restrict__ table, long long ldt, const long long* __restrict__ ids, long long n, int width,
                     long long vocab, __nv_bfloat16* __restrict__ out, long long ldo, int* __restrict__ bad) {
+    pdl_launch_dependents();
     const int vec = width >> 3;
     const long long total = n * vec;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {

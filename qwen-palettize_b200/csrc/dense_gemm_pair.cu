@@ -27,6 +27,7 @@ constexpr uint32_t kDpBarOff = kDpEpiOff + kDpEpiWarps * kDpEpiBytes;
 constexpr uint32_t kDpSmemBytes = kDpBarOff + 1024 + 256;
 
 struct DpParams {
+    int lets_next;           // let the next kernel start behind this one's wait
     int M, J, R, out_cols;
     int n_extra;             // 0 or 1 extra 64-wide reduction block from (A2, B2)
     int tiles_m, tiles_j, tile_w, n_whole, n_items;   // plan_pair_tiles
@@ -85,6 +86,8 @@ dense_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
     cluster_sync_all();   // both CTAs' barriers are initialised before anyone arrives on the other's
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
+    pdl_wait();
+    if (p.lets_next) pdl_launch_dependents();
 
     auto item_width = [&](int t) { return t < p.n_whole ? p.tile_w : 128; };
     auto item_origin = [&](int t, int& m0, int& j0) {
@@ -278,6 +281,7 @@ int launch_dp(const LutGemmArgs& a, int sms, cudaStream_t stream) {
     p.M = a.M; p.J = a.J; p.R = a.R; p.out_cols = GLU ? a.J / 2 : a.J; p.n_extra = a.r2 > 0 ? 1 : 0;
     p.alpha = a.alpha; p.bias = (const __nv_bfloat16*)a.bias; p.relu2 = a.fuse == 3 && a.act == 1;
     p.status = device_status_ptr();
+    p.lets_next = !g_smallm_overlap;
     int pairs = sms / 2;
     // columns of a row-major B come in boxes of 64, so there other widths would read what they do not use
     const PairTiles pt = GLU ? plan_pair_tiles(a.M, a.J, pairs, 64) : BMN ? plan_pair_tiles(a.M, a.J, pairs, 32) : plan_pair_waves(a.M, a.J, pairs, 16);
@@ -312,8 +316,7 @@ int launch_dp(const LutGemmArgs& a, int sms, cudaStream_t stream) {
         PLZ_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kDpSmemBytes));
         attr_set[dev & 63] = true;
     }
-    kern<<<2 * pairs, kDpThreads, kDpSmemBytes, stream>>>(tmA, tmB, tmBh, tmA2, tmB2, tmD, tmD16, p);
-    PLZ_LAUNCH_CHECK();
+    PLZ_LAUNCH_BEHIND(kern, dim3(2 * pairs), dim3(kDpThreads), kDpSmemBytes, stream, tmA, tmB, tmBh, tmA2, tmB2, tmD, tmD16, p);
     return PLZ_OK;
 }
 

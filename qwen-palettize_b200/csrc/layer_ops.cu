@@ -219,6 +219,7 @@ __global__ void __launch_bounds__(256)
 qknorm_rope_bwd_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, const __nv_bfloat16* __restrict__ w, const float* __restrict__ cs,
                        const float* __restrict__ sn, const __nv_bfloat16* __restrict__ dy, long long lddy, long long rows, int H, int S,
                        float eps, __nv_bfloat16* __restrict__ dx, long long lddx, float* __restrict__ dw) {
+    pdl_launch_dependents();
     __shared__ float acc[8][128];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     float g0 = 0.f, g1 = 0.f, g2 = 0.f, g3 = 0.f;   // this lane's four weight-gradient partials
@@ -263,6 +264,7 @@ __global__ void __launch_bounds__(256, 2)
 qknorm_rope_bwd16_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, const __nv_bfloat16* __restrict__ w, const float* __restrict__ cs,
                          const float* __restrict__ sn, const __nv_bfloat16* __restrict__ dy, long long lddy, long long units, int quads, int H, int S, float eps,
                          __nv_bfloat16* __restrict__ dx, long long lddx, float* __restrict__ dw) {
+    pdl_launch_dependents();
     __shared__ float acc[8][128];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, hl = lane >> 3, l = lane & 7;
     const Lanes16 wv = load_weight16(w, l);
@@ -395,11 +397,11 @@ int launch_add_rmsnorm(const void* x, long long ldx, const void* addend, long lo
     const bool block = M <= 4 * sm_count_here();   // few rows: a block per row
     const dim3 grid(block ? M : grid_for(M, 8));
     if (addend) {
-        if (block) PLZ_LAUNCH_CHAIN(rms_kernel<true, true>, grid, dim3(256), 0, stream, xp, ldx, ap, lda, sp, lds, gp, M, K, eps, hp, ldh, rstd);
-        else PLZ_LAUNCH_CHAIN(rms_kernel<false, true>, grid, dim3(256), 0, stream, xp, ldx, ap, lda, sp, lds, gp, M, K, eps, hp, ldh, rstd);
+        if (block) PLZ_LAUNCH_CHAIN_BEHIND(rms_kernel<true, true>, grid, dim3(256), 0, stream, xp, ldx, ap, lda, sp, lds, gp, M, K, eps, hp, ldh, rstd);
+        else PLZ_LAUNCH_CHAIN_BEHIND(rms_kernel<false, true>, grid, dim3(256), 0, stream, xp, ldx, ap, lda, sp, lds, gp, M, K, eps, hp, ldh, rstd);
     } else {
-        if (block) PLZ_LAUNCH_CHAIN(rms_kernel<true, false>, grid, dim3(256), 0, stream, xp, ldx, ap, lda, sp, lds, gp, M, K, eps, hp, ldh, rstd);
-        else PLZ_LAUNCH_CHAIN(rms_kernel<false, false>, grid, dim3(256), 0, stream, xp, ldx, ap, lda, sp, lds, gp, M, K, eps, hp, ldh, rstd);
+        if (block) PLZ_LAUNCH_CHAIN_BEHIND(rms_kernel<true, false>, grid, dim3(256), 0, stream, xp, ldx, ap, lda, sp, lds, gp, M, K, eps, hp, ldh, rstd);
+        else PLZ_LAUNCH_CHAIN_BEHIND(rms_kernel<false, false>, grid, dim3(256), 0, stream, xp, ldx, ap, lda, sp, lds, gp, M, K, eps, hp, ldh, rstd);
     }
     return PLZ_OK;
 }
@@ -443,7 +445,7 @@ int launch_qknorm_rope2(const void* x1, long long ldx1, const void* w1, int H1, 
         per = per < 1 ? 1 : per > quads ? quads : per;
         const int parts = (quads + (int)per - 1) / (int)per;
         const long long units = tokens * parts;
-        PLZ_LAUNCH_CHAIN(qknorm_rope_fwd16_kernel, dim3((unsigned)((units + 7) / 8)), dim3(256), 0, stream, a, b, cs, sn, units, parts, (int)per, S, eps);
+        PLZ_LAUNCH_CHAIN_BEHIND(qknorm_rope_fwd16_kernel, dim3((unsigned)((units + 7) / 8)), dim3(256), 0, stream, a, b, cs, sn, units, parts, (int)per, S, eps);
         return PLZ_OK;
     }
     PLZ_LAUNCH_CHAIN(qknorm_rope_fwd_kernel, dim3((unsigned)blocks), dim3(256), 0, stream, a, b, cs, sn, rows, S, eps);
@@ -451,14 +453,14 @@ int launch_qknorm_rope2(const void* x1, long long ldx1, const void* w1, int H1, 
 }
 int launch_swiglu_fwd(const void* gate, long long ldg, const void* up, long long ldu, int M, int N, void* act, long long lda, cudaStream_t stream) {
     if (M <= 0 || N <= 0) return PLZ_OK;
-    PLZ_LAUNCH_CHAIN(swiglu_fwd_kernel, dim3(grid_for((long long)M * (N >> 3), 256)), dim3(256), 0, stream, (const __nv_bfloat16*)gate, ldg,
+    PLZ_LAUNCH_CHAIN_BEHIND(swiglu_fwd_kernel, dim3(grid_for((long long)M * (N >> 3), 256)), dim3(256), 0, stream, (const __nv_bfloat16*)gate, ldg,
                      (const __nv_bfloat16*)up, ldu, M, N, (__nv_bfloat16*)act, lda);
     return PLZ_OK;
 }
 int launch_add(const void* a, long long lda, const void* b, long long ldb, const void* c, long long ldc, int M, int N, void* out, long long ldo,
                cudaStream_t stream) {
     if (M <= 0 || N <= 0) return PLZ_OK;
-    PLZ_LAUNCH_CHAIN(add_kernel, dim3(grid_for((long long)M * (N >> 3), 256)), dim3(256), 0, stream, (const __nv_bfloat16*)a, lda,
+    PLZ_LAUNCH_CHAIN_BEHIND(add_kernel, dim3(grid_for((long long)M * (N >> 3), 256)), dim3(256), 0, stream, (const __nv_bfloat16*)a, lda,
                      (const __nv_bfloat16*)b, ldb, (const __nv_bfloat16*)c, ldc, M, N, (__nv_bfloat16*)out, ldo);
     return PLZ_OK;
 }

@@ -44,6 +44,7 @@ int g_pair_gemm = 1;  // 0: never use the CTA-pair kernel (comparisons, tests of
 namespace {
 
 struct PairParams {
+    int lets_next;           // let the next kernel start behind this one's wait
     int M, J, R;
     int n_extra;             // 0 or 1 extra 64-wide reduction block from (A2, B2)
     int tiles_j, tile_w;     // column tiles of tile_w columns
@@ -131,6 +132,8 @@ lut_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
     cluster_sync_all();   // both CTAs' barriers are initialised before anyone arrives on the other's
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
+    pdl_wait();
+    if (p.lets_next) pdl_launch_dependents();
 
     auto item_width = [&](int t) { return t < p.n_whole ? p.tile_w : 128; };
     auto item_origin = [&](int t, int& m0, int& j0) {
@@ -489,6 +492,7 @@ int launch_pair_t(const LutGemmArgs& a, cudaStream_t stream) {
     p.Wn = a.Wn; p.Wk = a.Wk;
     p.alpha = a.alpha; p.bias = (const __nv_bfloat16*)a.bias;
     p.status = device_status_ptr();
+    p.lets_next = !g_smallm_overlap;
     p.prof = (unsigned long long*)a.prof;
     auto kern = lut_gemm_pair_kernel<BMODE, GLU>;
     static bool attr_set[64] = {};
@@ -513,6 +517,8 @@ int launch_pair_t(const LutGemmArgs& a, cudaStream_t stream) {
     cfg.blockDim = dim3(kThreads);
     cfg.dynamicSmemBytes = kSmemBytes;
     cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    cfg.attrs = attr; cfg.numAttrs = behind_attr(stream, attr);
     PLZ_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kern, tmA, tmA2, tmB2, tmD, tmD32, p));
     ++g_launch_count;
     return PLZ_OK;

@@ -52,6 +52,7 @@ struct NarrowParams {
     int count; NarrowMat mat[kNgMaxMats];
     int gs_n, gs_k, n_kgroups;
     int glu;                       // a tile is 64 rows of mat[0] and the same rows of mat[1]
+    int early;                     // W is read ahead of the wait for the kernel before
     const __nv_bfloat16* bias; int act, y_f32; float alpha;
     StatusWord* status;
 };
@@ -166,6 +167,7 @@ narrow_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
         mbar_fence_init();
         tma_prefetch_desc(&tmX);
         if (p.n_blocks > p.nkb) { tma_prefetch_desc(&tmX2); tma_prefetch_desc(&tmW2); }
+        if (!p.early) pdl_wait();
         for (int it = 0; it < pre; ++it) load_w(it, it);
     }
     if (warp == 1) { tmem_alloc(smem_u32((const void*)tmem_slot), p.tmem_cols); tmem_relinquish(); }
@@ -174,6 +176,7 @@ narrow_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
     const uint32_t tmem_w = tmem_base + (uint32_t)(p.n_acc * p.npad);      // LUT: 32 columns per stage
+    if (!p.early) pdl_wait();
     pdl_launch_dependents();
 
     // every wait below that x holds up starts after the previous kernel of the stream has finished: its time is not the wait's
@@ -459,7 +462,7 @@ int cluster_size(int tiles, int blocks, int sms, int fixed) {
 int turned_parts(int n_blocks) { return n_blocks >= 64 ? 8 : n_blocks >= 32 ? 4 : n_blocks >= 16 ? 2 : 1; }
 
 template <bool LUT>
-int launch_ng(const NarrowParams& p, int tiles, int ranks, bool early, const CUtensorMap (&tm)[4], cudaStream_t stream) {
+int launch_ng(const NarrowParams& p, int tiles, int ranks, const CUtensorMap (&tm)[4], cudaStream_t stream) {
     auto kern = narrow_gemm_kernel<LUT>;
     constexpr uint32_t smem = kNgRingBytes<LUT> + kNgBarBytes + 1024;
     static bool attr_set[64] = {};
@@ -472,11 +475,10 @@ int launch_ng(const NarrowParams& p, int tiles, int ranks, bool early, const CUt
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(tiles * ranks)); cfg.blockDim = dim3(kNgThreads<LUT>); cfg.dynamicSmemBytes = smem; cfg.stream = stream;
     cudaLaunchAttribute attr[2];
+    const unsigned behind = behind_attr(stream, &attr[1]);
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = (unsigned)ranks; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[1].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr; cfg.numAttrs = g_smallm_overlap && early ? 2 : 1;   // else W may be what the previous kernel writes: it is read ahead of the wait
+    cfg.attrs = attr; cfg.numAttrs = 1 + (p.early ? 1u : behind);
     PLZ_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kern, tm[0], tm[1], tm[2], tm[3], p));
     ++g_launch_count;
     return PLZ_OK;
@@ -537,8 +539,8 @@ int launch_narrow_gemm(const NarrowArgs& a, cudaStream_t stream) {
         if ((rc = make_tmap_bf16(&tm[3], a.w2, a.mat[0].N, a.r2, a.ldw2, 64, 128))) return rc;
     }
     const int ranks = a.transposed ? turned_parts(p.n_blocks) : cluster_size(tiles, p.n_blocks, seq_sm_count(), 12);
-    const bool early = a.early && !a.transposed;
-    return lut ? launch_ng<true>(p, tiles, ranks, early, tm, stream) : launch_ng<false>(p, tiles, ranks, early, tm, stream);
+    p.early = g_smallm_overlap && a.early && !a.transposed;       // else W may be what the previous kernel writes
+    return lut ? launch_ng<true>(p, tiles, ranks, tm, stream) : launch_ng<false>(p, tiles, ranks, tm, stream);
 }
 
 namespace {
@@ -590,6 +592,8 @@ turned_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
+    pdl_wait();
+    pdl_launch_dependents();
 
     int issued = 0;                        // stages the producing thread has filled
     if (warp == 0) {
@@ -710,8 +714,7 @@ int launch_tg(const NarrowArgs& a, const CUtensorMap& tmX, const CUtensorMap& tm
         PLZ_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
         attr_set[dev & 63] = true;
     }
-    kern<<<p.tiles < ctas ? p.tiles : ctas, kTgThreads, smem, stream>>>(tmX, tmW, p);
-    PLZ_LAUNCH_CHECK();
+    PLZ_LAUNCH_BEHIND(kern, dim3(p.tiles < ctas ? p.tiles : ctas), dim3(kTgThreads), smem, stream, tmX, tmW, p);
     return PLZ_OK;
 }
 

@@ -115,6 +115,8 @@ delta_chunk_kernel(const ChunkParams p) {
     const float* qg = (const float*)p.q + (row0 * p.G + hk) * p.dk;
     const float* kg = (const float*)p.k + (row0 * p.G + hk) * p.dk;
     const float* gg = p.logg + (row0 * p.H + h) * p.dk;
+    pdl_wait();
+    pdl_launch_dependents();
 
     if (p.vec) {
 #pragma unroll
@@ -372,7 +374,7 @@ delta_chunk_kernel(const ChunkParams p) {
                 if (is_w) f[ks][x] = -s.k[j][c];
                 else if (v_in_smem) f[ks][x] = s.q[j][c];
                 // past the last token T's column has beta = 0, past the last value column nobody reads: any finite value will do
-                else f[ks][x] = __ldg(vg + (long long)min(j, L - 1) * ldv + min(c, p.dv - 1));
+                else f[ks][x] = vg[(long long)min(j, L - 1) * ldv + min(c, p.dv - 1)];
             }
         float acc0[4] = {0.f, 0.f, 0.f, 0.f}, acc1[4] = {0.f, 0.f, 0.f, 0.f};
         uint32_t bh[4][2], bl[4][2];
@@ -427,6 +429,8 @@ decay_chunk_kernel(const ChunkParams p) {
     const __nv_bfloat16* qg = (const __nv_bfloat16*)p.q + row0 * p.ld + (long long)h * p.dk;
     const __nv_bfloat16* kg = (const __nv_bfloat16*)p.k + row0 * p.ld + (long long)h * p.dk;
     const __nv_bfloat16* vg = (const __nv_bfloat16*)p.v + row0 * p.ld + (long long)h * p.dv;
+    pdl_wait();
+    pdl_launch_dependents();
     if (tid <= kC) s.pw[tid] = powf(p.decay[h], (float)tid);
     if (p.vec) {
 #pragma unroll 4
@@ -540,9 +544,7 @@ int launch_chunked(ChunkParams p, int B, void* ws, long long ws_bytes, cudaStrea
     for (int c0 = 0; c0 < all; c0 += (int)seg) {
         p.t_begin = c0 * kC;
         p.chunks = all - c0 < (int)seg ? all - c0 : (int)seg;
-        if (DELTA) delta_chunk_kernel<DK><<<dim3(p.chunks, p.H, B), 256, smem, stream>>>(p);
-        else decay_chunk_kernel<DK><<<dim3(p.chunks, p.H, B), 256, smem, stream>>>(p);
-        PLZ_LAUNCH_CHECK();
+        PLZ_LAUNCH_BEHIND((DELTA ? delta_chunk_kernel<DK> : decay_chunk_kernel<DK>), dim3(p.chunks, p.H, B), dim3(256), smem, stream, p);
         const ScanArgs a = {p.ws, p.ws_stride, p.state, p.o, B, p.n, p.t_begin, p.chunks, p.H, p.dk, p.dv, p.dvp};
         const int rc = launch_chunk_scan(a, DELTA, DK / 64, stream);
         if (rc) return rc;

@@ -737,11 +737,11 @@ int launch_seq_rows_norm(int dtype, const float* x, const long long* idx, const 
 
 template <typename T>
 static int norm_gate4(dim3 grid, const float* o, const T* gate, long long ldg, const float* w, float eps, int groups, int L, T* out, cudaStream_t stream) {
-    if (L <= 128) PLZ_LAUNCH_CHAIN((norm_gate4_kernel<T, 1, 32>), grid, dim3(256), 0, stream, o, gate, ldg, w, eps, groups, L, out);
-    else if (L <= 256) PLZ_LAUNCH_CHAIN((norm_gate4_kernel<T, 2, 32>), grid, dim3(256), 0, stream, o, gate, ldg, w, eps, groups, L, out);
-    else if (L <= 1024) PLZ_LAUNCH_CHAIN((norm_gate4_kernel<T, 1, 256>), grid, dim3(256), 0, stream, o, gate, ldg, w, eps, groups, L, out);
-    else if (L <= 3072) PLZ_LAUNCH_CHAIN((norm_gate4_kernel<T, 3, 256>), grid, dim3(256), 0, stream, o, gate, ldg, w, eps, groups, L, out);
-    else PLZ_LAUNCH_CHAIN((norm_gate4_kernel<T, 4, 256>), grid, dim3(256), 0, stream, o, gate, ldg, w, eps, groups, L, out);
+    if (L <= 128) PLZ_LAUNCH_CHAIN_BEHIND((norm_gate4_kernel<T, 1, 32>), grid, dim3(256), 0, stream, o, gate, ldg, w, eps, groups, L, out);
+    else if (L <= 256) PLZ_LAUNCH_CHAIN_BEHIND((norm_gate4_kernel<T, 2, 32>), grid, dim3(256), 0, stream, o, gate, ldg, w, eps, groups, L, out);
+    else if (L <= 1024) PLZ_LAUNCH_CHAIN_BEHIND((norm_gate4_kernel<T, 1, 256>), grid, dim3(256), 0, stream, o, gate, ldg, w, eps, groups, L, out);
+    else if (L <= 3072) PLZ_LAUNCH_CHAIN_BEHIND((norm_gate4_kernel<T, 3, 256>), grid, dim3(256), 0, stream, o, gate, ldg, w, eps, groups, L, out);
+    else PLZ_LAUNCH_CHAIN_BEHIND((norm_gate4_kernel<T, 4, 256>), grid, dim3(256), 0, stream, o, gate, ldg, w, eps, groups, L, out);
     return PLZ_OK;
 }
 int launch_seq_norm_gate(int dtype, const float* o, const void* gate, long long ldg, const float* w, float eps, long long rows, int groups, int L,
@@ -777,15 +777,15 @@ int launch_delta_prep(int dtype, const DeltaPrepArgs& a, cudaStream_t stream) {
                        a.off_q % 4 == 0 && a.off_k % 4 == 0 && a.off_v % 4 == 0 && !(((uintptr_t)a.proj | (uintptr_t)a.a | (uintptr_t)a.conv | (uintptr_t)a.q | (uintptr_t)a.k | (uintptr_t)a.v | (uintptr_t)a.logg) & 15);
     if (rows4) {
         const dim3 g4((unsigned)((long long)a.B * ((a.n + kPrepRows - 1) / kPrepRows)), grid.y);
-        if (dtype == 1) PLZ_LAUNCH_CHAIN(delta_prep_rows_kernel<float>, g4, dim3(256), 0, stream, p);
-        else PLZ_LAUNCH_CHAIN(delta_prep_rows_kernel<bf>, g4, dim3(256), 0, stream, p);
+        if (dtype == 1) PLZ_LAUNCH_CHAIN_BEHIND(delta_prep_rows_kernel<float>, g4, dim3(256), 0, stream, p);
+        else PLZ_LAUNCH_CHAIN_BEHIND(delta_prep_rows_kernel<bf>, g4, dim3(256), 0, stream, p);
     } else if (dtype == 1) PLZ_LAUNCH_CHAIN(delta_prep_kernel<float>, grid, dim3(256), 0, stream, p);
     else PLZ_LAUNCH_CHAIN(delta_prep_kernel<bf>, grid, dim3(256), 0, stream, p);
     if (a.n > 1 && a.n_taps > 1) {
         const int qk = a.G * a.dk, C = 2 * qk + a.H * a.dv;
         const dim3 g2((C + 255) / 256, a.B);
-        if (dtype == 1) PLZ_LAUNCH_CHAIN(conv_state_kernel<float>, g2, dim3(256), 0, stream, (const float*)a.proj, a.ldp, a.off_q, a.off_k, a.off_v, qk, C, a.n_taps - 1, a.n, (float*)a.conv);
-        else PLZ_LAUNCH_CHAIN(conv_state_kernel<bf>, g2, dim3(256), 0, stream, (const bf*)a.proj, a.ldp, a.off_q, a.off_k, a.off_v, qk, C, a.n_taps - 1, a.n, (bf*)a.conv);
+        if (dtype == 1) PLZ_LAUNCH_CHAIN_BEHIND(conv_state_kernel<float>, g2, dim3(256), 0, stream, (const float*)a.proj, a.ldp, a.off_q, a.off_k, a.off_v, qk, C, a.n_taps - 1, a.n, (float*)a.conv);
+        else PLZ_LAUNCH_CHAIN_BEHIND(conv_state_kernel<bf>, g2, dim3(256), 0, stream, (const bf*)a.proj, a.ldp, a.off_q, a.off_k, a.off_v, qk, C, a.n_taps - 1, a.n, (bf*)a.conv);
     }
     return PLZ_OK;
 }
@@ -802,11 +802,11 @@ int launch_attn_prep(int dtype, const AttnPrepArgs& a, cudaStream_t stream) {
         const bool narrow = p.qw <= 2048 && p.kw <= 2048;
         const dim3 grid((unsigned)rows), block(256);
         if (dtype == 1) {
-            if (narrow) PLZ_LAUNCH_CHAIN((attn_prep4_kernel<float, 2>), grid, block, 0, stream, p);
-            else PLZ_LAUNCH_CHAIN((attn_prep4_kernel<float, 4>), grid, block, 0, stream, p);
+            if (narrow) PLZ_LAUNCH_CHAIN_BEHIND((attn_prep4_kernel<float, 2>), grid, block, 0, stream, p);
+            else PLZ_LAUNCH_CHAIN_BEHIND((attn_prep4_kernel<float, 4>), grid, block, 0, stream, p);
         } else {
-            if (narrow) PLZ_LAUNCH_CHAIN((attn_prep4_kernel<bf, 2>), grid, block, 0, stream, p);
-            else PLZ_LAUNCH_CHAIN((attn_prep4_kernel<bf, 4>), grid, block, 0, stream, p);
+            if (narrow) PLZ_LAUNCH_CHAIN_BEHIND((attn_prep4_kernel<bf, 2>), grid, block, 0, stream, p);
+            else PLZ_LAUNCH_CHAIN_BEHIND((attn_prep4_kernel<bf, 4>), grid, block, 0, stream, p);
         }
         return PLZ_OK;
     }

@@ -65,6 +65,8 @@ scan_kernel(const ScanArgs p, StatusWord* status) {
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem = *tmem_slot;
+    pdl_wait();
+    pdl_launch_dependents();
 
     if (warp == 9) {
         if (lane == 0) {
@@ -252,8 +254,7 @@ int launch_t(const ScanArgs& a, cudaStream_t stream) {
     int dev = 0;
     PLZ_CUDA_CHECK(cudaGetDevice(&dev));
     if (!once[dev & 63]) { PLZ_CUDA_CHECK(cudaFuncSetAttribute((scan_kernel<KB, HASW>), cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM)); once[dev & 63] = true; }
-    scan_kernel<KB, HASW><<<dim3((a.dv + 127) / 128, a.H, a.B), kScanThreads, C::SMEM, stream>>>(a, device_status_ptr());
-    PLZ_LAUNCH_CHECK();
+    PLZ_LAUNCH_BEHIND((scan_kernel<KB, HASW>), dim3((a.dv + 127) / 128, a.H, a.B), dim3(kScanThreads), C::SMEM, stream, a, device_status_ptr());
     return PLZ_OK;
 }
 

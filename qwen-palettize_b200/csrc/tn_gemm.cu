@@ -186,6 +186,7 @@ tn_gemm_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant__ 
     if (PAIR) cluster_sync_all();   // both CTAs' barriers exist before anyone arrives on the partner's
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
+    pdl_wait();                     // and no launch of dependents: gradients, and the indices it may write, are read as weights
 
     // tile -> (split, i tile, j tile); i fastest so that one wave of CTAs covers every i tile
     // item -> (split, i tile, j tile, first column inside the tile, columns); i fastest so that one wave of CTAs
@@ -851,11 +852,12 @@ static int launch_tn_t(const TnArgs& a, const TnParams& p, const CUtensorMap& tm
     cfg.blockDim = dim3(tn_threads(EW));
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
+    cfg.attrs = attr; cfg.numAttrs = behind_attr(stream, attr);
     if (PAIR) {
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-        cfg.attrs = attr; cfg.numAttrs = 1;
+        attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+        attr[cfg.numAttrs].val.clusterDim.x = 2; attr[cfg.numAttrs].val.clusterDim.y = 1; attr[cfg.numAttrs].val.clusterDim.z = 1;
+        ++cfg.numAttrs;
     }
     PLZ_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kern, tmP, tmQ, tmS0, tmS1, p));
     ++g_launch_count;

@@ -221,6 +221,7 @@ __global__ void __launch_bounds__(256)
 swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ gate, long long ldg, const __nv_bfloat16* __restrict__ up, long long ldu,
                   const __nv_bfloat16* __restrict__ dact, long long ldd, int M, int N, __nv_bfloat16* __restrict__ dgate,
                   long long lddg, __nv_bfloat16* __restrict__ dup, long long lddu) {
+    pdl_launch_dependents();
     const int vec_per_row = N >> 3;
     const long long total = (long long)M * vec_per_row;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
@@ -274,6 +275,7 @@ __global__ void __launch_bounds__(256)
 rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, const __nv_bfloat16* __restrict__ dh, long long lddh,
                    const float* __restrict__ rstd, const __nv_bfloat16* __restrict__ g, int M, int K,
                    __nv_bfloat16* __restrict__ dx, long long lddx, float* __restrict__ dg) {
+    pdl_launch_dependents();
     __shared__ float red[8];
     const int t = threadIdx.x, lane = t & 31, wib = t >> 5;
     float gk[kNormPairs][2], acc[kNormPairs][2];
@@ -336,6 +338,7 @@ constexpr int kNorm8MaxK = 8192;
 __global__ void __launch_bounds__(1024)
 rmsnorm_bwd8_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, const __nv_bfloat16* __restrict__ dh, long long lddh, const float* __restrict__ rstd,
                     const __nv_bfloat16* __restrict__ g, int M, int K, __nv_bfloat16* __restrict__ dx, long long lddx, float* __restrict__ dg) {
+    pdl_launch_dependents();
     __shared__ float2 red[2][32];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, n_warps = blockDim.x >> 5, c = threadIdx.x * 8;
     const bool in = c < K;
@@ -460,6 +463,8 @@ struct ZeroParams { uint4* p[4]; long long bytes[4]; };
 __global__ void __launch_bounds__(256)
 zero_kernel(const ZeroParams z) {
     const long long first = (long long)blockIdx.x * 256 + threadIdx.x, step = (long long)gridDim.x * 256;
+    pdl_wait();
+    pdl_launch_dependents();
 #pragma unroll
     for (int b = 0; b < 4; ++b) {
         const long long units = z.bytes[b] >> 4;
@@ -480,8 +485,7 @@ int launch_zero(void* const* ptrs, const long long* bytes, int count, cudaStream
     long long blocks = (most / 16 + 255) / 256;
     const long long cap = (long long)sm_count_of_current_device() * 8;
     if (blocks < 1) blocks = 1;
-    zero_kernel<<<(unsigned)(blocks < cap ? blocks : cap), 256, 0, stream>>>(z);
-    PLZ_LAUNCH_CHECK();
+    PLZ_LAUNCH_BEHIND(zero_kernel, dim3((unsigned)(blocks < cap ? blocks : cap)), dim3(256), 0, stream, z);
     return PLZ_OK;
 }
 
