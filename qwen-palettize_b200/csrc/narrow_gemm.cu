@@ -27,13 +27,13 @@ namespace plz {
 namespace {
 
 constexpr int kNgMaxMats = 4;
-constexpr int kNgDecodeWarps = 8;                 // two groups of 128 threads, blocks alternate between them
+constexpr int kNgDecodeWarps = 8;                 // two groups of 128 threads, pairs of blocks alternate between them
 constexpr uint32_t kNgWBytes = 128 * 64 * 2;
 // shared memory of the stages; two CTAs per SM. LUT: four x tiles of 128 tokens and the W tile of the extra block
 template <bool LUT>
 constexpr uint32_t kNgRingBytes = LUT ? 80 * 1024 : 96 * 1024;
 constexpr int kNgMaxStages = 16;                  // slots for copies
-constexpr int kNgMaxW = 8;                        // blocks of decoded W in TMEM
+constexpr int kNgMaxW = 3;                        // pairs of blocks of decoded W in TMEM
 constexpr uint32_t kNgBarBytes = 512;
 constexpr int kNgAhead = 4;                       // blocks of packed indices a decode thread has in flight
 
@@ -43,7 +43,7 @@ struct NarrowMat {
     void* y; long long ldy;
 };
 struct NarrowParams {
-    int M, npad, n_acc, stages, w_stages;   // slots for copies (dense: W and x, LUT: x), LUT: blocks of W in TMEM
+    int M, npad, n_acc, stages, w_stages;   // slots for copies (dense: W and x of a block; LUT: x of two blocks, a power of two of them), LUT: pairs of blocks of W in TMEM
     int x_mn, transposed;
     uint32_t x_bytes;              // of a tile of x
     uint32_t tmem_cols;
@@ -85,15 +85,14 @@ narrow_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
     const uint32_t raw = smem_u32(smem_raw);
     const uint32_t base = (raw + 1023u) & ~1023u;
     uint8_t* smem = smem_raw + (base - raw);
-    // dense: a stage is a W tile and an x tile; LUT: x tiles, behind them one W tile for the extra block (W is decoded to TMEM)
-    const uint32_t x_bytes = p.x_bytes, stage_bytes = (LUT ? 0u : kNgWBytes) + x_bytes;
-    const uint32_t w2_off = LUT ? (uint32_t)p.stages * x_bytes : 0u;
+    // dense: a stage is a W tile and an x tile; LUT: the x tiles of two blocks, behind the stages one W tile for the extra block (W is decoded to TMEM)
+    const uint32_t x_bytes = p.x_bytes, stage_bytes = LUT ? 2u * x_bytes : kNgWBytes + x_bytes;
+    const uint32_t w2_off = LUT ? (uint32_t)p.stages * stage_bytes : 0u;
     const uint32_t bar_off = kNgRingBytes<LUT>;
     auto full = [&](int s) { return base + bar_off + 8u * s; };
     auto empty = [&](int s) { return base + bar_off + 8u * (kNgMaxStages + s); };
-    auto full_w = [&](int s) { return base + bar_off + 8u * (2 * kNgMaxStages + s); };             // LUT only
-    auto empty_w = [&](int s) { return base + bar_off + 8u * (2 * kNgMaxStages + kNgMaxW + s); };
-    constexpr int kBars = 2 * kNgMaxStages + 2 * kNgMaxW + 1;
+    auto empty_w = [&](int s) { return base + bar_off + 8u * (2 * kNgMaxStages + s); };            // LUT only
+    constexpr int kBars = 2 * kNgMaxStages + kNgMaxW + 1;
     static_assert(8 * kBars + 8 <= kNgBarBytes, "barriers");
     const uint32_t acc_full = base + bar_off + 8u * (kBars - 1);
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem + bar_off + 8 * kBars);
@@ -113,20 +112,26 @@ narrow_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
     const int b_begin = (int)((long long)rank * p.n_blocks / n_ranks), b_end = (int)((long long)(rank + 1) * p.n_blocks / n_ranks);
     const int nb = b_end - b_begin;        // at least one: the cluster is no larger than the number of blocks
 
-    // the bytes of both copies of a stage are announced with the first one
-    auto load_w = [&](int it, int s) {
-        const int b = b_begin + it;
-        const bool extra = b >= p.nkb, by_tma = !LUT || extra;
-        mbar_arrive_expect_tx(full(s), x_bytes + (by_tma ? kNgWBytes : 0u));
+    // Steps: a block (dense), or a pair of blocks (LUT). What the issuing warp does once per step (a wait, the election, the commits: 470 clocks beside the 90 that four
+    // MMAs take) and what a decoding group does once (waits, the store's completion, an arrival: 450 beside 430 of decoding) made 650 clocks a block. By blocks / by pairs, 64 rows in a row of
+    // launches, us: 19456 x 2560 23.6 / 20.4, 12288 x 4096 19.4 / 17.4, 9728 x 2560 12.6 / 11.0, 2560 x 9728 14.6 / 12.7.
+    const int steps = LUT ? (nb + 1) >> 1 : nb;
+    // the bytes of all copies of a stage are announced with the first one
+    auto load_w = [&](int st, int s) {
+        const int b = b_begin + (LUT ? 2 * st : st), n = LUT && 2 * st + 1 < nb ? 2 : 1;
+        const bool extra = b + n > p.nkb, by_tma = !LUT || extra;
+        mbar_arrive_expect_tx(full(s), n * x_bytes + (by_tma ? kNgWBytes : 0u));
         if (by_tma) tma_load_2d(base + (LUT ? w2_off : s * stage_bytes), extra ? &tmW2 : &tmW, full(s), extra ? 0 : b * 64, n0);
     };
-    auto load_x = [&](int it, int s) {
-        const int b = b_begin + it;
+    auto load_x = [&](int st, int s) {
+        const int b = b_begin + (LUT ? 2 * st : st);
         const bool extra = b >= p.nkb;
         const bool mn = !LUT && p.x_mn;
-        tma_load_2d(base + s * stage_bytes + (LUT ? 0u : kNgWBytes), extra ? &tmX2 : &tmX, full(s), extra || mn ? 0 : b * 64, mn ? b * 64 : 0);
+        const uint32_t to = base + s * stage_bytes + (LUT ? 0u : kNgWBytes);
+        tma_load_2d(to, extra ? &tmX2 : &tmX, full(s), extra || mn ? 0 : b * 64, mn ? b * 64 : 0);
+        if (LUT && 2 * st + 1 < nb) tma_load_2d(to + x_bytes, b + 1 >= p.nkb ? &tmX2 : &tmX, full(s), b + 1 >= p.nkb ? 0 : (b + 1) * 64, 0);
     };
-    const int pre = nb < p.stages ? nb : p.stages;
+    const int pre = steps < p.stages ? steps : p.stages;
 
     // weights do not depend on the previous kernel and do not wait for this block's own set-up either
     constexpr int kAhead = LUT ? kNgAhead : 1;
@@ -150,18 +155,16 @@ narrow_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
         }
     };
     if (LUT && warp >= 2) {
+        if (!p.early) pdl_wait();
 #pragma unroll
-        for (int j = 0; j < kAhead; ++j) fetch(grp + 2 * j, j);
+        for (int j = 0; j < kAhead; ++j) fetch(4 * (j >> 1) + 2 * grp + (j & 1), j);
     }
     if (threadIdx.x == 0) {
         for (int s = 0; s < kNgMaxStages; ++s) {
-            mbar_init(full(s), 1);
+            mbar_init(full(s), LUT ? 1 + kNgDecodeWarps / 2 : 1);    // LUT: the copies and the decoded weights
             mbar_init(empty(s), 1);
         }
-        for (int s = 0; LUT && s < kNgMaxW; ++s) {
-            mbar_init(full_w(s), kNgDecodeWarps / 2);
-            mbar_init(empty_w(s), 1);
-        }
+        for (int s = 0; LUT && s < kNgMaxW; ++s) mbar_init(empty_w(s), 1);
         mbar_init(acc_full, 1);
         *abort_flag = 0;
         mbar_fence_init();
@@ -185,7 +188,7 @@ narrow_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
         if (lane == 0) {
             pdl_wait();
             for (int it = 0; it < pre; ++it) load_x(it, it);
-            for (int it = pre; it < nb; ++it) {
+            for (int it = pre; it < steps; ++it) {
                 const int s = it % p.stages;
                 if (!mbar_wait(empty(s), ((it / p.stages) & 1) ^ 1u, abort_flag, p.status, ST_TIMEOUT_EMPTY, 0)) break;
                 load_w(it, s);
@@ -205,67 +208,93 @@ narrow_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
                        d3 = p.n_acc > 2 ? tmem_base + 3u * (uint32_t)p.npad : d1;
         bool ok = true;
         int s = 0, iw = 0;
-        uint32_t ph = 0, phw = 0, lo = lo0;
+        uint32_t ph = 0, lo = lo0;
+        // a block: accumulators start with their first MMA
+        auto block = [&](bool from_tmem, uint32_t wt, uint32_t wd, uint32_t xd, uint32_t first) {
+            const uint32_t m1 = p.n_acc > 1 ? first : 1u, m2 = p.n_acc > 2 ? first : 1u;
+            if (from_tmem) {
+                umma_ts(tmem_base, wt, xd, hi, idesc, first);
+                umma_ts(d1, wt + 8u, xd + 2u, hi, idesc, m1);
+                umma_ts(d2, wt + 16u, xd + 4u, hi, idesc, m2);
+                umma_ts(d3, wt + 24u, xd + 6u, hi, idesc, m2);
+            } else {
+                umma_bf16_words<1>(tmem_base, wd, hi, xd, hi, idesc, first);
+                umma_bf16_words<1>(d1, wd + 2u, hi, xd + x_step, hi, idesc, m1);
+                umma_bf16_words<1>(d2, wd + 4u, hi, xd + 2u * x_step, hi, idesc, m2);
+                umma_bf16_words<1>(d3, wd + 6u, hi, xd + 3u * x_step, hi, idesc, m2);
+            }
+        };
         pdl_wait();
-        for (int it = 0; it < nb; ++it) {
-            ok = mbar_wait(full(s), ph, abort_flag, p.status, ST_TIMEOUT_FULL, 1);
-            if (LUT && ok) ok = mbar_wait(full_w(iw), phw, abort_flag, p.status, ST_TIMEOUT_FULL, 1);
-            ok = __all_sync(0xFFFFFFFFu, ok);
+        for (int st = 0; st < steps; ++st) {
+            ok = mbar_wait_warp(full(s), ph, abort_flag, p.status, ST_TIMEOUT_FULL, 1);
             if (!ok) break;
             tc_fence_after_sync();
-            const bool from_tmem = LUT && b_begin + it < p.nkb;
-            const uint32_t xd = lo + x_off, wd = LUT ? lo0 + (w2_off >> 4) : lo, wt = tmem_w + iw * 32u;
-            const uint32_t first = it > 0 ? 1u : 0u;             // accumulators start with their first MMA
-            const uint32_t m1 = p.n_acc > 1 ? first : 1u, m2 = p.n_acc > 2 ? first : 1u;
-            if (elect_one()) {
-                if (from_tmem) {
-                    umma_ts(tmem_base, wt, xd, hi, idesc, first);
-                    umma_ts(d1, wt + 8u, xd + 2u, hi, idesc, m1);
-                    umma_ts(d2, wt + 16u, xd + 4u, hi, idesc, m2);
-                    umma_ts(d3, wt + 24u, xd + 6u, hi, idesc, m2);
-                } else {
-                    umma_bf16_words<1>(tmem_base, wd, hi, xd, hi, idesc, first);
-                    umma_bf16_words<1>(d1, wd + 2u, hi, xd + x_step, hi, idesc, m1);
-                    umma_bf16_words<1>(d2, wd + 4u, hi, xd + 2u * x_step, hi, idesc, m2);
-                    umma_bf16_words<1>(d3, wd + 6u, hi, xd + 3u * x_step, hi, idesc, m2);
+            if (LUT) {
+                const int b = b_begin + 2 * st;
+                const uint32_t wt = tmem_w + iw * 64u, w2 = lo0 + (w2_off >> 4);
+                if (b + 1 < p.nkb && 2 * st + 1 < nb) {
+                    if (elect_one()) {
+                        block(true, wt, 0u, lo, st > 0 ? 1u : 0u);
+                        block(true, wt + 32u, 0u, lo + (x_bytes >> 4), 1u);
+                        umma_commit(empty(s));
+                        umma_commit(empty_w(iw));
+                    }
+                } else if (elect_one()) {           // the last step: one block, or the extra one
+                    block(b < p.nkb, wt, w2, lo, st > 0 ? 1u : 0u);
+                    if (2 * st + 1 < nb) block(b + 1 < p.nkb, wt + 32u, w2, lo + (x_bytes >> 4), 1u);
+                    umma_commit(empty(s));
+                    umma_commit(empty_w(iw));
                 }
+                if (++iw == p.w_stages) iw = 0;
+            } else if (elect_one()) {
+                block(false, 0u, lo, lo + x_off, st > 0 ? 1u : 0u);
                 umma_commit(empty(s));
-                if (LUT) umma_commit(empty_w(iw));
             }
             __syncwarp();
             lo += slot;
             if (++s == p.stages) { s = 0; ph ^= 1u; lo = lo0; }
-            if (LUT && ++iw == p.w_stages) { iw = 0; phw ^= 1u; }
         }
         if (ok && elect_one()) umma_commit(acc_full);
         __syncwarp();
     } else {
         bool ok = true;
         if (LUT) {
-            // ------------------------------------------------------ decode; the two groups of four warps take blocks in turn
-            for (int it0 = grp; it0 < nb && ok; it0 += 2 * kAhead) {
+            // ------------------------------------------------------ decode: the two groups of four warps take pairs of blocks in turn
+            const uint32_t lanes = tmem_w + ((uint32_t)((warp & 3) * 32) << 16);
+            int iw = grp;
+            uint32_t phw = 1;                       // the slots are free at first
+            for (int st0 = grp; st0 < steps && ok; st0 += kAhead) {
 #pragma unroll
-                for (int j = 0; j < kAhead; ++j) {
-                    const int it = it0 + 2 * j;
-                    if (it >= nb || !ok) continue;
-                    const int s = it % p.w_stages;       // an even number of blocks: a group always writes the same ones
-                    if (it >= p.w_stages) pdl_wait();
-                    ok = mbar_wait(empty_w(s), ((it / p.w_stages) & 1) ^ 1u, abort_flag, p.status, ST_TIMEOUT_EMPTY, 3);
+                for (int j = 0; j < kAhead; j += 2) {
+                    const int st = st0 + j, it = 2 * st;
+                    if (st >= steps || !ok) continue;
+                    if (st >= 2 && st < 4) pdl_wait();
+                    uint32_t o[32];
+                    auto decode = [&](int i) {
+                        const PalRegs pl = pal_split(pr[i].x, pr[i].y);
+                        decode16(w[i].x, pl, o);
+                        decode16(w[i].y, pl, o + 8);
+                        decode16(w[i].z, pl, o + 16);
+                        decode16(w[i].w, pl, o + 24);
+                    };
+                    if (it < nw) decode(j);
+                    fetch(it + 2 * kAhead, j);
+                    ok = mbar_wait_warp(empty_w(iw), phw, abort_flag, p.status, ST_TIMEOUT_EMPTY, 3);
                     if (!ok) continue;
-                    if (it < nw) {
-                        uint32_t o[32];
-                        const PalRegs pl = pal_split(pr[j].x, pr[j].y);
-                        decode16(w[j].x, pl, o);
-                        decode16(w[j].y, pl, o + 8);
-                        decode16(w[j].z, pl, o + 16);
-                        decode16(w[j].w, pl, o + 24);
-                        fetch(it + 2 * kAhead, j);
-                        tc_fence_after_sync();
-                        tmem_st_32x32(tmem_w + ((uint32_t)((warp & 3) * 32) << 16) + s * 32u, o);
-                        tc_fence_before_sync();
+                    const uint32_t to = lanes + iw * 64u;
+                    tc_fence_after_sync();
+                    if (it < nw) tmem_st_32x32_begin(to, o);
+                    if (it + 1 < nw) {
+                        decode(j + 1);
+                        tmem_st_32x32_begin(to + 32u, o);
                     }
+                    fetch(it + 1 + 2 * kAhead, j + 1);
+                    tmem_wait_st();
+                    tc_fence_before_sync();
                     __syncwarp();
-                    if (lane == 0) mbar_arrive(full_w(s));
+                    if (lane == 0) mbar_arrive(full(st & (p.stages - 1)));
+                    iw += 2;
+                    if (iw >= p.w_stages) { iw -= p.w_stages; phw ^= 1u; }
                 }
             }
         }
@@ -457,6 +486,26 @@ int cluster_size(int tiles, int blocks, int sms, int fixed) {
     return best;
 }
 
+// The same for packed W, whose blocks come out of a CTA at 0.25 us: start, sum and end are 14 of them, 18 in clusters of more than four, which moreover share SMs
+// from about three fifths of one CTA per SM on; pairs fill every place; and without clusters one SM with two CTAs sets the time. us at 64 rows in a row of launches, by clusters
+// of 1 / 2 / 3 / 4 / 6 / 8: 2560 x 2560 13.4 / 8.5 / 7.8 / 6.6 / 7.3 / 7.7, x 9728 39 / 21 / 18 / 15.6 / 13.4 / 12.7, 4096 x 4096 19 / 11.8 / 10.5 / 9.4 / 10.3 / 10.8, 6144 x 2560 13.9 / 9.3 /
+// 9.4 / 8.8 / 15 / 16, 9728 x 2560 14.3 / 11.5 / 10.9 / 15 / 18 / 23, 18944 x 2560 (148 tiles) 15.4 / 14.4 / 21 / 24 / 34 / 41, 19456 x 2560 (152) 20.4 / 20.7 / 21 / 25 / 35 / 42.
+int cluster_size_packed(int tiles, int blocks, int sms) {
+    int best = 1;
+    double best_cost = 0;
+    for (int c = 1; c <= 8; ++c) {
+        if (c > 1 && blocks / c < 2) break;
+        if (c == 5 || c == 7) continue;
+        const long long ctas = (long long)tiles * c, places = c <= 2 ? 2 * sms : 2 * sms * 9 / 10;
+        const double alone = c > 4 ? 0.6 * sms : sms;
+        double shared = ctas <= alone ? 0.0 : ctas >= alone + sms ? 1.0 : (ctas - alone) / sms;
+        if (c == 1 && shared > 0.0) shared = 1.0;
+        const double cost = (double)((ctas + places - 1) / places) * ((blocks + c - 1) / c + (c > 4 ? 18 : 14)) * (1.0 + 0.3 * shared);
+        if (c == 1 || cost < best_cost) { best = c; best_cost = cost; }
+    }
+    return best;
+}
+
 // Parts of the reduction of a turned product: by the reduction alone, so that a row's result does not depend on how many rows there are (a step over
 // all tokens and the sum of steps over parts of them then agree); eight to twenty blocks per part.
 int turned_parts(int n_blocks) { return n_blocks >= 64 ? 8 : n_blocks >= 32 ? 4 : n_blocks >= 16 ? 2 : 1; }
@@ -500,9 +549,9 @@ int launch_narrow_gemm(const NarrowArgs& a, cudaStream_t stream) {
     p.x_mn = a.x_mn; p.transposed = a.transposed;
     p.x_bytes = a.x_mn ? 64u * 128u : (uint32_t)p.npad * 128u;       // x_mn: 64 reduction rows of 64 columns
     if (lut) {      // 256 TMEM columns: accumulators, then 32 columns per stage
-        p.n_acc = p.npad <= 32 ? 4 : p.npad == 64 ? 2 : 1;
-        p.w_stages = (256 - p.n_acc * p.npad) / 32;                              // 4 or 6
-        p.stages = (int)((kNgRingBytes<true> - kNgWBytes) / p.x_bytes);      // behind them the W tile of the extra block
+        p.n_acc = p.npad == 16 ? 4 : p.npad == 32 ? 2 : 1;
+        p.w_stages = (256 - p.n_acc * p.npad) / 64;                              // 3, or 2 beyond 64 rows: never more than the slots for copies
+        p.stages = (int)((kNgRingBytes<true> - kNgWBytes) / (2u * p.x_bytes));   // 2 to 16, behind them the W tile of the extra block
         p.tmem_cols = 256;
         p.group_blocks = a.gs_k / 64; p.group_shift = -1;
         for (int i = 0; i < 16; ++i) if (p.group_blocks == 1 << i) p.group_shift = i;
@@ -538,7 +587,7 @@ int launch_narrow_gemm(const NarrowArgs& a, cudaStream_t stream) {
         if ((rc = make_tmap_bf16(&tm[2], a.x2, a.M, a.r2, a.ldx2, 64, (uint32_t)p.npad))) return rc;
         if ((rc = make_tmap_bf16(&tm[3], a.w2, a.mat[0].N, a.r2, a.ldw2, 64, 128))) return rc;
     }
-    const int ranks = a.transposed ? turned_parts(p.n_blocks) : cluster_size(tiles, p.n_blocks, seq_sm_count(), 12);
+    const int ranks = a.transposed ? turned_parts(p.n_blocks) : lut ? cluster_size_packed(tiles, p.n_blocks, seq_sm_count()) : cluster_size(tiles, p.n_blocks, seq_sm_count(), 12);
     p.early = g_smallm_overlap && a.early && !a.transposed;       // else W may be what the previous kernel writes
     return lut ? launch_ng<true>(p, tiles, ranks, tm, stream) : launch_ng<false>(p, tiles, ranks, tm, stream);
 }
