@@ -34,6 +34,7 @@ struct TcParams {
     float scale_log2e;
     const float* bias; long long ldb; int n_bias; const float* bias_top;
     int sink; const float* sinks;
+    int heads_first;
     const __nv_bfloat16* gate; long long ldg; int dv;
     StatusWord* status;
 };
@@ -237,10 +238,12 @@ attn_bias_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     const int warp = __shfl_sync(0xFFFFFFFFu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;   // uniform to the compiler too
     const int n_qt = (p.n + kT - 1) / kT;
     const int n_pairs = (n_qt + 1) / 2;
-    const int pi = n_pairs - 1 - (int)blockIdx.x;   // heavy pairs first
+    // heavy pairs first: over all heads where the CTAs make more than a wave, else within a head, whose pairs then share keys and values in L2
+    const int heads = gridDim.x / n_pairs, order = (int)blockIdx.x;
+    const int pi = n_pairs - 1 - (p.heads_first ? order / heads : order % n_pairs), hb = p.heads_first ? order % heads : order / n_pairs;
     const int qtA = 2 * pi, qtB = 2 * pi + 1;
     const bool hasB = qtB < n_qt;
-    const int h = blockIdx.y, b = blockIdx.z;
+    const int h = hb % p.H, b = hb / p.H;
     const int hk = h / (p.H / p.G);
     auto kv_tiles = [&](int qt) { return (p.pos + min(p.n, (qt + 1) * kT) + kT - 1) / kT; };
     const int n_kvA = kv_tiles(qtA);
@@ -372,7 +375,11 @@ int launch_t(const AttnBiasArgs& a, cudaStream_t stream) {
     PLZ_CUDA_CHECK(cudaGetDevice(&dev));
     if (!once[dev & 63]) { PLZ_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM)); once[dev & 63] = true; }
     const int n_qt = (a.n + kT - 1) / kT;
-    PLZ_LAUNCH_BEHIND(kern, dim3((n_qt + 1) / 2, a.H, a.B), dim3(kThreads), C::SMEM, stream, tmQ, tmK, tmV, tmO, tmQ2, tmK2, p);
+    const long long ctas = (long long)(n_qt + 1) / 2 * a.H * a.B;
+    if (ctas > 0x7FFFFFFF) { set_last_error("attention: too many query tiles"); return PLZ_ERR_TOO_LARGE; }
+    // us by pairs of a head / by heads: 4 x 1024 tokens, 32 heads over 8, 82 / 71; 2048, 20 heads (160 CTAs) 56 / 49; one wave: 2048, 16 heads over 2 of 64 48.5 / 51.7
+    p.heads_first = ctas > seq_sm_count();
+    PLZ_LAUNCH_BEHIND(kern, dim3((unsigned)ctas), dim3(kThreads), C::SMEM, stream, tmQ, tmK, tmV, tmO, tmQ2, tmK2, p);
     return PLZ_OK;
 }
 

@@ -49,3 +49,18 @@ def test_scores_that_grow_along_the_sequence(S, growth):
     s = s.masked_fill(~torch.ones(S, S, dtype=torch.bool, device="cuda").tril(), float("-inf"))
     assert_close(o, (torch.softmax(s, -1) @ v.double()).transpose(0, 1).reshape(S, Hq * D).float(), "o")
     assert_close(lse, torch.logsumexp(s, -1).float().view(B, Hq, S), "log-sum-exp", rel=1e-3)
+
+
+@pytest.mark.parametrize("B,n,pos", [(1, 300, 0), (3, 300, 0), (3, 520, 70)])      # 64, 192 and 288 CTAs: within a wave and beyond
+def test_order_of_the_query_tiles(B, n, pos):
+    import seq_ops as S
+    H, G, d, T, g = 32, 8, 64, pos + n, torch.Generator(device="cuda").manual_seed(n + B)
+    q, k, v = (torch.randn(B, t, h * d, generator=g, device="cuda").bfloat16() for t, h in ((n, H), (T, G), (T, G)))
+    tab = torch.randn(H, 100, generator=g, device="cuda")
+    o = S.attention_bias(q.view(B * n, H * d), k, v, S.DistanceBias.from_distances(tab), torch.tensor([pos], dtype=torch.int32, device="cuda"), pos, B, n, H, G, d, d, d ** -0.5, True)
+    check_status()
+    kf, vf = (t.double().view(B, T, G, d).repeat_interleave(H // G, 2) for t in (k, v))
+    at = torch.arange(pos, T, device="cuda")[:, None] - torch.arange(T, device="cuda")
+    s = torch.einsum("bihd,bjhd->bhij", q.double().view(B, n, H, d), kf) * d ** -0.5 + tab.double()[:, at.clamp(0, 99)]
+    s = torch.cat([s.masked_fill(at < 0, float("-inf")), torch.zeros_like(s[..., :1])], -1)
+    assert_close(o, torch.einsum("bhij,bjhd->bihd", torch.softmax(s, -1)[..., :-1], vf).reshape(B * n, H * d).float(), "o")
