@@ -56,8 +56,8 @@ class PalettizedQwen:
         """layers: list of dicts with the seven PackedWeight under LINEARS and bf16 vectors 'input_ln', 'post_ln', 'q_norm', 'k_norm'."""
         self.cfg, self.layers, self.embed, self.final_norm = cfg, layers, embed, final_norm
         self.cos, self.sin = ops.rope_tables(max_positions, cfg.head_dim, cfg.rope_theta, embed.device)
-        self.fused_mlp = False    # prefill: gate + up + SwiGLU as ONE single-CTA launch instead of two CTA-pair GEMMs + an element-wise
-                                  # pass; measured slower at 8 x 2048 tokens (4.0 against 3.4 ms per layer), so off
+        self.fused_mlp = False    # prefill: gate + up + SwiGLU as one single-CTA launch with the RMSNorm folded in; measured slower at 8 x 2048
+                                  # tokens (4.0 ms per layer against 3.4 of two CTA-pair products and a pass) than what prefill does, so off
 
     @classmethod
     def random(cls, cfg: ModelConfig, device, seed: int = 0, max_positions: int = 4096):
