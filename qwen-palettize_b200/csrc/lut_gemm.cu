@@ -655,10 +655,10 @@ static int launch_t(const LutGemmArgs& a, cudaStream_t stream) {
 // Products of at most 128 rows that a 128 x 256 tile per CTA serves as well as narrow_gemm.cu, whose start, sum over a cluster and end grow with the rows it
 // pads to (16, 32, 64, 128) and with the waves its 128-column tiles make: reductions of up to so many blocks of 64, by tiles that fill a quarter of the
 // chip / the chip / more. us here / there, 64 rows: dense 1024 x 256 5.9 / 7.6, x 512 6.9 / 6.8, x 2560 16 / 7.6; 9728 x 512 7.1 / 9.3, x 1536 11.7 / 11.2; packed 1024 x 128
-// 6.1 / 8.0, x 256 7.3 / 7.5, x 2560 31 / 8.5; 9728 x 512 10.4 / 10.9, x 1024 15.7 / 12.6; 128 rows: packed 24576 x 1536 22 / 25, x 2560 33 / 33. Up to 16 rows the kernels part at 128
+// 5.8 / 7.3, x 256 7.1 / 6.6, x 2560 31 / 7.6; 9728 x 384 8.4 / 8.8, x 512 10.0 / 8.9, x 1024 15.5 / 10.6; 19456 x 768 12.6 / 12.9, x 1024 15.6 / 14.3; 128 rows: packed 24576 x 1024 16.2 / 18.3, x 1536 21.3 / 21.1. Up to 16 rows the kernels part at 128
 // columns. Dense: also where the tiles alone fill the chip (32 rows and more) and, beyond 64 rows, wider outputs of reductions below 2048.
 static bool few_rows_short(const LutGemmArgs& a, bool decode, int sms) {
-    static const int dense_line[3][4] = {{2, 4, 6, 8}, {4, 8, 16, 32}, {4, 8, 32, 32}}, packed_line[3][4] = {{2, 2, 4, 4}, {4, 4, 8, 8}, {6, 10, 16, 28}};
+    static const int dense_line[3][4] = {{2, 4, 6, 8}, {4, 8, 16, 32}, {4, 8, 32, 32}}, packed_line[3][4] = {{2, 2, 3, 4}, {4, 4, 6, 8}, {6, 8, 13, 22}};
     const int tiles = (a.J + 127) / 128, wide = 4 * tiles <= sms ? 0 : tiles <= sms ? 1 : 2, pad = a.M <= 16 ? 0 : a.M <= 32 ? 1 : a.M <= 64 ? 2 : 3;
     if (!decode && ((a.M >= 32 && a.J >= 128 * sms) || (a.M > 64 && a.R < 2048 && a.J > 1024))) return true;
     return (a.R + 63) / 64 <= (decode ? packed_line : dense_line)[wide][pad];
