@@ -260,6 +260,9 @@ narrow_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
         bool ok = true;
         if (LUT) {
             // ------------------------------------------------------ decode: the two groups of four warps take pairs of blocks in turn
+            // The groups share three slots (two beyond 64 rows, then one each): a group that comes to a slot has, one of its steps before, waited for a product issued behind the
+            // slot's last but one use, so the barrier's parity tells the rounds apart. Three groups gain nothing (64 rows of 19456 x 2560 20.4 / 19.8 us, 6144 x 2560 8.8 / 9.0), and on two
+            // slots one of them could be a whole round ahead.
             const uint32_t lanes = tmem_w + ((uint32_t)((warp & 3) * 32) << 16);
             int iw = grp;
             uint32_t phw = 1;                       // the slots are free at first
