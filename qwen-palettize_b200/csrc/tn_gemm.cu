@@ -356,6 +356,11 @@ tn_gemm_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant__ 
         const int lane_group = warp & 3;
         const int col_part = (warp - 2) >> 2;
         const int ew = warp - 2;  // 0..EW - 1
+        // Places of this warp's columns in `red`, first the palettes that it works with, then its sums: its own whatever the width of the tile. Without a
+        // palette gradient no barrier keeps the warps of a lane group at the same tile, and one that came to a narrower part of a tile ahead of the others would
+        // otherwise write where they still read.
+        constexpr int kOwnCols = 256 / (EW / 4);
+        const int own_cols = lane_group * 256 + col_part * kOwnCols;
         bool ok = true;
         int lt = 0;
         // requests of the ring: the next kRingCols columns of this warp's part, on to the next tile behind the last one. They run ahead of the columns
@@ -430,12 +435,12 @@ tn_gemm_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant__ 
             m_range(sp, job, m_begin, nkb);
             const int buf = lt & 1;
             if (EPI == EPI_SOFT && ROWS_K && job < 0) {
-                // the palettes of this warp's columns, in the places of `red` that their partial sums take later
+                // the palettes of this warp's columns
                 const int part = c_num / (EW / 4), first = col_part * part, kgi = (ti * 128 < p.I ? ti * 128 : 0) / p.gs_k;
                 for (int c = lane; c < part; c += 32) {
                     const int n = tj * 256 + c_off + first + c;
                     const uint2 raw = n < p.J ? __ldg(reinterpret_cast<const uint2*>(p.palette + ((long long)n * p.n_kgroups + kgi) * 4)) : make_uint2(0u, 0u);
-                    *reinterpret_cast<float4*>(red + (lane_group * 256 + first + c) * 4) =
+                    *reinterpret_cast<float4*>(red + (own_cols + c) * 4) =
                         make_float4(__uint_as_float(raw.x << 16), __uint_as_float(raw.x & 0xFFFF0000u), __uint_as_float(raw.y << 16), __uint_as_float(raw.y & 0xFFFF0000u));
                 }
                 __syncwarp();
@@ -476,7 +481,7 @@ tn_gemm_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant__ 
                 // running address of the batch's first column
                 float* dcol = p.dlogits ? reinterpret_cast<float*>(p.dlogits) + (long long)k * p.ls_row + (long long)colbase * p.ls_col : nullptr;
                 if (EPI == EPI_SOFT && !row_ok) {     // all of a warp's rows are there or none
-                    for (int c = lane; c < wcols; c += 32) *reinterpret_cast<float4*>(red + (lane_group * 256 + col_part * wcols + c) * 4) = make_float4(0.f, 0.f, 0.f, 0.f);
+                    for (int c = lane; c < wcols; c += 32) *reinterpret_cast<float4*>(red + (own_cols + c) * 4) = make_float4(0.f, 0.f, 0.f, 0.f);
                 }
 #pragma unroll 1
                 for (int c0 = EPI == EPI_SOFT && !row_ok ? wcols : 0; c0 < wcols; c0 += kBatch) {
@@ -512,7 +517,7 @@ tn_gemm_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant__ 
                                 const bool valid = n < p.J;
                                 // rows and columns beyond the operands came as zeros, so their sums are zero
                                 const f32x2 dw = pair2(__uint_as_float(v[c]), __uint_as_float(v[c]));
-                                const ulonglong2 praw = *reinterpret_cast<const ulonglong2*>(red + (lane_group * 256 + col_part * wcols + c0 + c) * 4);
+                                const ulonglong2 praw = *reinterpret_cast<const ulonglong2*>(red + (own_cols + c0 + c) * 4);
                                 const f32x2 cp[2] = {praw.x, praw.y};
                                 if (p.pack_out != nullptr) {
                                     float l[4];
@@ -585,7 +590,7 @@ tn_gemm_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant__ 
                             for (int j = 0; j + 1 < h; j += 2) split2(add2(pair2(part[j], part[j + 1]), pair2(got[j], got[j + 1])), part[j], part[j + 1]);
                             if (h == 1) part[0] += got[0];
                         }
-                        if (lane % (32 / kVals) == 0) red[(lane_group * 256 + col_part * wcols + c0) * 4 + lane / (32 / kVals)] = part[0];
+                        if (lane % (32 / kVals) == 0) red[(own_cols + c0) * 4 + lane / (32 / kVals)] = part[0];
                     }
                     if (dcol != nullptr) dcol += kBatch * p.ls_col;
                 }
@@ -597,10 +602,11 @@ tn_gemm_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant__ 
                     const int k0 = ti * 128;
                     if (et < c_num && n < p.J && k0 < p.I) {
                         const long long pg = ((long long)n * p.n_kgroups + k0 / p.gs_k) * 4;
+                        const int at = et / wcols * kOwnCols + et % wcols;
 #pragma unroll
                         for (int q = 0; q < 4; ++q) {
-                            const float s = ((red[(0 * 256 + et) * 4 + q] + red[(1 * 256 + et) * 4 + q]) +
-                                             red[(2 * 256 + et) * 4 + q]) + red[(3 * 256 + et) * 4 + q];
+                            const float s = ((red[(0 * 256 + at) * 4 + q] + red[(1 * 256 + at) * 4 + q]) +
+                                             red[(2 * 256 + at) * 4 + q]) + red[(3 * 256 + at) * 4 + q];
                             atomicAdd(p.dpalette + pg + q, s);
                         }
                     }

@@ -57,6 +57,24 @@ def test_weight_gradient_writes_the_indices(M, N, K, limit, noise, rank):
         assert_close(db, dy.float().t() @ t.float(), "dB")
 
 
+# Without a palette gradient nothing holds the epilogue's warps at the same tile: whole tiles followed by quarters and by halves (as above), by quarters of all 74 pairs, and
+# one pair that walks whole tiles alone. The logits' gradients have the bits that they have with one, every time.
+@pytest.mark.parametrize("M,N,K,limit", [(70, 1256, 256, 8), (70, 1256, 256, 4), (64, 9728, 2560, 0), (10304, 1256, 256, 8), (96, 776, 512, 2)])
+@pytest.mark.parametrize("noise", ["none", "tensor"])
+def test_logit_gradient_alone(M, N, K, limit, noise):
+    import plz_ops as ops
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    x, dy = (torch.randn(M, n, generator=g, device="cuda").bfloat16() for n in (K, N))
+    w = ops.PackedWeight(ops.empty_packed(N, K, "cuda"), torch.randn(N * (K // 128), 4, generator=g, device="cuda").bfloat16(), N, K, 1, 128)
+    logits = torch.randn(N, K, 4, generator=g, device="cuda") * 2
+    nz = None if noise == "none" else torch.randn(N, K, 4, generator=g, device="cuda")
+    with _ctas(limit):
+        want = ops.backward_dw_soft(w, x, dy, logits, "nk4", noise=nz, tau=0.7)[0]
+        got = [ops.backward_dw_soft(w, x, dy, logits, "nk4", noise=nz, tau=0.7, want_dpalette=False) for _ in range(5)]
+    check_status()
+    assert all(p is None and torch.equal(d, want) for d, p in got)
+
+
 def test_no_rows_still_select():
     import plz_ops as ops
     N, K = 264, 384
