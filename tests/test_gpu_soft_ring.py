@@ -75,6 +75,35 @@ def test_logit_gradient_alone(M, N, K, limit, noise):
     assert all(p is None and torch.equal(d, want) for d, p in got)
 
 
+# logits far beyond any temperature: large ones, the type's lowest in one and in all four entries, the same large value four times
+@pytest.mark.parametrize("tau", [1.0, 0.01])
+@pytest.mark.parametrize("layout,dtype", [("nk4", torch.float32), ("4kn", torch.float32), ("4kn", torch.float16)])
+def test_extreme_logits(layout, dtype, tau):
+    import plz_ops as ops
+    M, N, K = 65, 264, 384
+    g = torch.Generator().manual_seed(7)
+    x, dy = torch.randn(M, K, generator=g).bfloat16(), torch.randn(M, N, generator=g).bfloat16()
+    pal = (torch.randn(N, 4, generator=g) * 0.02).bfloat16()
+    big, lowest = (6e4 if dtype == torch.float16 else 1e10), torch.finfo(dtype).min
+    logits = (torch.randn(N, K, 4, generator=g) * 2).round() / 2
+    logits[0::6] = torch.tensor([big, 0.0, 0.0, 0.0])
+    logits[1::6] = lowest
+    logits[2::6, :, 1] = lowest
+    logits[3::6] = -big
+    logits[4::6] = (logits[4::6] * 1e9).clamp(-big, big)
+    logits = logits.to(dtype)
+    p = torch.softmax(logits.double() / tau, -1).float()
+    _, want_log, want_pal, _ = O.soft_backward(x, dy, torch.zeros(N, K).bfloat16(), p, pal, 1, K)
+    lg = (logits if layout == "nk4" else O.from_nk_logits(logits)).cuda()
+    w = ops.PackedWeight(ops.empty_packed(N, K, "cuda"), pal.cuda(), N, K, 1, K)
+    w_soft = ops.soft_select(w, lg, layout, tau=tau, want_soft=True)
+    dlog, dpal = ops.backward_dw_soft(w, x.cuda(), dy.cuda(), lg, layout, tau=tau)
+    check_status()
+    assert_close(w_soft, (p * O.group_palette(pal, N, K, 1, K)).sum(-1), "W_soft")
+    assert_close(dlog, want_log if layout == "nk4" else O.from_nk_logits(want_log), "dLogits")
+    assert_close(dpal, want_pal, "dPalette")
+
+
 def test_no_rows_still_select():
     import plz_ops as ops
     N, K = 264, 384
