@@ -13,11 +13,11 @@
 
 namespace {
 
-// an exact torch.Tensor or Parameter on a GPU, or nullptr
+// an exact torch.Tensor or Parameter on a GPU with memory of its own (under vmap and jvp there are some without), or nullptr
 const at::Tensor* tensor(PyObject* o) {
     if (!THPVariable_CheckExact(o)) return nullptr;
     const at::Tensor& t = THPVariable_Unpack(o);
-    return t.defined() && t.is_cuda() && t.layout() == at::kStrided ? &t : nullptr;
+    return t.defined() && t.is_cuda() && t.layout() == at::kStrided && t.has_storage() ? &t : nullptr;
 }
 const at::Tensor* matrix(PyObject* o, int64_t cols = -1) {
     const at::Tensor* t = tensor(o);
@@ -54,19 +54,24 @@ bool weight(PyObject* const* a, plz_weight_t& w) {
 }
 int64_t palette_groups(const plz_weight_t& w) { return (int64_t)(w.N / w.gs_n) * (w.K / w.gs_k); }
 bool rows(const at::Tensor& t) { return t.size(0) <= 0x7FFFFFFF; }
+struct Rows { void* p; int64_t ld; int32_t n; };
+Rows rows_of(const at::Tensor& t) { return {t.data_ptr(), t.stride(0), (int32_t)t.size(0)}; }
 at::Tensor result(const at::Tensor& like, at::IntArrayRef sizes, at::ScalarType type = at::kBFloat16) { return at::empty(sizes, like.options().dtype(type)); }
 
+// gives the interpreter's lock up for its lifetime; an exception takes it back too
+struct Unlocked {
+    PyThreadState* state = PyEval_SaveThread();
+    ~Unlocked() { PyEval_RestoreThread(state); }
+};
+// call: addresses and library calls only, tensors are looked at before
 template <typename F>
 bool launch(F call) {
     void* stream = c10::cuda::getCurrentCUDAStream().stream();
-    PyThreadState* state = PyEval_SaveThread();
-    const int32_t rc = call(stream);
-    PyEval_RestoreThread(state);
-    return rc == PLZ_OK;
+    Unlocked unlocked;
+    return call(stream) == PLZ_OK;
 }
-bool clear(at::Tensor& t, void* stream) {   // fp32
-    void* p = t.data_ptr();
-    const int64_t bytes = t.numel() * 4;
+bool clear(void* p, int64_t words, void* stream) {   // fp32
+    const int64_t bytes = words * 4;
     return plz_zero(&p, &bytes, 1, stream) == PLZ_OK;
 }
 
@@ -77,7 +82,8 @@ PyObject* hard_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const at::Tensor* x;
     if (n != kWeightArgs + 1 || !weight(a, w) || !(x = matrix(a[6], w.K)) || !rows(*x)) Py_RETURN_NONE;
     at::Tensor y = result(*x, {x->size(0), w.N});
-    if (!launch([&](void* s) { return plz_hard_fwd(&w, x->data_ptr(), x->stride(0), (int32_t)x->size(0), nullptr, nullptr, y.data_ptr(), w.N, s); })) Py_RETURN_NONE;
+    const Rows xr = rows_of(*x), yr = rows_of(y);
+    if (!launch([&](void* s) { return plz_hard_fwd(&w, xr.p, xr.ld, xr.n, nullptr, nullptr, yr.p, w.N, s); })) Py_RETURN_NONE;
     return THPVariable_Wrap(std::move(y));
     END_HANDLE_TH_ERRORS
 }
@@ -89,7 +95,8 @@ PyObject* hard_forward_smallm(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const at::Tensor* x;
     if (n != kWeightArgs + 1 || !weight(a, w) || !(x = matrix(a[6], w.K)) || x->size(0) > 64) Py_RETURN_NONE;
     at::Tensor y = result(*x, {x->size(0), w.N});
-    if (!launch([&](void* s) { return plz_hard_fwd_smallm(&w, x->data_ptr(), x->stride(0), (int32_t)x->size(0), y.data_ptr(), w.N, s); })) Py_RETURN_NONE;
+    const Rows xr = rows_of(*x), yr = rows_of(y);
+    if (!launch([&](void* s) { return plz_hard_fwd_smallm(&w, xr.p, xr.ld, xr.n, yr.p, w.N, s); })) Py_RETURN_NONE;
     return THPVariable_Wrap(std::move(y));
     END_HANDLE_TH_ERRORS
 }
@@ -102,10 +109,9 @@ PyObject* hard_forward_bias(PyObject*, PyObject* const* a, Py_ssize_t n) {
     if (n != kWeightArgs + 2 || !weight(a, w) || !(x = matrix(a[6], w.K)) || !rows(*x)) Py_RETURN_NONE;
     if (a[7] != Py_None && (!(bias = tensor(a[7])) || bias->scalar_type() != at::kBFloat16 || !bias->is_contiguous() || bias->numel() != w.N)) Py_RETURN_NONE;
     at::Tensor y = result(*x, {x->size(0), w.N});
-    if (!launch([&](void* s) {
-            return plz_hard_fwd_bias(&w, x->data_ptr(), x->stride(0), (int32_t)x->size(0), bias ? bias->data_ptr() : nullptr, y.data_ptr(), w.N, s);
-        }))
-        Py_RETURN_NONE;
+    const Rows xr = rows_of(*x), yr = rows_of(y);
+    const void* bp = bias ? bias->data_ptr() : nullptr;
+    if (!launch([&](void* s) { return plz_hard_fwd_bias(&w, xr.p, xr.ld, xr.n, bp, yr.p, w.N, s); })) Py_RETURN_NONE;
     return THPVariable_Wrap(std::move(y));
     END_HANDLE_TH_ERRORS
 }
@@ -131,9 +137,11 @@ PyObject* eval_linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
         t = result(*x, {M, A->size(0)});
     }
     at::Tensor y = result(*x, shape);
+    const bool with_lora = t.defined();
+    void *const xp = x->data_ptr(), *const yp = y.data_ptr(), *const tp = with_lora ? t.data_ptr() : nullptr;
     if (!launch([&](void* s) {
-            if (lora.rank == 0 && M <= 64) return plz_hard_fwd_smallm(&w, x->data_ptr(), w.K, (int32_t)M, y.data_ptr(), w.N, s);
-            return plz_hard_fwd(&w, x->data_ptr(), w.K, (int32_t)M, t.defined() ? &lora : nullptr, t.defined() ? t.data_ptr() : nullptr, y.data_ptr(), w.N, s);
+            if (lora.rank == 0 && M <= 64) return plz_hard_fwd_smallm(&w, xp, w.K, (int32_t)M, yp, w.N, s);
+            return plz_hard_fwd(&w, xp, w.K, (int32_t)M, with_lora ? &lora : nullptr, tp, yp, w.N, s);
         }))
         Py_RETURN_NONE;
     return THPVariable_Wrap(std::move(y));
@@ -147,7 +155,8 @@ PyObject* backward_dx(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const at::Tensor* dy;
     if (n != kWeightArgs + 1 || !weight(a, w) || !(dy = matrix(a[6], w.N)) || !rows(*dy)) Py_RETURN_NONE;
     at::Tensor dx = result(*dy, {dy->size(0), w.K});
-    if (!launch([&](void* s) { return plz_bwd_dx(&w, dy->data_ptr(), dy->stride(0), (int32_t)dy->size(0), nullptr, nullptr, dx.data_ptr(), w.K, s); })) Py_RETURN_NONE;
+    const Rows dyr = rows_of(*dy), dxr = rows_of(dx);
+    if (!launch([&](void* s) { return plz_bwd_dx(&w, dyr.p, dyr.ld, dyr.n, nullptr, nullptr, dxr.p, w.K, s); })) Py_RETURN_NONE;
     return THPVariable_Wrap(std::move(dx));
     END_HANDLE_TH_ERRORS
 }
@@ -159,9 +168,12 @@ PyObject* backward_dw_hard(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const at::Tensor *x, *dy;
     if (n != kWeightArgs + 2 || !weight(a, w) || !(x = matrix(a[6], w.K)) || !(dy = matrix(a[7], w.N)) || !rows(*x) || dy->size(0) != x->size(0)) Py_RETURN_NONE;
     at::Tensor dpal = result(*x, {palette_groups(w), 4}, at::kFloat);
+    const Rows xr = rows_of(*x), dyr = rows_of(*dy);
+    float* const pp = (float*)dpal.data_ptr();
+    const int64_t words = dpal.numel();
     if (!launch([&](void* s) {
-            if (!clear(dpal, s)) return PLZ_ERR_CUDA;
-            return plz_bwd_dw_hard(&w, x->data_ptr(), x->stride(0), dy->data_ptr(), dy->stride(0), (int32_t)x->size(0), (float*)dpal.data_ptr(), s);
+            if (!clear(pp, words, s)) return PLZ_ERR_CUDA;
+            return plz_bwd_dw_hard(&w, xr.p, xr.ld, dyr.p, dyr.ld, xr.n, pp, s);
         }))
         Py_RETURN_NONE;
     return THPVariable_Wrap(std::move(dpal));
@@ -174,9 +186,12 @@ PyObject* col_sum(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const at::Tensor* dy;
     if (n != 1 || !(dy = matrix(a[0])) || !rows(*dy) || dy->size(1) > 0x7FFFFFFF) Py_RETURN_NONE;
     at::Tensor out = result(*dy, {dy->size(1)}, at::kFloat);
+    const Rows dyr = rows_of(*dy);
+    const int64_t cols = dy->size(1);
+    float* const sums = (float*)out.data_ptr();
     if (!launch([&](void* s) {
-            if (!clear(out, s)) return PLZ_ERR_CUDA;
-            return plz_col_sum(dy->data_ptr(), dy->stride(0), (int32_t)dy->size(0), (int32_t)dy->size(1), (float*)out.data_ptr(), s);
+            if (!clear(sums, cols, s)) return PLZ_ERR_CUDA;
+            return plz_col_sum(dyr.p, dyr.ld, dyr.n, (int32_t)cols, sums, s);
         }))
         Py_RETURN_NONE;
     return THPVariable_Wrap(std::move(out));
@@ -234,10 +249,13 @@ PyObject* backward_dw_soft(PyObject*, PyObject* const* a, Py_ssize_t n) {
         if (dlog.strides() != t->strides()) Py_RETURN_NONE;
     }
     if (want_p) dpal = result(*x, {palette_groups(w), 4}, at::kFloat);
+    const Rows xr = rows_of(*x), dyr = rows_of(*dy);
+    void* const lp = want_l ? dlog.data_ptr() : nullptr;
+    float* const pp = want_p ? (float*)dpal.data_ptr() : nullptr;
+    const int64_t words = want_p ? dpal.numel() : 0;
     if (!launch([&](void* s) {
-            if (want_p && !clear(dpal, s)) return PLZ_ERR_CUDA;
-            return plz_bwd_dw_soft(&w, x->data_ptr(), x->stride(0), dy->data_ptr(), dy->stride(0), (int32_t)x->size(0), &l, &z, (float)tau,
-                                   want_l ? dlog.data_ptr() : nullptr, want_p ? (float*)dpal.data_ptr() : nullptr, s);
+            if (want_p && !clear(pp, words, s)) return PLZ_ERR_CUDA;
+            return plz_bwd_dw_soft(&w, xr.p, xr.ld, dyr.p, dyr.ld, xr.n, &l, &z, (float)tau, lp, pp, s);
         }))
         Py_RETURN_NONE;
     PyObject* out = PyTuple_New(2);

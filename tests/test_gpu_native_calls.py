@@ -99,6 +99,26 @@ def test_what_is_refused(general):
         assert type(a.value) is type(b.value) and str(a.value) == str(b.value), i
 
 
+# tensors without memory: what a transform hands to the function that it works on
+@pytest.mark.parametrize("transform", [lambda f, x: torch.vmap(f)(torch.stack([x, x])), lambda f, x: torch.func.jvp(f, (x,), (torch.ones_like(x),)),
+                                       lambda f, x: torch.func.grad(lambda z: f(z).float().sum())(x)], ids=["vmap", "jvp", "grad"])
+def test_transforms_are_refused(transform, general):
+    g = torch.Generator(device="cuda").manual_seed(3)
+    w, w2 = _weight(g, 256, 256, 1, 256), _weight(g, 256, 256, 1, 256)
+    lg = torch.randn(256, 256, 4, generator=g, device="cuda")
+    plain, lora = (PL.PalettizedLinear(256, 256, rank=r).eval() for r in (0, 16))
+    d = _rnd(g, 80, 256)
+    fs = [lambda z: ops.hard_forward(w, z)[0], lambda z: ops.hard_forward_smallm(w, z), lambda z: ops.hard_forward_bias(w, z, None), lambda z: ops.hard_forward_bias(w, d, z[0]),
+          lambda z: ops.backward_dx(w, z)[0], lambda z: ops.backward_dw_hard(w, z, d), lambda z: ops.backward_dw_hard(w, d, z), ops.col_sum,
+          lambda z: ops.soft_select(w2, z.float()[:, :, None].expand(-1, -1, 4), "nk4"), lambda z: ops.backward_dw_soft(w, z, d, lg, "nk4")[0], plain, lora]
+    for i, f in enumerate(fs):
+        with pytest.raises(Exception) as a:
+            transform(f, d)
+        with pytest.raises(Exception) as b:
+            general(lambda: transform(f, d))
+        assert type(a.value) is type(b.value) and str(a.value) == str(b.value), i
+
+
 def test_own_stream_thread_and_subclass(general):
     g = torch.Generator(device="cuda").manual_seed(2)
     w = _weight(g, 512, 256, 1, 256)
