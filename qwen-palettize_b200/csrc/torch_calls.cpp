@@ -132,7 +132,7 @@ PyObject* eval_linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
     if (a[7] != Py_None) {
         const at::Tensor *A = matrix(a[7], w.K), *B = matrix(a[8]);
         double scale;
-        if (!A || !B || A->size(0) != B->size(1) || A->size(0) > 64 || B->size(0) != w.N || !real(a[9], scale)) Py_RETURN_NONE;
+        if (!A || !B || A->size(0) != B->size(1) || A->size(0) < 1 || A->size(0) > 64 || B->size(0) != w.N || !real(a[9], scale)) Py_RETURN_NONE;
         lora = {(int32_t)A->size(0), (float)scale, A->data_ptr(), A->stride(0), B->data_ptr(), B->stride(0)};
         t = result(*x, {M, A->size(0)});
     }
@@ -140,7 +140,7 @@ PyObject* eval_linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const bool with_lora = t.defined();
     void *const xp = x->data_ptr(), *const yp = y.data_ptr(), *const tp = with_lora ? t.data_ptr() : nullptr;
     if (!launch([&](void* s) {
-            if (lora.rank == 0 && M <= 64) return plz_hard_fwd_smallm(&w, xp, w.K, (int32_t)M, yp, w.N, s);
+            if (!with_lora && M <= 64) return plz_hard_fwd_smallm(&w, xp, w.K, (int32_t)M, yp, w.N, s);
             return plz_hard_fwd(&w, xp, w.K, (int32_t)M, with_lora ? &lora : nullptr, tp, yp, w.N, s);
         }))
         Py_RETURN_NONE;

@@ -91,6 +91,9 @@ def test_what_is_refused(general):
            lambda: ops.backward_dx(w, x), lambda: ops.backward_dw_hard(w, x, x), lambda: ops.col_sum(x.float()),
            lambda: ops.soft_select(w, lg, "nk4", tau=0.0), lambda: ops.soft_select(w, lg.double(), "nk4"), lambda: ops.soft_select(w, lg, "nk4", noise=lg.half()),
            lambda: ops.backward_dw_soft(w, x, _rnd(g, 80, 512), lg, "nk4", tau=-1.0)]
+    m = PL.PalettizedLinear(256, 512, rank=8).eval()
+    m.lora_A, m.lora_B = torch.nn.Parameter(m.lora_A.detach()[:0]), torch.nn.Parameter(m.lora_B.detach()[:, :0])
+    bad.append(lambda: m(x[:4]))                # LoRA factors of rank 0
     for i, f in enumerate(bad):
         with pytest.raises(Exception) as a:
             f()
