@@ -991,8 +991,10 @@ int launch_tn_gemm(const TnArgs& a, cudaStream_t stream) {
         const int rem = tiles % grid;
         if (tiles > grid && rem > 0 && 2 * rem <= grid) {
             // quarters where the soft epilogue is the longer part (1000 tokens of 2560 x 9728 218 -> 209 us): a product of 64 columns feeds on as many bytes of P as
-            // one of 256, so a long main loop would not gain
-            p.tail_shift = a.epi == EPI_SOFT && a.M < kTnLongLoop && 4 * rem <= grid ? 2 : 1;
+            // one of 256, so a long main loop would not gain. Not where the cut runs along k and a tile's columns are all of a palette's: four sums that meet at
+            // one address by atomics would round in another order from run to run, two do not.
+            const bool shared = !a.rows_are_k && a.gs_n <= 128 && a.gs_k <= 256;
+            p.tail_shift = a.epi == EPI_SOFT && !shared && a.M < kTnLongLoop && 4 * rem <= grid ? 2 : 1;
             p.n_whole = tiles - rem; p.n_items = p.n_whole + (rem << p.tail_shift);
         }
     }

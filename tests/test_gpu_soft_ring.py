@@ -104,6 +104,22 @@ def test_extreme_logits(layout, dtype, tau):
     assert_close(dpal, want_pal, "dPalette")
 
 
+# five tiles on four pairs, cut along k, a palette per row (or 128 of them) and 256 columns: what meets at an address adds up the same every time
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+@pytest.mark.parametrize("gs_n", [1, 128])
+def test_palette_gradient_repeats(dtype, gs_n):
+    import plz_ops as ops
+    M, N, K = 70, 256, 1280
+    g = torch.Generator(device="cuda").manual_seed(3)
+    x, dy = (torch.randn(M, n, generator=g, device="cuda").bfloat16() for n in (K, N))
+    w = ops.PackedWeight(ops.empty_packed(N, K, "cuda"), torch.randn(N // gs_n * (K // 256), 4, generator=g, device="cuda").bfloat16(), N, K, gs_n, 256)
+    lg = torch.randn(4, K, N, generator=g, device="cuda").to(dtype)
+    with _ctas(8):
+        first = ops.backward_dw_soft(w, x, dy, lg, "4kn", tau=0.7)[1]
+        assert all(torch.equal(ops.backward_dw_soft(w, x, dy, lg, "4kn", tau=0.7)[1], first) for _ in range(100))
+    check_status()
+
+
 def test_no_rows_still_select():
     import plz_ops as ops
     N, K = 264, 384
