@@ -64,3 +64,20 @@ def test_order_of_the_query_tiles(B, n, pos):
     s = torch.einsum("bihd,bjhd->bhij", q.double().view(B, n, H, d), kf) * d ** -0.5 + tab.double()[:, at.clamp(0, 99)]
     s = torch.cat([s.masked_fill(at < 0, float("-inf")), torch.zeros_like(s[..., :1])], -1)
     assert_close(o, torch.einsum("bhij,bjhd->bihd", torch.softmax(s, -1)[..., :-1], vf).reshape(B * n, H * d).float(), "o")
+
+
+# the entries in front of distance 0 are there to be read with a tile and may hold anything: a prompt, a portion behind cached tokens, more distances than the table has;
+# heads of either kind beside each other
+@pytest.mark.parametrize("n,pos,D", [(130, 0, 40), (300, 70, 100), (300, 70, 1000)])
+def test_what_stands_in_front_of_the_biases(n, pos, D):
+    import seq_ops as S
+    B, H, G, d, T, g = 1, 4, 2, 64, pos + n, torch.Generator(device="cuda").manual_seed(n)
+    q, k, v = (torch.randn(B, t, h * d, generator=g, device="cuda").bfloat16() for t, h in ((n, H), (T, G), (T, G)))
+    b = S.DistanceBias.from_distances(torch.randn(H, D, generator=g, device="cuda"))
+    out = []
+    for fill in (0.0, 1e29, float("nan"), float("inf"), torch.finfo(torch.float32).max):
+        b.rows[::2, :S.BIAS_FRONT] = fill
+        out.append(S.attention_bias(q.view(B * n, H * d), k, v, b, torch.tensor([pos], dtype=torch.int32, device="cuda"), pos, B, n, H, G, d, d, d ** -0.5, True))
+    check_status()
+    # the other pass over a masked tile adds its weights in another order: 128 fp32 sums, then bf16
+    assert torch.isfinite(out[0]).all() and torch.equal(out[0], out[1]) and all((o.float() - out[0].float()).abs().max() <= 2.0 ** -7 * out[0].float().abs().max() for o in out)
