@@ -234,7 +234,8 @@ def latent_attention(q: torch.Tensor, c: torch.Tensor, kr, sinks, pos: torch.Ten
 
 def put(dst: torch.Tensor, values: torch.Tensor):
     """dst.copy_(values), for the few int64 numbers in host memory that a step starts with without waiting for the work before it."""
-    if values.device.type == "cpu" and values.dtype == dst.dtype == torch.int64 and values.shape == dst.shape and 0 < values.numel() <= 4096 and dst.is_contiguous():
+    if (values.device.type == "cpu" and values.dtype == dst.dtype == torch.int64 and values.shape == dst.shape and 0 < values.numel() <= 4096 and dst.is_contiguous()
+            and not torch.cuda.is_current_stream_capturing()):     # a graph would replay the numbers of its capture
         values = values.contiguous()
         P.check(P.lib().plz_put_words(dst.data_ptr(), values.data_ptr(), values.numel(), P.stream_ptr()), "plz_put_words")
     else:

@@ -14,3 +14,17 @@ def test_declines_what_it_does_not_take(built_lib):
         assert f(*rest) is None
         assert f() is None and f(*(None for _ in rest)) is None and f(*(7 for _ in rest)) is None and f(*rest, 1) is None
         assert f(*(2 ** 80 for _ in rest)) is None
+
+
+def test_host_numbers_are_not_frozen_into_a_graph(built_lib, monkeypatch):
+    """While the stream is captured, numbers from the host go by the copy, which a capture refuses; a launch would replay these ones for good."""
+    import plz_native as P
+    import seq_ops as S
+
+    def no_launch():
+        raise AssertionError("launched")
+    monkeypatch.setattr(P, "lib", no_launch)
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: True)
+    dst, v = torch.zeros(3, dtype=torch.int64), torch.arange(3)
+    S.put(dst, v)
+    assert torch.equal(dst, v) and torch.equal(S.on_device(v, "cpu"), v)
