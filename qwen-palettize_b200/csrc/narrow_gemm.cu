@@ -53,6 +53,7 @@ struct NarrowParams {
     int gs_n, gs_k, n_kgroups;
     int glu;                       // a tile is 64 rows of mat[0] and the same rows of mat[1]
     int early;                     // W is read ahead of the wait for the kernel before
+    int lets_next;                 // let the next kernel start behind this one's wait
     const __nv_bfloat16* bias; int act, y_f32; float alpha;
     StatusWord* status;
 };
@@ -180,7 +181,7 @@ narrow_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
     const uint32_t tmem_base = *tmem_slot;
     const uint32_t tmem_w = tmem_base + (uint32_t)(p.n_acc * p.npad);      // LUT: 32 columns per stage
     if (!p.early) pdl_wait();
-    pdl_launch_dependents();
+    if (p.lets_next) pdl_launch_dependents();
 
     // every wait below that x holds up starts after the previous kernel of the stream has finished: its time is not the wait's
     int issued = pre;                      // stages the producing thread has filled
@@ -591,7 +592,9 @@ int launch_narrow_gemm(const NarrowArgs& a, cudaStream_t stream) {
         if ((rc = make_tmap_bf16(&tm[3], a.w2, a.mat[0].N, a.r2, a.ldw2, 64, 128))) return rc;
     }
     const int ranks = a.transposed ? turned_parts(p.n_blocks) : lut ? cluster_size_packed(tiles, p.n_blocks, seq_sm_count()) : cluster_size(tiles, p.n_blocks, seq_sm_count(), 12);
-    p.early = g_smallm_overlap && a.early && !a.transposed;       // else W may be what the previous kernel writes
+    const bool chain = a.early && !a.transposed;                  // else W may be what the previous kernel writes, and the result what the next one reads as W
+    p.early = chain && g_smallm_overlap;
+    p.lets_next = chain || !g_smallm_overlap;
     return lut ? launch_ng<true>(p, tiles, ranks, tm, stream) : launch_ng<false>(p, tiles, ranks, tm, stream);
 }
 
@@ -607,6 +610,7 @@ constexpr int kTgMaxStages = 11;
 constexpr uint32_t kTgRingBytes = 200 * 1024;
 struct TurnedParams {
     int M, N, tiles, parts, n_blocks, x_mn, stages;
+    int lets_next;           // let the next kernel start behind this one's wait
     uint32_t x_bytes;
     __nv_bfloat16* y; long long ldy;
     float alpha;
@@ -645,7 +649,7 @@ turned_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
     pdl_wait();
-    pdl_launch_dependents();
+    if (p.lets_next) pdl_launch_dependents();
 
     int issued = 0;                        // stages the producing thread has filled
     if (warp == 0) {
@@ -757,6 +761,7 @@ int launch_tg(const NarrowArgs& a, const CUtensorMap& tmX, const CUtensorMap& tm
     p.stages = (int)(kTgRingBytes / (kNgWBytes + p.x_bytes));
     if (p.stages > kTgMaxStages) p.stages = kTgMaxStages;
     p.y = (__nv_bfloat16*)a.mat[0].y; p.ldy = a.mat[0].ldy; p.alpha = a.alpha; p.status = device_status_ptr();
+    p.lets_next = !g_smallm_overlap;
     auto kern = turned_gemm_kernel<NPAD>;
     constexpr uint32_t smem = kTgRingBytes + kNgBarBytes + 1024;
     static bool attr_set[64] = {};

@@ -75,7 +75,8 @@ inline cudaError_t launch_chain(void (*kernel)(KArgs...), dim3 grid, dim3 block,
 // memory, the cluster's first meeting) run under the end of the kernel before, whoever launched that and with the switch of the token chain on or off. us without / with it: training step
 // of a decoder layer, 8 x 512 tokens, 2880 / 2831; 2 x 1024 tokens through recurrent layers 1368 / 1332; step of one Linear over 1000 tokens 354 / 349.
 // Two rules keep the kernels of the token chain safe, which read weights ahead of their waits: a kernel that writes what may serve as weights, palettes or indices
-// (weight gradients, optimizer, selections) does not execute griddepcontrol.launch_dependents, and dense and palettized products only with that switch off.
+// (weight gradients, optimizer, selections) does not execute griddepcontrol.launch_dependents, and dense and palettized products only with that switch off, or as
+// products of the chain themselves (NarrowArgs::early, LutGemmArgs::early), whose results are activations.
 // Not while the stream is captured: there the switch alone decides which edges of the graph are programmatic.
 // Fills in the attribute; the number of them (0 or 1).
 inline unsigned behind_attr(cudaStream_t stream, cudaLaunchAttribute* attr) {

@@ -84,3 +84,21 @@ def test_captured_chain_has_plain_edges():
     graph.replay()
     torch.cuda.synchronize()
     assert torch.equal(got, want)
+
+
+# products outside the token chain (few rows; at most 64 columns, walked by tiles or in clusters) do not let a kernel of the chain, which reads its matrix ahead of the wait, start
+# before they have finished
+@pytest.mark.parametrize("M,N", [(128, 1024), (64, 4096), (2048, 64), (16384, 32), (96, 16)])
+def test_a_product_as_the_next_ones_matrix(M, N):
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    r = lambda *s: torch.randn(*s, generator=g, device="cuda").bfloat16()
+    x, wd, z = [r(M, 2560) for _ in range(4)], r(N, 2560), r(2, N)
+    want = [S.linear(z, ops.dense_forward(wd, v)[0]) for v in x]
+    torch.cuda.synchronize()
+    P.lib().plz_set_smallm_overlap(1)
+    try:
+        got = [S.linear(z, ops.dense_forward(wd, v)[0]) for _ in range(5) for v in x]
+    finally:
+        P.lib().plz_set_smallm_overlap(0)
+    P.device_status()
+    assert all(torch.equal(a, b) for a, b in zip(got, want * 5))
