@@ -3,6 +3,7 @@
 Usage: python build.py [--force] [--verbose]
 The library lands next to this file so that it travels with the source tree.
 """
+import importlib.metadata
 import importlib.util
 import os
 import subprocess
@@ -19,6 +20,7 @@ HEADERS = ["plz_sm100.cuh", "plz_host.h", "plz_launch.h", "soft_math.cuh", "seq_
 LIB = os.path.join(HERE, "libplz.so")
 CALLS_SRC = os.path.join(CSRC, "torch_calls.cpp")
 CALLS = os.path.join(HERE, "_plz_torch.so")   # Python module over libplz.so for torch tensors
+CALLS_FOR = os.path.join(HERE, "build", "_plz_torch.txt")   # what it was compiled against
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
          "-Xcompiler", "-fPIC", "--use_fast_math", "-Xptxas", "-v"]
@@ -37,9 +39,21 @@ def _stale():
     return _older(LIB, [os.path.join(CSRC, s) for s in SOURCES + HEADERS])
 
 
+def _calls_for():
+    """What the Python module is compiled against: torch's C++ interface and the interpreter's."""
+    return f"torch {importlib.metadata.version('torch')}, {sysconfig.get_config_var('SOABI')}\n"
+
+
+def _calls_stale():
+    if _older(CALLS, [CALLS_SRC, os.path.join(HERE, "..", "include", "plz.h")]) or not os.path.exists(CALLS_FOR):
+        return True
+    with open(CALLS_FOR) as f:
+        return f.read() != _calls_for()
+
+
 def _build_calls(force):
     """The Python module, compiled against the installed torch (host code only)."""
-    if not force and not _older(CALLS, [CALLS_SRC, os.path.join(HERE, "..", "include", "plz.h")]):
+    if not force and not _calls_stale():
         return
     root = os.path.dirname(importlib.util.find_spec("torch").origin)
     inc, lib = os.path.join(root, "include"), os.path.join(root, "lib")
@@ -51,6 +65,9 @@ def _build_calls(force):
     if r.returncode != 0:
         sys.stderr.write(r.stdout)
         raise RuntimeError("g++ failed on torch_calls.cpp")
+    os.makedirs(os.path.dirname(CALLS_FOR), exist_ok=True)
+    with open(CALLS_FOR, "w") as f:
+        f.write(_calls_for())
 
 
 def build(force=False, verbose=False):

@@ -28,3 +28,17 @@ def test_host_numbers_are_not_frozen_into_a_graph(built_lib, monkeypatch):
     dst, v = torch.zeros(3, dtype=torch.int64), torch.arange(3)
     S.put(dst, v)
     assert torch.equal(dst, v) and torch.equal(S.on_device(v, "cpu"), v)
+
+
+def test_module_is_rebuilt_for_another_torch_or_python(built_lib, monkeypatch):
+    import sysconfig
+
+    import build
+    assert not build._calls_stale()
+    with monkeypatch.context() as m:
+        m.setattr(build.importlib.metadata, "version", lambda name: "0.0")
+        assert build._calls_stale()
+    with monkeypatch.context() as m:
+        m.setattr(sysconfig, "get_config_var", lambda name: "cpython-00")
+        assert build._calls_stale()
+    assert not build._calls_stale()
