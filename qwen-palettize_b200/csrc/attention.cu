@@ -9,7 +9,7 @@
 // All products run on the 5th-generation tensor cores (tcgen05.mma, 128 x 128 x 16, accumulators in TMEM), operands
 // staged by TMA in 128-byte-swizzled tiles. One CTA handles one (batch, head) and one or two 128-token tiles:
 //   forward        two neighbouring query tiles per CTA: S = Q K^T -> online softmax by 128 threads per tile (one row each,
-//                  TMEM -> registers) -> P (bf16) to shared memory -> O += P V, O rescaled in TMEM when a row maximum has outgrown its reference;
+//                  TMEM -> registers) -> P (bf16) to shared memory -> O += P V, O rescaled in TMEM when a row maximum grows;
 //                  the softmax of one tile runs under the MMAs of the other; also writes the row log-sum-exp.
 //   backward dQ    per q tile: S, dP = dO V^T -> dS = P (dP - D) / sqrt(d) -> dQ += dS K
 //   backward dKdV  per kv tile and kv head, over the q heads of the group and the q tiles at or after it:
@@ -34,18 +34,18 @@ struct AttnParams {
 };
 
 // eight MMAs of one 128 x 128 x 128 product. A / B tiles are 128-row bf16 tiles of two 64-column blocks.
-//   K-major operand (rows = M or N index, reduction along the 128-byte row):  step ks -> block ks / 4, 32 bytes * (ks % 4)
-//   MN-major operand (rows = reduction index, M or N along the row): step ks -> 16 rows = 2048 bytes, blocks 16 KB apart
-__device__ __forceinline__ void mma_128(uint32_t d_tmem, uint32_t sA, bool a_mn, uint32_t sB, bool b_mn, bool accumulate) {
-    const uint32_t idesc = make_idesc(128, 128, a_mn ? 1 : 0, b_mn ? 1 : 0);
-    const uint64_t ad0 = a_mn ? make_sdesc(sA, kBlk, 1024u) : make_sdesc(sA, 16u, 1024u);
+//   K-major operand (A, and B unless b_mn; rows = M or N index, reduction along the 128-byte row):  step ks -> block ks / 4, 32 bytes * (ks % 4)
+//   MN-major B (rows = reduction index, N along the row): step ks -> 16 rows = 2048 bytes, blocks 16 KB apart
+__device__ __forceinline__ void mma_128(uint32_t d_tmem, uint32_t sA, uint32_t sB, bool b_mn, bool accumulate) {
+    const uint32_t idesc = make_idesc(128, 128, 0, b_mn ? 1 : 0);
+    const uint64_t ad0 = make_sdesc(sA, 16u, 1024u);
     const uint64_t bd0 = b_mn ? make_sdesc(sB, kBlk, 1024u) : make_sdesc(sB, 16u, 1024u);
     const uint32_t a_hi = (uint32_t)(ad0 >> 32), b_hi = (uint32_t)(bd0 >> 32), a_lo = (uint32_t)ad0, b_lo = (uint32_t)bd0;
 #pragma unroll
     for (int ks = 0; ks < 8; ++ks) {
         const uint32_t off_k = (uint32_t)((ks >> 2) * (kBlk >> 4) + (ks & 3) * 2);
         const uint32_t off_mn = (uint32_t)(ks * 128);
-        umma_bf16_words<1>(d_tmem, a_lo + (a_mn ? off_mn : off_k), a_hi, b_lo + (b_mn ? off_mn : off_k), b_hi, idesc,
+        umma_bf16_words<1>(d_tmem, a_lo + off_k, a_hi, b_lo + (b_mn ? off_mn : off_k), b_hi, idesc,
                            (ks > 0 || accumulate) ? 1u : 0u);
     }
 }
@@ -256,8 +256,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             if (elect_one()) { load_tile(sKV + s * kTile, is_k ? &tmK : &tmV, full(s), hk * kD, row); }
         }
     } else if (warp == 8) {
-        // the whole warp walks the tiles and one elected lane issues (narrow_gemm.cu: operands stay in uniform registers):
-        // 4 x 1024 tokens, 32 heads 87 -> 82 us; backward of 8 x 512: dK and dV 106 -> 101, dQ 71 -> 68
+        // the whole warp walks the tiles and one elected lane issues (narrow_gemm.cu: operands stay in uniform registers)
         auto ready = [&](int item) { return mbar_wait_warp(full(item % 3), (item / 3) & 1, abort_flag, p.status, ST_TIMEOUT_FULL, 11); };
         auto done = [&](int item) { if (item + 3 <= last && elect_one()) umma_commit(empty(item % 3)); };
         bool ok = mbar_wait_warp(q_full, 0, abort_flag, p.status, ST_TIMEOUT_FULL, 10);
@@ -271,7 +270,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                     if (j >= 0) ok = mbar_wait_warp(s_free(g), j & 1, abort_flag, p.status, ST_TIMEOUT_ACCUM, 12);
                     if (!ok) break;
                     tc_fence_after_sync();
-                    if (elect_one()) { mma_128(tS(g), sQ0 + g * kTile, false, sKV + item % 3 * kTile, false, false); }
+                    if (elect_one()) { mma_128(tS(g), sQ0 + g * kTile, sKV + item % 3 * kTile, false, false); }
                     if (elect_one()) { umma_commit(s_full(g)); }
                 }
                 if (!ok) break;
@@ -286,7 +285,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                     ok = mbar_wait_warp(p_full(g), j & 1, abort_flag, p.status, ST_TIMEOUT_FULL, 13);
                     if (!ok) break;
                     tc_fence_after_sync();
-                    if (elect_one()) { mma_128(tO(g), sP0 + g * kTile, false, sKV + item % 3 * kTile, true, j > 0); } // V: rows = kv = reduction index
+                    if (elect_one()) { mma_128(tO(g), sP0 + g * kTile, sKV + item % 3 * kTile, true, j > 0); } // V: rows = kv = reduction index
                     if (elect_one()) { umma_commit(o_full(g)); }
                 }
                 if (!ok) break;

@@ -21,7 +21,7 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t,
 EncodeTiledFn get_encode_fn();
 
 // 2-D bf16 row-major tensor [rows, cols] with row pitch `ld` elements; box = [box_cols, box_rows],
-// box_cols 64: 128-byte swizzle, 32: 64-byte swizzle; out-of-range elements read as zero.
+// box_cols 64: 128-byte swizzle, 32: 64-byte swizzle, 16: none; out-of-range elements read as zero.
 int make_tmap_bf16(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint64_t ld,
                    uint32_t box_cols, uint32_t box_rows);
 
