@@ -549,8 +549,8 @@ PairTiles plan_pair_tiles(int M, int J, int pairs, int step) {
 
 // One or two waves of narrower tiles where they are fewer columns in all: 2048 x 2560 outputs are 80 tiles of 256 on 74 pairs, a wave and one of halves, 384
 // columns; or 144 tiles of 144, two nearly full waves, 288. For the dense kernel (packed weights are decoded in chains that cost 160 columns at least).
-// us plan_pair_tiles / here: 2048 rows, 2560 x 2560 26.5 / 22.4, 2560 x 9728 87.6 / 84.8, 2560 x 4096 40.8 / 38.9; 1000 rows, 7680 x 2560 34.0 / 31.7; 512 rows, 9728 x 2560
-// 30.0 / 28.2. More waves or more rows do not pay, as narrow tiles read more of both operands: 1536 rows, 9728 x 2560 in four waves of 208 columns 57.6 / 62.5, 4096 rows,
+// us plan_pair_tiles / here, one after the other: 2048 rows, 2560 x 2560 27.1 / 25.6, 2560 x 4096 39.3 / 37.5, 2560 x 9728 87.4 / 84.8; 1000 rows, 7680 x 2560 33.6 / 31.6; 512 rows,
+// 9728 x 2560 28.7 / 27.6. More waves or more rows do not pay, as narrow tiles read more of both operands: 1536 rows, 9728 x 2560 in four waves of 208 columns 57.6 / 62.5, 4096 rows,
 // 2560 x 9728 in four of 144 151 / 178; nor do gated outputs (512 rows, 19456 x 2560 44.2 / 45.4).
 PairTiles plan_pair_waves(int M, int J, int pairs, int step) {
     PairTiles best = plan_pair_tiles(M, J, pairs, 32);

@@ -1,5 +1,5 @@
 // Per-weight arithmetic of the Gumbel-Softmax relaxation, shared by the pass that builds W_soft and by the gradient epilogue so that forward and
-// backward see identical numbers (soft_tensors.cu has steps of its own, for tensors that a caller asks for).
+// backward see identical numbers (soft_tensors.cu has steps of its own, for tensors that a caller asks for: their last bits may differ).
 //
 // Semantics follow the reference's PyTorch/Triton path:
 //   P = softmax((logits + g) / tau) in fp32, max-subtracted   (scripts/triton_soft_forward.py:119-141)
@@ -65,8 +65,8 @@ struct Soft4 {
 
 // s: logits plus noise; c: palette entries in fp32; scale: soft_scale(tau). exp(x / tau) is 2 to the scaled x. The largest is subtracted before anything is
 // scaled: of logits of any size the largest then weighs exactly 1, where a product that is rounded, or overflows, by itself would leave its error as an
-// exponent (one instruction less; a step of 1000 tokens through 9728 x 2560 353 against 354 us). 150 instructions per weight of the weight gradient's epilogue
-// with single numbers, 106 with pairs.
+// exponent (one instruction less; a step of 1000 tokens through 9728 x 2560 353 against 354 us). Pairs in place of single numbers took the weight gradient's
+// epilogue from 150 to 105 instructions per weight.
 __device__ __forceinline__ Soft4 soft4(const f32x2 (&s)[2], const f32x2 (&c)[2], float scale) {
     float x[4], e[4];
     split2(s[0], x[0], x[1]);

@@ -74,7 +74,7 @@ __device__ __forceinline__ void palette4(const __nv_bfloat16* palette, long long
 }
 
 // The tensors' own arithmetic, one rounding per step: the index taken from P (hard_from_noisy) depends on every one of them where two entries are close,
-// so soft_math.cuh's fused form would change it.
+// so soft_math.cuh's order of them would change it.
 __device__ __forceinline__ float gumbel_hash(uint32_t seed, uint32_t idx) {
     uint32_t x = seed ^ (idx * 0x9E3779B9u);
     x ^= x >> 13;

@@ -51,7 +51,7 @@ struct TnParams {
         float* out; long long out_si, out_sj;
     } side[2];
     int n_side_items;
-    // Tail of the persistent schedule (halves or quarters). After the whole tiles come the half tiles (one per work unit, n_items - n_whole of
+    // Tail of the persistent schedule. After the whole tiles come their halves or quarters, here both called half tiles (one per work unit, n_items - n_whole of
     // them) and then the side items, which are dealt only to the units that did not get a half tile: tail slots that fall on
     // a unit with a half tile stay empty, so that no unit carries a half tile AND a second side item while others idle.
     // tail_free = units without a half tile (0: the side items simply follow the halves); n_total = items including holes.
@@ -190,7 +190,7 @@ tn_gemm_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant__ 
 
     // tile -> (split, i tile, j tile); i fastest so that one wave of CTAs covers every i tile
     // item -> (split, i tile, j tile, first column inside the tile, columns); i fastest so that one wave of CTAs
-    // covers every i tile. Items past n_whole are the two 128-column halves of a tile.
+    // covers every i tile. Items past n_whole are halves or quarters of a tile's columns.
     auto tile_coords = [&](int item, int& sp, int& ti, int& tj, int& c_off, int& c_num, int& job) {
         c_off = 0; c_num = 256; job = -1;
         if (item >= p.n_items) {
@@ -835,9 +835,10 @@ tn_gemm_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant__ 
 // ---------------------------------------------------------------------------------------------
 
 // Epilogue warps of the interleaved soft epilogue: sixteen, or eight and a stage more for the main loop where that is what takes the time, in a launch of more
-// than one wave. us at 9728 x 2560, sixteen / eight warps (before the ring of requests: sixteen below 10241 tokens, else eight), noise tensor: 1000 tokens 215 (277),
-// 4096 tokens 273 / 295 (310), 6144 348 / 351 (355), 8192 422 / 391 (405), 10240 499 / 463 (483), 16384 - / 691 (738); sampled noise: 1000 tokens 183 (248), 4096 262 / 325 (294),
-// 8192 390 / 416 (402), 10240 474 / 468 (488), 16384 - / 694 (732). One wave (1024 x 2560), 10240 tokens: 107 / 109 (109) and 115 / 121 (114).
+// than one wave. us, sixteen / eight warps (before the ring of requests: sixteen below 10241 tokens, else eight), noise tensor: 9728 x 2560, 1000 tokens 215 (277), 4096 271 / 291 (306), 6144 347 / 357 (356),
+// 8192 422 / 423 (430), 10240 497 / 498 (505), 12288 572 / 574 (583); 2560 x 9728 293 / 307 (323), 374 / 375 (377), 452 / 447 (457), 531 / 528 (539), 612 / 611 (624); 6144 x 2560 175 / 185 (201),
+// 225 / 226 (229), 272 / 271 (273), 320 / 319 (322), 369 / 365 (374); 4096 x 2560 124 / 129 (148), 157 / 153 (163), 192 / 182 (188), 225 / 216 (222), 260 / 251 (258). Sampled noise, 9728 x 2560: 1000 tokens 183 (248),
+// 4096 262 / 325 (294), 8192 390 / 416 (402), 10240 474 / 468 (488), 16384 - / 694 (732). One wave (1024 x 2560), 10240 tokens: 107 / 109 (109) and 115 / 121 (114).
 // Planar fp16 logits: always sixteen. The hard epilogue has 45 us with sixteen against 40 at 512 tokens: always eight.
 constexpr int kTnLongLoopNoise = 7168, kTnLongLoop = 10241;
 
