@@ -472,8 +472,8 @@ int32_t plz_bwd_dw_hard_lora(const plz_weight_t* w, const void* x, int64_t ldx, 
  * plz_attn_prep: RMS norm of the whole q and k projections, optional value mixing with the first mixing layer's values, and the
  *   write of keys and values into the cache at *pos + t.
  * plz_attn_bias: causal attention of the n new tokens against the cache (which already holds them), score * scale + bias by distance
- *   (bias points at distance 0 of head 0; entry n_bias - 1 holds for everything farther; rows ldb apart, readable, whatever stands there, from 256 entries
- *   before distance 0 to 256 entries past n_bias - 1), optional sink in the denominator (score sinks[h], or 0 when sinks is NULL).
+ *   (bias points at distance 0 of head 0; entry n_bias - 1 holds for everything farther; rows ldb apart, readable from 256 entries before
+ *   distance 0, which may hold anything, to 256 entries past n_bias - 1, which repeat it), optional sink in the denominator (score sinks[h], or 0 when sinks is NULL).
  *   The last dk2 of the dk query / key columns may come from a second key tensor that all heads share; the output may be multiplied by
  *   sigmoid(gate). host_pos = *pos when the caller knows it, or
  *   -1 (n == 1 only). ws: plz_attn_bias_ws_bytes bytes for n == 1, else unused. */
